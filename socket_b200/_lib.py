@@ -103,6 +103,16 @@ class ResidualParams(C.Structure):
     ]
 
 
+class LinearParams(C.Structure):
+    """Mirror of `sk_linear_params`."""
+    _fields_ = [
+        ("x", _p), ("w", _p), ("res", _p), ("out", _p), ("act", _p),
+        ("x_ld", _i64), ("w_ld", _i64), ("res_ld", _i64), ("out_ld", _i64), ("act_ld", _i64), ("gate_row", _i64), ("up_row", _i64),
+        ("rows", _i), ("n", _i), ("k", _i), ("ff", _i), ("dtype", _i), ("out_f32", _i), ("glu", _i), ("chained", _i),
+        ("limit", _f), ("slope", _f),
+    ]
+
+
 class AttnParams(C.Structure):
     """Mirror of `sk_attn_params`."""
     _fields_ = [
@@ -163,6 +173,8 @@ BLOCK_SIGNATURES = {
     "skb_last_error": (C.c_char_p, []),
     "skb_embed_rows": (_i, [_p, _p, _i, _i64, _i64, _i, _f, _p, _p, _p, _p]),
     "skb_residual_norm": (_i, [C.POINTER(ResidualParams), _p]),
+    "skb_linear_rows_applicable": (_i, [C.POINTER(LinearParams)]),
+    "skb_linear_rows": (_i, [C.POINTER(LinearParams), _p]),
     "skb_glu": (_i, [_p, _p, _i, _i64, _i, _i64, _i, _f, _f, _p, _i64, _p]),
     "skb_ring_append": (_i, [_p, _p, _i, _i, _i, _i64, _i64, _i64, _i64, _i, _i, _i, _i, _p, _i64, _p, _p, _p]),
     "skb_rotary_rows": (_i, [C.POINTER(RotaryRowsParams), _p]),

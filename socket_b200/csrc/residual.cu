@@ -33,6 +33,7 @@ residual_norm_kernel(sk_residual_params p) {
     __shared__ float red[3][32];
     const int64_t row = blockIdx.x;
     const int W = p.width, nt = blockDim.x, t = threadIdx.x;
+    pdl_launch_dependents();                              // the projection that reads `out` may request its weights
     float* xr = p.x + row * W;
     const T* w_in = (const T*)p.w_in;
     const T* w_out = (const T*)p.w_out;

@@ -53,11 +53,14 @@ def vector(n: int) -> nn.Parameter:
     return nn.Parameter(torch.zeros(n), requires_grad=False)
 
 
+# Products inside a decoder's stack: the kernel before each of them is one of the stack's own, which write no weights
+def matmul(x: Tensor, w: Tensor) -> Tensor:
+    return ops.linear(x, w, chained=True)
+
+
 def matmul_f32(x: Tensor, w: Tensor) -> Tensor:
     """x w^T whose fp32 sums are not rounded."""
-    if x.dtype == torch.float32:
-        return torch.mm(x, w.t())
-    return torch.mm(x, w.t(), out_dtype=torch.float32)
+    return ops.linear(x, w, f32=True, chained=True)
 
 
 # ---------------------------------------------------------------------------------- attention
@@ -118,7 +121,7 @@ class ChunkedAttention(nn.Module):
 
     def forward(self, h: Tensor, cache: RingCache, at: Portion) -> Tensor:
         B, S = at.B, at.S
-        qkv = torch.mm(h, self.wqkv.t()).view(B, S, -1)
+        qkv = matmul(h, self.wqkv).view(B, S, -1)
         a, b, c = self.sizes
         q = qkv[..., :a].unflatten(-1, (self.H, self.D))
         k = qkv[..., a:a + b].unflatten(-1, (self.G, self.D))
@@ -136,7 +139,7 @@ class ChunkedAttention(nn.Module):
                 ka, va = k, v
             y = ops.attn(q, ka, va, start=at.start, kv_start=lo, **args)
             ops.ring_append(k, v, cache.k[:B], cache.v[:B], start=at.start)
-        return torch.mm(y.view(B * S, self.H * self.E), self.wo.t())
+        return matmul(y.view(B * S, self.H * self.E), self.wo)
 
 
 # ---------------------------------------------------------------------------------- latent attention
@@ -227,7 +230,7 @@ class LatentAttention(nn.Module):
 
     def forward(self, h: Tensor, cache: LatentCache, at: Portion) -> Tensor:
         B, S = at.B, at.S
-        qd = torch.mm(h, self.wqd.t())
+        qd = matmul(h, self.wqd)
         q = qd[:, :self.q_rows]
         dkv = qd[:, self.q_rows:self.q_rows + self.K + self.R]
         rows = cache.rows[:B]
@@ -244,7 +247,7 @@ class LatentAttention(nn.Module):
             k = kv[..., :self.q_rows].unflatten(-1, (self.H, self.D + self.R))
             v = kv[..., self.q_rows:].unflatten(-1, (self.H, self.E))
             y = ops.attn(q.view(B, S, -1).unflatten(-1, (self.H, self.D + self.R)), k, v, **args)
-        return torch.mm(y.view(B * S, self.H * self.E), self.wo.t())
+        return matmul(y.view(B * S, self.H * self.E), self.wo)
 
 
 # ---------------------------------------------------------------------------------- window attention
@@ -397,11 +400,11 @@ class Mamba2(nn.Module):
         return 0
 
     def forward(self, h: Tensor, cache: StateCache, at: Portion) -> Tensor:
-        proj = torch.mm(h, self.w_in.t())
+        proj = matmul(h, self.w_in)
         y = ops.ssm(proj, self.inner, self.conv_w, self.conv_b, self.dt_bias_f32, self.A_log_f32, self.skip_f32,
                     cache.conv[:at.B], cache.state[:at.B], S=at.S, groups=self.G, start=at.start, pos=at.pos)
         y = ops.gated_group_norm(y, proj, self.norm_w, self.parts, self.eps)
-        return torch.mm(y, self.wo.t())
+        return matmul(y, self.wo)
 
 
 # ---------------------------------------------------------------------------------- feed-forward
@@ -419,7 +422,9 @@ class ClampedFeedForward(nn.Module):
         return {"gate": self.w13[:self.ff], "up": self.w13[self.ff:2 * self.ff], "down": self.w2}
 
     def forward(self, h: Tensor) -> Tensor:
-        return torch.mm(ops.glu_clamped(torch.mm(h, self.w13.t()), self.ff, self.limit), self.w2.t())
+        unit = ops.linear_glu(h, self.w13, 0, self.ff, self.ff, ops.GLU_CLAMPED, limit=self.limit, slope=ops.GLU_SLOPE, chained=True)
+        act = ops.glu_clamped(matmul(h, self.w13), self.ff, self.limit) if unit is None else unit[1]
+        return matmul(act, self.w2)
 
 
 class ParallelLayer(nn.Module):
@@ -454,11 +459,16 @@ class ParallelLayer(nn.Module):
         return out
 
     def forward(self, h: Tensor, cache, at: Portion) -> Tensor:
-        proj = torch.mm(h, self.w_in.t())
-        parts = [proj[:, s] for s in self.in_slices]
         make = torch.zeros if self.gaps else torch.empty           # columns between the two parts meet zero weights
         inner = make(h.shape[0], self.cols, dtype=h.dtype, device=h.device)
-        self.mixer.mix(parts[:len(self.mixer.in_sizes)], h, cache, at, inner[:, :self.mixer.out_size])
-        if self.ff:
-            ops.glu_silu(*parts[-2:], out=inner[:, self.ff_at:self.ff_at + self.ff])
+        act = inner[:, self.ff_at:self.ff_at + self.ff]
+        fused = None
+        if self.ff:                                                # few rows: projections and unit in one launch
+            gate, up = self.in_slices[-2:]
+            fused = ops.linear_glu(h, self.w_in, gate.start, up.start, self.ff, ops.GLU_SILU, plain=gate.start, act=act, chained=True)
+        proj = matmul(h, self.w_in) if fused is None else fused[0]
+        n_mix = len(self.mixer.in_sizes)
+        self.mixer.mix([proj[:, s] for s in self.in_slices[:n_mix]], h, cache, at, inner[:, :self.mixer.out_size])
+        if self.ff and fused is None:
+            ops.glu_silu(proj[:, gate], proj[:, up], out=act)
         return matmul_f32(inner, self.w_out)

@@ -1,0 +1,64 @@
+"""Projections of a few rows against float64: edges of tiles (16 and 32 weight rows), of the pieces of 64 along k, of the
+division of k among 8 and 16 warps, several tiles per CTA, and the gated unit beside plain rows."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _bound(x, w, dtype, f32):
+    """fp32 sums of k products, each step off by at most 2^-23 of the sum of magnitudes; then one rounding to the type."""
+    mag = x.double().abs() @ w.double().abs().t()
+    eps = 0.0 if f32 else {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
+    return mag * x.shape[1] * 2.0 ** -23, eps
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,n,k", [(1, 1, 16), (8, 16, 64), (3, 17, 48), (2, 33, 1040), (5, 2369, 528), (8, 4752, 128), (1, 2368, 2064),
+                                      (7, 9600, 192), (4, 19008, 64), (8, 100, 14336)])
+def test_plain_products(rows, n, k, dtype):
+    from socket_b200 import block_ops as ops
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    x = torch.randn(rows, k + 8, generator=g, device="cuda").to(dtype)[:, :k]          # strided rows
+    w = torch.randn(n, k + 16, generator=g, device="cuda").to(dtype)[:, :k]
+    res = torch.randn(rows, n, generator=g, device="cuda").to(dtype)
+    assert ops._linear_params(x, w, False) is not None
+    want = x.double() @ w.double().t()
+    for f32, r, chained in ((True, None, False), (False, None, True), (False, res, False)):
+        got = ops.linear(x, w, f32=f32, res=r, chained=chained).double()
+        ref = want if r is None else want + r.double()
+        tol, eps = _bound(x, w, dtype, f32)
+        assert got.shape == ref.shape and bool(((got - ref).abs() <= tol + eps * ref.abs() + 1e-7).all())
+
+
+@pytest.mark.parametrize("rows,k,ff,plain", [(1, 64, 16, 0), (8, 128, 33, 40), (3, 1040, 5632, 3072), (8, 512, 100, 4800)])
+@pytest.mark.parametrize("kind", [0, 1])
+def test_gated_unit(rows, k, ff, plain, kind):
+    from socket_b200 import block_ops as ops
+    g = torch.Generator(device="cuda").manual_seed(ff)
+    x = torch.randn(rows, k, generator=g, device="cuda").bfloat16()
+    w = (torch.randn(plain + 2 * ff + 8, k, generator=g, device="cuda") * 2 * k ** -0.5).bfloat16()
+    wide = torch.full((rows, ff + 24), 3.0, device="cuda", dtype=torch.bfloat16)
+    out, act = ops.linear_glu(x, w, plain, plain + ff + 8, ff, kind, limit=1.5, slope=1.7, plain=plain, act=wide[:, 8:8 + ff])
+    y = x.double() @ w.double().t()
+    gate, up = y[:, plain:plain + ff], y[:, plain + ff + 8:plain + 2 * ff + 8]
+    if kind == ops.GLU_CLAMPED:
+        a, b = gate.clamp(max=1.5), up.clamp(-1.5, 1.5)
+        want = a * torch.sigmoid(1.7 * a) * (b + 1)
+    else:
+        want = gate * torch.sigmoid(gate) * up
+    # sums: 2^-23 k of the magnitudes (at most 8 here after the scaling), times the unit's slopes (below 10); one rounding
+    mag = (x.double().abs() @ w.double().abs().t()).max()
+    assert bool(((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + mag * k * 2.0 ** -23 * 10 + 1e-6 * (1 + want.abs())).all())
+    assert bool((wide[:, :8] == 3).all()) and bool((wide[:, 8 + ff:] == 3).all())
+    tol, eps = _bound(x, w[:plain], torch.bfloat16, False)
+    assert bool(((out.double() - y[:, :plain]).abs() <= tol + eps * y[:, :plain].abs() + 1e-7).all())
+
+
+def test_shapes_outside_go_to_the_library():
+    from socket_b200 import block_ops as ops
+    x, w = torch.randn(9, 64, device="cuda").bfloat16(), torch.randn(24, 64, device="cuda").bfloat16()
+    for a, b in ((x, w), (x[:2, :40], w[:, :40]), (x[:2].float(), w.float())):
+        assert ops._linear_params(a, b, False) is None
+        torch.testing.assert_close(ops.linear(a, b), torch.mm(a, b.t()))
+        assert ops.linear_glu(a, b, 0, 8, 8, ops.GLU_SILU) is None
