@@ -128,7 +128,7 @@ attn_decode_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_const
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int split = blockIdx.x, g = blockIdx.y / groups, grp = blockIdx.y % groups, b = blockIdx.z;
     const int rep = p.H / p.G, n_rows = p.S * rep, r_first = grp * ROWS;
-    pdl_launch_dependents();
+    pdl_begin();                                                // queries, the newest key and the position come from kernels before
     const DmRange rg = dm_range(p, splits);
     if (split == 0 && grp == 0 && tid == 0 && p.status != nullptr && rg.outside)
         atomicOr(p.status, SK_DEV_POS_OUT_OF_RANGE);
@@ -349,7 +349,7 @@ attn_decode_wide_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int split = blockIdx.x, g = blockIdx.y / groups, grp = blockIdx.y % groups, b = blockIdx.z;
     const int rep = p.H / p.G, n_rows = p.S * rep, r_first = grp * ROWS;
-    pdl_launch_dependents();
+    pdl_begin();                                                // queries, the newest key and the position come from kernels before
     const DmRange rg = dm_range(p, splits);
     if (split == 0 && grp == 0 && tid == 0 && p.status != nullptr && rg.outside)
         atomicOr(p.status, SK_DEV_POS_OUT_OF_RANGE);
@@ -583,11 +583,11 @@ attn_decode_merge_kernel(sk_attn_params p, int splits, int groups, int rows_per_
     const int warp = t >> 5, lane = t & 31, c = (blockIdx.x - row * col_blocks) * DG_COLS + 4 * lane;
     const int s = row / rep, h = g * rep + row - s * rep, grp = row / rows_per_group, r = row - grp * rows_per_group;
     const float sink = p.sink != nullptr ? p.sink[h] * DM_LOG2E : -INFINITY;
+    pdl_begin();
     const DmRange rg = dm_range(p, splits);
     const int n = rg.tiles > 0 ? (rg.tiles + rg.per_split - 1) / rg.per_split : 0;      // <= DM_MAX_SPLITS
     const float* part = (const float*)p.workspace + (((int64_t)b * p.G + g) * groups + grp) * splits * part_floats;
     const float* stat = part + (int64_t)rows_per_group * p.dv + r;
-    pdl_wait();
     float mk = -INFINITY, lk = 0.f;
     if (t < n) {
         mk = __ldcg(stat + t * part_floats);
@@ -651,7 +651,8 @@ int launch_splits(const sk_attn_params& p, const DmPlan& d, const CUtensorMap& m
         auto kern = kernel;                                                                                              \
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d.smem);      \
         if (e != cudaSuccess) return fail(SK_ERR_CUDA, "attn_decode kernel smem attribute: %s", cudaGetErrorString(e));  \
-        kern<<<grid, DM_WARPS * 32, d.smem, st>>>(mk, mv, p, d.splits, d.groups, d.np, d.nvp, d.k_off, __VA_ARGS__);     \
+        return check_chained(launch_after(kern, grid, dim3(DM_WARPS * 32), d.smem, st, mk, mv, p, d.splits, d.groups, d.np, d.nvp, d.k_off, \
+                                          __VA_ARGS__), "attn_decode_kernel");                                           \
     } while (0)
 #define SK_DM_WIDE(KS)                                                                                    \
     do {                                                                                                  \
@@ -670,7 +671,6 @@ int launch_splits(const sk_attn_params& p, const DmPlan& d, const CUtensorMap& m
     }
 #undef SK_DM_WIDE
 #undef SK_DM
-    return check_launch("attn_decode_kernel");
 }
 
 }  // namespace

@@ -17,6 +17,7 @@ __device__ __forceinline__ void rotate_pair(float& u, float& v, const float* cs)
 template <typename T>
 __global__ void __launch_bounds__(256)
 latent_append_kernel(sk_latent_params p) {
+    pdl_begin();
     __shared__ float red[32];
     const int s = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
     const int64_t i = first_position(p.pos, p.start) + s;
@@ -61,8 +62,9 @@ latent_append_kernel(sk_latent_params p) {
 constexpr int AB_ROWS = 8;
 template <typename T>
 __global__ void __launch_bounds__(256)
-latent_absorb_kernel(const T* __restrict__ q, int64_t q_ld, const T* __restrict__ uk, int64_t rows, int H, int dim, int rot,
+latent_absorb_kernel(const T* q, int64_t q_ld, const T* __restrict__ uk, int64_t rows, int H, int dim, int rot,
                      int rank, int out_ld, T* __restrict__ out) {
+    pdl_begin();
     extern __shared__ float sm[];                                // q [AB_ROWS][dim], partials [8][AB_ROWS][64]
     float* part = sm + AB_ROWS * dim;
     const int h = blockIdx.x, c0 = blockIdx.y * 64, t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -125,8 +127,9 @@ latent_absorb_kernel(const T* __restrict__ q, int64_t q_ld, const T* __restrict_
 // (8 columns each) and 16 along the head's rows of W_uk, so that a thread's loads are few, wide and in flight together.
 template <int ROWS>
 __global__ void __launch_bounds__(256)
-latent_absorb_vec_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_ld, const __nv_bfloat16* __restrict__ uk, int64_t rows,
+latent_absorb_vec_kernel(const __nv_bfloat16* q, int64_t q_ld, const __nv_bfloat16* __restrict__ uk, int64_t rows,
                          int H, int dim, int rot, int rank, int out_ld, __nv_bfloat16* __restrict__ out) {
+    pdl_begin();
     extern __shared__ float sm[];                                // q [ROWS][dim], partials [16][ROWS][128]
     float* part = sm + ROWS * dim;
     const int h = blockIdx.x, c0 = blockIdx.y * 128, t = threadIdx.x, cl = t & 15, dg = t >> 4;
@@ -196,8 +199,9 @@ latent_absorb_vec_kernel(const __nv_bfloat16* __restrict__ q, int64_t q_ld, cons
 // out[row, h * vdim + e] for bf16 and a rank that is a multiple of 8: one warp per output element and row group
 template <int ROWS>
 __global__ void __launch_bounds__(128)
-latent_up_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ uv, int64_t rows, int H, int vdim,
+latent_up_vec_kernel(const __nv_bfloat16* o, const __nv_bfloat16* __restrict__ uv, int64_t rows, int H, int vdim,
                      int rank, __nv_bfloat16* __restrict__ out) {
+    pdl_begin();
     const int lane = threadIdx.x & 31;
     const int e = blockIdx.x * 4 + (threadIdx.x >> 5);
     const int64_t r0 = (int64_t)blockIdx.y * ROWS;
@@ -235,7 +239,8 @@ latent_up_vec_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* _
 // out[row, h * vdim + e] = <W_uv[h * vdim + e, :], o[row, h, :]>: one warp per output element and row group
 template <typename T>
 __global__ void __launch_bounds__(256)
-latent_up_kernel(const T* __restrict__ o, const T* __restrict__ uv, int64_t rows, int H, int vdim, int rank, T* __restrict__ out) {
+latent_up_kernel(const T* o, const T* __restrict__ uv, int64_t rows, int H, int vdim, int rank, T* __restrict__ out) {
+    pdl_begin();
     const int lane = threadIdx.x & 31;
     const int e = blockIdx.x * 8 + (threadIdx.x >> 5);           // flat (head, value dimension)
     const int64_t r0 = (int64_t)blockIdx.y * AB_ROWS;
@@ -278,9 +283,8 @@ latent_up_kernel(const T* __restrict__ o, const T* __restrict__ uv, int64_t rows
 
 int launch_latent_append(const sk_latent_params& p, cudaStream_t st) {
     dim3 grid((unsigned)p.S, (unsigned)p.B);
-    if (p.dtype == SK_BF16) latent_append_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p);
-    else latent_append_kernel<float><<<grid, 256, 0, st>>>(p);
-    return check_launch("latent_append_kernel");
+    auto kern = p.dtype == SK_BF16 ? latent_append_kernel<__nv_bfloat16> : latent_append_kernel<float>;
+    return check_chained(launch_after(kern, grid, dim3(256), 0, st, p), "latent_append_kernel");
 }
 
 int launch_latent_absorb(const void* q, int64_t q_ld, int dtype, const void* uk, int64_t rows, int H, int dim, int rot,
@@ -290,20 +294,19 @@ int launch_latent_absorb(const void* q, int64_t q_ld, int dtype, const void* uk,
         const int R = rows == 1 ? 1 : 4;
         dim3 grid((unsigned)H, (unsigned)((out_ld + 127) / 128), (unsigned)((rows + R - 1) / R));
         const size_t smem = (size_t)(R * dim + 16 * R * 128) * sizeof(float);
-        if (R == 1) latent_absorb_vec_kernel<1><<<grid, 256, smem, st>>>(qb, q_ld, ub, rows, H, dim, rot, rank, out_ld, (__nv_bfloat16*)out);
-        else latent_absorb_vec_kernel<4><<<grid, 256, smem, st>>>(qb, q_ld, ub, rows, H, dim, rot, rank, out_ld, (__nv_bfloat16*)out);
-        return check_launch("latent_absorb_vec_kernel");
+        auto kern = R == 1 ? latent_absorb_vec_kernel<1> : latent_absorb_vec_kernel<4>;
+        return check_chained(launch_after(kern, grid, dim3(256), smem, st, qb, q_ld, ub, rows, H, dim, rot, rank, out_ld, (__nv_bfloat16*)out),
+                             "latent_absorb_vec_kernel");
     }
     dim3 grid((unsigned)H, (unsigned)((out_ld + 63) / 64), (unsigned)((rows + AB_ROWS - 1) / AB_ROWS));
     const size_t smem = (size_t)(AB_ROWS * dim + 8 * AB_ROWS * 64) * sizeof(float);
     if (smem > 48 * 1024) return fail(SK_ERR_UNSUPPORTED, "sk_latent_absorb: head size %d is too large", dim);
     if (dtype == SK_BF16)
-        latent_absorb_kernel<<<grid, 256, smem, st>>>((const __nv_bfloat16*)q, q_ld, (const __nv_bfloat16*)uk, rows, H, dim,
-                                                      rot, rank, out_ld, (__nv_bfloat16*)out);
-    else
-        latent_absorb_kernel<<<grid, 256, smem, st>>>((const float*)q, q_ld, (const float*)uk, rows, H, dim, rot, rank,
-                                                      out_ld, (float*)out);
-    return check_launch("latent_absorb_kernel");
+        return check_chained(launch_after(latent_absorb_kernel<__nv_bfloat16>, grid, dim3(256), smem, st, (const __nv_bfloat16*)q, q_ld,
+                                          (const __nv_bfloat16*)uk, rows, H, dim, rot, rank, out_ld, (__nv_bfloat16*)out),
+                             "latent_absorb_kernel");
+    return check_chained(launch_after(latent_absorb_kernel<float>, grid, dim3(256), smem, st, (const float*)q, q_ld, (const float*)uk,
+                                      rows, H, dim, rot, rank, out_ld, (float*)out), "latent_absorb_kernel");
 }
 
 int launch_latent_up(const void* o, int dtype, const void* uv, int64_t rows, int H, int vdim, int rank, void* out,
@@ -312,17 +315,16 @@ int launch_latent_up(const void* o, int dtype, const void* uv, int64_t rows, int
         const __nv_bfloat16 *ob = (const __nv_bfloat16*)o, *ub = (const __nv_bfloat16*)uv;
         const int R = rows == 1 ? 1 : 4;
         dim3 grid((unsigned)((H * vdim + 3) / 4), (unsigned)((rows + R - 1) / R));
-        if (R == 1) latent_up_vec_kernel<1><<<grid, 128, 0, st>>>(ob, ub, rows, H, vdim, rank, (__nv_bfloat16*)out);
-        else latent_up_vec_kernel<4><<<grid, 128, 0, st>>>(ob, ub, rows, H, vdim, rank, (__nv_bfloat16*)out);
-        return check_launch("latent_up_vec_kernel");
+        auto kern = R == 1 ? latent_up_vec_kernel<1> : latent_up_vec_kernel<4>;
+        return check_chained(launch_after(kern, grid, dim3(128), 0, st, ob, ub, rows, H, vdim, rank, (__nv_bfloat16*)out),
+                             "latent_up_vec_kernel");
     }
     dim3 grid((unsigned)((H * vdim + 7) / 8), (unsigned)((rows + AB_ROWS - 1) / AB_ROWS));
     if (dtype == SK_BF16)
-        latent_up_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)uv, rows, H, vdim, rank,
-                                               (__nv_bfloat16*)out);
-    else
-        latent_up_kernel<<<grid, 256, 0, st>>>((const float*)o, (const float*)uv, rows, H, vdim, rank, (float*)out);
-    return check_launch("latent_up_kernel");
+        return check_chained(launch_after(latent_up_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, (const __nv_bfloat16*)o,
+                                          (const __nv_bfloat16*)uv, rows, H, vdim, rank, (__nv_bfloat16*)out), "latent_up_kernel");
+    return check_chained(launch_after(latent_up_kernel<float>, grid, dim3(256), 0, st, (const float*)o, (const float*)uv, rows, H, vdim,
+                                      rank, (float*)out), "latent_up_kernel");
 }
 
 }  // namespace sk

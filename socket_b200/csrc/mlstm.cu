@@ -19,6 +19,7 @@ constexpr int MS_COLS = 16, MS_GROUPS = 16;
 template <typename T, int NPT>
 __global__ void __launch_bounds__(MS_COLS * MS_GROUPS)
 mlstm_steps_kernel(sk_mlstm_params p) {
+    pdl_begin();
     __shared__ float red[2][8][MS_COLS];
     const int t = threadIdx.x, c = t & (MS_COLS - 1), grp = t >> 4, warp = t >> 5, lane = t & 31;
     const int col = blockIdx.x * MS_COLS + c, h = blockIdx.y, b = blockIdx.z;
@@ -78,6 +79,7 @@ mlstm_steps_kernel(sk_mlstm_params p) {
 template <typename T, int V, int NV>
 __global__ void __launch_bounds__(1024)
 mlstm_finish_kernel(sk_mlstm_params p) {
+    pdl_begin();
     __shared__ float red[32];
     const int64_t row = blockIdx.x;
     const int h = blockIdx.y, nt = blockDim.x, t = threadIdx.x;
@@ -122,24 +124,18 @@ template <typename T, int V> int finish_dispatch(const sk_mlstm_params& p, cudaS
     while (nt < 1024 && (vecs + nt - 1) / nt > 8) nt *= 2;
     const int nv = (vecs + nt - 1) / nt;
     dim3 grid((unsigned)((int64_t)p.B * p.S), (unsigned)p.H);
-    if (nv <= 1) mlstm_finish_kernel<T, V, 1><<<grid, nt, 0, st>>>(p);
-    else if (nv <= 2) mlstm_finish_kernel<T, V, 2><<<grid, nt, 0, st>>>(p);
-    else if (nv <= 8) mlstm_finish_kernel<T, V, 8><<<grid, nt, 0, st>>>(p);
-    else return fail(SK_ERR_UNSUPPORTED, "skb_mlstm: value size %d is too large", p.P);
-    return check_launch("mlstm_finish_kernel");
+    if (nv > 8) return fail(SK_ERR_UNSUPPORTED, "skb_mlstm: value size %d is too large", p.P);
+    auto kern = nv <= 1 ? mlstm_finish_kernel<T, V, 1> : nv <= 2 ? mlstm_finish_kernel<T, V, 2> : mlstm_finish_kernel<T, V, 8>;
+    return check_chained(launch_after(kern, grid, dim3((unsigned)nt), 0, st, p), "mlstm_finish_kernel");
 }
 
 template <typename T> int steps_dispatch(const sk_mlstm_params& p, cudaStream_t st) {
     dim3 grid((unsigned)((p.P + MS_COLS) / MS_COLS), (unsigned)p.H, (unsigned)p.B);      // P + 1 columns
     const int npt = (p.N + MS_GROUPS - 1) / MS_GROUPS;
-    if (npt <= 2) mlstm_steps_kernel<T, 2><<<grid, 256, 0, st>>>(p);
-    else if (npt <= 4) mlstm_steps_kernel<T, 4><<<grid, 256, 0, st>>>(p);
-    else if (npt <= 8) mlstm_steps_kernel<T, 8><<<grid, 256, 0, st>>>(p);
-    else if (npt <= 16) mlstm_steps_kernel<T, 16><<<grid, 256, 0, st>>>(p);
-    else if (npt <= 32) mlstm_steps_kernel<T, 32><<<grid, 256, 0, st>>>(p);
-    else if (npt <= 64) mlstm_steps_kernel<T, 64><<<grid, 256, 0, st>>>(p);
-    else return fail(SK_ERR_UNSUPPORTED, "skb_mlstm: key size %d is too large", p.N);
-    return check_launch("mlstm_steps_kernel");
+    if (npt > 64) return fail(SK_ERR_UNSUPPORTED, "skb_mlstm: key size %d is too large", p.N);
+    auto kern = npt <= 2 ? mlstm_steps_kernel<T, 2> : npt <= 4 ? mlstm_steps_kernel<T, 4> : npt <= 8 ? mlstm_steps_kernel<T, 8>
+              : npt <= 16 ? mlstm_steps_kernel<T, 16> : npt <= 32 ? mlstm_steps_kernel<T, 32> : mlstm_steps_kernel<T, 64>;
+    return check_chained(launch_after(kern, grid, dim3(256), 0, st, p), "mlstm_steps_kernel");
 }
 
 }  // namespace

@@ -10,6 +10,8 @@ template <typename T, int V>
 __global__ void __launch_bounds__(256)
 embed_rows_kernel(const int64_t* __restrict__ tokens, const T* __restrict__ table, int64_t vocab, int width, float scale,
                   float* __restrict__ x, float* __restrict__ x_copy, int32_t* status) {
+    // launched unchained, the first kernel of a stack: those behind it may rely on all earlier work being complete
+    pdl_launch_dependents();
     const int64_t row = blockIdx.x;
     const int i = (blockIdx.y * 256 + threadIdx.x) * V;
     const int64_t tok = tokens[row];
@@ -33,7 +35,7 @@ residual_norm_kernel(sk_residual_params p) {
     __shared__ float red[3][32];
     const int64_t row = blockIdx.x;
     const int W = p.width, nt = blockDim.x, t = threadIdx.x;
-    pdl_launch_dependents();                              // the projection that reads `out` may request its weights
+    pdl_begin();                                          // the projection that reads `out` may request its weights
     float* xr = p.x + row * W;
     const T* w_in = (const T*)p.w_in;
     const T* w_out = (const T*)p.w_out;
@@ -124,8 +126,9 @@ residual_norm_kernel(sk_residual_params p) {
 // KIND SKB_GLU_CLAMPED: y = g * sigmoid(slope * g) * (u + 1), g and u clamped; SKB_GLU_SILU: y = g * sigmoid(g) * u
 template <typename T, int V, int KIND>
 __global__ void __launch_bounds__(256)
-glu_kernel(const T* __restrict__ gate, const T* __restrict__ up, int64_t rows, int ff, int64_t ld, float limit, float slope,
-           T* __restrict__ out, int64_t out_ld) {
+glu_kernel(const T* gate, const T* up, int64_t rows, int ff, int64_t ld, float limit, float slope, T* __restrict__ out,
+           int64_t out_ld) {
+    pdl_begin();
     const int i = (blockIdx.x * 256 + threadIdx.x) * V;
     if (i >= ff) return;
     for (int64_t row = blockIdx.y; row < rows; row += gridDim.y) {
@@ -149,9 +152,10 @@ glu_kernel(const T* __restrict__ gate, const T* __restrict__ up, int64_t rows, i
 // s0 leaves out what no later token sees, so that no two tokens of a portion meet in one row.
 template <typename T>
 __global__ void __launch_bounds__(256)
-ring_append_kernel(const T* __restrict__ k, const T* __restrict__ v, int64_t k_bs, int64_t k_ss, int64_t v_bs,
+ring_append_kernel(const T* k, const T* v, int64_t k_bs, int64_t k_ss, int64_t v_bs,
                    int64_t v_ss, int k_row, int v_row, int ring, const int64_t* __restrict__ pos, int64_t start, int s0,
                    T* __restrict__ k_cache, T* __restrict__ v_cache) {
+    pdl_begin();
     const int s = s0 + blockIdx.x, b = blockIdx.y;
     const int64_t slot = (first_position(pos, start) + s) % ring;
     const T* ks = k + b * k_bs + s * k_ss;
@@ -173,12 +177,13 @@ int residual_dispatch(const sk_residual_params& p, cudaStream_t st) {
     while (nt < 1024 && (vecs + nt - 1) / nt > 8) nt *= 2;
     const int nv = (vecs + nt - 1) / nt;
     dim3 grid((unsigned)p.rows);
-    if (nv <= 1) residual_norm_kernel<T, TY, V, 1><<<grid, nt, 0, st>>>(p);
-    else if (nv <= 2) residual_norm_kernel<T, TY, V, 2><<<grid, nt, 0, st>>>(p);
-    else if (nv <= 4) residual_norm_kernel<T, TY, V, 4><<<grid, nt, 0, st>>>(p);
-    else if (nv <= 8) residual_norm_kernel<T, TY, V, 8><<<grid, nt, 0, st>>>(p);
+    void (*kern)(sk_residual_params) = nullptr;
+    if (nv <= 1) kern = residual_norm_kernel<T, TY, V, 1>;
+    else if (nv <= 2) kern = residual_norm_kernel<T, TY, V, 2>;
+    else if (nv <= 4) kern = residual_norm_kernel<T, TY, V, 4>;
+    else if (nv <= 8) kern = residual_norm_kernel<T, TY, V, 8>;
     else return fail(SK_ERR_UNSUPPORTED, "sk_residual_norm: width %d is too large", p.width);
-    return check_launch("residual_norm_kernel");
+    return check_chained(launch_after(kern, grid, dim3((unsigned)nt), 0, st, p), "residual_norm_kernel");
 }
 
 }  // namespace
@@ -215,12 +220,12 @@ int launch_glu(const void* gate, const void* up, int dtype, int64_t rows, int ff
 #define SK_GLU(T, V)                                                                                                       \
     do {                                                                                                                   \
         auto kern = kind == SKB_GLU_CLAMPED ? glu_kernel<T, V, SKB_GLU_CLAMPED> : glu_kernel<T, V, SKB_GLU_SILU>;          \
-        kern<<<grid, 256, 0, st>>>((const T*)gate, (const T*)up, rows, ff, ld, limit, slope, (T*)out, out_ld);             \
+        return check_chained(launch_after(kern, grid, dim3(256), 0, st, (const T*)gate, (const T*)up, rows, ff, ld, limit, slope, \
+                                          (T*)out, out_ld), "glu_kernel");                                                 \
     } while (0)
     if (dtype == SK_BF16) { if (v8) SK_GLU(__nv_bfloat16, 8); else if (v4) SK_GLU(__nv_bfloat16, 4); else SK_GLU(__nv_bfloat16, 1); }
     else { if (v4) SK_GLU(float, 4); else SK_GLU(float, 1); }
 #undef SK_GLU
-    return check_launch("glu_kernel");
 }
 
 int launch_ring_append(const void* k, const void* v, int dtype, int B, int S, int64_t k_bs, int64_t k_ss, int64_t v_bs,
@@ -231,13 +236,12 @@ int launch_ring_append(const void* k, const void* v, int dtype, int B, int S, in
     const int s0 = pos == nullptr && first > start ? (int)(first - start) : 0;   // a device position: one token
     dim3 grid((unsigned)(S - s0), (unsigned)B);
     if (dtype == SK_BF16)
-        ring_append_kernel<<<grid, 256, 0, st>>>((const __nv_bfloat16*)k, (const __nv_bfloat16*)v, k_bs, k_ss, v_bs, v_ss,
-                                                 k_row, v_row, ring, pos, start, s0, (__nv_bfloat16*)k_cache,
-                                                 (__nv_bfloat16*)v_cache);
-    else
-        ring_append_kernel<<<grid, 256, 0, st>>>((const float*)k, (const float*)v, k_bs, k_ss, v_bs, v_ss, k_row, v_row,
-                                                 ring, pos, start, s0, (float*)k_cache, (float*)v_cache);
-    return check_launch("ring_append_kernel");
+        return check_chained(launch_after(ring_append_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, (const __nv_bfloat16*)k,
+                                          (const __nv_bfloat16*)v, k_bs, k_ss, v_bs, v_ss, k_row, v_row, ring, pos, start, s0,
+                                          (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache), "ring_append_kernel");
+    return check_chained(launch_after(ring_append_kernel<float>, grid, dim3(256), 0, st, (const float*)k, (const float*)v, k_bs, k_ss,
+                                      v_bs, v_ss, k_row, v_row, ring, pos, start, s0, (float*)k_cache, (float*)v_cache),
+                         "ring_append_kernel");
 }
 
 }  // namespace sk

@@ -13,6 +13,7 @@ constexpr int RR_THREADS = 256;
 template <typename T, int V>
 __global__ void __launch_bounds__(RR_THREADS)
 rotary_rows_kernel(const sk_rotary_rows_params p) {
+    pdl_begin();
     const int row = blockIdx.x, b = blockIdx.y, t = threadIdx.x;
     const int rot = p.rot_dims, half = rot / 2, rest = p.dim - rot, hrow = p.dim + rot;
     const int64_t first = first_position(p.pos, p.start);
@@ -78,7 +79,7 @@ int launch_rotary_rows(const sk_rotary_rows_params& p, cudaStream_t st) {
                ((uintptr_t)p.q_in | (uintptr_t)p.k_in | (uintptr_t)p.ring | (uintptr_t)p.q_out | (uintptr_t)p.rows_out) % (v * es) == 0;
     };
     dim3 grid((unsigned)(p.prev + p.S), (unsigned)p.B);
-#define SK_RR(T, V) rotary_rows_kernel<T, V><<<grid, RR_THREADS, 0, st>>>(p)
+#define SK_RR(T, V) return check_chained(launch_after(rotary_rows_kernel<T, V>, grid, dim3(RR_THREADS), 0, st, p), "rotary_rows_kernel")
     if (p.dtype == SK_BF16) {
         if (vec(8)) SK_RR(__nv_bfloat16, 8);
         else if (vec(4)) SK_RR(__nv_bfloat16, 4);
@@ -88,7 +89,6 @@ int launch_rotary_rows(const sk_rotary_rows_params& p, cudaStream_t st) {
         else SK_RR(float, 1);
     }
 #undef SK_RR
-    return check_launch("rotary_rows_kernel");
 }
 
 }  // namespace sk

@@ -27,6 +27,7 @@ __device__ __forceinline__ void conv_tap_input(const sk_ssm_params& p, int b, in
 template <typename T, int V, int TAPS>      // TAPS: 0 = any number
 __global__ void __launch_bounds__(128)
 ssm_conv_kernel(sk_ssm_params p) {
+    pdl_begin();
     const int channels = p.H * p.P + 2 * p.G * p.N;
     const int ch = (blockIdx.x * 128 + threadIdx.x) * V, b = blockIdx.z, s0 = blockIdx.y * CONV_TOK;
     if (ch >= channels) return;
@@ -96,6 +97,7 @@ ssm_conv_kernel(sk_ssm_params p) {
 template <typename T>
 __global__ void __launch_bounds__(128)
 ssm_conv_state_kernel(sk_ssm_params p) {
+    pdl_begin();
     const int channels = p.H * p.P + 2 * p.G * p.N;
     const int ch = blockIdx.x * 128 + threadIdx.x, b = blockIdx.y;
     if (ch >= channels) return;
@@ -117,6 +119,7 @@ constexpr int ST_COLS = 16, ST_GROUPS = 16;
 template <typename T, int NPT>
 __global__ void __launch_bounds__(ST_COLS * ST_GROUPS)
 ssm_steps_kernel(sk_ssm_params p) {
+    pdl_begin();
     __shared__ float red[2][8][ST_COLS];
     const int t = threadIdx.x, c = t & (ST_COLS - 1), grp = t >> 4, warp = t >> 5, lane = t & 31;
     const int col = blockIdx.x * ST_COLS + c, h = blockIdx.y, b = blockIdx.z;
@@ -170,8 +173,9 @@ ssm_steps_kernel(sk_ssm_params p) {
 // ---------------------------------------------------------------- gate, then RMS norm of each part
 template <typename T, int V, int NV>
 __global__ void __launch_bounds__(1024)
-gated_group_norm_kernel(const T* __restrict__ y, const T* __restrict__ z, int64_t z_ld, const T* __restrict__ w, int inner,
-                        int part, float eps, T* __restrict__ out) {
+gated_group_norm_kernel(const T* y, const T* z, int64_t z_ld, const T* __restrict__ w, int inner, int part, float eps,
+                        T* __restrict__ out) {
+    pdl_begin();
     __shared__ float red[32];
     const int64_t row = blockIdx.x;
     const int c0 = blockIdx.y * part, nt = blockDim.x, t = threadIdx.x;
@@ -213,25 +217,23 @@ int norm_dispatch(const void* y, const void* z, int64_t z_ld, const void* w, int
     while (nt < 1024 && (vecs + nt - 1) / nt > 8) nt *= 2;
     const int nv = (vecs + nt - 1) / nt;
     dim3 grid((unsigned)rows, (unsigned)parts);
-#define SK_GN(NV) gated_group_norm_kernel<T, V, NV><<<grid, nt, 0, st>>>((const T*)y, (const T*)z, z_ld, (const T*)w, inner, part, eps, (T*)out)
+#define SK_GN(NV)                                                                                                        \
+    return check_chained(launch_after(gated_group_norm_kernel<T, V, NV>, grid, dim3((unsigned)nt), 0, st, (const T*)y,   \
+                                      (const T*)z, z_ld, (const T*)w, inner, part, eps, (T*)out), "gated_group_norm_kernel")
     if (nv <= 1) SK_GN(1);
     else if (nv <= 2) SK_GN(2);
     else if (nv <= 4) SK_GN(4);
     else if (nv <= 8) SK_GN(8);
     else return fail(SK_ERR_UNSUPPORTED, "sk_gated_group_norm: part of %d elements is too large", part);
 #undef SK_GN
-    return check_launch("gated_group_norm_kernel");
 }
 
 template <typename T> int steps_dispatch(const sk_ssm_params& p, cudaStream_t st) {
     dim3 grid((unsigned)((p.P + ST_COLS - 1) / ST_COLS), (unsigned)p.H, (unsigned)p.B);
     const int npt = (p.N + ST_GROUPS - 1) / ST_GROUPS;
-    if (npt <= 2) ssm_steps_kernel<T, 2><<<grid, 256, 0, st>>>(p);
-    else if (npt <= 4) ssm_steps_kernel<T, 4><<<grid, 256, 0, st>>>(p);
-    else if (npt <= 8) ssm_steps_kernel<T, 8><<<grid, 256, 0, st>>>(p);
-    else if (npt <= 16) ssm_steps_kernel<T, 16><<<grid, 256, 0, st>>>(p);
-    else return fail(SK_ERR_UNSUPPORTED, "sk_ssm: state size %d is too large", p.N);
-    return check_launch("ssm_steps_kernel");
+    if (npt > 16) return fail(SK_ERR_UNSUPPORTED, "sk_ssm: state size %d is too large", p.N);
+    auto kern = npt <= 2 ? ssm_steps_kernel<T, 2> : npt <= 4 ? ssm_steps_kernel<T, 4> : npt <= 8 ? ssm_steps_kernel<T, 8> : ssm_steps_kernel<T, 16>;
+    return check_chained(launch_after(kern, grid, dim3(256), 0, st, p), "ssm_steps_kernel");
 }
 
 template <typename T> int conv_dispatch(const sk_ssm_params& p, cudaStream_t st) {
@@ -242,16 +244,13 @@ template <typename T> int conv_dispatch(const sk_ssm_params& p, cudaStream_t st)
     };
     const int V = p.S == 1 ? 1 : sizeof(T) == 2 && vec(8) && p.taps == 4 ? 8 : (vec(4) ? 4 : 1);
     dim3 grid((unsigned)((channels + 128 * V - 1) / (128 * V)), (unsigned)((p.S + CONV_TOK - 1) / CONV_TOK), (unsigned)p.B);
-    if (V == 8) {
-        if constexpr (sizeof(T) == 2) ssm_conv_kernel<T, 8, 4><<<grid, 128, 0, st>>>(p);
-    } else if (V == 4 && p.taps == 4) ssm_conv_kernel<T, 4, 4><<<grid, 128, 0, st>>>(p);
-    else if (V == 4) ssm_conv_kernel<T, 4, 0><<<grid, 128, 0, st>>>(p);
-    else ssm_conv_kernel<T, 1, 0><<<grid, 128, 0, st>>>(p);
-    if (int rc = check_launch("ssm_conv_kernel")) return rc;
-    if (p.S > 1 && p.taps > 1) {
-        ssm_conv_state_kernel<T><<<dim3((unsigned)((channels + 127) / 128), (unsigned)p.B), 128, 0, st>>>(p);
-        return check_launch("ssm_conv_state_kernel");
-    }
+    auto kern = V == 4 && p.taps == 4 ? ssm_conv_kernel<T, 4, 4> : V == 4 ? ssm_conv_kernel<T, 4, 0> : ssm_conv_kernel<T, 1, 0>;
+    if constexpr (sizeof(T) == 2)
+        if (V == 8) kern = ssm_conv_kernel<T, 8, 4>;
+    if (int rc = check_chained(launch_after(kern, grid, dim3(128), 0, st, p), "ssm_conv_kernel")) return rc;
+    if (p.S > 1 && p.taps > 1)
+        return check_chained(launch_after(ssm_conv_state_kernel<T>, dim3((unsigned)((channels + 127) / 128), (unsigned)p.B), dim3(128), 0,
+                                          st, p), "ssm_conv_state_kernel");
     return SK_OK;
 }
 
