@@ -1,0 +1,64 @@
+"""Prefill attention where its rules change: heads in groups with a shorter last group, biases whose table ends inside, at
+and far before a half tile of 64 keys, rows that end anywhere in a query tile, head sizes with a ragged last MMA step."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(S, H, G, D, E, start, kv_start, bias_len, chunk, window, cap, sink, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    T = start + S - kv_start
+    q, k, v = r(1, S, H, D).bfloat16(), r(1, T, G, D).bfloat16(), r(1, T, G, E).bfloat16()
+    kw = dict(scale=2.0 * D ** -0.5, start=start, kv_start=kv_start, chunk=chunk, window=window, softcap=cap)
+    if bias_len:
+        kw["bias"] = 2.0 * r(H, bias_len)
+    if sink:
+        kw["sink"] = r(H)
+    return q, k, v, kw
+
+
+def _plain(q, k, v, kw, i, h):
+    """Row i of head h in float64, and the sum of weights times |v|."""
+    g = h // (q.shape[2] // k.shape[2])
+    s = k[0, :, g].double() @ q[0, i, h].double() * kw["scale"]
+    if kw["softcap"]:
+        s = kw["softcap"] * torch.tanh(s / kw["softcap"])
+    pos, j = kw["start"] + i, kw["kv_start"] + torch.arange(k.shape[1], device="cuda")
+    if "bias" in kw:
+        s = s + kw["bias"][h].double()[(pos - j).clamp(0, kw["bias"].shape[1] - 1)]
+    seen = j <= pos
+    if kw["chunk"]:
+        seen &= j // kw["chunk"] == pos // kw["chunk"]
+    if kw["window"]:
+        seen &= pos - j < kw["window"]
+    s = s.masked_fill(~seen, -float("inf"))
+    if "sink" in kw:
+        s = torch.cat([s, kw["sink"][h:h + 1].double()])
+    p = torch.softmax(s, 0)[:k.shape[1]]
+    return p @ v[0, :, g].double(), p @ v[0, :, g].double().abs()
+
+
+@pytest.mark.parametrize("S,H,G,D,E,start,kv_start,bias_len,chunk,window,cap,sink", [
+    (300, 11, 11, 192, 128, 9000, 0, 0, 0, 0, 0.0, True),        # 6 MB of keys and values a head: groups of 8 and 3
+    (515, 20, 10, 192, 128, 14000, 0, 0, 0, 0, 0.0, False),      # groups of 5 key/value heads, two queries heads each
+    (700, 4, 2, 128, 128, 0, 0, 33, 0, 0, 0.0, False),           # bias constant beyond 32, inside the diagonal tiles
+    (385, 4, 2, 128, 128, 640, 512, 193, 512, 0, 0.0, False),    # and at a half tile's edge, behind the chunk's first rows
+    (257, 2, 2, 128, 64, 511, 0, 5000, 512, 0, 0.0, True),       # table longer than any distance
+    (129, 3, 1, 72, 40, 200, 0, 70, 0, 0, 0.0, True),            # ragged head sizes
+    (640, 2, 1, 128, 128, 900, 773, 0, 0, 128, 30.0, True),      # window as long as a tile, weights relative to zero
+    (640, 2, 1, 128, 128, 900, 773, 100, 0, 128, 30.0, False),   # the same with a bias: running maximum under a cap
+    (200, 2, 1, 144, 128, 100, 0, 0, 0, 65, 200.0, False),       # a cap too high for that
+])
+def test_forms(S, H, G, D, E, start, kv_start, bias_len, chunk, window, cap, sink):
+    from socket_b200 import block_ops as ops
+    q, k, v, kw = _case(S, H, G, D, E, start, kv_start, bias_len, chunk, window, cap, sink, S + D)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    got = ops.attn(q, k, v, path="prefill_tc", status=status, **kw)[0].double()
+    assert int(status) == 0
+    for i in sorted({0, 1, 31, 32, 63, 64, 127, 128, 255, 256, S // 2, S - 1} & set(range(S))):
+        for h in range(H):
+            want, mag = _plain(q, k, v, kw, i, h)
+            # weights rounded to bf16 (2^-9 each, their sum is not), fp32 scores of at most 2^7 off by 2^-17, the result rounded
+            assert bool(((got[i, h] - want).abs() <= 2.0 ** -8 * mag + 2.0 ** -8 * want.abs() + 1e-6).all()), (i, h)
