@@ -358,40 +358,46 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             if (lane == 0) mbar_arrive(&sh.v_full[stage]);
             if (c + 2 < p.chunks) load(c + 2, raw[stage], e[stage], mi[stage], tp[stage]);
         }
-    } else if (lane == 0) {
-        // ---- K by TMA, MMAs: S += K^T (weighted V)
+    } else {
+        // ---- K by TMA, MMAs: S += K^T (weighted V).  The warp stays converged, one lane issues (see umma_ss_by)
+        const bool leader = elect_one();
+        auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(FULL, mbar_wait_bounded(bar, parity)) != 0; };
         auto fetch = [&](int c) {
             const int s = c % ST_KSTAGES;
             char* dst = k_s + s * 2 * MT_PANEL;
-            mbar_expect(&sh.k_full[s], 2 * MT_PANEL);
-            for (int q = 0; q < 2; ++q) tma_load_4d(dst + q * MT_PANEL, &map_k, n0 + q * 64, h, c * MT_TOK, b, &sh.k_full[s]);
+            if (leader) {
+                mbar_expect(&sh.k_full[s], 2 * MT_PANEL);
+                for (int q = 0; q < 2; ++q) tma_load_4d(dst + q * MT_PANEL, &map_k, n0 + q * 64, h, c * MT_TOK, b, &sh.k_full[s]);
+            }
+            __syncwarp();
         };
         const uint32_t idesc = umma_idesc_bf16(ST_P, true) | UMMA_A_MN;
-        const uint32_t ka = smem_addr(k_s), va = smem_addr(v_s);
+        const uint64_t k_desc = umma_desc_sw128_mn(smem_addr(k_s), MT_PANEL), v_desc = umma_desc_sw128_mn(smem_addr(v_s), MT_PANEL);
         int sent = 0;
         for (; sent < p.chunks && sent < ST_KSTAGES; ++sent) fetch(sent);
         bool ok = true;
         int c = 0;
-        for (; c < p.chunks && !*failed; ++c) {
+        for (; c < p.chunks && !__any_sync(FULL, *failed != 0); ++c) {
             const int stage = c & 1;
-            ok = mbar_wait_bounded(&sh.s_ready, (uint32_t)(c & 1));           // which follows the MMAs of chunk c - 1
+            ok = wait_all(&sh.s_ready, (uint32_t)(c & 1));                    // which follows the MMAs of chunk c - 1
             if (!ok) break;
             if (c >= 1 && sent < p.chunks) fetch(sent++);                     // into the stage chunk c - 1 has left
-            ok = mbar_wait_bounded(&sh.k_full[c % ST_KSTAGES], (uint32_t)((c / ST_KSTAGES) & 1)) &&
-                 mbar_wait_bounded(&sh.v_full[stage], (uint32_t)((c >> 1) & 1));
+            ok = wait_all(&sh.k_full[c % ST_KSTAGES], (uint32_t)((c / ST_KSTAGES) & 1)) && wait_all(&sh.v_full[stage], (uint32_t)((c >> 1) & 1));
             if (!ok) break;
             tc_fence_after();
+            const uint64_t kd = umma_desc_at(k_desc, (c % ST_KSTAGES) * (2 * MT_PANEL >> 4)), vd = umma_desc_at(v_desc, stage * (2 * MT_PANEL >> 4));
+#pragma unroll
             for (int part = 0; part < 2; ++part)
+#pragma unroll
                 for (int k = 0; k < MT_TOK / 16; ++k)
-                    umma_ss(tmem, umma_desc_sw128_mn(ka + (c % ST_KSTAGES) * 2 * MT_PANEL + k * 2048, MT_PANEL),
-                            umma_desc_sw128_mn(va + (stage * 2 + part) * MT_PANEL + k * 2048, MT_PANEL), idesc, 1);
-            umma_commit(&sh.mma_done);
-            umma_commit(&sh.v_empty[stage]);
+                    umma_ss_by(leader, tmem, umma_desc_at(kd, k * (2048 >> 4)), umma_desc_at(vd, part * (MT_PANEL >> 4) + k * (2048 >> 4)), idesc, 1);
+            umma_commit_by(leader, &sh.mma_done);
+            umma_commit_by(leader, &sh.v_empty[stage]);
         }
-        if (!ok) *failed = 1;
+        if (!ok && lane == 0) *failed = 1;
         if (c < p.chunks)                                     // left early: no copy stays in flight
             for (int q = c; q < sent; ++q) mbar_wait_bounded(&sh.k_full[q % ST_KSTAGES], (uint32_t)((q / ST_KSTAGES) & 1));
-        umma_commit(&sh.drained);
+        umma_commit_by(leader, &sh.drained);
         mbar_wait_bounded(&sh.drained, 0);
     }
     __syncthreads();
@@ -486,43 +492,53 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
         }
     } else if (warp == 5) {
-        if (lane == 0) {
-            const uint32_t id_k = umma_idesc_bf16(MT_TOK, false), id_mn = umma_idesc_bf16(OT_P, true);
-            const uint32_t qa = smem_addr(q_s), ra = smem_addr(ring);
-            const int k16 = (p.N + 15) / 16;
-            bool ok = mbar_wait_bounded(&sh.q_full, 0);
-            int i = 0;
-            for (; ok && i < items && !*failed; ++i) {
-                const int s = i % OT_STAGES;
-                if (i == items - 1) ok = mbar_wait_bounded(&sh.p_full, 0);
-                ok = ok && mbar_wait_bounded(&sh.full[s], (uint32_t)((i / OT_STAGES) & 1));
-                if (!ok) break;
-                tc_fence_after();
-                const uint32_t sa = ra + s * OT_STAGE;
-                if (i < k_items) {                            // scores
-                    for (int k = i * 8; k < k16 && k < i * 8 + 8; ++k) {
-                        const uint32_t off = (uint32_t)(k >> 2) * MT_PANEL + (k & 3) * 32;
-                        umma_ss(t_sc, umma_desc_sw128(qa + off), umma_desc_sw128(sa + off - i * 2 * MT_PANEL), id_k, k > 0);
-                    }
-                    if (i == k_items - 1) umma_commit(&sh.s_full);
-                } else if (i < items - 1) {                   // Q S_in, value and remainder
-                    const int j = i - k_items;
-                    for (int part = 0; part < 2; ++part)
-                        for (int k = j * 4; k < k16 && k < j * 4 + 4; ++k)
-                            umma_ss(t_qs, umma_desc_sw128(qa + (uint32_t)j * MT_PANEL + (k & 3) * 32),
-                                    umma_desc_sw128_mn(sa + part * 2 * OT_S_PANEL + (k & 3) * 2048, OT_S_PANEL), id_mn, k > 0 || part > 0);
-                } else {                                      // weights V, value and remainder
-                    for (int part = 0; part < 2; ++part)
-                        for (int k = 0; k < MT_TOK / 16; ++k)
-                            umma_ts(t_wv, t_w + part * 64 + k * 8, umma_desc_sw128_mn(sa + k * 2048, MT_PANEL), id_mn, k > 0 || part > 0);
-                    umma_commit(&sh.done);
+        // the warp stays converged, one lane issues (see umma_ss_by)
+        const bool leader = elect_one();
+        auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(FULL, mbar_wait_bounded(bar, parity)) != 0; };
+        const uint32_t id_k = umma_idesc_bf16(MT_TOK, false), id_mn = umma_idesc_bf16(OT_P, true);
+        const uint64_t q_desc = umma_desc_sw128(smem_addr(q_s)), ring_k = umma_desc_sw128(smem_addr(ring)),
+                       ring_s = umma_desc_sw128_mn(smem_addr(ring), OT_S_PANEL), ring_v = umma_desc_sw128_mn(smem_addr(ring), MT_PANEL);
+        const int k16 = (p.N + 15) / 16;
+        bool ok = wait_all(&sh.q_full, 0);
+        for (int i = 0; ok && i < items && !__any_sync(FULL, *failed != 0); ++i) {
+            const int s = i % OT_STAGES;
+            const uint32_t at = s * (OT_STAGE >> 4);
+            if (i == items - 1) ok = wait_all(&sh.p_full, 0);
+            ok = ok && wait_all(&sh.full[s], (uint32_t)((i / OT_STAGES) & 1));
+            if (!ok) break;
+            tc_fence_after();
+            if (i < k_items) {                                // scores
+                const uint64_t qd = umma_desc_at(q_desc, i * (2 * MT_PANEL >> 4)), kd = umma_desc_at(ring_k, at);
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const uint32_t off = (uint32_t)(k >> 2) * (MT_PANEL >> 4) + (k & 3) * 2;
+                    if (i * 8 + k < k16) umma_ss_by(leader, t_sc, umma_desc_at(qd, off), umma_desc_at(kd, off), id_k, i > 0 || k > 0);
                 }
-                umma_commit(&sh.empty[s]);
+                if (i == k_items - 1) umma_commit_by(leader, &sh.s_full);
+            } else if (i < items - 1) {                       // Q S_in, value and remainder
+                const int j = i - k_items;
+                const uint64_t qd = umma_desc_at(q_desc, j * (MT_PANEL >> 4)), sd = umma_desc_at(ring_s, at);
+#pragma unroll
+                for (int part = 0; part < 2; ++part)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k)
+                        if (j * 4 + k < k16)
+                            umma_ss_by(leader, t_qs, umma_desc_at(qd, k * 2), umma_desc_at(sd, (part * 2 * OT_S_PANEL + k * 2048) >> 4),
+                                       id_mn, j > 0 || k > 0 || part > 0);
+            } else {                                          // weights V, value and remainder
+                const uint64_t vd = umma_desc_at(ring_v, at);
+#pragma unroll
+                for (int part = 0; part < 2; ++part)
+#pragma unroll
+                    for (int k = 0; k < MT_TOK / 16; ++k)
+                        umma_ts_by(leader, t_wv, t_w + part * 64 + k * 8, umma_desc_at(vd, k * (2048 >> 4)), id_mn, k > 0 || part > 0);
+                umma_commit_by(leader, &sh.done);
             }
-            if (!ok) *failed = 1;
-            umma_commit(&sh.drained);                         // leave no MMA and no barrier arrival in flight
-            mbar_wait_bounded(&sh.drained, 0);
+            umma_commit_by(leader, &sh.empty[s]);
         }
+        if (!ok && lane == 0) *failed = 1;
+        umma_commit_by(leader, &sh.drained);                  // leave no MMA and no barrier arrival in flight
+        mbar_wait_bounded(&sh.drained, 0);
     } else {
         // ---- thread = token
         const int t = warp * 32 + lane;

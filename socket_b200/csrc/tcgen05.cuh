@@ -177,8 +177,10 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int n, bool b_mn_major) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn_major ? 1u << 16 : 0u) | ((uint32_t)(n >> 3) << 17) |
            ((128u >> 4) << 24);
 }
-// The same, and the commit, for a warp that stays converged: the lane with `leader` set issues.  Operands then are
-// warp-uniform values to the compiler, which the instruction needs; inside one lane's branch each would be moved there.
+// D (tensor memory) (+)= A B with A in shared memory (ss) or in tensor memory, two bf16 per column (ts), B in shared
+// memory; and the commit.  For a warp that stays converged, of which the lane with `leader` set issues: operands then are
+// warp-uniform values to the compiler, which the instruction needs.  Inside one lane's branch each is moved there by itself,
+// and an MMA costs about 200 cycles to issue.
 __device__ __forceinline__ void umma_ss_by(bool leader, uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
@@ -220,23 +222,5 @@ __device__ __forceinline__ bool elect_one() {
     return r != 0;
 }
 constexpr uint32_t UMMA_A_MN = 1u << 15;             // the K index of A runs over the rows, as b_mn_major says of B
-// D (tensor memory) (+)= A (shared memory) B (shared memory)
-__device__ __forceinline__ void umma_ss(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// D (tensor memory) (+)= A (tensor memory, two bf16 per column) B (shared memory)
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
 
 }  // namespace sk
