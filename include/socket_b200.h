@@ -411,6 +411,37 @@ SK_API int sk_decode_step(const sk_decode_params* p, void* stream);
 SK_API int64_t sk_decode_step_rescored_rows_offset(int B, int H, int Hkv, int D, int L, int R, int64_t T_max,
                                             int64_t M, int sink, int window);
 
+/* out [rows, n] = x [rows, k] W^T, W [n, k] with rows w_ld elements apart: the projections of a decode step, at most 8
+ * rows, bf16 or fp16, fp32 sums.  `res` (or NULL; element type of x) is added to the sums; out has the element type of
+ * x, or fp32 with out_f32.  With ff > 0 the same launch also takes x through a gated unit (SKB_GLU_CLAMPED: g * sigmoid(slope * g) * (u + 1) of g = min(gate, limit),
+ * u = clamp(up, -limit, limit); SKB_GLU_SILU: gate * sigmoid(gate) * up):
+ *   act [rows, ff] = unit(x G^T, x U^T), G and U the ff rows of W from gate_row and from up_row on
+ * whose sums are not rounded in between; n may then be 0.  `chained`: the caller vouches that the kernel before this one
+ * on the stream does not write W, and the weights may be requested before that kernel has ended.
+ * sk_linear_rows_applicable: whether shapes, strides and alignment are taken (k and w_ld multiples of 16, W 32-byte
+ * aligned, x rows 16-byte aligned). */
+enum { SKB_GLU_CLAMPED = 0, SKB_GLU_SILU = 1 };
+typedef struct sk_linear_params {
+    const void* x;
+    const void* w;
+    const void* res;
+    void* out;
+    void* act;
+    int64_t x_ld, w_ld, res_ld, out_ld, act_ld, gate_row, up_row;
+    int rows, n, k, ff, dtype, out_f32, glu, chained;
+    float limit, slope;
+} sk_linear_params;
+SK_API int sk_linear_rows_applicable(const sk_linear_params* p);
+SK_API int sk_linear_rows(const sk_linear_params* p, void* stream);
+
+/* out [rows, width] = x / sqrt(mean(x^2) + eps) * w per row, fp32 arithmetic. */
+SK_API int sk_rms_norm(const void* x, const void* w, int dtype, int64_t rows, int width, float eps, void* out, void* stream);
+
+/* The end of a greedy decode step: token[b] = index of the largest of logits [b, :vocab] (rows ld elements apart; the
+ * first of equal ones, NaN before all), then pos[0] += 1 and seqlens[b] += 1. */
+SK_API int sk_pick_token(const void* logits, int dtype, int64_t ld, int batch, int vocab, int64_t* token, int64_t* pos,
+                         int32_t* seqlens, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

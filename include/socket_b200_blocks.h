@@ -56,31 +56,17 @@ typedef struct sk_residual_params {
 } sk_residual_params;
 SK_API int skb_residual_norm(const sk_residual_params* p, void* stream);
 
-/* out [rows, n] = x [rows, k] W^T, W [n, k] with rows w_ld elements apart: the projections of a decode step, at most 8
- * rows, bf16 or fp16, fp32 sums.  `res` (or NULL; element type of x) is added to the sums; out has the element type of
- * x, or fp32 with out_f32.  With ff > 0 the same launch also takes x through a gated unit (see skb_glu):
- *   act [rows, ff] = unit(x G^T, x U^T), G and U the ff rows of W from gate_row and from up_row on
- * whose sums are not rounded in between; n may then be 0.  `chained`: the caller vouches that the kernel before this one
- * on the stream does not write W, and the weights may be requested before that kernel has ended.
- * skb_linear_rows_applicable: whether shapes, strides and alignment are taken (k and w_ld multiples of 16, W 32-byte
- * aligned, x rows 16-byte aligned). */
-typedef struct sk_linear_params {
-    const void* x;
-    const void* w;
-    const void* res;
-    void* out;
-    void* act;
-    int64_t x_ld, w_ld, res_ld, out_ld, act_ld, gate_row, up_row;
-    int rows, n, k, ff, dtype, out_f32, glu, chained;
-    float limit, slope;
-} sk_linear_params;
+/* The few rows' projections of socket_b200.h. */
 SK_API int skb_linear_rows_applicable(const sk_linear_params* p);
 SK_API int skb_linear_rows(const sk_linear_params* p, void* stream);
+
+/* The end of a greedy decode step, as sk_pick_token of socket_b200.h. */
+SK_API int skb_pick_token(const void* logits, int dtype, int64_t ld, int batch, int vocab, int64_t* token, int64_t* pos,
+                          int32_t* seqlens, void* stream);
 
 /* Gated unit of a feed-forward; gate and up rows are `ld` elements apart, out rows out_ld:
  *   SKB_GLU_CLAMPED  out = g * sigmoid(slope * g) * (u + 1), g = min(gate, limit), u = clamp(up, -limit, limit)
  *   SKB_GLU_SILU     out = gate * sigmoid(gate) * up */
-enum { SKB_GLU_CLAMPED = 0, SKB_GLU_SILU = 1 };
 SK_API int skb_glu(const void* gate, const void* up, int dtype, int64_t rows, int ff, int64_t ld, int kind, float limit,
                    float slope, void* out, int64_t out_ld, void* stream);
 

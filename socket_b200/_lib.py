@@ -45,6 +45,16 @@ class DecodeParams(C.Structure):
 
 _i, _i64, _p, _f, _sz = C.c_int, C.c_int64, C.c_void_p, C.c_float, C.c_size_t
 
+class LinearParams(C.Structure):
+    """Mirror of `sk_linear_params`."""
+    _fields_ = [
+        ("x", _p), ("w", _p), ("res", _p), ("out", _p), ("act", _p),
+        ("x_ld", _i64), ("w_ld", _i64), ("res_ld", _i64), ("out_ld", _i64), ("act_ld", _i64), ("gate_row", _i64), ("up_row", _i64),
+        ("rows", _i), ("n", _i), ("k", _i), ("ff", _i), ("dtype", _i), ("out_f32", _i), ("glu", _i), ("chained", _i),
+        ("limit", _f), ("slope", _f),
+    ]
+
+
 # name -> (restype, argtypes); the order follows include/socket_b200.h
 SIGNATURES = {
     "sk_abi_version": (_i, []),
@@ -91,6 +101,10 @@ SIGNATURES = {
     "sk_decode_step_workspace_bytes": (_sz, [_i, _i, _i, _i, _i, _i, _i64, _i64, _i, _i]),
     "sk_decode_step_rescored_rows_offset": (_i64, [_i, _i, _i, _i, _i, _i, _i64, _i64, _i, _i]),
     "sk_decode_step": (_i, [C.POINTER(DecodeParams), _p]),
+    "sk_linear_rows_applicable": (_i, [C.POINTER(LinearParams)]),
+    "sk_linear_rows": (_i, [C.POINTER(LinearParams), _p]),
+    "sk_rms_norm": (_i, [_p, _p, _i, _i64, _i, _f, _p, _p]),
+    "sk_pick_token": (_i, [_p, _i, _i64, _i, _i, _p, _p, _p, _p]),
 }
 
 
@@ -100,16 +114,6 @@ class ResidualParams(C.Structure):
         ("x", _p), ("y", _p), ("w_in", _p), ("x0", _p), ("w_out", _p), ("out", _p),
         ("rows", _i64), ("y_ld", _i64),
         ("width", _i), ("in_mode", _i), ("out_mode", _i), ("dtype", _i), ("y_dtype", _i), ("eps", _f),
-    ]
-
-
-class LinearParams(C.Structure):
-    """Mirror of `sk_linear_params`."""
-    _fields_ = [
-        ("x", _p), ("w", _p), ("res", _p), ("out", _p), ("act", _p),
-        ("x_ld", _i64), ("w_ld", _i64), ("res_ld", _i64), ("out_ld", _i64), ("act_ld", _i64), ("gate_row", _i64), ("up_row", _i64),
-        ("rows", _i), ("n", _i), ("k", _i), ("ff", _i), ("dtype", _i), ("out_f32", _i), ("glu", _i), ("chained", _i),
-        ("limit", _f), ("slope", _f),
     ]
 
 
@@ -175,6 +179,7 @@ BLOCK_SIGNATURES = {
     "skb_residual_norm": (_i, [C.POINTER(ResidualParams), _p]),
     "skb_linear_rows_applicable": (_i, [C.POINTER(LinearParams)]),
     "skb_linear_rows": (_i, [C.POINTER(LinearParams), _p]),
+    "skb_pick_token": (_i, [_p, _i, _i64, _i, _i, _p, _p, _p, _p]),
     "skb_glu": (_i, [_p, _p, _i, _i64, _i, _i64, _i, _f, _f, _p, _i64, _p]),
     "skb_ring_append": (_i, [_p, _p, _i, _i, _i, _i64, _i64, _i64, _i64, _i, _i, _i, _i, _p, _i64, _p, _p, _p]),
     "skb_rotary_rows": (_i, [C.POINTER(RotaryRowsParams), _p]),

@@ -11,13 +11,13 @@ from torch import Tensor
 
 from . import _lib
 from ._lib import blocks, check_blocks, dtype_code, ptr, stream_ptr
+from .few_rows import GLU_CLAMPED, GLU_SILU, _linear_params, linear, linear_glu  # noqa: F401
 from .ops import _require_cuda
 
 ATTN_PATHS = {"auto": 0, "rows": 1, "prefill_tc": 2, "decode": 3}
 SSM_PATHS = {"auto": 0, "steps": 1, "chunks": 2, "tensor": 3}
 IN_NONE, IN_ADD_NORM, IN_REPLACE, IN_ADD = 0, 1, 2, 3
 OUT_NONE, OUT_NORM, OUT_CONCAT, OUT_LAYER_NORM = 0, 1, 2, 3
-GLU_CLAMPED, GLU_SILU = 0, 1
 RING_KEEP = {"chunk": 0, "window": 1}
 GLU_SLOPE = 1.702
 
@@ -71,54 +71,6 @@ def residual_norm(x: Tensor, eps: float, *, y: Optional[Tensor] = None, w_in: Op
     p.out = ptr(out)
     check_blocks(blocks().skb_residual_norm(C.byref(p), stream_ptr(x.device)), "skb_residual_norm")
     return out
-
-
-def _linear_params(x: Tensor, w: Tensor, chained: bool) -> Optional[_lib.LinearParams]:
-    """The parameter block of a product of a few rows, or None when the kernel does not take these shapes."""
-    rows, k = x.shape
-    if rows > 8 or x.dtype == torch.float32 or not x.is_cuda or x.stride(1) != 1 or w.stride(1) != 1:
-        return None
-    p = _lib.LinearParams()
-    p.x, p.w, p.x_ld, p.w_ld, p.rows, p.k, p.dtype = ptr(x), ptr(w), x.stride(0) if rows > 1 else max(x.stride(0), k), w.stride(0), rows, k, dtype_code(x)
-    p.chained = int(chained)
-    return p if blocks().skb_linear_rows_applicable(C.byref(p)) else None
-
-
-def linear(x: Tensor, w: Tensor, *, f32: bool = False, res: Optional[Tensor] = None, chained: bool = False) -> Tensor:
-    """x [rows, k] w^T (+ res [rows, n]) with fp32 sums, rounded to x's type unless `f32`.  Few rows (a decode step) go to
-    the kernel that streams the weights, others to the library.  `chained`: the kernel before this call on the stream
-    does not write w (see `skb_linear_rows`)."""
-    assert x.shape[1] == w.shape[1] and x.dtype == w.dtype and x.device == w.device
-    p = _linear_params(x, w, chained)
-    if p is None:
-        out = torch.mm(x, w.t(), out_dtype=torch.float32) if f32 and x.dtype != torch.float32 else torch.mm(x, w.t())
-        return out if res is None else out + res
-    n = w.shape[0]
-    out = torch.empty(x.shape[0], n, dtype=torch.float32 if f32 else x.dtype, device=x.device)
-    p.out, p.out_ld, p.n, p.out_f32 = ptr(out), n, n, int(f32)
-    if res is not None:
-        assert res.shape == out.shape and res.dtype == x.dtype and res.stride(1) == 1
-        p.res, p.res_ld = ptr(res), max(res.stride(0), n)
-    check_blocks(blocks().skb_linear_rows(C.byref(p), stream_ptr(x.device)), "skb_linear_rows")
-    return out
-
-
-def linear_glu(x: Tensor, w: Tensor, gate_row: int, up_row: int, ff: int, kind: int, *, limit: float = 0.0, slope: float = 1.0,
-               plain: int = 0, act: Optional[Tensor] = None, chained: bool = False):
-    """(x w[:plain]^T, unit(x G^T, x U^T)) with G, U the ff rows of w from `gate_row` and `up_row` on, in one launch; `act`
-    may be a slice of wider rows.  None when the shapes are not the kernel's."""
-    assert x.shape[1] == w.shape[1] and x.dtype == w.dtype and max(gate_row, up_row) + ff <= w.shape[0] and plain <= w.shape[0]
-    p = _linear_params(x, w, chained)
-    if p is None:
-        return None
-    out = torch.empty(x.shape[0], plain, dtype=x.dtype, device=x.device)
-    if act is None:
-        act = torch.empty(x.shape[0], ff, dtype=x.dtype, device=x.device)
-    assert act.shape == (x.shape[0], ff) and act.dtype == x.dtype and act.stride(1) == 1
-    p.out, p.out_ld, p.n, p.act, p.act_ld = ptr(out) if plain else 0, plain, plain, ptr(act), max(act.stride(0), ff)
-    p.ff, p.gate_row, p.up_row, p.glu, p.limit, p.slope = ff, gate_row, up_row, kind, float(limit), float(slope)
-    check_blocks(blocks().skb_linear_rows(C.byref(p), stream_ptr(x.device)), "skb_linear_rows")
-    return out, act
 
 
 def _glu(gate: Tensor, up: Tensor, kind: int, limit: float, slope: float, out: Optional[Tensor]) -> Tensor:

@@ -3,6 +3,7 @@
 #include <cstring>
 
 #include "abi_check.cuh"
+#include "blocks.cuh"
 
 namespace sk {
 
@@ -619,6 +620,18 @@ int sk_decode_step(const sk_decode_params* p, void* stream) {
                               up256(sparse_decode_workspace_bytes(p->B, p->H, p->D, lay.list_stride)),
                               p->status, st);
     return rc;
+}
+
+int sk_linear_rows_applicable(const sk_linear_params* p) { return p != nullptr && linear_rows_applicable(*p) ? 1 : 0; }
+int sk_linear_rows(const sk_linear_params* p, void* stream) { return linear_rows(p, (cudaStream_t)stream); }
+
+int sk_rms_norm(const void* x, const void* w, int dtype, int64_t rows, int width, float eps, void* out, void* stream) {
+    return rms_norm_rows(x, w, dtype, rows, width, eps, out, (cudaStream_t)stream);
+}
+
+int sk_pick_token(const void* logits, int dtype, int64_t ld, int batch, int vocab, int64_t* token, int64_t* pos, int32_t* seqlens,
+                  void* stream) {
+    return pick_token(logits, dtype, ld, batch, vocab, token, pos, seqlens, (cudaStream_t)stream);
 }
 
 }  // extern "C"

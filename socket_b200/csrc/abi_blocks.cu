@@ -104,16 +104,11 @@ int skb_residual_norm(const sk_residual_params* p, void* stream) {
 
 int skb_linear_rows_applicable(const sk_linear_params* p) { return p != nullptr && linear_rows_applicable(*p) ? 1 : 0; }
 
-int skb_linear_rows(const sk_linear_params* p, void* stream) {
-    SK_REQUIRE(p && p->x && p->w && p->rows > 0 && p->k > 0 && p->n >= 0 && p->ff >= 0 && p->n + p->ff > 0,
-               "skb_linear_rows: null pointer or empty product");
-    SK_REQUIRE((p->n == 0 || (p->out && p->out_ld >= p->n)) && (p->res == nullptr || p->res_ld >= p->n) && p->x_ld >= p->k && p->w_ld >= p->k,
-               "skb_linear_rows: output missing or row stride smaller than row");
-    SK_REQUIRE(p->ff == 0 || (p->act && p->act_ld >= p->ff && p->gate_row >= 0 && p->up_row >= 0 &&
-                              (p->glu == SKB_GLU_CLAMPED || p->glu == SKB_GLU_SILU)), "skb_linear_rows: gated unit incomplete");
-    if (!linear_rows_applicable(*p))
-        return fail(SK_ERR_UNSUPPORTED, "skb_linear_rows: at most 8 rows of bf16 or fp16, k and the weights' row stride multiples of 16, aligned rows");
-    return launch_linear_rows(*p, (cudaStream_t)stream);
+int skb_linear_rows(const sk_linear_params* p, void* stream) { return linear_rows(p, (cudaStream_t)stream); }
+
+int skb_pick_token(const void* logits, int dtype, int64_t ld, int batch, int vocab, int64_t* token, int64_t* pos, int32_t* seqlens,
+                   void* stream) {
+    return pick_token(logits, dtype, ld, batch, vocab, token, pos, seqlens, (cudaStream_t)stream);
 }
 
 int skb_glu(const void* gate, const void* up, int dtype, int64_t rows, int ff, int64_t ld, int kind, float limit, float slope,

@@ -98,7 +98,10 @@ int launch_embed_rows(const int64_t* tokens, const void* table, int dtype, int64
                       float scale, float* x, float* x_copy, int32_t* status, cudaStream_t st);
 int launch_residual_norm(const sk_residual_params& p, cudaStream_t st);
 bool linear_rows_applicable(const sk_linear_params& p);
-int launch_linear_rows(const sk_linear_params& p, cudaStream_t st);
+int linear_rows(const sk_linear_params* p, cudaStream_t st);             // both libraries' entry point, with its checks
+int pick_token(const void* logits, int dtype, int64_t ld, int batch, int vocab, int64_t* token, int64_t* pos, int32_t* seqlens,
+               cudaStream_t st);                                         // the same
+int rms_norm_rows(const void* x, const void* w, int dtype, int64_t rows, int width, float eps, void* out, cudaStream_t st);
 int launch_glu(const void* gate, const void* up, int dtype, int64_t rows, int ff, int64_t ld, int kind, float limit, float slope,
                void* out, int64_t out_ld, cudaStream_t st);
 int launch_ring_append(const void* k, const void* v, int dtype, int B, int S, int64_t k_bs, int64_t k_ss, int64_t v_bs,

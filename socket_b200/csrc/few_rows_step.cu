@@ -1,0 +1,3 @@
+// The kernels of a decode step's few rows, for the step library.
+#include "linear_rows_body.cuh"
+#include "token_rows_body.cuh"

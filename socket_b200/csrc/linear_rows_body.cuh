@@ -16,6 +16,8 @@
 // Measured (one row, cold weights, back to back in a graph; chained / not / cuBLAS): 4096 x 14336 20.1 / 21.7 / 24.4 us
 // (5.9 TB/s), 28672 x 4096 38.2 / 39.6 / 39.1 us, 4096 x 4096 6.2 / 8.2 / 12.9 us, 2048 x 2048 2.4 / 4.0 / 7.3 us; with
 // 8 rows within 3% of that.
+#pragma once
+#include "abi_check.cuh"
 #include "blocks.cuh"
 
 namespace sk {
@@ -228,8 +230,16 @@ bool linear_rows_applicable(const sk_linear_params& p) {
            (uintptr_t)p.w % 32 == 0 && (uintptr_t)p.x % 16 == 0;
 }
 
-int launch_linear_rows(const sk_linear_params& p, cudaStream_t st) {
-    return p.dtype == SK_BF16 ? linear_dispatch<__nv_bfloat16>(p, st) : linear_dispatch<__half>(p, st);
+int linear_rows(const sk_linear_params* p, cudaStream_t st) {
+    SK_REQUIRE(p && p->x && p->w && p->rows > 0 && p->k > 0 && p->n >= 0 && p->ff >= 0 && p->n + p->ff > 0,
+               "linear_rows: null pointer or empty product");
+    SK_REQUIRE((p->n == 0 || (p->out && p->out_ld >= p->n)) && (p->res == nullptr || p->res_ld >= p->n) && p->x_ld >= p->k && p->w_ld >= p->k,
+               "linear_rows: output missing or row stride smaller than row");
+    SK_REQUIRE(p->ff == 0 || (p->act && p->act_ld >= p->ff && p->gate_row >= 0 && p->up_row >= 0 &&
+                              (p->glu == SKB_GLU_CLAMPED || p->glu == SKB_GLU_SILU)), "linear_rows: gated unit incomplete");
+    if (!linear_rows_applicable(*p))
+        return fail(SK_ERR_UNSUPPORTED, "linear_rows: at most 8 rows of bf16 or fp16, k and the weights' row stride multiples of 16, aligned rows");
+    return p->dtype == SK_BF16 ? linear_dispatch<__nv_bfloat16>(*p, st) : linear_dispatch<__half>(*p, st);
 }
 
 }  // namespace sk

@@ -17,6 +17,8 @@ import torch
 import torch.nn as nn
 from torch import Tensor
 
+from . import few_rows
+
 
 def find_multiple(n: int, k: int) -> int:
     return n if n % k == 0 else n + k - (n % k)
@@ -108,6 +110,9 @@ class Decoder(nn.Module):
     def _decode_body(self, mode: str) -> None:
         logits = self._decode_logits(mode)
         self._logits = logits
+        if logits.is_cuda:
+            few_rows.pick_token(logits, self._tok, self._pos, self._seqlens, self.libraries[0])
+            return
         self._tok.copy_(torch.argmax(logits, dim=-1, keepdim=True))
         self._pos.add_(1)
         self._seqlens.add_(1)

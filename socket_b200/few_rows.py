@@ -1,0 +1,89 @@
+"""Operators on the few rows of a decode step that every decoder uses: projections that stream the weights once, an RMS
+norm of rows in the model's type, the greedy pick.  Both libraries hold the kernels; a model calls those of the library
+it is built on (`library`: "step" or "blocks")."""
+from __future__ import annotations
+
+import ctypes as C
+from typing import Optional
+
+import torch
+from torch import Tensor
+
+from . import _lib
+from ._lib import blocks, check, check_blocks, dtype_code, lib, ptr, stream_ptr
+
+GLU_CLAMPED, GLU_SILU = 0, 1
+
+
+def _call(library: str, name: str, *args) -> int:
+    return getattr(lib(), "sk_" + name)(*args) if library == "step" else getattr(blocks(), "skb_" + name)(*args)
+
+
+def _launch(library: str, name: str, *args) -> None:
+    (check if library == "step" else check_blocks)(_call(library, name, *args), name)
+
+
+def _linear_params(x: Tensor, w: Tensor, chained: bool, library: str = "blocks") -> Optional[_lib.LinearParams]:
+    """The parameter block of a product of a few rows, or None when the kernel does not take these shapes."""
+    rows, k = x.shape
+    if rows > 8 or x.dtype == torch.float32 or not x.is_cuda or x.stride(1) != 1 or w.stride(1) != 1:
+        return None
+    p = _lib.LinearParams()
+    p.x, p.w, p.x_ld, p.w_ld, p.rows, p.k, p.dtype = ptr(x), ptr(w), x.stride(0) if rows > 1 else max(x.stride(0), k), w.stride(0), rows, k, dtype_code(x)
+    p.chained = int(chained)
+    return p if _call(library, "linear_rows_applicable", C.byref(p)) else None
+
+
+def linear(x: Tensor, w: Tensor, *, f32: bool = False, res: Optional[Tensor] = None, chained: bool = False,
+           library: str = "blocks") -> Tensor:
+    """x [rows, k] w^T (+ res [rows, n]) with fp32 sums, rounded to x's type unless `f32`.  Few rows (a decode step) go to
+    the kernel that streams the weights, others to the library.  `chained`: the kernel before this call on the stream
+    does not write w (see `skb_linear_rows`)."""
+    assert x.shape[1] == w.shape[1] and x.dtype == w.dtype and x.device == w.device
+    p = _linear_params(x, w, chained, library)
+    if p is None:
+        out = torch.mm(x, w.t(), out_dtype=torch.float32) if f32 and x.dtype != torch.float32 else torch.mm(x, w.t())
+        return out if res is None else out + res
+    n = w.shape[0]
+    out = torch.empty(x.shape[0], n, dtype=torch.float32 if f32 else x.dtype, device=x.device)
+    p.out, p.out_ld, p.n, p.out_f32 = ptr(out), n, n, int(f32)
+    if res is not None:
+        assert res.shape == out.shape and res.dtype == x.dtype and res.stride(1) == 1
+        p.res, p.res_ld = ptr(res), max(res.stride(0), n)
+    _launch(library, "linear_rows", C.byref(p), stream_ptr(x.device))
+    return out
+
+
+def linear_glu(x: Tensor, w: Tensor, gate_row: int, up_row: int, ff: int, kind: int, *, limit: float = 0.0, slope: float = 1.0,
+               plain: int = 0, act: Optional[Tensor] = None, chained: bool = False, library: str = "blocks"):
+    """(x w[:plain]^T, unit(x G^T, x U^T)) with G, U the ff rows of w from `gate_row` and `up_row` on, in one launch; `act`
+    may be a slice of wider rows.  None when the shapes are not the kernel's."""
+    assert x.shape[1] == w.shape[1] and x.dtype == w.dtype and max(gate_row, up_row) + ff <= w.shape[0] and plain <= w.shape[0]
+    p = _linear_params(x, w, chained, library)
+    if p is None:
+        return None
+    out = torch.empty(x.shape[0], plain, dtype=x.dtype, device=x.device)
+    if act is None:
+        act = torch.empty(x.shape[0], ff, dtype=x.dtype, device=x.device)
+    assert act.shape == (x.shape[0], ff) and act.dtype == x.dtype and act.stride(1) == 1
+    p.out, p.out_ld, p.n, p.act, p.act_ld = ptr(out) if plain else 0, plain, plain, ptr(act), max(act.stride(0), ff)
+    p.ff, p.gate_row, p.up_row, p.glu, p.limit, p.slope = ff, gate_row, up_row, kind, float(limit), float(slope)
+    _launch(library, "linear_rows", C.byref(p), stream_ptr(x.device))
+    return out, act
+
+
+def rms_norm(x: Tensor, w: Tensor, eps: float) -> Tensor:
+    """x [..., width] -> x / rms(x) * w in x's type, fp32 arithmetic (the step library's)."""
+    assert x.is_cuda and x.is_contiguous() and w.is_contiguous() and w.shape == x.shape[-1:] and w.dtype == x.dtype
+    out = torch.empty_like(x)
+    check(lib().sk_rms_norm(ptr(x), ptr(w), dtype_code(x), x.numel() // x.shape[-1], x.shape[-1], float(eps), ptr(out),
+                            stream_ptr(x.device)), "sk_rms_norm")
+    return out
+
+
+def pick_token(logits: Tensor, token: Tensor, pos: Tensor, seqlens: Tensor, library: str) -> None:
+    """token [batch, 1] = index of the largest of logits [batch, vocab]; pos and seqlens count one token more."""
+    assert logits.is_cuda and logits.dim() == 2 and logits.stride(1) == 1 and token.is_contiguous() and token.numel() == logits.shape[0]
+    assert token.dtype == pos.dtype == torch.int64 and seqlens.dtype == torch.int32 and seqlens.numel() == logits.shape[0]
+    _launch(library, "pick_token", ptr(logits), dtype_code(logits), max(logits.stride(0), logits.shape[1]), logits.shape[0],
+            logits.shape[1], ptr(token), ptr(pos), ptr(seqlens), stream_ptr(logits.device))

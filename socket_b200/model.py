@@ -31,7 +31,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch import Tensor
 
-from . import ops, tp
+from . import few_rows, ops, tp
 from .attention import KVCache
 from .decoder import Decoder, find_multiple, generate  # noqa: F401  (generate: the public entry point)
 from .synth import hypercube_protos
@@ -99,6 +99,12 @@ class RMSNorm(nn.Module):
         xf = x.float()
         return (xf * torch.rsqrt(torch.mean(xf * xf, dim=-1, keepdim=True) + self.eps)).type_as(x) * self.weight
 
+    def few_rows(self, x: Tensor) -> Tensor:
+        """The same for the rows of a decode step on a GPU."""
+        if x.dtype != self.weight.dtype:
+            return self.forward(x)
+        return few_rows.rms_norm(x.contiguous(), self.weight, self.eps)
+
 
 def precompute_freqs_cis(seq_len: int, n_elem: int, base: float = 10000, device=None) -> Tensor:
     """[seq_len, n_elem/2, 2] (cos, sin) in bf16, as GPT-FAST/model.py:617-623."""
@@ -117,6 +123,19 @@ def apply_rotary_emb(x: Tensor, freqs_cis: Tensor, out: Optional[Tensor] = None)
         return y.type_as(x)
     out.copy_(y.view(out.shape))
     return out
+
+
+def few_rows_here(x: Tensor, world: int) -> bool:
+    """Whether a decode step's projections go to the kernel that streams the weights: one GPU's whole matrices, at most
+    8 rows of a 16-bit type.  (Widths outside its rules still go to the library, inside `few_rows.linear`.)"""
+    return x.is_cuda and world == 1 and x.shape[0] * x.shape[1] <= 8 and x.dtype in (torch.bfloat16, torch.float16)
+
+
+def project_rows(x: Tensor, layer: nn.Linear, res: Optional[Tensor] = None) -> Tensor:
+    """layer(x) (+ res) of the rows [B, 1, width] of a decode step.  The kernel before it is one that made x: no weights."""
+    y = few_rows.linear(x.reshape(-1, x.shape[-1]), layer.weight, res=None if res is None else res.reshape(-1, res.shape[-1]),
+                        chained=True, library="step")
+    return y.view(*x.shape[:-1], -1)
 
 
 class FeedForward(nn.Module):
@@ -144,6 +163,13 @@ class FeedForward(nn.Module):
     def forward(self, x: Tensor) -> Tensor:
         return self.w2(self.hidden(x))
 
+    def decode(self, x: Tensor, res: Tensor) -> Tensor:
+        """res + forward(x) for a few rows: gate, up and unit in one launch, the residual in the other."""
+        unit = few_rows.linear_glu(x.reshape(-1, x.shape[-1]), self.w13.weight, 0, self.inter, self.inter, few_rows.GLU_SILU,
+                                   chained=True, library="step")
+        hidden = self.hidden(x) if unit is None else unit[1].view(*x.shape[:-1], -1)
+        return project_rows(hidden, self.w2, res)
+
 
 class Attention(nn.Module):
     """`wqkv` / `wo` around the SOCKET state (planes, protos_T, the cache with codes and norms).
@@ -170,6 +196,7 @@ class Attention(nn.Module):
         self.register_buffer("planes", torch.randn(self.L, self.K, self.head_dim))
         self.register_buffer("protos_T", hypercube_protos(self.K) if self.R == 1 << self.K
                              else torch.randn(self.K, self.R))
+        self.world = world
         self.kv_cache: Optional[KVCache] = None
         self._step = None
 
@@ -211,7 +238,7 @@ class Attention(nn.Module):
         keys already cached (dense mode); `freqs_cis` the position's rotary row (CPU flow),
         `rope_table` the whole table (GPU flow: the row is picked on the device)."""
         B = x.shape[0]
-        qkv = self.wqkv(x)
+        qkv = project_rows(x, self.wqkv) if few_rows_here(x, self.world) else self.wqkv(x)
         if x.is_cuda:
             # split + rotary embedding of q and k in one launch, straight into the step's inputs
             ops.rope_split(qkv, rope_table, pos, self.n_head, self.n_local_heads, self.q_s, self.k_s, self.v_s)
@@ -282,6 +309,10 @@ class TransformerBlock(nn.Module):
             y = self.attention.decode(self.attention_norm(x), freqs_cis, pos, seqlens, mode, rope_table, project=False)
             h = fused(y, self.attention.wo.weight, res=x.contiguous())
             return fused(self.feed_forward.hidden(self.ffn_norm(h)), self.feed_forward.w2.weight, res=h)
+        if few_rows_here(x, self.world):
+            y = self.attention.decode(self.attention_norm.few_rows(x), freqs_cis, pos, seqlens, mode, rope_table, project=False)
+            h = project_rows(y, self.attention.wo, x)
+            return self.feed_forward.decode(self.ffn_norm.few_rows(h), h)
         h = x + self._sum(self.attention.decode(self.attention_norm(x), freqs_cis, pos, seqlens, mode, rope_table))
         return h + self._sum(self.feed_forward(self.ffn_norm(h)))
 
@@ -369,6 +400,8 @@ class Transformer(Decoder):
         fc = None if x.is_cuda else self.freqs_cis[self._pos]   # [1,D/2,2]
         for layer in self.layers:
             x = layer.decode(x, fc, self._pos, self._seqlens, mode, self.freqs_cis)
+        if few_rows_here(x, 1):                                 # every rank holds the whole vocabulary projection
+            return project_rows(self.norm.few_rows(x), self.output)[:, -1]
         return self.output(self.norm(x))[:, -1]
 
     def _setup_decode_layers(self, batch: int, mode: str) -> None:

@@ -62,3 +62,38 @@ def test_shapes_outside_go_to_the_library():
         assert ops._linear_params(a, b, False) is None
         torch.testing.assert_close(ops.linear(a, b), torch.mm(a, b.t()))
         assert ops.linear_glu(a, b, 0, 8, 8, ops.GLU_SILU) is None
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("batch,vocab", [(1, 1), (3, 33), (2, 4096), (8, 32768), (1, 50257)])
+def test_pick_token(batch, vocab, dtype):
+    from socket_b200 import few_rows
+    g = torch.Generator(device="cuda").manual_seed(vocab)
+    wide = torch.randn(batch, vocab + 8, generator=g, device="cuda").to(dtype)
+    logits = wide[:, :vocab]
+    rows = [logits.clone() for _ in range(4)]
+    rows[1][:, vocab // 2:] = rows[1].amax()                      # equal largest ones: the first of them
+    rows[2][:] = -float("inf")
+    rows[3][:, vocab // 3] = float("nan")
+    for library in ("step", "blocks"):
+        for x in [logits] + rows:
+            tok = torch.full((batch, 1), -1, dtype=torch.int64, device="cuda")
+            pos = torch.tensor([41], device="cuda")
+            seq = torch.arange(batch, dtype=torch.int32, device="cuda")
+            few_rows.pick_token(x, tok, pos, seq, library)
+            v = x.double().cpu()
+            v = torch.where(v.isnan(), torch.full_like(v, float("inf")), v)
+            want = torch.tensor([[int((r == r.max()).nonzero()[0])] for r in v])
+            assert torch.equal(tok.cpu(), want) and int(pos) == 42 and torch.equal(seq.cpu(), torch.arange(1, batch + 1, dtype=torch.int32))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,width", [(1, 8), (2, 33), (8, 4096), (3, 5000), (1, 16384)])
+def test_rms_norm_rows(rows, width, dtype):
+    from socket_b200 import few_rows
+    g = torch.Generator(device="cuda").manual_seed(width)
+    x, w = torch.randn(rows, width, generator=g, device="cuda").to(dtype), torch.randn(width, generator=g, device="cuda").to(dtype)
+    want = x.double() / torch.sqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-5) * w.double()
+    # the sum of squares in fp32 (relative error below 2^-20 after the tree), a few fp32 roundings, one to the type
+    eps = {torch.float32: 0.0, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype] + 2.0 ** -20
+    assert bool(((few_rows.rms_norm(x, w, 1e-5).double() - want).abs() <= eps * want.abs() + 6e-8).all())
