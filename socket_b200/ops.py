@@ -233,7 +233,8 @@ def select_list(scores: torch.Tensor, T: int, M: int, sink: int, window: int,
     assert scores.stride(0) == H * scores.stride(1)
     if allowed is not None:
         assert allowed.shape == (B, H, T)
-        allowed = allowed.to(torch.uint8).contiguous() if allowed.dtype != torch.uint8 else allowed.contiguous()
+        allowed = allowed.contiguous()
+        allowed = allowed.view(torch.uint8) if allowed.dtype == torch.bool else allowed.to(torch.uint8)      # a bool is a byte 0 or 1
     Ktot = list_len(T, sink, window, M)
     lst = torch.empty(B, H, Ktot, dtype=torch.int32, device=scores.device)
     ln = torch.empty(B, H, dtype=torch.int32, device=scores.device)
