@@ -11,7 +11,7 @@ from torch import Tensor
 
 from . import _lib
 from ._lib import blocks, check_blocks, dtype_code, ptr, stream_ptr
-from .few_rows import GLU_CLAMPED, GLU_SILU, _linear_params, linear, linear_glu  # noqa: F401
+from .few_rows import FEW_ROWS, GLU_CLAMPED, GLU_SILU, _linear_params, linear, linear_glu  # noqa: F401
 from .ops import _require_cuda
 
 ATTN_PATHS = {"auto": 0, "rows": 1, "prefill_tc": 2, "decode": 3}

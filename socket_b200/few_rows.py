@@ -13,6 +13,7 @@ from . import _lib
 from ._lib import blocks, check, check_blocks, dtype_code, lib, ptr, stream_ptr
 
 GLU_CLAMPED, GLU_SILU = 0, 1
+FEW_ROWS = 8                # the most that the streaming projection takes
 
 
 def _call(library: str, name: str, *args) -> int:
@@ -26,7 +27,7 @@ def _launch(library: str, name: str, *args) -> None:
 def _linear_params(x: Tensor, w: Tensor, chained: bool, library: str = "blocks") -> Optional[_lib.LinearParams]:
     """The parameter block of a product of a few rows, or None when the kernel does not take these shapes."""
     rows, k = x.shape
-    if rows > 8 or x.dtype == torch.float32 or not x.is_cuda or x.stride(1) != 1 or w.stride(1) != 1:
+    if rows > FEW_ROWS or x.dtype == torch.float32 or not x.is_cuda or x.stride(1) != 1 or w.stride(1) != 1:
         return None
     p = _lib.LinearParams()
     p.x, p.w, p.x_ld, p.w_ld, p.rows, p.k, p.dtype = ptr(x), ptr(w), x.stride(0) if rows > 1 else max(x.stride(0), k), w.stride(0), rows, k, dtype_code(x)

@@ -54,12 +54,17 @@ def vector(n: int) -> nn.Parameter:
 
 
 # Products inside a decoder's stack: the kernel before each of them is one of the stack's own, which write no weights
+# (a prompt's go straight to the library: short ones are bound by the host's time per call)
 def matmul(x: Tensor, w: Tensor) -> Tensor:
+    if x.shape[0] > ops.FEW_ROWS:
+        return torch.mm(x, w.t())
     return ops.linear(x, w, chained=True)
 
 
 def matmul_f32(x: Tensor, w: Tensor) -> Tensor:
     """x w^T whose fp32 sums are not rounded."""
+    if x.shape[0] > ops.FEW_ROWS:
+        return torch.mm(x, w.t()) if x.dtype == torch.float32 else torch.mm(x, w.t(), out_dtype=torch.float32)
     return ops.linear(x, w, f32=True, chained=True)
 
 
@@ -422,7 +427,9 @@ class ClampedFeedForward(nn.Module):
         return {"gate": self.w13[:self.ff], "up": self.w13[self.ff:2 * self.ff], "down": self.w2}
 
     def forward(self, h: Tensor) -> Tensor:
-        unit = ops.linear_glu(h, self.w13, 0, self.ff, self.ff, ops.GLU_CLAMPED, limit=self.limit, slope=ops.GLU_SLOPE, chained=True)
+        unit = None
+        if h.shape[0] <= ops.FEW_ROWS:                             # projections and unit in one launch
+            unit = ops.linear_glu(h, self.w13, 0, self.ff, self.ff, ops.GLU_CLAMPED, limit=self.limit, slope=ops.GLU_SLOPE, chained=True)
         act = ops.glu_clamped(matmul(h, self.w13), self.ff, self.limit) if unit is None else unit[1]
         return matmul(act, self.w2)
 
@@ -465,7 +472,8 @@ class ParallelLayer(nn.Module):
         fused = None
         if self.ff:                                                # few rows: projections and unit in one launch
             gate, up = self.in_slices[-2:]
-            fused = ops.linear_glu(h, self.w_in, gate.start, up.start, self.ff, ops.GLU_SILU, plain=gate.start, act=act, chained=True)
+            if h.shape[0] <= ops.FEW_ROWS:
+                fused = ops.linear_glu(h, self.w_in, gate.start, up.start, self.ff, ops.GLU_SILU, plain=gate.start, act=act, chained=True)
         proj = matmul(h, self.w_in) if fused is None else fused[0]
         n_mix = len(self.mixer.in_sizes)
         self.mixer.mix([proj[:, s] for s in self.in_slices[:n_mix]], h, cache, at, inner[:, :self.mixer.out_size])

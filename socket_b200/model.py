@@ -17,7 +17,8 @@ What differs from the reference, on purpose:
   `GPT-FAST/tp.py:124-137` does) and the sum over ranks after `wo` and after the feed-forward is
   issued explicitly (`tp.py`'s forward hook does not fire on the reference's sparse path).
 
-The GEMMs, norms and the dense baseline attention are torch / library kernels: they surround the
+A decode step's projections and norms run on the kernels of `few_rows.py` (one GPU, at most 8 rows of a 16-bit
+type); other GEMMs and norms and the dense baseline attention are torch / library kernels: they surround the
 path, they are not it.  `mode="dense"` attends over the whole cache with a split-KV flash decode
 and is the full-attention baseline of the tokens/s comparison.
 """
@@ -128,7 +129,7 @@ def apply_rotary_emb(x: Tensor, freqs_cis: Tensor, out: Optional[Tensor] = None)
 def few_rows_here(x: Tensor, world: int) -> bool:
     """Whether a decode step's projections go to the kernel that streams the weights: one GPU's whole matrices, at most
     8 rows of a 16-bit type.  (Widths outside its rules still go to the library, inside `few_rows.linear`.)"""
-    return x.is_cuda and world == 1 and x.shape[0] * x.shape[1] <= 8 and x.dtype in (torch.bfloat16, torch.float16)
+    return x.is_cuda and world == 1 and x.shape[0] * x.shape[1] <= few_rows.FEW_ROWS and x.dtype in (torch.bfloat16, torch.float16)
 
 
 def project_rows(x: Tensor, layer: nn.Linear, res: Optional[Tensor] = None) -> Tensor:
