@@ -24,13 +24,24 @@ def _launch(library: str, name: str, *args) -> None:
     (check if library == "step" else check_blocks)(_call(library, name, *args), name)
 
 
+def _ld(t: Tensor) -> int:
+    """Elements from one row of t [rows, n] to the next; a single row's own stride says nothing."""
+    return t.stride(0) if t.shape[0] > 1 else max(t.stride(0), t.shape[1])
+
+
+def _separate_rows(t: Tensor) -> Tensor:
+    """t itself if its rows are dense and do not overlap, as the kernels read them, else a copy: rows that are expanded or
+    turned from another layout."""
+    return t if t.stride(1) == 1 and _ld(t) >= t.shape[1] else t.contiguous()
+
+
 def _linear_params(x: Tensor, w: Tensor, chained: bool, library: str = "blocks") -> Optional[_lib.LinearParams]:
     """The parameter block of a product of a few rows, or None when the kernel does not take these shapes."""
     rows, k = x.shape
     if rows > FEW_ROWS or x.dtype == torch.float32 or not x.is_cuda or x.stride(1) != 1 or w.stride(1) != 1:
         return None
     p = _lib.LinearParams()
-    p.x, p.w, p.x_ld, p.w_ld, p.rows, p.k, p.dtype = ptr(x), ptr(w), x.stride(0) if rows > 1 else max(x.stride(0), k), w.stride(0), rows, k, dtype_code(x)
+    p.x, p.w, p.x_ld, p.w_ld, p.rows, p.k, p.dtype = ptr(x), ptr(w), _ld(x), w.stride(0), rows, k, dtype_code(x)
     p.chained = int(chained)
     return p if _call(library, "linear_rows_applicable", C.byref(p)) else None
 
@@ -49,8 +60,9 @@ def linear(x: Tensor, w: Tensor, *, f32: bool = False, res: Optional[Tensor] = N
     out = torch.empty(x.shape[0], n, dtype=torch.float32 if f32 else x.dtype, device=x.device)
     p.out, p.out_ld, p.n, p.out_f32 = ptr(out), n, n, int(f32)
     if res is not None:
-        assert res.shape == out.shape and res.dtype == x.dtype and res.stride(1) == 1
-        p.res, p.res_ld = ptr(res), max(res.stride(0), n)
+        assert res.shape == out.shape and res.dtype == x.dtype
+        res = _separate_rows(res)                             # lives until the launch
+        p.res, p.res_ld = ptr(res), _ld(res)
     _launch(library, "linear_rows", C.byref(p), stream_ptr(x.device))
     return out
 
@@ -67,7 +79,7 @@ def linear_glu(x: Tensor, w: Tensor, gate_row: int, up_row: int, ff: int, kind: 
     if act is None:
         act = torch.empty(x.shape[0], ff, dtype=x.dtype, device=x.device)
     assert act.shape == (x.shape[0], ff) and act.dtype == x.dtype and act.stride(1) == 1
-    p.out, p.out_ld, p.n, p.act, p.act_ld = ptr(out) if plain else 0, plain, plain, ptr(act), max(act.stride(0), ff)
+    p.out, p.out_ld, p.n, p.act, p.act_ld = ptr(out) if plain else 0, plain, plain, ptr(act), _ld(act)
     p.ff, p.gate_row, p.up_row, p.glu, p.limit, p.slope = ff, gate_row, up_row, kind, float(limit), float(slope)
     _launch(library, "linear_rows", C.byref(p), stream_ptr(x.device))
     return out, act

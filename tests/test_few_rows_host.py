@@ -1,0 +1,46 @@
+"""What the operators on few rows hand to their kernels: the launch is caught and the addresses are read back on the host."""
+import ctypes as C
+
+import pytest
+import torch
+
+from socket_b200 import _lib, few_rows
+
+
+def _read(address, ld, rows, n):
+    """rows x n bf16 as a kernel given (address, ld) reads them."""
+    raw = torch.tensor([[C.c_uint16.from_address(address + 2 * (r * ld + i)).value for i in range(n)] for r in range(rows)])
+    return raw.to(torch.int32).to(torch.int16).view(torch.bfloat16)
+
+
+@pytest.fixture
+def caught(monkeypatch):
+    """Every launch of the module, by name: what `read` makes of the parameters while the call is still running."""
+    seen, read = [], {}
+
+    def launch(library, name, *args):
+        seen.append(read[name](*args))
+
+    def params(x, w, chained, library="blocks"):
+        p = _lib.LinearParams()
+        p.rows, p.k = x.shape
+        return p
+
+    monkeypatch.setattr(few_rows, "_launch", launch)
+    monkeypatch.setattr(few_rows, "_linear_params", params)
+    monkeypatch.setattr(few_rows, "stream_ptr", lambda device=None: 0)
+    return seen, read
+
+
+@pytest.mark.parametrize("rows", [1, 2, 8])
+@pytest.mark.parametrize("layout", ["dense", "strided", "broadcast", "turned"])
+def test_residual_rows(caught, rows, layout):
+    seen, read = caught
+    n, k = 24, 16
+    x, w = torch.randn(rows, k).bfloat16(), torch.randn(n, k).bfloat16()
+    big = torch.randn(9, n + 8).bfloat16()                        # what lies behind a broadcast row belongs to this buffer too
+    res = {"dense": torch.randn(rows, n).bfloat16(), "strided": big[:rows, :n], "broadcast": big[:1, 8:].expand(rows, n),
+           "turned": torch.randn(n, rows).bfloat16().t()}[layout]
+    read["linear_rows"] = lambda p, stream: _read(p._obj.res, p._obj.res_ld, rows, n)
+    few_rows.linear(x, w, res=res)
+    assert torch.equal(seen[0], res)

@@ -97,3 +97,19 @@ def test_rms_norm_rows(rows, width, dtype):
     # the sum of squares in fp32 (relative error below 2^-20 after the tree), a few fp32 roundings, one to the type
     eps = {torch.float32: 0.0, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype] + 2.0 ** -20
     assert bool(((few_rows.rms_norm(x, w, 1e-5).double() - want).abs() <= eps * want.abs() + 6e-8).all())
+
+
+@pytest.mark.parametrize("rows", [1, 2, 8, 9])
+@pytest.mark.parametrize("layout", ["strided", "broadcast", "turned"])
+def test_residual_layouts(rows, layout):
+    from socket_b200 import block_ops as ops
+    n, k = 72, 128
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    x, w = r(rows, k), r(n, k)
+    res = {"strided": r(rows, n + 8)[:, 8:], "broadcast": r(1, n).expand(rows, n), "turned": r(n, rows).t()}[layout]
+    want = x.double() @ w.double().t() + res.double()
+    tol, eps = _bound(x, w, torch.bfloat16, False)
+    if rows > 8:                                                  # the library rounds the product before the sum
+        tol = tol + eps * (want - res.double()).abs()
+    assert bool(((ops.linear(x, w, res=res).double() - want).abs() <= tol + eps * want.abs() + 1e-7).all())
