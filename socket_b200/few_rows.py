@@ -11,6 +11,7 @@ from torch import Tensor
 
 from . import _lib
 from ._lib import blocks, check, check_blocks, dtype_code, lib, ptr, stream_ptr
+from .ops import _require_cuda
 
 GLU_CLAMPED, GLU_SILU = 0, 1
 FEW_ROWS = 8                # the most that the streaming projection takes
@@ -96,7 +97,9 @@ def rms_norm(x: Tensor, w: Tensor, eps: float) -> Tensor:
 
 def pick_token(logits: Tensor, token: Tensor, pos: Tensor, seqlens: Tensor, library: str) -> None:
     """token [batch, 1] = index of the largest of logits [batch, vocab]; pos and seqlens count one token more."""
-    assert logits.is_cuda and logits.dim() == 2 and logits.stride(1) == 1 and token.is_contiguous() and token.numel() == logits.shape[0]
+    _require_cuda(logits)
+    assert logits.dim() == 2 and token.is_contiguous() and token.numel() == logits.shape[0]
     assert token.dtype == pos.dtype == torch.int64 and seqlens.dtype == torch.int32 and seqlens.numel() == logits.shape[0]
-    _launch(library, "pick_token", ptr(logits), dtype_code(logits), max(logits.stride(0), logits.shape[1]), logits.shape[0],
-            logits.shape[1], ptr(token), ptr(pos), ptr(seqlens), stream_ptr(logits.device))
+    logits = _separate_rows(logits)                               # lives until the launch
+    _launch(library, "pick_token", ptr(logits), dtype_code(logits), _ld(logits), logits.shape[0], logits.shape[1], ptr(token), ptr(pos),
+            ptr(seqlens), stream_ptr(logits.device))

@@ -28,6 +28,7 @@ def caught(monkeypatch):
 
     monkeypatch.setattr(few_rows, "_launch", launch)
     monkeypatch.setattr(few_rows, "_linear_params", params)
+    monkeypatch.setattr(few_rows, "_require_cuda", lambda *tensors: None)
     monkeypatch.setattr(few_rows, "stream_ptr", lambda device=None: 0)
     return seen, read
 
@@ -44,3 +45,17 @@ def test_residual_rows(caught, rows, layout):
     read["linear_rows"] = lambda p, stream: _read(p._obj.res, p._obj.res_ld, rows, n)
     few_rows.linear(x, w, res=res)
     assert torch.equal(seen[0], res)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 8, 9])
+@pytest.mark.parametrize("layout", ["dense", "strided", "broadcast", "turned"])
+def test_logit_rows(caught, rows, layout):
+    seen, read = caught
+    n = 24
+    big = torch.randn(10, n + 8).bfloat16()
+    logits = {"dense": torch.randn(rows, n).bfloat16(), "strided": big[:rows, :n], "broadcast": big[:1, 8:].expand(rows, n),
+              "turned": torch.randn(n, rows).bfloat16().t()}[layout]
+    read["pick_token"] = lambda address, dtype, ld, batch, vocab, *rest: _read(address, ld, batch, vocab)
+    few_rows.pick_token(logits, torch.zeros(rows, 1, dtype=torch.int64), torch.zeros(1, dtype=torch.int64),
+                        torch.zeros(rows, dtype=torch.int32), "blocks")
+    assert torch.equal(seen[0], logits)

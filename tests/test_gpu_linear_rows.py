@@ -113,3 +113,16 @@ def test_residual_layouts(rows, layout):
     if rows > 8:                                                  # the library rounds the product before the sum
         tol = tol + eps * (want - res.double()).abs()
     assert bool(((ops.linear(x, w, res=res).double() - want).abs() <= tol + eps * want.abs() + 1e-7).all())
+
+
+@pytest.mark.parametrize("rows", [1, 2, 8, 9])
+@pytest.mark.parametrize("layout", ["broadcast", "turned"])
+def test_pick_token_layouts(rows, layout):
+    from socket_b200 import few_rows
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    logits = r(1, 1000).expand(rows, 1000) if layout == "broadcast" else r(1000, rows).t()
+    tok = torch.zeros(rows, 1, dtype=torch.int64, device="cuda")
+    pos, seq = torch.zeros(1, dtype=torch.int64, device="cuda"), torch.zeros(rows, dtype=torch.int32, device="cuda")
+    few_rows.pick_token(logits, tok, pos, seq, "step")
+    assert torch.equal(tok, logits.argmax(-1, keepdim=True))
