@@ -418,8 +418,8 @@ SK_API int64_t sk_decode_step_rescored_rows_offset(int B, int H, int Hkv, int D,
  *   act [rows, ff] = unit(x G^T, x U^T), G and U the ff rows of W from gate_row and from up_row on
  * whose sums are not rounded in between; n may then be 0.  `chained`: the caller vouches that the kernel before this one
  * on the stream does not write W, and the weights may be requested before that kernel has ended.
- * sk_linear_rows_applicable: whether shapes, strides and alignment are taken (k and w_ld multiples of 16, W 32-byte
- * aligned, x rows 16-byte aligned). */
+ * sk_linear_rows_applicable: whether rows, shapes, strides and alignment are taken (1 to 8 rows that do not overlap, k and
+ * w_ld multiples of 16, W 32-byte aligned, x rows 16-byte aligned). */
 enum { SKB_GLU_CLAMPED = 0, SKB_GLU_SILU = 1 };
 typedef struct sk_linear_params {
     const void* x;

@@ -226,8 +226,8 @@ int linear_dispatch(const sk_linear_params& p, cudaStream_t st) {
 }  // namespace
 
 bool linear_rows_applicable(const sk_linear_params& p) {
-    return p.rows <= LR_MAX_ROWS && (p.dtype == SK_BF16 || p.dtype == SK_F16) && p.k % 16 == 0 && p.w_ld % 16 == 0 && p.x_ld % 8 == 0 &&
-           (uintptr_t)p.w % 32 == 0 && (uintptr_t)p.x % 16 == 0;
+    return p.rows > 0 && p.rows <= LR_MAX_ROWS && p.k > 0 && p.x_ld >= p.k && p.w_ld >= p.k && (p.dtype == SK_BF16 || p.dtype == SK_F16) &&
+           p.k % 16 == 0 && p.w_ld % 16 == 0 && p.x_ld % 8 == 0 && (uintptr_t)p.w % 32 == 0 && (uintptr_t)p.x % 16 == 0;
 }
 
 int linear_rows(const sk_linear_params* p, cudaStream_t st) {

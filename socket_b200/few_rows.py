@@ -39,10 +39,10 @@ def _separate_rows(t: Tensor) -> Tensor:
 def _linear_params(x: Tensor, w: Tensor, chained: bool, library: str = "blocks") -> Optional[_lib.LinearParams]:
     """The parameter block of a product of a few rows, or None when the kernel does not take these shapes."""
     rows, k = x.shape
-    if rows > FEW_ROWS or x.dtype == torch.float32 or not x.is_cuda or x.stride(1) != 1 or w.stride(1) != 1:
+    if rows > FEW_ROWS or x.dtype not in (torch.bfloat16, torch.float16) or not x.is_cuda or x.stride(1) != 1 or w.stride(1) != 1:
         return None
     p = _lib.LinearParams()
-    p.x, p.w, p.x_ld, p.w_ld, p.rows, p.k, p.dtype = ptr(x), ptr(w), _ld(x), w.stride(0), rows, k, dtype_code(x)
+    p.x, p.w, p.x_ld, p.w_ld, p.rows, p.k, p.dtype = ptr(x), ptr(w), _ld(x), _ld(w), rows, k, dtype_code(x)
     p.chained = int(chained)
     return p if _call(library, "linear_rows_applicable", C.byref(p)) else None
 
@@ -53,11 +53,11 @@ def linear(x: Tensor, w: Tensor, *, f32: bool = False, res: Optional[Tensor] = N
     the kernel that streams the weights, others to the library.  `chained`: the kernel before this call on the stream
     does not write w (see `skb_linear_rows`)."""
     assert x.shape[1] == w.shape[1] and x.dtype == w.dtype and x.device == w.device
-    p = _linear_params(x, w, chained, library)
+    n = w.shape[0]
+    p = _linear_params(x, w, chained, library) if n else None
     if p is None:
         out = torch.mm(x, w.t(), out_dtype=torch.float32) if f32 and x.dtype != torch.float32 else torch.mm(x, w.t())
         return out if res is None else out + res
-    n = w.shape[0]
     out = torch.empty(x.shape[0], n, dtype=torch.float32 if f32 else x.dtype, device=x.device)
     p.out, p.out_ld, p.n, p.out_f32 = ptr(out), n, n, int(f32)
     if res is not None:

@@ -59,3 +59,15 @@ def test_logit_rows(caught, rows, layout):
     few_rows.pick_token(logits, torch.zeros(rows, 1, dtype=torch.int64), torch.zeros(1, dtype=torch.int64),
                         torch.zeros(rows, dtype=torch.int32), "blocks")
     assert torch.equal(seen[0], logits)
+
+
+@pytest.mark.parametrize("taken,change", [(1, {}), (1, dict(rows=8)), (1, dict(x_ld=72)), (0, dict(rows=0)), (0, dict(rows=9)), (0, dict(k=0)),
+                                          (0, dict(x_ld=0)), (0, dict(w_ld=0)), (0, dict(w_ld=48)), (0, dict(x_ld=56)), (0, dict(k=56)),
+                                          (0, dict(dtype=_lib.SK_F32)), (0, dict(w=4096 + 16)), (0, dict(x=4096 + 8))])
+def test_what_the_projection_takes(taken, change):
+    """What linear_rows would refuse is not applicable, so that linear() sends it to the library."""
+    p = _lib.LinearParams(x=4096, w=4096, out=4096, x_ld=64, w_ld=64, out_ld=32, rows=2, n=32, k=64, dtype=_lib.SK_BF16)
+    for name, value in change.items():
+        setattr(p, name, value)
+    assert _lib.blocks().skb_linear_rows_applicable(C.byref(p)) == taken
+    assert _lib.lib().sk_linear_rows_applicable(C.byref(p)) == taken

@@ -126,3 +126,26 @@ def test_pick_token_layouts(rows, layout):
     pos, seq = torch.zeros(1, dtype=torch.int64, device="cuda"), torch.zeros(rows, dtype=torch.int32, device="cuda")
     few_rows.pick_token(logits, tok, pos, seq, "step")
     assert torch.equal(tok, logits.argmax(-1, keepdim=True))
+
+
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("form", ["expanded rows", "expanded weights", "no rows", "no columns", "no weights", "one weight row"])
+def test_what_only_the_library_takes(form, f32):
+    from socket_b200 import block_ops as ops
+    r = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    x, w = r(3, 64), r(24, 64)
+    x, w = {"expanded rows": (x[:1].expand(3, 64), w), "expanded weights": (x, w[:1].expand(24, 64)), "no rows": (x[:0], w),
+            "no columns": (x[:, :0], w[:, :0]), "no weights": (x, w[:0]), "one weight row": (x, r(64, 1).t())}[form]
+    got = ops.linear(x, w, f32=f32)
+    assert got.shape == (x.shape[0], w.shape[0]) and got.dtype == (torch.float32 if f32 else torch.bfloat16)
+    want = x.double() @ w.double().t()
+    tol, eps = _bound(x, w, torch.bfloat16, f32)
+    assert bool(((got.double() - want).abs() <= tol + eps * want.abs() + 1e-7).all())
+    if form in ("expanded rows", "no rows", "no columns"):
+        assert ops.linear_glu(x, w, 0, 8, 8, ops.GLU_SILU) is None
+
+
+def test_doubles_go_to_the_library():
+    from socket_b200 import block_ops as ops
+    x, w = torch.randn(2, 64, device="cuda", dtype=torch.float64), torch.randn(24, 64, device="cuda", dtype=torch.float64)
+    torch.testing.assert_close(ops.linear(x, w), x @ w.t())
