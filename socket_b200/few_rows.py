@@ -25,6 +25,13 @@ def _launch(library: str, name: str, *args) -> None:
     (check if library == "step" else check_blocks)(_call(library, name, *args), name)
 
 
+def _require_on(device: torch.device, *tensors: Optional[Tensor]) -> None:
+    """The kernels read and write addresses: every tensor of a call lies on the device of its rows."""
+    for t in tensors:
+        if t is not None and t.device != device:
+            raise RuntimeError(f"tensors of one call on {device} and {t.device}")
+
+
 def _ld(t: Tensor) -> int:
     """Elements from one row of t [rows, n] to the next; a single row's own stride says nothing."""
     return t.stride(0) if t.shape[0] > 1 else max(t.stride(0), t.shape[1])
@@ -52,7 +59,8 @@ def linear(x: Tensor, w: Tensor, *, f32: bool = False, res: Optional[Tensor] = N
     """x [rows, k] w^T (+ res [rows, n]) with fp32 sums, rounded to x's type unless `f32`.  Few rows (a decode step) go to
     the kernel that streams the weights, others to the library.  `chained`: the kernel before this call on the stream
     does not write w (see `skb_linear_rows`)."""
-    assert x.shape[1] == w.shape[1] and x.dtype == w.dtype and x.device == w.device
+    assert x.shape[1] == w.shape[1] and x.dtype == w.dtype
+    _require_on(x.device, w, res)
     n = w.shape[0]
     p = _linear_params(x, w, chained, library) if n else None
     if p is None:
@@ -72,6 +80,7 @@ def linear_glu(x: Tensor, w: Tensor, gate_row: int, up_row: int, ff: int, kind: 
                plain: int = 0, act: Optional[Tensor] = None, chained: bool = False, library: str = "blocks"):
     """(x w[:plain]^T, unit(x G^T, x U^T)) with G, U the ff rows of w from `gate_row` and `up_row` on, in one launch; `act`
     may be a slice of wider rows.  None when the shapes are not the kernel's."""
+    _require_on(x.device, w, act)
     assert x.shape[1] == w.shape[1] and x.dtype == w.dtype and max(gate_row, up_row) + ff <= w.shape[0] and plain <= w.shape[0]
     p = _linear_params(x, w, chained, library)
     if p is None:
@@ -88,7 +97,9 @@ def linear_glu(x: Tensor, w: Tensor, gate_row: int, up_row: int, ff: int, kind: 
 
 def rms_norm(x: Tensor, w: Tensor, eps: float) -> Tensor:
     """x [..., width] -> x / rms(x) * w in x's type, fp32 arithmetic (the step library's)."""
-    assert x.is_cuda and x.is_contiguous() and w.is_contiguous() and w.shape == x.shape[-1:] and w.dtype == x.dtype
+    _require_cuda(x)
+    _require_on(x.device, w)
+    assert x.is_contiguous() and w.is_contiguous() and w.shape == x.shape[-1:] and w.dtype == x.dtype
     out = torch.empty_like(x)
     check(lib().sk_rms_norm(ptr(x), ptr(w), dtype_code(x), x.numel() // x.shape[-1], x.shape[-1], float(eps), ptr(out),
                             stream_ptr(x.device)), "sk_rms_norm")
@@ -98,8 +109,9 @@ def rms_norm(x: Tensor, w: Tensor, eps: float) -> Tensor:
 def pick_token(logits: Tensor, token: Tensor, pos: Tensor, seqlens: Tensor, library: str) -> None:
     """token [batch, 1] = index of the largest of logits [batch, vocab]; pos and seqlens count one token more."""
     _require_cuda(logits)
-    assert logits.dim() == 2 and token.is_contiguous() and token.numel() == logits.shape[0]
-    assert token.dtype == pos.dtype == torch.int64 and seqlens.dtype == torch.int32 and seqlens.numel() == logits.shape[0]
+    _require_on(logits.device, token, pos, seqlens)
+    assert logits.dim() == 2 and token.is_contiguous() and seqlens.is_contiguous() and pos.numel() == 1
+    assert token.dtype == pos.dtype == torch.int64 and seqlens.dtype == torch.int32 and token.numel() == seqlens.numel() == logits.shape[0]
     logits = _separate_rows(logits)                               # lives until the launch
     _launch(library, "pick_token", ptr(logits), dtype_code(logits), _ld(logits), logits.shape[0], logits.shape[1], ptr(token), ptr(pos),
             ptr(seqlens), stream_ptr(logits.device))

@@ -71,3 +71,24 @@ def test_what_the_projection_takes(taken, change):
         setattr(p, name, value)
     assert _lib.blocks().skb_linear_rows_applicable(C.byref(p)) == taken
     assert _lib.lib().sk_linear_rows_applicable(C.byref(p)) == taken
+
+
+def test_tensors_elsewhere_are_refused(caught):
+    """One tensor of each call on another device; nothing is launched (a launch would find no reader here)."""
+    x, w, there = torch.randn(2, 64).bfloat16(), torch.randn(24, 64).bfloat16(), dict(dtype=torch.bfloat16, device="meta")
+    tok, pos, seq = torch.zeros(2, 1, dtype=torch.int64), torch.zeros(1, dtype=torch.int64), torch.zeros(2, dtype=torch.int32)
+    for call in (lambda: few_rows.linear(x, w.to("meta")), lambda: few_rows.linear(x, w, res=torch.empty(2, 24, **there)),
+                 lambda: few_rows.linear_glu(x, w, 0, 8, 8, 0, act=torch.empty(2, 8, **there)),
+                 lambda: few_rows.rms_norm(x, torch.empty(64, **there), 1e-5),
+                 lambda: few_rows.pick_token(x, tok.to("meta"), pos, seq, "step"),
+                 lambda: few_rows.pick_token(x, tok, pos.to("meta"), seq, "step"),
+                 lambda: few_rows.pick_token(x, tok, pos, seq.to("meta"), "step")):
+        with pytest.raises(RuntimeError, match="tensors of one call"):
+            call()
+
+
+def test_counts_of_another_layout_are_refused(caught):
+    logits, tok, pos = torch.randn(2, 64).bfloat16(), torch.zeros(2, 1, dtype=torch.int64), torch.zeros(1, dtype=torch.int64)
+    for p, seq in ((pos, torch.zeros(4, dtype=torch.int32)[::2]), (torch.zeros(2, dtype=torch.int64), torch.zeros(2, dtype=torch.int32))):
+        with pytest.raises(AssertionError):
+            few_rows.pick_token(logits, tok, p, seq, "step")
