@@ -22,8 +22,6 @@
 #include "tcgen05.cuh"
 #include "tensor_map.cuh"
 
-#include <climits>
-
 namespace sk {
 namespace {
 
@@ -70,12 +68,12 @@ enum { FP_CAP_NONE = 0, FP_CAP = 1, FP_CAP_BOUND = 2 };
 constexpr float FP_CAP_BOUND_LOG2 = 80.f;
 constexpr double FP_GROUP_BYTES = 48e6;      // 32 heads of 192 / 128 on 8000 rows, 164 MB: 978 us side by side, 937 in groups
 
-// first key row (in key-row coordinates, may be negative) that query row i sees
+// first key row (counted from kv_start: rows of the call, below 2^30, whatever the positions are) that query row i sees
 __device__ __forceinline__ int fp_first_row(const FpShape& p, int i) {
     int64_t lo = -p.kv_start;
     if (p.chunk > 0) lo = (i + p.kv_start) / p.chunk * p.chunk - p.kv_start;
     if (p.window > 0 && i - p.window + 1 > lo) lo = i - p.window + 1;
-    return (int)max(lo, (int64_t)INT_MIN);
+    return (int)max(lo, (int64_t)0);
 }
 
 // s <- cap_out tanh(s cap_in) for 16 scores from c0 on; the caller's loops are unrolled
@@ -134,8 +132,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     for (int t = 0; t < 2; ++t) {
         const int first = q0 + t * FP_TILE;
         i0[t] = (int)(p.start - p.kv_start) + first;
-        int lo = fp_first_row(p, i0[t]);
-        if (lo < 0) lo = 0;
+        const int lo = fp_first_row(p, i0[t]);
         if (t == 0) base = lo;
         const int rows = p.S - first < FP_TILE ? p.S - first : FP_TILE;
         beg[t] = (lo - base) / FP_TILE;

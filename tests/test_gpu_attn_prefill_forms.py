@@ -62,3 +62,16 @@ def test_forms(S, H, G, D, E, start, kv_start, bias_len, chunk, window, cap, sin
             want, mag = _plain(q, k, v, kw, i, h)
             # weights rounded to bf16 (2^-9 each, their sum is not), fp32 scores of at most 2^7 off by 2^-17, the result rounded
             assert bool(((got[i, h] - want).abs() <= 2.0 ** -8 * mag + 2.0 ** -8 * want.abs() + 1e-6).all()), (i, h)
+
+
+@pytest.mark.parametrize("kv_start", [2 ** 31 - 300, 2 ** 31 + 7, 2 ** 40])
+@pytest.mark.parametrize("chunk,window,cap", [(0, 0, 0.0), (0, 200, 30.0), (2 ** 30, 0, 0.0)])
+def test_positions_beyond_two_billion(kv_start, chunk, window, cap):
+    """Key rows count from kv_start; where the first position lies must not matter without a chunk's edge in between."""
+    from socket_b200 import block_ops as ops
+    if chunk and kv_start < 2 ** 31:
+        kv_start = 2 ** 31 - 2 ** 20                              # its chunk begins and ends far from these rows
+    q, k, v, kw = _case(300, 2, 1, 128, 64, 250, 0, 0, 0, window, cap, False, 7)
+    want = ops.attn(q, k, v, path="prefill_tc", **kw)
+    kw.update(start=kv_start + 250, kv_start=kv_start, chunk=chunk)
+    assert torch.equal(ops.attn(q, k, v, path="prefill_tc", **kw), want)
