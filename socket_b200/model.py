@@ -88,6 +88,19 @@ transformer_configs = {
 }
 
 
+# Hooks on every module: a torch that does not tell has them, for all this module knows
+_any_global_hook = getattr(torch.nn.modules.module, "_has_any_global_hook", lambda: True)
+
+
+def untouched(module: nn.Module, kind: type) -> bool:
+    """Whether calling `module` is what `kind` does with its own dense weights and nothing else: not wrapped, replaced or
+    compiled, no hooks, no bias.  Only then may a kernel take the weights and leave the call out."""
+    hooks = (module._forward_hooks, module._forward_pre_hooks, module._backward_hooks, module._backward_pre_hooks)
+    own = type(module) is kind and "forward" not in module.__dict__ and getattr(module, "_compiled_call_impl", None) is None
+    return (own and not any(hooks) and not _any_global_hook() and getattr(module, "bias", None) is None and
+            all(type(p) is nn.Parameter for p in module._parameters.values() if p is not None))
+
+
 class RMSNorm(nn.Module):
     def __init__(self, dim: int, eps: float = 1e-5):
         super().__init__()
@@ -100,11 +113,12 @@ class RMSNorm(nn.Module):
         xf = x.float()
         return (xf * torch.rsqrt(torch.mean(xf * xf, dim=-1, keepdim=True) + self.eps)).type_as(x) * self.weight
 
-    def few_rows(self, x: Tensor) -> Tensor:
-        """The same for the rows of a decode step on a GPU."""
-        if x.dtype != self.weight.dtype:
-            return self.forward(x)
-        return few_rows.rms_norm(x.contiguous(), self.weight, self.eps)
+
+def norm_rows(norm: nn.Module, x: Tensor) -> Tensor:
+    """norm(x) of the rows of a decode step on a GPU."""
+    if not untouched(norm, RMSNorm) or x.dtype != norm.weight.dtype:
+        return norm(x)
+    return few_rows.rms_norm(x.contiguous(), norm.weight, norm.eps)
 
 
 def precompute_freqs_cis(seq_len: int, n_elem: int, base: float = 10000, device=None) -> Tensor:
@@ -128,12 +142,15 @@ def apply_rotary_emb(x: Tensor, freqs_cis: Tensor, out: Optional[Tensor] = None)
 
 def few_rows_here(x: Tensor, world: int) -> bool:
     """Whether a decode step's projections go to the kernel that streams the weights: one GPU's whole matrices, at most
-    8 rows of a 16-bit type.  (Widths outside its rules still go to the library, inside `few_rows.linear`.)"""
-    return x.is_cuda and world == 1 and x.shape[0] * x.shape[1] <= few_rows.FEW_ROWS and x.dtype in (torch.bfloat16, torch.float16)
+    8 rows of a 16-bit type, no gradients.  (Widths outside its rules still go to the library, inside `few_rows.linear`;
+    modules that do more than a product are called.)"""
+    return x.is_cuda and world == 1 and not torch.is_grad_enabled() and x.shape[0] * x.shape[1] <= few_rows.FEW_ROWS and x.dtype in (torch.bfloat16, torch.float16)
 
 
 def project_rows(x: Tensor, layer: nn.Linear, res: Optional[Tensor] = None) -> Tensor:
     """layer(x) (+ res) of the rows [B, 1, width] of a decode step.  The kernel before it is one that made x: no weights."""
+    if not untouched(layer, nn.Linear):
+        return layer(x) if res is None else res + layer(x)
     y = few_rows.linear(x.reshape(-1, x.shape[-1]), layer.weight, res=None if res is None else res.reshape(-1, res.shape[-1]),
                         chained=True, library="step")
     return y.view(*x.shape[:-1], -1)
@@ -166,8 +183,10 @@ class FeedForward(nn.Module):
 
     def decode(self, x: Tensor, res: Tensor) -> Tensor:
         """res + forward(x) for a few rows: gate, up and unit in one launch, the residual in the other."""
-        unit = few_rows.linear_glu(x.reshape(-1, x.shape[-1]), self.w13.weight, 0, self.inter, self.inter, few_rows.GLU_SILU,
-                                   chained=True, library="step")
+        unit = None
+        if untouched(self.w13, nn.Linear):
+            unit = few_rows.linear_glu(x.reshape(-1, x.shape[-1]), self.w13.weight, 0, self.inter, self.inter, few_rows.GLU_SILU,
+                                       chained=True, library="step")
         hidden = self.hidden(x) if unit is None else unit[1].view(*x.shape[:-1], -1)
         return project_rows(hidden, self.w2, res)
 
@@ -311,9 +330,11 @@ class TransformerBlock(nn.Module):
             h = fused(y, self.attention.wo.weight, res=x.contiguous())
             return fused(self.feed_forward.hidden(self.ffn_norm(h)), self.feed_forward.w2.weight, res=h)
         if few_rows_here(x, self.world):
-            y = self.attention.decode(self.attention_norm.few_rows(x), freqs_cis, pos, seqlens, mode, rope_table, project=False)
+            y = self.attention.decode(norm_rows(self.attention_norm, x), freqs_cis, pos, seqlens, mode, rope_table, project=False)
             h = project_rows(y, self.attention.wo, x)
-            return self.feed_forward.decode(self.ffn_norm.few_rows(h), h)
+            if not untouched(self.feed_forward, FeedForward):
+                return h + self.feed_forward(norm_rows(self.ffn_norm, h))
+            return self.feed_forward.decode(norm_rows(self.ffn_norm, h), h)
         h = x + self._sum(self.attention.decode(self.attention_norm(x), freqs_cis, pos, seqlens, mode, rope_table))
         return h + self._sum(self.feed_forward(self.ffn_norm(h)))
 
@@ -402,7 +423,7 @@ class Transformer(Decoder):
         for layer in self.layers:
             x = layer.decode(x, fc, self._pos, self._seqlens, mode, self.freqs_cis)
         if few_rows_here(x, 1):                                 # every rank holds the whole vocabulary projection
-            return project_rows(self.norm.few_rows(x), self.output)[:, -1]
+            return project_rows(norm_rows(self.norm, x), self.output)[:, -1]
         return self.output(self.norm(x))[:, -1]
 
     def _setup_decode_layers(self, batch: int, mode: str) -> None:

@@ -92,3 +92,53 @@ def test_fused_rope_split_equals_the_tensor_formulation(dtype):
     ops.rope_split(qkv, table, torch.tensor([n_pos], device=DEV), H, Hkv, q, k, v, status=status)
     torch.cuda.synchronize()
     assert int(status) == 1 and (q == 0).all()
+
+
+def _one_token(model, B=2, T=300):
+    prompt = torch.randint(0, model.config.vocab_size, (B, T), generator=torch.Generator().manual_seed(5)).to(DEV)
+    model.setup_caches(B, T + 16)
+    model.setup_decode(B, "sparse", use_graph=False)
+    model.prefill(prompt, chunk=512)
+    return model.decode_given_token(prompt[:, :1], T).float()
+
+
+NAMES = ("attention_norm", "attention.wqkv", "attention.wo", "ffn_norm", "feed_forward", "feed_forward.w13", "feed_forward.w2")
+
+
+@pytest.mark.parametrize("name", [f"layers.1.{n}" for n in NAMES] + ["norm", "output"])
+def test_a_hook_on_any_module_acts_on_the_decoded_token(name):
+    model = _model()
+    plain = _one_token(model)
+    module, calls = model.get_submodule(name), []
+    handle = module.register_forward_hook(lambda mod, args, out: calls.append(tuple(out.shape)))
+    same = _one_token(model)
+    handle.remove()
+    assert len(calls) == 2 and calls[-1][:2] == (2, 1)            # the prompt's portion, then the token
+    # one product or norm by the library in place of the kernel: bf16 roundings of one module in a model of two layers
+    assert (same - plain).norm() <= 2e-2 * plain.norm()
+    handle = module.register_forward_hook(lambda mod, args, out: torch.zeros_like(out))
+    other = _one_token(model)
+    handle.remove()
+    assert (other - plain).norm() >= 5e-2 * plain.norm()
+
+
+def test_wrapped_and_replaced_modules_act_on_the_decoded_token():
+    class Scaled(torch.nn.Module):
+        def __init__(self, inner, by):
+            super().__init__()
+            self.inner, self.by = inner, by
+
+        def forward(self, x):
+            return self.by * self.inner(x)
+
+    model = _model()
+    want = model.layers[0].feed_forward.w2.weight.data
+    want.mul_(0.5)                                                # exact in bf16
+    half = _one_token(model)
+    want.mul_(2.0)
+    model.layers[0].feed_forward.w2 = Scaled(model.layers[0].feed_forward.w2, 0.5)
+    got = _one_token(model)
+    assert (got - half).norm() <= 2e-2 * half.norm()
+    model.layers[1].feed_forward = Scaled(model.layers[1].feed_forward, 0.0)
+    off = _one_token(model)
+    assert (off - got).norm() >= 5e-2 * got.norm()
