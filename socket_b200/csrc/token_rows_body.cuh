@@ -38,6 +38,31 @@ rms_norm_rows_kernel(const T* x, const T* __restrict__ w, int width, float eps, 
     }
 }
 
+// Rows too long for registers: read twice, the second time mostly from L2.
+template <typename T, int V>
+__global__ void __launch_bounds__(512)
+rms_norm_long_rows_kernel(const T* x, const T* __restrict__ w, int width, float eps, T* __restrict__ out) {
+    pdl_begin();
+    __shared__ float red[32];
+    const int64_t row = blockIdx.x, step = (int64_t)blockDim.x * V;
+    float ss = 0.f;
+    for (int64_t i = threadIdx.x * V; i < width; i += step) {
+        float v[V];
+        load_vec<T, V>(x + row * width + i, v);
+#pragma unroll
+        for (int e = 0; e < V; ++e) ss = fmaf(v[e], v[e], ss);
+    }
+    const float inv = 1.f / sqrtf(block_sum(ss, red) / (float)width + eps);
+    for (int64_t i = threadIdx.x * V; i < width; i += step) {
+        float v[V], g[V];
+        load_vec<T, V>(x + row * width + i, v);
+        load_vec<T, V>(w + i, g);
+#pragma unroll
+        for (int e = 0; e < V; ++e) v[e] *= inv * g[e];
+        store_vec<T, V>(out + row * width + i, v);
+    }
+}
+
 template <typename T>
 int rms_dispatch(const void* x, const void* w, int64_t rows, int width, float eps, void* out, cudaStream_t st) {
     constexpr int V = 16 / sizeof(T);
@@ -46,13 +71,12 @@ int rms_dispatch(const void* x, const void* w, int64_t rows, int width, float ep
     int nt = 512;
     while (nt > 32 && nt / 2 >= vecs) nt /= 2;
     const int nv = (vecs + nt - 1) / nt;
-    if (nv > 32) return fail(SK_ERR_UNSUPPORTED, "sk_rms_norm: width %d is too large", width);
     auto run = [&](auto kern) {
         return check_chained(launch_after(kern, dim3((unsigned)rows), dim3((unsigned)nt), 0, st, (const T*)x, (const T*)w, width, eps, (T*)out),
                              "rms_norm_rows_kernel");
     };
-    if (vec) return nv <= 1 ? run(rms_norm_rows_kernel<T, V, 1>) : nv <= 4 ? run(rms_norm_rows_kernel<T, V, 4>) : run(rms_norm_rows_kernel<T, V, 32>);
-    return nv <= 4 ? run(rms_norm_rows_kernel<T, 1, 4>) : run(rms_norm_rows_kernel<T, 1, 32>);
+    if (vec) return nv <= 1 ? run(rms_norm_rows_kernel<T, V, 1>) : nv <= 4 ? run(rms_norm_rows_kernel<T, V, 4>) : run(rms_norm_long_rows_kernel<T, V>);
+    return nv <= 4 ? run(rms_norm_rows_kernel<T, 1, 4>) : run(rms_norm_long_rows_kernel<T, 1>);
 }
 
 // Is (a, i) picked over (b, j): NaN before all, then the larger value, then the smaller index
