@@ -413,11 +413,14 @@ SK_API int64_t sk_decode_step_rescored_rows_offset(int B, int H, int Hkv, int D,
 
 /* out [rows, n] = x [rows, k] W^T, W [n, k] with rows w_ld elements apart: the projections of a decode step, at most 8
  * rows, bf16 or fp16, fp32 sums.  `res` (or NULL; element type of x) is added to the sums; out has the element type of
- * x, or fp32 with out_f32.  With ff > 0 the same launch also takes x through a gated unit (SKB_GLU_CLAMPED: g * sigmoid(slope * g) * (u + 1) of g = min(gate, limit),
- * u = clamp(up, -limit, limit); SKB_GLU_SILU: gate * sigmoid(gate) * up):
+ * x, or fp32 with out_f32.  With ff > 0 the same launch also takes x through a gated unit:
  *   act [rows, ff] = unit(x G^T, x U^T), G and U the ff rows of W from gate_row and from up_row on
- * whose sums are not rounded in between; n may then be 0.  `chained`: the caller vouches that the kernel before this one
- * on the stream does not write W, and the weights may be requested before that kernel has ended.
+ *   SKB_GLU_CLAMPED: g * sigmoid(slope * g) * (u + 1) of g = min(gate, limit), u = clamp(up, -limit, limit)
+ *   SKB_GLU_SILU: gate * sigmoid(gate) * up
+ * whose sums are not rounded in between; n may then be 0.
+ * `chained`: the kernel may start, and request W, while kernels before it on the stream still run.  The caller vouches
+ * that W is complete by then: neither the stream's last unchained launch nor any kernel behind it writes W.  (That the
+ * kernel directly before does not is not enough: it may have let this one in before its own wait.)
  * sk_linear_rows_applicable: whether rows, shapes, strides and alignment are taken (1 to 8 rows that do not overlap, k and
  * w_ld multiples of 16, W 32-byte aligned, x rows 16-byte aligned). */
 enum { SKB_GLU_CLAMPED = 0, SKB_GLU_SILU = 1 };

@@ -9,9 +9,10 @@
 // were loaded, without a shuffle or a pass through shared memory.  The warps' sums meet in shared memory, in warp
 // order, in fp32.
 //
-// Weights do not depend on the kernel before this one.  With `chained` the kernel may start while that kernel still
-// runs, fills its ring with weights, and only then waits for x: the caller vouches that the kernel before it on the
-// stream does not write the weights.
+// Weights do not depend on the kernel before this one.  With `chained` the kernel may start while kernels before it still
+// run, fills its ring with weights, and only then waits for x.  It lets its own successor in before that wait, and so do the
+// kernels of the sparse step: a chained projection can reach back over several kernels.  The caller vouches that neither
+// the stream's last unchained launch nor anything behind it writes the weights.
 //
 // Measured (one row, cold weights, back to back in a graph; chained / not / cuBLAS): 4096 x 14336 20.1 / 21.7 / 24.4 us
 // (5.9 TB/s), 28672 x 4096 38.2 / 39.6 / 39.1 us, 4096 x 4096 6.2 / 8.2 / 12.9 us, 2048 x 2048 2.4 / 4.0 / 7.3 us; with

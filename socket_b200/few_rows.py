@@ -57,8 +57,8 @@ def _linear_params(x: Tensor, w: Tensor, chained: bool, library: str = "blocks")
 def linear(x: Tensor, w: Tensor, *, f32: bool = False, res: Optional[Tensor] = None, chained: bool = False,
            library: str = "blocks") -> Tensor:
     """x [rows, k] w^T (+ res [rows, n]) with fp32 sums, rounded to x's type unless `f32`.  Few rows (a decode step) go to
-    the kernel that streams the weights, others to the library.  `chained`: the kernel before this call on the stream
-    does not write w (see `skb_linear_rows`)."""
+    the kernel that streams the weights, others to the library.  `chained`: w may be read while kernels
+    before this call still run; neither the stream's last unchained launch nor any kernel behind it writes w."""
     assert x.shape[1] == w.shape[1] and x.dtype == w.dtype
     _require_on(x.device, w, res)
     n = w.shape[0]

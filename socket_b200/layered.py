@@ -102,14 +102,14 @@ class LayeredDecoder(Decoder):
     # ------------------------------------------------------------------------------- the decoder's hooks
     def _portion(self, idx: Tensor, start: int, collect: Optional[list] = None) -> Tensor:
         B, S = idx.shape
-        at = Portion(B, S, start, status=self._status, workspace=self._workspace)
+        at = Portion(B, S, start, status=self._status, workspace=self._workspace, chained=True)
         return self._stack(idx, at, collect).view(B, S, -1)
 
     def _head(self, hidden: Tensor) -> Tensor:
-        logits = matmul_f32(hidden.reshape(-1, hidden.shape[-1]), self.head)
+        logits = matmul_f32(hidden.reshape(-1, hidden.shape[-1]), self.head, chained=True)
         return logits.view(*hidden.shape[:-1], -1)
 
     def _decode_logits(self, mode: str) -> Tensor:
         B = self._tok.shape[0]
-        at = Portion(B, 1, 0, pos=self._pos, status=self._status, workspace=self._workspace)
+        at = Portion(B, 1, 0, pos=self._pos, status=self._status, workspace=self._workspace, chained=True)
         return self._head(self._stack(self._tok, at))

@@ -34,6 +34,9 @@ class Portion:
     pos: Optional[Tensor] = None
     status: Optional[Tensor] = None       # device int32, collects flags of the kernels
     workspace: Optional[Tensor] = None    # scratch of the split decode kernel, shared by all layers
+    # set by a decoder's stack, whose kernels write no weights and whose first is launched unchained: its products may
+    # request weights while kernels before them still run.  A mixer called by itself may stand right behind such a write
+    chained: bool = False
 
     @property
     def end(self) -> int:
@@ -53,19 +56,19 @@ def vector(n: int) -> nn.Parameter:
     return nn.Parameter(torch.zeros(n), requires_grad=False)
 
 
-# Products inside a decoder's stack: the kernel before each of them is one of the stack's own, which write no weights
-# (a prompt's go straight to the library: short ones are bound by the host's time per call)
-def matmul(x: Tensor, w: Tensor) -> Tensor:
+# `chained`: see `few_rows.linear`.  A prompt's products go straight to the library: short ones are bound by the host's time
+# per call
+def matmul(x: Tensor, w: Tensor, chained: bool = False) -> Tensor:
     if x.shape[0] > ops.FEW_ROWS:
         return torch.mm(x, w.t())
-    return ops.linear(x, w, chained=True)
+    return ops.linear(x, w, chained=chained)
 
 
-def matmul_f32(x: Tensor, w: Tensor) -> Tensor:
+def matmul_f32(x: Tensor, w: Tensor, chained: bool = False) -> Tensor:
     """x w^T whose fp32 sums are not rounded."""
     if x.shape[0] > ops.FEW_ROWS:
         return torch.mm(x, w.t()) if x.dtype == torch.float32 else torch.mm(x, w.t(), out_dtype=torch.float32)
-    return ops.linear(x, w, f32=True, chained=True)
+    return ops.linear(x, w, f32=True, chained=chained)
 
 
 # ---------------------------------------------------------------------------------- attention
@@ -126,7 +129,7 @@ class ChunkedAttention(nn.Module):
 
     def forward(self, h: Tensor, cache: RingCache, at: Portion) -> Tensor:
         B, S = at.B, at.S
-        qkv = matmul(h, self.wqkv).view(B, S, -1)
+        qkv = matmul(h, self.wqkv, at.chained).view(B, S, -1)
         a, b, c = self.sizes
         q = qkv[..., :a].unflatten(-1, (self.H, self.D))
         k = qkv[..., a:a + b].unflatten(-1, (self.G, self.D))
@@ -144,7 +147,7 @@ class ChunkedAttention(nn.Module):
                 ka, va = k, v
             y = ops.attn(q, ka, va, start=at.start, kv_start=lo, **args)
             ops.ring_append(k, v, cache.k[:B], cache.v[:B], start=at.start)
-        return matmul(y.view(B * S, self.H * self.E), self.wo)
+        return matmul(y.view(B * S, self.H * self.E), self.wo, at.chained)
 
 
 # ---------------------------------------------------------------------------------- latent attention
@@ -235,7 +238,7 @@ class LatentAttention(nn.Module):
 
     def forward(self, h: Tensor, cache: LatentCache, at: Portion) -> Tensor:
         B, S = at.B, at.S
-        qd = matmul(h, self.wqd)
+        qd = matmul(h, self.wqd, at.chained)
         q = qd[:, :self.q_rows]
         dkv = qd[:, self.q_rows:self.q_rows + self.K + self.R]
         rows = cache.rows[:B]
@@ -252,7 +255,7 @@ class LatentAttention(nn.Module):
             k = kv[..., :self.q_rows].unflatten(-1, (self.H, self.D + self.R))
             v = kv[..., self.q_rows:].unflatten(-1, (self.H, self.E))
             y = ops.attn(q.view(B, S, -1).unflatten(-1, (self.H, self.D + self.R)), k, v, **args)
-        return matmul(y.view(B * S, self.H * self.E), self.wo)
+        return matmul(y.view(B * S, self.H * self.E), self.wo, at.chained)
 
 
 # ---------------------------------------------------------------------------------- window attention
@@ -358,7 +361,7 @@ class MatrixMemory(nn.Module):
 
     def mix(self, parts: List[Tensor], h: Tensor, cache: MemoryState, at: Portion, out: Tensor) -> None:
         B = at.B
-        ops.mlstm(*parts, matmul_f32(h, self.w_gates), self.i_b_f32, self.f_b_f32, self.norm_w, cache.S[:B], cache.n[:B],
+        ops.mlstm(*parts, matmul_f32(h, self.w_gates, at.chained), self.i_b_f32, self.f_b_f32, self.norm_w, cache.S[:B], cache.n[:B],
                   cache.m[:B], out, S=at.S, cap=self.cap, q_scale=self.N ** -0.5, eps=self.eps, start=at.start, pos=at.pos,
                   status=at.status)
 
@@ -405,11 +408,11 @@ class Mamba2(nn.Module):
         return 0
 
     def forward(self, h: Tensor, cache: StateCache, at: Portion) -> Tensor:
-        proj = matmul(h, self.w_in)
+        proj = matmul(h, self.w_in, at.chained)
         y = ops.ssm(proj, self.inner, self.conv_w, self.conv_b, self.dt_bias_f32, self.A_log_f32, self.skip_f32,
                     cache.conv[:at.B], cache.state[:at.B], S=at.S, groups=self.G, start=at.start, pos=at.pos)
         y = ops.gated_group_norm(y, proj, self.norm_w, self.parts, self.eps)
-        return matmul(y, self.wo)
+        return matmul(y, self.wo, at.chained)
 
 
 # ---------------------------------------------------------------------------------- feed-forward
@@ -426,12 +429,13 @@ class ClampedFeedForward(nn.Module):
     def tensors(self) -> dict:
         return {"gate": self.w13[:self.ff], "up": self.w13[self.ff:2 * self.ff], "down": self.w2}
 
-    def forward(self, h: Tensor) -> Tensor:
+    def forward(self, h: Tensor, chained: bool = False) -> Tensor:
         unit = None
         if h.shape[0] <= ops.FEW_ROWS:                             # projections and unit in one launch
-            unit = ops.linear_glu(h, self.w13, 0, self.ff, self.ff, ops.GLU_CLAMPED, limit=self.limit, slope=ops.GLU_SLOPE, chained=True)
-        act = ops.glu_clamped(matmul(h, self.w13), self.ff, self.limit) if unit is None else unit[1]
-        return matmul(act, self.w2)
+            unit = ops.linear_glu(h, self.w13, 0, self.ff, self.ff, ops.GLU_CLAMPED, limit=self.limit, slope=ops.GLU_SLOPE,
+                                  chained=chained)
+        act = ops.glu_clamped(matmul(h, self.w13, chained), self.ff, self.limit) if unit is None else unit[1]
+        return matmul(act, self.w2, chained)
 
 
 class ParallelLayer(nn.Module):
@@ -473,10 +477,11 @@ class ParallelLayer(nn.Module):
         if self.ff:                                                # few rows: projections and unit in one launch
             gate, up = self.in_slices[-2:]
             if h.shape[0] <= ops.FEW_ROWS:
-                fused = ops.linear_glu(h, self.w_in, gate.start, up.start, self.ff, ops.GLU_SILU, plain=gate.start, act=act, chained=True)
-        proj = matmul(h, self.w_in) if fused is None else fused[0]
+                fused = ops.linear_glu(h, self.w_in, gate.start, up.start, self.ff, ops.GLU_SILU, plain=gate.start, act=act,
+                                       chained=at.chained)
+        proj = matmul(h, self.w_in, at.chained) if fused is None else fused[0]
         n_mix = len(self.mixer.in_sizes)
         self.mixer.mix([proj[:, s] for s in self.in_slices[:n_mix]], h, cache, at, inner[:, :self.mixer.out_size])
         if self.ff and fused is None:
             ops.glu_silu(proj[:, gate], proj[:, up], out=act)
-        return matmul_f32(inner, self.w_out)
+        return matmul_f32(inner, self.w_out, at.chained)

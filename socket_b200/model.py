@@ -148,7 +148,8 @@ def few_rows_here(x: Tensor, world: int) -> bool:
 
 
 def project_rows(x: Tensor, layer: nn.Linear, res: Optional[Tensor] = None) -> Tensor:
-    """layer(x) (+ res) of the rows [B, 1, width] of a decode step.  The kernel before it is one that made x: no weights."""
+    """layer(x) (+ res) of the rows [B, 1, width] of a decode step.  Chained: the step's kernels write no
+    weights, and the norm in front of it (or a library kernel) has waited for everything before the step."""
     if not untouched(layer, nn.Linear):
         return layer(x) if res is None else res + layer(x)
     y = few_rows.linear(x.reshape(-1, x.shape[-1]), layer.weight, res=None if res is None else res.reshape(-1, res.shape[-1]),

@@ -153,14 +153,14 @@ class Radapel(LayeredDecoder):
             layer = self.layers[run.layer]
             if run.new_pass is not None:
                 joined = ops.residual_norm(x, eps, y=y, w_in=w, x0=x0, dtype=dt)
-                y = matmul_f32(joined, self.loop_in)
+                y = matmul_f32(joined, self.loop_in, at.chained)
                 h = ops.residual_norm(x, eps, y=y, w_in=self.loop_step[run.new_pass], replace=True, w_out=layer.norm1)
             else:
                 h = ops.residual_norm(x, eps, y=y, w_in=w, w_out=layer.norm1)
             y, w = layer.mixer(h, cache, at), layer.norm1b
             if layer.mlp is not None:
                 h = ops.residual_norm(x, eps, y=y, w_in=w, w_out=layer.norm2)
-                y, w = layer.mlp(h), layer.norm2b
+                y, w = layer.mlp(h, at.chained) if type(layer.mlp) is ClampedFeedForward else layer.mlp(h), layer.norm2b
             if collect is not None:
                 ops.residual_norm(x, eps, y=y, w_in=w)
                 collect.append(x.clone())

@@ -92,3 +92,33 @@ def test_counts_of_another_layout_are_refused(caught):
     for p, seq in ((pos, torch.zeros(4, dtype=torch.int32)[::2]), (torch.zeros(2, dtype=torch.int64), torch.zeros(2, dtype=torch.int32))):
         with pytest.raises(AssertionError):
             few_rows.pick_token(logits, tok, p, seq, "step")
+
+
+@pytest.mark.parametrize("chained", [False, True])
+def test_products_are_chained_only_inside_a_stack(monkeypatch, chained):
+    """A mixer called by itself may stand right behind a kernel that wrote its weights; a decoder's stack says it does not."""
+    from socket_b200 import mixers as m
+
+    seen = []
+
+    class Stop(Exception):
+        pass
+
+    def product(x, w, *args, chained=False, **kw):
+        seen.append(chained)
+        raise Stop
+
+    monkeypatch.setattr(m.ops, "linear", product)
+    monkeypatch.setattr(m.ops, "linear_glu", product)
+    h, at = torch.zeros(2, 64), m.Portion(2, 1, 0, **({"chained": True} if chained else {}))
+    memory = m.MatrixMemory(64, 2, 8, 8, 15.0, 1e-5)
+    calls = [lambda: m.ChunkedAttention(64, 2, 1, 8, 8, 16, 1.0, 8, 4.0)(h, None, at),
+             lambda: m.LatentAttention(64, 2, 8, 8, 8, 16, 8, 1e4, 1.0, 1e-5)(h, None, at),
+             lambda: m.Mamba2(64, 2, 8, 8, 1, 4, 1, 1e-5)(h, None, at),
+             lambda: m.ParallelLayer(64, memory, 16)(h, None, at), lambda: m.ParallelLayer(64, memory, 0)(h, None, at),
+             lambda: memory.mix([], h, m.MemoryState(2, 2, 8, 8, "cpu"), at, h),
+             lambda: m.ClampedFeedForward(64, 16, 7.0)(h, *([True] if chained else []))]
+    for call in calls:
+        with pytest.raises(Stop):
+            call()
+    assert seen == [chained] * len(calls)
