@@ -67,7 +67,7 @@ __device__ __forceinline__ int effective_len(int64_t T, const int32_t* T_dev) {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // First statement of a kernel that is always launched chained: everything behind it sees what an unchained launch
-// would see, and only the cost of launching overlaps the kernel before.  Data of earlier kernels is read through
+// would see, and only the cost of launching overlaps the kernel before.  Inputs, weights among them, are read through
 // pointers without __restrict__, so that no load is moved in front of the wait.
 // The successor is let in only now: a projection (linear_rows_body.cuh) that got in while the projection before still runs
 // would find its places SM by SM as that one's blocks end, two on some SMs and none on others (28672 x 4096 inside a

@@ -62,7 +62,7 @@ latent_append_kernel(sk_latent_params p) {
 constexpr int AB_ROWS = 8;
 template <typename T>
 __global__ void __launch_bounds__(256)
-latent_absorb_kernel(const T* q, int64_t q_ld, const T* __restrict__ uk, int64_t rows, int H, int dim, int rot,
+latent_absorb_kernel(const T* q, int64_t q_ld, const T* uk, int64_t rows, int H, int dim, int rot,
                      int rank, int out_ld, T* __restrict__ out) {
     pdl_begin();
     extern __shared__ float sm[];                                // q [AB_ROWS][dim], partials [8][AB_ROWS][64]
@@ -127,7 +127,7 @@ latent_absorb_kernel(const T* q, int64_t q_ld, const T* __restrict__ uk, int64_t
 // (8 columns each) and 16 along the head's rows of W_uk, so that a thread's loads are few, wide and in flight together.
 template <int ROWS>
 __global__ void __launch_bounds__(256)
-latent_absorb_vec_kernel(const __nv_bfloat16* q, int64_t q_ld, const __nv_bfloat16* __restrict__ uk, int64_t rows,
+latent_absorb_vec_kernel(const __nv_bfloat16* q, int64_t q_ld, const __nv_bfloat16* uk, int64_t rows,
                          int H, int dim, int rot, int rank, int out_ld, __nv_bfloat16* __restrict__ out) {
     pdl_begin();
     extern __shared__ float sm[];                                // q [ROWS][dim], partials [16][ROWS][128]
@@ -199,7 +199,7 @@ latent_absorb_vec_kernel(const __nv_bfloat16* q, int64_t q_ld, const __nv_bfloat
 // out[row, h * vdim + e] for bf16 and a rank that is a multiple of 8: one warp per output element and row group
 template <int ROWS>
 __global__ void __launch_bounds__(128)
-latent_up_vec_kernel(const __nv_bfloat16* o, const __nv_bfloat16* __restrict__ uv, int64_t rows, int H, int vdim,
+latent_up_vec_kernel(const __nv_bfloat16* o, const __nv_bfloat16* uv, int64_t rows, int H, int vdim,
                      int rank, __nv_bfloat16* __restrict__ out) {
     pdl_begin();
     const int lane = threadIdx.x & 31;
@@ -239,7 +239,7 @@ latent_up_vec_kernel(const __nv_bfloat16* o, const __nv_bfloat16* __restrict__ u
 // out[row, h * vdim + e] = <W_uv[h * vdim + e, :], o[row, h, :]>: one warp per output element and row group
 template <typename T>
 __global__ void __launch_bounds__(256)
-latent_up_kernel(const T* o, const T* __restrict__ uv, int64_t rows, int H, int vdim, int rank, T* __restrict__ out) {
+latent_up_kernel(const T* o, const T* uv, int64_t rows, int H, int vdim, int rank, T* __restrict__ out) {
     pdl_begin();
     const int lane = threadIdx.x & 31;
     const int e = blockIdx.x * 8 + (threadIdx.x >> 5);           // flat (head, value dimension)

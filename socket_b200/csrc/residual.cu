@@ -153,7 +153,7 @@ glu_kernel(const T* gate, const T* up, int64_t rows, int ff, int64_t ld, float l
 template <typename T>
 __global__ void __launch_bounds__(256)
 ring_append_kernel(const T* k, const T* v, int64_t k_bs, int64_t k_ss, int64_t v_bs,
-                   int64_t v_ss, int k_row, int v_row, int ring, const int64_t* __restrict__ pos, int64_t start, int s0,
+                   int64_t v_ss, int k_row, int v_row, int ring, const int64_t* pos, int64_t start, int s0,
                    T* __restrict__ k_cache, T* __restrict__ v_cache) {
     pdl_begin();
     const int s = s0 + blockIdx.x, b = blockIdx.y;

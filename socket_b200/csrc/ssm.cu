@@ -173,7 +173,7 @@ ssm_steps_kernel(sk_ssm_params p) {
 // ---------------------------------------------------------------- gate, then RMS norm of each part
 template <typename T, int V, int NV>
 __global__ void __launch_bounds__(1024)
-gated_group_norm_kernel(const T* y, const T* z, int64_t z_ld, const T* __restrict__ w, int inner, int part, float eps,
+gated_group_norm_kernel(const T* y, const T* z, int64_t z_ld, const T* w, int inner, int part, float eps,
                         T* __restrict__ out) {
     pdl_begin();
     __shared__ float red[32];
