@@ -243,11 +243,17 @@ def ptr(t) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+# Not a public name of torch: where a torch has no such function, the stream is asked for the public way
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_ptr(device=None) -> int:
     """torch's current stream of a device that has been used already (the operators' tensors live on it).  Read without
     making a Stream object: an operator call costs the host 1 to 2 us less, and a short prompt is some 60 of them."""
+    if _raw_stream is None:
+        return torch.cuda.current_stream(device).cuda_stream
     index = None if device is None else device.index
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
+    return _raw_stream(torch.cuda.current_device() if index is None else index)
 
 
 def dtype_code(t: torch.Tensor) -> int:
