@@ -337,7 +337,7 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
                     for (int c = 0; c < FP_HALF; c += 2) unpack2(fma2(pack2(s[c], s[c + 1]), sc2, far2), s[c], s[c + 1]);
                 } else {
-const float* at = bt + lane + FP_HALF - 1;
+                    const float* at = bt + lane + FP_HALF - 1;
 #pragma unroll
                     for (int c = 0; c < FP_HALF; ++c) s[c] = fmaf(s[c], sc, at[-c]);
                 }

@@ -34,6 +34,7 @@
 // reads for call n, and a word left by call n-2 never carries call n's number.  The per-CTA call
 // counter lives in this GPU's own memory, so a CUDA graph can replay the call.
 #include "common.cuh"
+#include "warp_mma.cuh"
 
 namespace sk {
 namespace {
@@ -73,19 +74,6 @@ __device__ __forceinline__ void unpack8(const uint4& w, const __half*, float (&f
     }
 }
 
-// D (16 x 8, fp32) += A (16 x 16, row-major) * B (16 x 8, column-major)
-__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1, const __nv_bfloat16*) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void mma16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                         uint32_t b0, uint32_t b1, const __half*) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 template <typename T, int GA_COLS>
 __global__ void __launch_bounds__(GA_THREADS, 1)

@@ -4,10 +4,10 @@
 // flight all the time.  A CTA walks tiles of 16 RT weight rows; its 8 warps divide k.  A lane holds 32 consecutive
 // bytes of two rows of each 16-row tile (four lanes: 128 bytes of a row) in a ring of registers, refilled as soon as a
 // piece has been used and across the ends of tiles, so the stream does not stop at a tile's reduction: 64 KB in flight
-// per CTA, two CTAs per SM (or one of 16 warps, when there is at most one tile per SM).  The products are m16n8k16 MMAs, weight rows against the (up to) 8 rows of x; a sum over k
-// may be taken in any order as long as both operands take the same one, so a lane's own 16 elements serve as they
-// were loaded, without a shuffle or a pass through shared memory.  The warps' sums meet in shared memory, in warp
-// order, in fp32.
+// per CTA, two CTAs per SM (or one of 16 warps, when there is at most one tile per SM).  The products are m16n8k16 MMAs,
+// weight rows against the (up to) 8 rows of x; a sum over k may be taken in any order as long as both operands take the
+// same one, so a lane's own 16 elements serve as they were loaded, without a shuffle or a pass through shared memory.
+// The warps' sums meet in shared memory, in warp order, in fp32.
 //
 // Weights do not depend on the kernel before this one.  With `chained` the kernel may start while kernels before it still
 // run, fills its ring with weights, and only then waits for x.  It lets its own successor in before that wait, and so do the
@@ -20,24 +20,13 @@
 #pragma once
 #include "abi_check.cuh"
 #include "blocks.cuh"
+#include "warp_mma.cuh"
 
 namespace sk {
 namespace {
 
 constexpr int LR_MAX_ROWS = 8;
 
-__device__ __forceinline__ void lr_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                       uint32_t b1, const __nv_bfloat16*) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void lr_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                       uint32_t b1, const __half*) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 __device__ __forceinline__ void lr_load_weights(const void* p, bool live, uint32_t (&r)[8]) {
     if (live) {
         asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -187,7 +176,7 @@ linear_rows_kernel(const __grid_constant__ sk_linear_params p, int plain_tiles, 
                     for (int j = 0; j < 4; ++j)
 #pragma unroll
                         for (int rt = 0; rt < RT; ++rt)
-                            lr_mma(acc[rt], wf[s][c][2 * rt][2 * j], wf[s][c][2 * rt + 1][2 * j], wf[s][c][2 * rt][2 * j + 1],
+                            mma16816(acc[rt], wf[s][c][2 * rt][2 * j], wf[s][c][2 * rt + 1][2 * j], wf[s][c][2 * rt][2 * j + 1],
                                    wf[s][c][2 * rt + 1][2 * j + 1], xf[s][c][2 * j], xf[s][c][2 * j + 1], (const T*)nullptr);
                 if (base + s + NS < total) {
                     load_w(s);

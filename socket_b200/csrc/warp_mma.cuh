@@ -1,4 +1,4 @@
-// Warp-level matrix helpers: 16-byte asynchronous copies, ldmatrix fragments, m16n8k16 bf16 MMA.
+// Warp-level matrix helpers: 16-byte asynchronous copies, ldmatrix fragments, m16n8k16 MMAs.
 // Fragment of a 16 x 8 fp32 tile: lane holds (row lane / 4, columns 2 (lane % 4) and + 1) in c[0..1] and
 // the same columns of row + 8 in c[2..3].
 #pragma once
@@ -25,6 +25,17 @@ __device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], 
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// The same for either 16-bit type, fragment by fragment
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1,
+                                         const __nv_bfloat16*) {
+    mma16816(c, {a0, a1, a2, a3}, b0, b1);
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1,
+                                         const __half*) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 // two fp32 values as bf16 pairs: the values rounded, and what rounding left
