@@ -6,11 +6,20 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _bound(x, w, dtype, f32):
-    """fp32 sums of k products, each step off by at most 2^-23 of the sum of magnitudes; then one rounding to the type."""
-    mag = x.double().abs() @ w.double().abs().t()
-    eps = 0.0 if f32 else {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}[dtype]
-    return mag * x.shape[1] * 2.0 ** -23, eps
+EPS = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11, torch.float32: 2.0 ** -23}
+
+
+def _sums(x, w, library=False):
+    """Per result, how far an fp32 sum may be off: each addition at most 2^-23 of the magnitudes added.  The kernel adds a
+    warp's part of k (an eighth of its pieces of up to 128 elements), then 16 warps; of the library's order nothing is known."""
+    k = x.shape[1]
+    adds = k if library else min(k, k // 8 + 128) + 16
+    return x.double().abs() @ w.double().abs().t() * adds * 2.0 ** -23
+
+
+def _bound(x, w, dtype, f32, library=False):
+    """Those sums, then one rounding to the type."""
+    return _sums(x, w, library), 0.0 if f32 else EPS[dtype]
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
@@ -31,28 +40,67 @@ def test_plain_products(rows, n, k, dtype):
         assert got.shape == ref.shape and bool(((got - ref).abs() <= tol + eps * ref.abs() + 1e-7).all())
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows,k,ff,plain", [(1, 64, 16, 0), (8, 128, 33, 40), (3, 1040, 5632, 3072), (8, 512, 100, 4800)])
 @pytest.mark.parametrize("kind", [0, 1])
-def test_gated_unit(rows, k, ff, plain, kind):
+def test_gated_unit(rows, k, ff, plain, kind, dtype):
     from socket_b200 import block_ops as ops
     g = torch.Generator(device="cuda").manual_seed(ff)
-    x = torch.randn(rows, k, generator=g, device="cuda").bfloat16()
-    w = (torch.randn(plain + 2 * ff + 8, k, generator=g, device="cuda") * 2 * k ** -0.5).bfloat16()
-    wide = torch.full((rows, ff + 24), 3.0, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(rows, k, generator=g, device="cuda").to(dtype)
+    w = (torch.randn(plain + 2 * ff + 8, k, generator=g, device="cuda") * 2 * k ** -0.5).to(dtype)
+    wide = torch.full((rows, ff + 24), 3.0, device="cuda", dtype=dtype)
     out, act = ops.linear_glu(x, w, plain, plain + ff + 8, ff, kind, limit=1.5, slope=1.7, plain=plain, act=wide[:, 8:8 + ff])
-    y = x.double() @ w.double().t()
-    gate, up = y[:, plain:plain + ff], y[:, plain + ff + 8:plain + 2 * ff + 8]
-    if kind == ops.GLU_CLAMPED:
-        a, b = gate.clamp(max=1.5), up.clamp(-1.5, 1.5)
-        want = a * torch.sigmoid(1.7 * a) * (b + 1)
-    else:
-        want = gate * torch.sigmoid(gate) * up
-    # sums: 2^-23 k of the magnitudes (at most 8 here after the scaling), times the unit's slopes (below 10); one rounding
-    mag = (x.double().abs() @ w.double().abs().t()).max()
-    assert bool(((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + mag * k * 2.0 ** -23 * 10 + 1e-6 * (1 + want.abs())).all())
+    y, off = x.double() @ w.double().t(), _sums(x, w)
+    gates, ups = slice(plain, plain + ff), slice(plain + ff + 8, plain + 2 * ff + 8)
+    slope, a, b = (1.7, y[:, gates].clamp(max=1.5), y[:, ups].clamp(-1.5, 1.5) + 1) if kind == ops.GLU_CLAMPED else (1.0, y[:, gates], y[:, ups])
+    want = a * torch.sigmoid(slope * a) * b
+    # a sigmoid(slope a) has slopes up to 1.1 and is at most |a|; the exponential is off by 2 + 1.18 |slope a| units in the last
+    # place, the division by 2, three more roundings; then one to the type (fp16: at least half a denormal step)
+    d_gate, d_up = off[:, gates], off[:, ups]
+    unit = 1.1 * d_gate * (b.abs() + d_up) + a.abs() * d_up + want.abs() * (8 + 1.2 * (slope * a).abs()) * 2.0 ** -23
+    assert bool(((act.double() - want).abs() <= unit + EPS[dtype] * (want.abs() + unit) + 2.0 ** -25).all())
     assert bool((wide[:, :8] == 3).all()) and bool((wide[:, 8 + ff:] == 3).all())
-    tol, eps = _bound(x, w[:plain], torch.bfloat16, False)
+    tol, eps = _bound(x, w[:plain], dtype, False)
     assert bool(((out.double() - y[:, :plain]).abs() <= tol + eps * y[:, :plain].abs() + 1e-7).all())
+
+
+@pytest.mark.parametrize("rows", [1, 8])
+@pytest.mark.parametrize("graph", [False, True])
+def test_chained_products_behind_one_another(rows, graph):
+    """Projections of all forms (16 and 32 rows a tile, 16 warps, the unit), each reading what the one before wrote: chained or
+    not, the same bits."""
+    from socket_b200 import block_ops as ops
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda")
+    sizes = [512, 9600, 2048, 4800, 256, 512]
+    ws = [(r(n, k) * k ** -0.5).bfloat16() for k, n in zip(sizes, sizes[1:])]
+    glu = (r(1024, 512) * 512 ** -0.5).bfloat16()
+
+    def chain(x, chained):
+        for _ in range(3):
+            for w in ws:
+                x = ops.linear(x, w, chained=chained)
+            x = ops.linear_glu(x, glu, 0, 512, 512, ops.GLU_SILU, chained=chained)[1]
+        return x
+
+    x0 = r(rows, 512).bfloat16()
+    want = chain(x0, False)
+    x = x0.clone()                                                # unchained, behind everything that made the weights
+    if not graph:
+        assert torch.equal(chain(x, True), want)
+        return
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        chain(x, True)
+        recorded = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(recorded, stream=side):
+            got = chain(x.clone(), True)
+    torch.cuda.current_stream().wait_stream(side)
+    for _ in range(3):
+        got.zero_()
+        recorded.replay()
+        assert torch.equal(got, want)
 
 
 def test_shapes_outside_go_to_the_library():
@@ -111,7 +159,7 @@ def test_residual_layouts(rows, layout):
     x, w = r(rows, k), r(n, k)
     res = {"strided": r(rows, n + 8)[:, 8:], "broadcast": r(1, n).expand(rows, n), "turned": r(n, rows).t()}[layout]
     want = x.double() @ w.double().t() + res.double()
-    tol, eps = _bound(x, w, torch.bfloat16, False)
+    tol, eps = _bound(x, w, torch.bfloat16, False, library=rows > 8)
     if rows > 8:                                                  # the library rounds the product before the sum
         tol = tol + eps * (want - res.double()).abs()
     assert bool(((ops.linear(x, w, res=res).double() - want).abs() <= tol + eps * want.abs() + 1e-7).all())
@@ -141,7 +189,7 @@ def test_what_only_the_library_takes(form, f32):
     got = ops.linear(x, w, f32=f32)
     assert got.shape == (x.shape[0], w.shape[0]) and got.dtype == (torch.float32 if f32 else torch.bfloat16)
     want = x.double() @ w.double().t()
-    tol, eps = _bound(x, w, torch.bfloat16, f32)
+    tol, eps = _bound(x, w, torch.bfloat16, f32, library=True)
     assert bool(((got.double() - want).abs() <= tol + eps * want.abs() + 1e-7).all())
     if form in ("expanded rows", "no rows", "no columns"):
         assert ops.linear_glu(x, w, 0, 8, 8, ops.GLU_SILU) is None
