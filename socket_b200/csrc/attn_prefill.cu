@@ -15,9 +15,9 @@
 //
 // Bound: the softmax arithmetic of a tile (the exponential's unit and the issue slots of 16 warps) beside 2 x 512 cycles of
 // MMAs.  Measured, one GPU, L2 flushed (with four warps per tile, one thread per row, and the MMAs built and issued in one
-// lane's loop: in brackets): 8000 tokens, 32 / 8 heads of 128, chunk and bias 599 us (996); 32 heads of 192 / 128 with
-// sinks 702 us (1098); 32000 tokens, 16 heads, window 4096 and cap 1150 us (1739); 1501 tokens behind 2500, 16 heads,
-// bias 97 us (133).
+// lane's loop: in brackets): 8000 tokens, 32 / 8 heads of 128, chunk and bias 586 us (996); 32 heads of 192 / 128 with
+// sinks 677 us (1098); 32000 tokens, 16 heads, window 4096 and cap 1136 us (1739); 1501 tokens behind 2500, 16 heads,
+// bias 94 us (133).
 #include "blocks.cuh"
 #include "tcgen05.cuh"
 #include "tensor_map.cuh"
@@ -31,7 +31,8 @@ constexpr int FP_SOFTMAX_WARPS = 16;                          // warp: 8 tile + 
 constexpr int FP_TMA_WARP = 16, FP_MMA_WARP = 17;
 constexpr int FP_THREADS = 32 * (FP_SOFTMAX_WARPS + 4);       // the last two warps idle: registers are dealt to groups of four
 // Registers a thread: 96 at launch (640 threads), then 112 for the softmax warps and 32 for the others
-// (512 x 112 + 128 x 32 = 61440, all that the block was launched with; with 104 and 64: 675 and 931 us below)
+// (512 x 112 + 128 x 32 = 61440, all that the block was launched with; with 104 and 64 the first two figures above are 655
+// and 900 us).  64 scores and their weights do not quite fit: 270 to 360 bytes a thread are spilled in every form.
 constexpr int FP_REGS_SOFTMAX = 112, FP_REGS_OTHER = 32;
 constexpr uint32_t FP_PANEL = FP_TILE * 128;                  // 128 rows x 64 bf16
 constexpr int FP_BIAS_SPAN = 96;                              // distances a warp's 32 rows x 64 keys can have
@@ -59,14 +60,13 @@ struct FpShape {            // what the kernel needs beside the tensor maps
     int32_t* status;
     int64_t o_bs, o_ss, o_hs, start, kv_start, bias_len;
     int S, H, G, dqk, dv, chunk, window, nk, nv;      // nk, nv: stages of the K and V rings
-    int q_blocks, head_group;                 // blocks of 256 queries; heads walked side by side
+    int q_blocks;                             // blocks of 256 queries
     float scale_log2, cap_in, cap_out;        // softcap: s <- cap_out tanh(s cap_in), log2 units
     float cap_poly[5], cap_small;             // the same for s^2 <= cap_small: s times a polynomial in s^2
 };
 // Softcap: none, any, or one so low that exp of a capped score and sums of it stay far inside the fp32 range
 enum { FP_CAP_NONE = 0, FP_CAP = 1, FP_CAP_BOUND = 2 };
 constexpr float FP_CAP_BOUND_LOG2 = 80.f;
-constexpr double FP_GROUP_BYTES = 48e6;      // 32 heads of 192 / 128 on 8000 rows, 164 MB: 978 us side by side, 937 in groups
 
 // first key row (counted from kv_start: rows of the call, below 2^30, whatever the positions are) that query row i sees
 __device__ __forceinline__ int fp_first_row(const FpShape& p, int i) {
@@ -114,10 +114,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     extern __shared__ __align__(1024) char fp_raw[];
     char* tiles = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(fp_raw) + 1023) & ~(uintptr_t)1023);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // groups of heads in order; in a group heads side by side, long rows first
-    const int b = blockIdx.y, group = blockIdx.x / (p.head_group * p.q_blocks), in_group = blockIdx.x - group * p.head_group * p.q_blocks;
-    const int heads = min(p.head_group, p.H - group * p.head_group), back = in_group / heads;
-    const int h = group * p.head_group + in_group - back * heads, g = h / (p.H / p.G);
+    // heads side by side, long rows first: the last blocks to start are short ones.  (Heads in groups whose keys and values fit
+    // the L2 end in a short group of long rows: 24000 tokens, 16 heads of 192 / 128 in groups of 3: 2975 us, so 2643; 8000
+    // tokens, 32 heads in groups of 9: 699 us, so 677.  16000 tokens, 16 heads were 1177 us in groups and are 1207 so.)
+    const int b = blockIdx.y, back = blockIdx.x / p.H, h = blockIdx.x - back * p.H, g = h / (p.H / p.G);
     const int np = (p.dqk + 63) / 64, nvp = (p.dv + 63) / 64;
     char* q_s = tiles;                                        // [tile][panel]
     char* k_s = q_s + 2 * np * FP_PANEL;                      // [stage][panel]
@@ -497,13 +497,7 @@ int launch_attn_prefill_tc(const sk_attn_params& p, cudaStream_t st) {
                                  : (f.cap_out <= FP_CAP_BOUND_LOG2 ? attn_prefill_kernel<false, FP_CAP_BOUND> : attn_prefill_kernel<false, FP_CAP>);
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(SK_ERR_CUDA, "attn_prefill_kernel smem attribute: %s", cudaGetErrorString(e));
-    // Heads side by side, so that the last blocks to start are short ones, but only as many as have keys and values for
-    // FP_GROUP_BYTES of the L2 together
     f.q_blocks = (p.S + 2 * FP_TILE - 1) / (2 * FP_TILE);
-    const int rep = p.H / p.G;
-    const double kv_bytes = (double)p.kv_rows * (p.dqk + p.dv) * 2;
-    const int kv_heads = (int)(FP_GROUP_BYTES / kv_bytes < p.G ? FP_GROUP_BYTES / kv_bytes : p.G);
-    f.head_group = rep * (kv_heads < 1 ? 1 : kv_heads);
     dim3 grid((unsigned)(p.H * f.q_blocks), (unsigned)p.B);
     kern<<<grid, FP_THREADS, smem, st>>>(mq, mk, mv, f);
     return check_launch("attn_prefill_kernel");

@@ -1,4 +1,4 @@
-"""Prefill attention where its rules change: heads in groups with a shorter last group, biases whose table ends inside, at
+"""Prefill attention where its rules change: many heads of few key/value heads or of their own, biases whose table ends inside, at
 and far before a half tile of 64 keys, rows that end anywhere in a query tile, head sizes with a ragged last MMA step."""
 import pytest
 import torch
@@ -41,8 +41,8 @@ def _plain(q, k, v, kw, i, h):
 
 
 @pytest.mark.parametrize("S,H,G,D,E,start,kv_start,bias_len,chunk,window,cap,sink", [
-    (300, 11, 11, 192, 128, 9000, 0, 0, 0, 0, 0.0, True),        # 6 MB of keys and values a head: groups of 8 and 3
-    (515, 20, 10, 192, 128, 14000, 0, 0, 0, 0, 0.0, False),      # groups of 5 key/value heads, two queries heads each
+    (300, 11, 11, 192, 128, 9000, 0, 0, 0, 0, 0.0, True),        # an odd number of heads, each its own keys, 6 MB a head
+    (515, 20, 10, 192, 128, 14000, 0, 0, 0, 0, 0.0, False),      # two query heads a key/value head, a ragged last block
     (700, 4, 2, 128, 128, 0, 0, 33, 0, 0, 0.0, False),           # bias constant beyond 32, inside the diagonal tiles
     (385, 4, 2, 128, 128, 640, 512, 193, 512, 0, 0.0, False),    # and at a half tile's edge, behind the chunk's first rows
     (257, 2, 2, 128, 64, 511, 0, 5000, 512, 0, 0.0, True),       # table longer than any distance
