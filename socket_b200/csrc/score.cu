@@ -834,9 +834,11 @@ int launch_score_compat(const float* q_probs, const int16_t* key_buckets, const 
     const int use_smem = smem <= 160 * 1024;
     if (use_smem && smem > 48 * 1024)
         cudaFuncSetAttribute(score_compat_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    // 16 and 32 tables: the unrolled form, while its blocks fill the SMs at least once (else shorter blocks spread better)
+    // 16 and 32 tables (the unrolled form is compiled for those that the configurations and tests have) that fit shared memory,
+    // at every size, the call between events: 1 row x 700 keys 11 us (the other form 27), 8 x 12345 12 (25), 32 x 4096 13 (29), 32 x 32768 53 (107);
+    // 16 tables 8 (17), 10 (16), 10 (19), 25 (49)
     const int64_t blocks = (T + SC_COMPAT_KEYS - 1) / SC_COMPAT_KEYS;
-    if ((L == 32 || L == 16) && smem <= 48 * 1024 && blocks <= INT_MAX && blocks * B * H >= sm_count()) {
+    if ((L == 32 || L == 16) && smem <= 48 * 1024 && blocks <= INT_MAX) {
         auto kern = L == 32 ? score_compat_tables_kernel<32> : score_compat_tables_kernel<16>;
         kern<<<dim3((unsigned)blocks, (unsigned)(B * H)), SC_COMPAT_THREADS, smem, st>>>(q_probs, key_buckets, allowed, v_hist, out, R, T);
         return check_launch("score_compat_tables_kernel");

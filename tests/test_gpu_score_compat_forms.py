@@ -1,4 +1,4 @@
-"""The original-layout scorer at the edges of its blocks of 1024 keys and on both sides of its rule (tables, size): the same
+"""The original-layout scorer at the edges of its blocks of 1024 keys and on both sides of its rule (tables, table size): the same
 bits as adding the tables one by one in fp32."""
 import pytest
 import torch
@@ -7,7 +7,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("H,L,R,T", [(148, 32, 256, 1), (148, 32, 256, 511), (160, 32, 64, 513), (150, 16, 256, 1024), (75, 32, 256, 1025),
-                                     (37, 16, 128, 4096), (3, 32, 256, 1500), (149, 24, 256, 700), (150, 32, 512, 600)])
+                                     (37, 16, 128, 4096), (3, 32, 256, 1500), (149, 24, 256, 700), (150, 32, 512, 600), (1, 32, 256, 1),
+                                     (2, 16, 256, 1025), (1, 32, 384, 2048), (1, 32, 385, 2048)])
 def test_same_bits_as_table_by_table(H, L, R, T):
     from socket_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(T)
