@@ -14,9 +14,9 @@
 // kernels of the sparse step: a chained projection can reach back over several kernels.  The caller vouches that neither
 // the stream's last unchained launch nor anything behind it writes the weights.
 //
-// Measured (one row, cold weights, back to back in a graph; chained / not / cuBLAS): 4096 x 14336 20.1 / 21.7 / 24.4 us
-// (5.9 TB/s), 28672 x 4096 38.2 / 39.6 / 39.1 us, 4096 x 4096 6.2 / 8.2 / 12.9 us, 2048 x 2048 2.4 / 4.0 / 7.3 us; with
-// 8 rows within 3% of that.
+// Measured (one row, cold weights, back to back in a graph; chained / not / cuBLAS): 4096 x 14336 19.2 / 20.8 / 24.4 us
+// (6.1 TB/s), 28672 x 4096 37.0 / 38.7 / 39.1 us, 4096 x 4096 6.1 / 7.9 / 12.9 us, 2048 x 2048 2.4 / 4.0 / 7.3 us; 8 rows:
+// 4096 x 14336 19.6 / 21.4 us, 2048 x 5632 5.4 / 7.2 us (one row 4.6 / 6.7).
 #pragma once
 #include "abi_check.cuh"
 #include "blocks.cuh"

@@ -1,6 +1,6 @@
 """Operators on the few rows of a decode step that every decoder uses: projections that stream the weights once, an RMS
-norm of rows in the model's type, the greedy pick.  Both libraries hold the projections and the pick; a model calls those of the library
-it is built on (`library`: "step" or "blocks")."""
+norm of rows in the model's type, the greedy pick.  Both libraries hold the projections and the pick, the step library
+the norm; a model calls those of the library it is built on (`library`: "step" or "blocks")."""
 from __future__ import annotations
 
 import ctypes as C
