@@ -388,3 +388,18 @@ def test_bias_table_of_a_layer_reaches_every_bucket():
     want = distance_buckets(100, 12, 100)
     assert sorted(set(want.tolist())) == list(range(12))
     assert torch.equal(m.bias.cpu(), torch.arange(24.).view(12, 2)[want].t())
+
+
+@pytest.mark.parametrize("rows", [511, 512, 513, 1100])
+def test_gated_norm_on_both_sides_of_the_signal_rule(rows):
+    """Grids up to 4096 blocks let the kernel behind them in early, larger ones do not: the same bits as row by row groups, and a
+    successor that is launched chained reads what the whole grid wrote."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    r = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()
+    y, z, w = r(rows, 256), r(rows, 256), r(256)
+    for _ in range(5):
+        whole = ops.gated_group_norm(y, z, w, 8, 1e-5)
+        again = ops.gated_group_norm(whole, z, w, 8, 1e-5)
+    parts = [ops.gated_group_norm(a, b, w, 8, 1e-5) for a, b in zip(y.split(100), z.split(100))]
+    assert torch.equal(whole, torch.cat(parts))
+    assert torch.equal(again, torch.cat([ops.gated_group_norm(a, b, w, 8, 1e-5) for a, b in zip(parts, z.split(100))]))
