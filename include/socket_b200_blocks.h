@@ -161,7 +161,8 @@ SK_API int skb_latent_up(const void* o, int dtype, const void* uv, int64_t rows,
  * (conv_w [channels, taps], last tap = current token) + silu into xbc rows (xbc_ld apart), carried
  * inputs conv_state [B, taps - 1, channels].  skb_ssm_scan: the recurrence on those rows,
  * state [B, H, N, P] fp32, y [B, S, H P] (with the skip D x).  Position 0 starts from zero state.
- * `path`: SKB_SSM_STEPS walks token by token, SKB_SSM_CHUNKS uses matrix products per block of tokens. */
+ * `path`: SKB_SSM_STEPS walks token by token, SKB_SSM_CHUNKS uses matrix products per block of 64 tokens; SKB_SSM_AUTO
+ * also has chunks of 128 tokens on the tensor cores (skb_ssm_path then says SKB_SSM_TENSOR). */
 enum { SKB_SSM_AUTO = 0, SKB_SSM_STEPS = 1, SKB_SSM_CHUNKS = 2, SKB_SSM_TENSOR = 3 };
 typedef struct sk_ssm_params {
     const void *xbc_in, *dt_in, *conv_w, *conv_b;

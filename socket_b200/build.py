@@ -30,7 +30,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std
          "--expt-relaxed-constexpr"]
 LIBRARIES = {"step": LIB, "blocks": BLOCKS_LIB}
 BLOCK_SOURCES = ("abi_blocks", "attn_decode", "attn_prefill", "attn_rows", "few_rows", "latent", "mlstm", "mlstm_tc",
-                 "recurrence_chunks", "residual", "rotary_rows", "ssm")
+                 "recurrence_chunks", "residual", "rotary_rows", "ssm", "ssm_tc")
 SHARED_SOURCES = ("host",)
 
 

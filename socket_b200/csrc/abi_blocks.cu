@@ -46,9 +46,17 @@ int check_ssm(const sk_ssm_params* p) {
     return SK_OK;
 }
 
+// From two blocks of 64 tokens on, one chunk of 128 on the tensor cores is faster: 65 to 127 tokens of 128 heads with the
+// convolution 35 us in blocks, 27 in a chunk (4 x 64 heads: 50 and 34 to 37); up to 64 tokens, one block, 29.
+constexpr int SSM_TC_TOKENS = 65;
 int ssm_path(const sk_ssm_params& p) {
     if (p.path != SKB_SSM_AUTO) return p.path;
+    if (p.S >= SSM_TC_TOKENS && ssm_tc_applicable(p)) return SKB_SSM_TENSOR;
     return p.S >= 16 && ssm_chunks_applicable(p) ? SKB_SSM_CHUNKS : SKB_SSM_STEPS;
+}
+size_t ssm_workspace(const sk_ssm_params& p) {
+    const int path = ssm_path(p);
+    return path == SKB_SSM_TENSOR ? ssm_tc_workspace(p) : path == SKB_SSM_CHUNKS ? ssm_chunks_workspace(p) : 0;
 }
 
 int check_mlstm(const sk_mlstm_params* p) {
@@ -195,22 +203,18 @@ int skb_ssm_conv(const sk_ssm_params* p, void* stream) {
     return launch_ssm_conv(*p, (cudaStream_t)stream);
 }
 
-size_t skb_ssm_workspace_bytes(const sk_ssm_params* p) {
-    return p != nullptr && ssm_path(*p) == SKB_SSM_CHUNKS ? ssm_chunks_workspace(*p) : 0;
-}
+size_t skb_ssm_workspace_bytes(const sk_ssm_params* p) { return p != nullptr ? ssm_workspace(*p) : 0; }
 
 int skb_ssm_path(const sk_ssm_params* p) { return p != nullptr ? ssm_path(*p) : SKB_SSM_STEPS; }
 
 int skb_ssm_scan(const sk_ssm_params* p, void* stream) {
     if (int rc = check_ssm(p)) return rc;
-    if (ssm_path(*p) == SKB_SSM_CHUNKS) {
-        if (!ssm_chunks_applicable(*p)) return fail(SK_ERR_UNSUPPORTED, "skb_ssm_scan: shape outside the block kernel");
-        if (ssm_chunks_workspace(*p) > 0 && (p->workspace == nullptr || p->workspace_bytes < ssm_chunks_workspace(*p)))
-            return fail(SK_ERR_WORKSPACE, "skb_ssm_scan: workspace of %zu bytes needed, %zu given", ssm_chunks_workspace(*p),
-                        p->workspace_bytes);
-        return launch_ssm_chunks(*p, (cudaStream_t)stream);
-    }
-    return launch_ssm_steps(*p, (cudaStream_t)stream);
+    const cudaStream_t st = (cudaStream_t)stream;
+    const int path = ssm_path(*p);
+    if (path == SKB_SSM_CHUNKS && !ssm_chunks_applicable(*p)) return fail(SK_ERR_UNSUPPORTED, "skb_ssm_scan: shape outside the block kernel");
+    if (ssm_workspace(*p) > 0 && (p->workspace == nullptr || p->workspace_bytes < ssm_workspace(*p)))
+        return fail(SK_ERR_WORKSPACE, "skb_ssm_scan: workspace of %zu bytes needed, %zu given", ssm_workspace(*p), p->workspace_bytes);
+    return path == SKB_SSM_TENSOR ? launch_ssm_tc(*p, st) : path == SKB_SSM_CHUNKS ? launch_ssm_chunks(*p, st) : launch_ssm_steps(*p, st);
 }
 
 size_t skb_mlstm_workspace_bytes(const sk_mlstm_params* p) {

@@ -124,6 +124,9 @@ int launch_ssm_steps(const sk_ssm_params& p, cudaStream_t st);
 bool ssm_chunks_applicable(const sk_ssm_params& p);
 size_t ssm_chunks_workspace(const sk_ssm_params& p);
 int launch_ssm_chunks(const sk_ssm_params& p, cudaStream_t st);
+bool ssm_tc_applicable(const sk_ssm_params& p);
+size_t ssm_tc_workspace(const sk_ssm_params& p);
+int launch_ssm_tc(const sk_ssm_params& p, cudaStream_t st);
 int launch_gated_group_norm(const void* y, const void* z, int64_t z_ld, const void* w, int dtype, int64_t rows,
                             int inner, int parts, float eps, void* out, cudaStream_t st);
 bool mlstm_chunks_applicable(const sk_mlstm_params& p);

@@ -1,5 +1,6 @@
 // Linear recurrences with a scalar decay per head and token, over a prompt portion, as matrix products per block of
-// 64 tokens (bf16 inputs): the state-space mixer and the matrix memory.  In both, with weights W that depend on the
+// 64 tokens (bf16 inputs): the state-space mixer and the matrix memory, for short portions (longer ones: ssm_tc.cu and
+// mlstm_tc.cu) and for shapes outside the tensor-core forms.  In both, with weights W that depend on the
 // head's gates only,
 //   y_t   = W_in(t) q_t^T S_in + sum_{s <= t} (q_t . k_s) W(t, s) v_s        S_out = W_in(end) S_in + sum_s W(end, s) k_s v_s^T
 // State space (k = B, q = C, v = x; cum_t the running sum of the log decays inside a block):

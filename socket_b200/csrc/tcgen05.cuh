@@ -13,6 +13,7 @@ __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)
 
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
     const uint32_t addr = smem_addr(bar);
+#pragma unroll 1
     for (uint32_t it = 0; it < TC_WAIT_LIMIT; ++it) {
         uint32_t done;
         asm volatile(
@@ -25,6 +26,19 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
         if (done) return true;
     }
     return false;
+}
+
+// one look at the barrier, the same answer for the whole (converged) warp
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    return __all_sync(FULL, done != 0) != 0;
 }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* bar) {
@@ -158,6 +172,13 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
         "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
         ::"r"(smem_addr(dst)), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_addr(bar))
         : "memory");
+}
+
+// untiled copy; both addresses and the size are multiples of 16 bytes
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_addr(dst)), "l"(src), "r"(bytes), "r"(smem_addr(bar))
+                 : "memory");
 }
 
 // Operand whose K index runs over the rows of 128 bytes (64 elements of the other index each), 128-byte
