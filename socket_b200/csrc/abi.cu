@@ -24,6 +24,10 @@ static int64_t list_len_host(int64_t T, int sink, int window, int64_t M) {
 
 using namespace sk;
 
+// Rows from which a cache append of 16-bit keys goes to the tensor cores: one persistent tile against one fp64 block per four
+// rows (256 rows 14 us both, bound by the call; 512 rows 15 and 21; 1024 rows 15 and 36).
+constexpr int64_t KV_TC_ROWS = 512;
+
 extern "C" {
 
 int sk_abi_version(void) { return SK_ABI_VERSION; }
@@ -57,6 +61,10 @@ int sk_kv_append(const void* k_new, const void* v_new, int kv_dtype, const int64
                "sk_kv_append: null pointer");
     SK_REQUIRE(valid_dtype(kv_dtype) && valid_dtype(plane_dtype), "sk_kv_append: bad dtype");
     SK_REQUIRE(P <= 8, "sk_kv_append: the cache stores uint8 codes, P must be <= 8 (got %d)", P);
+    const int64_t N = (int64_t)B * S * Hkv;
+    if (N >= KV_TC_ROWS && kv_append_tc_applicable(k_new, v_new, kv_dtype, planes, plane_dtype, k_cache, v_cache, codes, N, D, L, P))
+        return launch_kv_append_tc(k_new, v_new, kv_dtype, input_pos, planes, k_cache, v_cache, codes, v_norm, prefill_len, status, B,
+                                   S, Hkv, Tcap, (cudaStream_t)stream);
     return launch_kv_append(k_new, v_new, kv_dtype, input_pos, planes, plane_dtype, k_cache, v_cache,
                             codes, v_norm, prefill_len, status, B, S, Hkv, D, Tcap, L, P,
                             (cudaStream_t)stream);
@@ -79,8 +87,8 @@ int sk_hash_keys_tc(const void* keys, int64_t key_row_stride, const void* planes
     SK_ALIGNED(workspace, 256, "sk_hash_keys_tc: workspace");
     if (key_row_stride % 8 || code_row_stride % 16)
         return fail(SK_ERR_MISALIGNED, "sk_hash_keys_tc: key rows and code rows must start on 16-byte boundaries");
-    return launch_hash_keys_tc(keys, key_row_stride, planes, N, codes, code_row_stride, dst_row, workspace,
-                               workspace_bytes, status, (cudaStream_t)stream);
+    return launch_hash_keys_tc(keys, key_row_stride, planes, N, codes, code_row_stride, dst_row, workspace_bytes, status,
+                               (cudaStream_t)stream);
 }
 
 size_t sk_kv_append_tc_workspace_bytes(int B, int S, int Hkv) {
@@ -104,17 +112,10 @@ int sk_kv_append_tc(const void* k_new, const void* v_new, int kv_dtype, const in
     SK_ALIGNED(codes, 16, "sk_kv_append_tc: codes");
     if (workspace_bytes < sk_kv_append_tc_workspace_bytes(B, S, Hkv))
         return fail(SK_ERR_WORKSPACE, "sk_kv_append_tc: workspace too small");
-    cudaStream_t st = (cudaStream_t)stream;
-    const int64_t N = (int64_t)B * S * Hkv;
-    char* ws = static_cast<char*>(workspace);
-    int64_t* dst_row = reinterpret_cast<int64_t*>(ws);
-    const size_t off = up256((size_t)N * sizeof(int64_t));
-    int rc = launch_cache_rows(input_pos, B, S, Hkv, Tcap, dst_row, status, st);
-    if (rc != SK_OK) return rc;
-    rc = launch_kv_copy(k_new, v_new, kv_dtype, input_pos, k_cache, v_cache, v_norm, prefill_len, nullptr, B, S,
-                        Hkv, D, Tcap, st);
-    if (rc != SK_OK) return rc;
-    return launch_hash_keys_tc(k_new, D, planes, N, codes, L, dst_row, ws + off, workspace_bytes - off, status, st);
+    if ((((uintptr_t)v_new | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) != 0)
+        return fail(SK_ERR_MISALIGNED, "kv copy: K/V pointers must be 16-byte aligned");
+    return launch_kv_append_tc(k_new, v_new, kv_dtype, input_pos, planes, k_cache, v_cache, codes, v_norm, prefill_len, status, B, S,
+                               Hkv, Tcap, (cudaStream_t)stream);
 }
 
 int sk_rope_split(const void* qkv, int dtype, const void* freqs_cis, int freq_dtype, const int64_t* input_pos,

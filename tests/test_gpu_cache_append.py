@@ -1,0 +1,84 @@
+"""Cache appends of 16-bit rows in one tensor-core launch, against the exact fp64 kernel (which fp32 planes of the same values
+select): the same cache rows, codes, norms and length, bit for bit."""
+import pytest
+import torch
+
+from socket_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _cache(B, Hkv, T, dtype):
+    z = lambda *s, dt=dtype: torch.full(s, 7, dtype=dt, device=DEV)  # noqa: E731
+    return [z(B, Hkv, T, 128), z(B, Hkv, T, 128), z(B, Hkv, T, 32, dt=torch.uint8), z(B, Hkv, T, dt=torch.float16),
+            torch.zeros((), dtype=torch.int32, device=DEV)]
+
+
+def _both(B, S, Hkv, T, pos, k, v, planes):
+    got, want = _cache(B, Hkv, T, k.dtype), _cache(B, Hkv, T, k.dtype)
+    flags = [torch.zeros((), dtype=torch.int32, device=DEV) for _ in range(2)]
+    ops.kv_append(*got, pos, k, v, planes, status=flags[0])
+    ops.kv_append(*want, pos, k, v, planes.float(), status=flags[1])
+    for name, g, w in zip(("keys", "values", "codes", "norms", "length"), got, want):
+        assert torch.equal(g.view(torch.uint8) if g.dim() else g, w.view(torch.uint8) if w.dim() else w), name
+    assert int(flags[0]) == int(flags[1])
+    return got, int(flags[0])
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,S,Hkv,start", [(1, 1024, 1, 0), (1, 1025, 1, 3), (3, 347, 1, 0), (2, 257, 5, 100), (1, 8192, 8, 0),
+                                           (4, 1999, 8, 1)])
+def test_append_on_tensor_cores_equals_the_exact_kernel(B, S, Hkv, start, dtype):
+    g = torch.Generator(device=DEV).manual_seed(B * S + Hkv)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    k, v = (r(B, S, Hkv, 128) * torch.exp(r(128))).to(dtype), r(B, S, Hkv, 128).to(dtype)
+    pos = start + torch.randperm(S, generator=g, device=DEV)
+    _both(B, S, Hkv, start + S + 5, pos, k, v, r(32, 8, 128).to(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_append_of_hostile_rows_is_exact(dtype):
+    """Rows of zeros, orthogonal to planes, tiny, huge, infinite and NaN; planes of zeros and tiny ones; positions outside the
+    cache."""
+    g = torch.Generator(device=DEV).manual_seed(3)
+    S = 1300
+    planes = torch.randn(32, 8, 128, generator=g, device=DEV).to(dtype)
+    k = torch.randn(1, S, 1, 128, generator=g, device=DEV).to(dtype)
+    v = torch.randn(1, S, 1, 128, generator=g, device=DEV).to(dtype)
+    planes[0, 0] = 0
+    planes[1, 1] *= 1e-3
+    planes[5, :, 64:] = 0
+    k[0, 5] = 0
+    k[0, 6] = 0
+    k[0, 6, 0, 0], k[0, 6, 0, 1] = planes[3, 2, 1], -planes[3, 2, 0]
+    k[0, 200:600, :, :64] = 0                                # orthogonal to a whole table
+    k[0, 600:620] *= 1e-4 if dtype == torch.float16 else 1e-25
+    k[0, 620:640] *= 6e4 if dtype == torch.float16 else 1e37
+    k[0, 640, 0, 3] = float("inf")
+    k[0, 641, 0, 3] = float("-inf")
+    k[0, 642, 0, 3] = float("nan")
+    k[0, 643, 0, 3], k[0, 643, 0, 4] = float("inf"), float("inf")
+    pos = torch.arange(S, device=DEV)
+    pos[7], pos[9] = -1, S + 100
+    _, flags = _both(1, S, 1, S + 2, pos, k, v, planes)
+    assert flags != 0
+    if dtype == torch.bfloat16:                              # planes whose squares vanish in fp32
+        _both(1, S, 1, S + 2, torch.arange(S, device=DEV), k, v, (planes.float() * 1e-25).to(dtype))
+
+
+def test_append_where_every_projection_is_near_zero():
+    S, planes = 4000, torch.randn(32, 8, 128, device=DEV).bfloat16()
+    planes[:, :, 64:] = 0
+    k = torch.zeros(1, S, 1, 128, device=DEV)
+    k[..., 64:] = torch.randn(1, S, 1, 64, device=DEV)
+    (_, _, codes, _, _), _ = _both(1, S, 1, S, torch.arange(S, device=DEV), k.bfloat16(), k.bfloat16(), planes)
+    assert (codes[:, :, :S] == 255).all()
+
+
+def test_rows_that_do_not_start_on_16_bytes_take_the_general_kernel():
+    S = 1500
+    planes = torch.randn(32, 8, 128, device=DEV).half()
+    raw = torch.randn(2, S * 128 + 1, device=DEV).half()
+    k, v = (t[1:].view(1, S, 1, 128) for t in raw)
+    _both(1, S, 1, S, torch.arange(S, device=DEV), k, v, planes)
