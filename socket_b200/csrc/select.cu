@@ -34,20 +34,25 @@ constexpr int SEL_CHUNK1 = SEL_THREADS * SEL_EPT1;
 constexpr int SEL_SAMPLES = 8192;
 
 struct SelShared {
-    uint32_t hist[SEL_BINS];
+    __align__(16) uint32_t hist[SEL_BINS];
     uint32_t cand_key[SEL_CAP];
     int32_t cand_idx[SEL_CAP];
-    int scan_buf[2][40];
+    int scan_buf[2][SEL_WARPS];
     uint32_t red_lo[SEL_WARPS], red_hi[SEL_WARPS], red_x[SEL_WARPS];
+    uint32_t cut_key;
     int thr_bin, thr_above, thr_inbin;
 };
 
+// One CTA per row leaves most of the chip idle at a few rows, and a CTA of 32 warps is bound by its instructions (62 % of the
+// issue slots taken), so what every warp executes is kept short: one barrier per scan, 16-byte shared-memory accesses, and
+// the paths of degenerate rows out of line (the instruction cache holds what is left).
 struct Scan {
     int parity = 0;
     // exclusive prefix of v over the block in thread order; total returned through `total`
     __device__ __forceinline__ int excl(int v, int& total, SelShared& s) {
+        static_assert(SEL_WARPS == 32, "a warp looks at every warp's sum");
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        int* buf = s.scan_buf[parity];
+        int* buf = s.scan_buf[parity];                 // two in turn: the scan after next is behind a barrier
         parity ^= 1;
         int inc = v;
 #pragma unroll
@@ -57,20 +62,9 @@ struct Scan {
         }
         if (lane == 31) buf[warp] = inc;
         __syncthreads();
-        if (warp == 0) {
-            const int w = buf[lane];
-            int winc = w;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int n = __shfl_up_sync(FULL, winc, o);
-                if (lane >= o) winc += n;
-            }
-            buf[lane] = winc - w;
-            if (lane == 31) buf[32] = winc;
-        }
-        __syncthreads();
-        total = buf[32];
-        return buf[warp] + inc - v;
+        const int w = buf[lane];
+        total = __reduce_add_sync(FULL, w);
+        return __reduce_add_sync(FULL, lane < warp ? w : 0) + inc - v;
     }
 };
 
@@ -88,66 +82,38 @@ __device__ __forceinline__ float key_to_float(uint32_t key) {
     return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
 }
 
-// Block-wide min / max of one uint32 per thread; every thread gets the result.
+// Block-wide min / max of one uint32 per thread; every thread gets the result.  One barrier, after the values were
+// written: a caller has another one before red_lo / red_hi are used again.
 __device__ __forceinline__ void block_minmax(SelShared& s, uint32_t& lo, uint32_t& hi) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(FULL, lo, o));
-        hi = max(hi, __shfl_xor_sync(FULL, hi, o));
-    }
+    lo = __reduce_min_sync(FULL, lo);
+    hi = __reduce_max_sync(FULL, hi);
     if (lane == 0) {
         s.red_lo[warp] = lo;
         s.red_hi[warp] = hi;
     }
     __syncthreads();
-    lo = s.red_lo[lane];
-    hi = s.red_hi[lane];
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(FULL, lo, o));
-        hi = max(hi, __shfl_xor_sync(FULL, hi, o));
-    }
-    __syncthreads();                                   // red_lo / red_hi may be reused
+    lo = __reduce_min_sync(FULL, s.red_lo[lane]);
+    hi = __reduce_max_sync(FULL, s.red_hi[lane]);
 }
 
 // Same with a second minimum riding along.
 __device__ __forceinline__ void block_minmax3(SelShared& s, uint32_t& lo, uint32_t& hi, uint32_t& lo2) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(FULL, lo, o));
-        hi = max(hi, __shfl_xor_sync(FULL, hi, o));
-        lo2 = min(lo2, __shfl_xor_sync(FULL, lo2, o));
-    }
-    if (lane == 0) {
-        s.red_lo[warp] = lo;
-        s.red_hi[warp] = hi;
-        s.red_x[warp] = lo2;
-    }
-    __syncthreads();
-    lo = s.red_lo[lane];
-    hi = s.red_hi[lane];
-    lo2 = s.red_x[lane];
-#pragma unroll
-    for (int o = 16; o >= 1; o >>= 1) {
-        lo = min(lo, __shfl_xor_sync(FULL, lo, o));
-        hi = max(hi, __shfl_xor_sync(FULL, hi, o));
-        lo2 = min(lo2, __shfl_xor_sync(FULL, lo2, o));
-    }
-    __syncthreads();
+    lo2 = __reduce_min_sync(FULL, lo2);
+    if (lane == 0) s.red_x[warp] = lo2;
+    block_minmax(s, lo, hi);
+    lo2 = __reduce_min_sync(FULL, s.red_x[lane]);
 }
 
 // Over hist[0..SEL_BINS): the bin b with  #(bins > b) < target <= #(bins >= b)  (target >= 1,
 // total count >= target).  All threads take part (4 bins each, descending); result in shared
 // memory, valid after the trailing barrier.
 __device__ __forceinline__ void find_bin_desc(SelShared& s, Scan& scan, int target) {
-    int c[4], local = 0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        c[j] = (int)s.hist[SEL_BINS - 1 - (4 * threadIdx.x + j)];
-        local += c[j];
-    }
+    static_assert(SEL_BINS == 4 * SEL_THREADS, "four bins per thread");
+    const uint4 bins = *reinterpret_cast<const uint4*>(&s.hist[SEL_BINS - 4 - 4 * threadIdx.x]);
+    const int c[4] = {(int)bins.w, (int)bins.z, (int)bins.y, (int)bins.x};
+    const int local = c[0] + c[1] + c[2] + c[3];
     int total;
     int before = scan.excl(local, total, s);
 #pragma unroll
@@ -162,11 +128,23 @@ __device__ __forceinline__ void find_bin_desc(SelShared& s, Scan& scan, int targ
     __syncthreads();
 }
 
+// Histogram increment of a lane's bin.  Distinct bins cost an atomic each; a warp whose lanes all hit the same one adds once.
+__device__ __forceinline__ void hist_add(uint32_t* hist, uint32_t bin, bool active) {
+    const unsigned live = __ballot_sync(FULL, active);
+    const uint32_t first = __shfl_sync(FULL, bin, 0);
+    if (__all_sync(FULL, !active || bin == first)) {
+        if ((threadIdx.x & 31) == 0 && live != 0) atomicAdd(&hist[first], (uint32_t)__popc(live));
+    } else if (active) {
+        atomicAdd(&hist[bin], 1u);
+    }
+}
+
 // k-th largest (k >= 1) of keys[0..n) in shared memory, n >= k.  Returns the key; `quota` =
 // how many elements equal to it belong to the top k.  Radix select on (key - min) with up to
 // 12 bits per pass, so score keys that span a few octaves need two passes.
 __device__ __forceinline__ uint32_t smem_kth(SelShared& s, Scan& scan, const uint32_t* keys, int n,
                                              uint32_t k, uint32_t& quota) {
+    __syncthreads();
     uint32_t kmin = 0xffffffffu, kmax = 0u;
     for (int i = threadIdx.x; i < n; i += SEL_THREADS) {
         const uint32_t key = keys[i];
@@ -227,9 +205,11 @@ __device__ __forceinline__ void load_scores(const float* __restrict__ sc, int t0
 
 // Exact top-`need` of the n_cand candidates in shared memory (index order) -> heavy[out_pos..),
 // ties at the cut resolved towards the front (= the smallest indices).  Returns the k-th key.
-__device__ __forceinline__ uint32_t emit_from_candidates(SelShared& s, Scan& scan, int n_cand, int need,
-                                                         int out_pos, int Me, int32_t* __restrict__ heavy) {
+// The way of last resort, out of line; begins and ends with a barrier.
+__device__ __noinline__ uint32_t emit_from_candidates(SelShared& s, int n_cand, int need, int out_pos, int Me,
+                                                      int32_t* __restrict__ heavy) {
     const int tid = threadIdx.x;
+    Scan scan;
     uint32_t quota;
     const uint32_t kth = smem_kth(s, scan, s.cand_key, n_cand, (uint32_t)need, quota);
     int gt_base = 0, eq_base = 0;
@@ -252,57 +232,74 @@ __device__ __forceinline__ uint32_t emit_from_candidates(SelShared& s, Scan& sca
         gt_base += total & 0xffff;
         eq_base += total >> 16;
     }
+    __syncthreads();
     return kth;
 }
 
 // Same job as emit_from_candidates with fewer block-wide phases, for the common case of a few
 // thousand candidates: one 4096-bin histogram of (key - kmin) finds the bin holding the need-th
 // largest key; everything in higher bins is emitted by one ordered scan (consecutive candidates
-// per thread), and the handful of candidates inside that bin are ranked against each other
-// directly.  hist must be zero on entry.  Returns false (nothing written) if the threshold bin
-// holds more than 1024 candidates; the caller then uses the radix path.
-__device__ __forceinline__ bool emit_candidates_binned(SelShared& s, Scan& scan, int n, int need, int Me,
+// per thread, four to a load), and the handful of candidates inside that bin are ranked against each other
+// directly.  kmin and kmax bound the finite keys; what lies below kmin (-infinity) counts as bin 0.  hist must be
+// zero on entry, with a barrier behind the zeros and the candidates.  Returns false (nothing usable written) if the
+// threshold bin holds more than 1024 candidates; the caller then uses the radix path.
+__device__ __forceinline__ bool emit_candidates_binned(SelShared& s, Scan& scan, int n, int need, int out_pos, int Me,
                                                        uint32_t kmin, uint32_t kmax,
                                                        int32_t* __restrict__ heavy, uint32_t& kth_out) {
     const int tid = threadIdx.x;
-    const uint32_t range = kmax - kmin;
+    const uint32_t range = kmax > kmin ? kmax - kmin : 0u;
     const int bits = range == 0 ? 0 : 32 - __clz(range);
     const int shift = max(0, bits - 12);
+#pragma unroll 2
     for (int base = 0; base < n; base += SEL_THREADS) {
         const int i = base + tid;
         const uint32_t k = i < n ? s.cand_key[i] : kmin;
-        warp_hist_add(s.hist, (k - kmin) >> shift, i < n);
+        hist_add(s.hist, k > kmin ? min((k - kmin) >> shift, (uint32_t)(SEL_BINS - 1)) : 0u, i < n);
     }
     __syncthreads();
     find_bin_desc(s, scan, need);
     const int thr = s.thr_bin, above = s.thr_above, inbin = s.thr_inbin;
     if (inbin > 1024) return false;
-    __syncthreads();                                   // hist is reused for the tie list below
-    uint32_t* tie_key = s.hist;                        // [1024]
+    // edges of the threshold bin; the last bin has no upper one
+    const uint32_t lower = thr == 0 ? 0u : kmin + ((uint32_t)thr << shift);
+    const uint64_t upper64 = (uint64_t)kmin + (((uint64_t)thr + 1u) << shift) - 1u;
+    const uint32_t upper = thr == SEL_BINS - 1 || upper64 > 0xffffffffu ? 0xffffffffu : (uint32_t)upper64;
+    uint32_t* tie_key = s.hist;                        // [1024]; the bins have been read before the barrier in find_bin_desc
     int32_t* tie_idx = reinterpret_cast<int32_t*>(s.hist + 1024);
-    const int ept = (n + SEL_THREADS - 1) / SEL_THREADS;
-    const int i0 = tid * ept, i1 = min(n, i0 + ept);
-    int n_gt = 0, n_eq = 0;
-    for (int i = i0; i < i1; ++i) {
-        const int b = (int)((s.cand_key[i] - kmin) >> shift);
-        n_gt += b > thr;
-        n_eq += b == thr;
+    const int nq = (n + 4 * SEL_THREADS - 1) / (4 * SEL_THREADS), q0 = tid * nq;      // groups of four candidates; 16 at most
+    uint32_t gt = 0, eq = 0;                           // one bit per candidate of this thread
+#pragma unroll 1
+    for (int q = 0; q < nq; ++q) {
+        const int i = (q0 + q) * 4;
+        if (i >= n) break;
+        const uint4 k = reinterpret_cast<const uint4*>(s.cand_key)[q0 + q];
+        const uint32_t key[4] = {k.x, k.y, k.z, k.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (i + e < n && key[e] >= lower) {
+                if (key[e] > upper) gt |= 1u << (4 * q + e);
+                else eq |= 1u << (4 * q + e);
+            }
+        }
     }
     int total;
-    const int off = scan.excl(n_gt | (n_eq << 16), total, s);
-    int g = off & 0xffff, e = off >> 16;
-    for (int i = i0; i < i1; ++i) {
-        const uint32_t k = s.cand_key[i];
-        const int b = (int)((k - kmin) >> shift);
-        if (b > thr) {
-            if (g < Me) heavy[g] = s.cand_idx[i];
-            ++g;
-        } else if (b == thr) {
-            if (e < 1024) {
-                tie_key[e] = k;
-                tie_idx[e] = s.cand_idx[i];
+    const int off = scan.excl(__popc(gt) | (__popc(eq) << 16), total, s);
+    int g = out_pos + (off & 0xffff), e = off >> 16;
+#pragma unroll 1
+    for (int q = 0; q < nq; ++q, gt >>= 4, eq >>= 4) {
+        if (((gt | eq) & 15u) == 0u) continue;
+        const int4 ix = reinterpret_cast<const int4*>(s.cand_idx)[q0 + q];
+        const int32_t idx[4] = {ix.x, ix.y, ix.z, ix.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (gt >> c & 1u) {
+                if (g < Me) heavy[g] = idx[c];
+                ++g;
+            } else if (eq >> c & 1u) {
+                tie_key[e] = s.cand_key[(q0 + q) * 4 + c];
+                tie_idx[e] = idx[c];
+                ++e;
             }
-            ++e;
         }
     }
     __syncthreads();
@@ -310,11 +307,12 @@ __device__ __forceinline__ bool emit_candidates_binned(SelShared& s, Scan& scan,
     if (tid < inbin) {
         const uint32_t k = tie_key[tid];
         int rank = 0;
+#pragma unroll 4
         for (int j = 0; j < inbin; ++j) {
             const uint32_t kj = tie_key[j];
             rank += (kj > k) || (kj == k && j < tid);
         }
-        if (rank < want && above + rank < Me) heavy[above + rank] = tie_idx[tid];
+        if (rank < want && out_pos + above + rank < Me) heavy[out_pos + above + rank] = tie_idx[tid];
         if (rank == want - 1) s.red_lo[0] = k;
     }
     __syncthreads();
@@ -322,27 +320,212 @@ __device__ __forceinline__ bool emit_candidates_binned(SelShared& s, Scan& scan,
     return true;
 }
 
+// The candidates on chip -> heavy: range of their finite keys, then the binned emission, else the radix one.  Ends with a barrier.
+__device__ __forceinline__ void emit_candidates(SelShared& s, Scan& scan, int n, int need, int out_pos, int Me, uint32_t kmin,
+                                                uint32_t kmax, int32_t* __restrict__ heavy) {
+    block_minmax(s, kmin, kmax);
+    uint32_t kth;
+    if (!emit_candidates_binned(s, scan, n, need, out_pos, Me, kmin, kmax, heavy, kth))
+        emit_from_candidates(s, n, need, out_pos, Me, heavy);
+}
+constexpr uint32_t KEY_MINUS_INF = 0x007fffffu;        // order_key(-infinity)
+
+// Rows whose sample gave no usable cut: histogram of the whole row, the threshold bin kept on chip.  False if that bin does not
+// fit.  Out of line; begins and ends with a barrier.
+__device__ __noinline__ bool select_row_two_pass(SelShared& s, const float* __restrict__ sc, int T, int Me, int32_t* __restrict__ heavy) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool vec = (reinterpret_cast<uintptr_t>(sc) & 15u) == 0;
+    Scan scan;
+    __syncthreads();
+    // ---- two-pass path: sampled range, histogram, threshold bin
+    uint32_t kmin = 0xffffffffu, kmax = 0u;
+    const int sstride = T / (SEL_THREADS * 4);
+    for (int j = 0; j < 4; ++j) {
+        const float f = sc[(size_t)(tid * 4 + j) * sstride];
+        if (f > -INFINITY && f < INFINITY) {
+            const uint32_t k = order_key(f);
+            kmin = min(kmin, k);
+            kmax = max(kmax, k);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        kmin = min(kmin, __shfl_xor_sync(FULL, kmin, o));
+        kmax = max(kmax, __shfl_xor_sync(FULL, kmax, o));
+    }
+    if (lane == 0) {
+        s.red_lo[warp] = kmin;
+        s.red_hi[warp] = kmax;
+    }
+    for (int i = tid; i < SEL_BINS; i += SEL_THREADS) s.hist[i] = 0;
+    __syncthreads();
+    kmin = s.red_lo[lane];
+    kmax = s.red_hi[lane];
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        kmin = min(kmin, __shfl_xor_sync(FULL, kmin, o));
+        kmax = max(kmax, __shfl_xor_sync(FULL, kmax, o));
+    }
+    BinMap bin;
+    if (kmin > kmax) {  // no finite sample
+        bin.lo = 0;
+        bin.shift = 20;
+    } else {
+        const uint32_t range = kmax - kmin;
+        const int bits = 32 - __clz(range | 1u);
+        bin.lo = kmin;
+        bin.shift = max(0, bits - 11);
+    }
+    // pass 1: histogram; two independent groups per thread keep 4 x 16 B in flight
+    for (int base = 0; base < T; base += 2 * SEL_CHUNK) {
+        float fa[SEL_EPT], fb[SEL_EPT];
+        const int ta = base + tid * SEL_EPT, tb = ta + SEL_CHUNK;
+        load_scores<SEL_EPT>(sc, ta, T, vec, fa);
+        load_scores<SEL_EPT>(sc, tb, T, vec, fb);
+#pragma unroll
+        for (int j = 0; j < SEL_EPT; ++j)
+            warp_hist_add(s.hist, (uint32_t)bin(order_key(fa[j])), ta + j < T);
+#pragma unroll
+        for (int j = 0; j < SEL_EPT; ++j)
+            warp_hist_add(s.hist, (uint32_t)bin(order_key(fb[j])), tb + j < T);
+    }
+    __syncthreads();
+    find_bin_desc(s, scan, Me);
+    const int thr = s.thr_bin;
+    const int above = s.thr_above;
+    const int inbin = s.thr_inbin;
+    if (inbin > SEL_CAP) {
+        return false;
+    } else {
+        // pass 2: emit the sure ones, keep the threshold bin on chip (index order)
+        int sure_base = 0, cand_base = 0;
+        float cur[SEL_EPT], nxt[SEL_EPT];
+        load_scores<SEL_EPT>(sc, tid * SEL_EPT, T, vec, cur);
+        for (int base = 0; base < T; base += SEL_CHUNK) {
+            const int t0 = base + tid * SEL_EPT;
+            if (base + SEL_CHUNK < T) load_scores<SEL_EPT>(sc, t0 + SEL_CHUNK, T, vec, nxt);
+            uint32_t k[SEL_EPT];
+            int cls[SEL_EPT];  // 2 = sure, 1 = candidate
+            int n_sure = 0, n_cnd = 0;
+#pragma unroll
+            for (int j = 0; j < SEL_EPT; ++j) {
+                cls[j] = 0;
+                k[j] = order_key(cur[j]);
+                if (t0 + j < T) {
+                    const int b = bin(k[j]);
+                    cls[j] = b > thr ? 2 : (b == thr ? 1 : 0);
+                    n_sure += cls[j] == 2;
+                    n_cnd += cls[j] == 1;
+                }
+            }
+            int total;
+            const int off = scan.excl(n_sure | (n_cnd << 16), total, s);
+            int so = sure_base + (off & 0xffff), co = cand_base + (off >> 16);
+#pragma unroll
+            for (int j = 0; j < SEL_EPT; ++j) {
+                // bounds hold by construction; the guards keep a row whose scores
+                // change under the kernel from writing outside its buffers
+                if (cls[j] == 2) {
+                    if (so < Me) heavy[so] = t0 + j;
+                    ++so;
+                } else if (cls[j] == 1) {
+                    if (co < SEL_CAP) {
+                        s.cand_key[co] = k[j];
+                        s.cand_idx[co] = t0 + j;
+                    }
+                    ++co;
+                }
+            }
+            sure_base += total & 0xffff;
+            cand_base += total >> 16;
+#pragma unroll
+            for (int j = 0; j < SEL_EPT; ++j) cur[j] = nxt[j];
+        }
+        __syncthreads();
+        emit_from_candidates(s, inbin, Me - above, above, Me, heavy);
+        return true;
+    }
+}
+
+// Rows whose threshold bin overflows the chip (all scores equal): radix select over global memory.  The same conventions.
+__device__ __noinline__ void select_row_global(SelShared& s, const float* __restrict__ sc, int T, int Me, int32_t* __restrict__ heavy) {
+    const int tid = threadIdx.x;
+    Scan scan;
+    __syncthreads();
+    // ---- fallback: radix select over the whole row in global memory
+    uint32_t prefix = 0, mask = 0, remaining = (uint32_t)Me;
+    for (int shift = 24; shift >= 0; shift -= 8) {
+        for (int i = tid; i < SEL_BINS; i += SEL_THREADS) s.hist[i] = 0;
+        __syncthreads();
+        for (int base = 0; base < T; base += SEL_THREADS) {
+            const int t = base + tid;
+            const uint32_t k = t < T ? order_key(sc[t]) : 0u;
+            warp_hist_add_match(s.hist, (k >> shift) & 0xffu, t < T && (k & mask) == prefix);
+        }
+        __syncthreads();
+        find_bin_desc(s, scan, (int)remaining);
+        remaining -= (uint32_t)s.thr_above;
+        prefix |= (uint32_t)s.thr_bin << shift;
+        mask |= 0xffu << shift;
+        __syncthreads();
+    }
+    int gt_base = 0, eq_base = 0;
+    for (int base = 0; base < T; base += SEL_CHUNK) {
+        const int t0 = base + tid * SEL_EPT;
+        int gt[SEL_EPT], eq[SEL_EPT], n_gt = 0, n_eq = 0;
+#pragma unroll
+        for (int j = 0; j < SEL_EPT; ++j) {
+            gt[j] = eq[j] = 0;
+            if (t0 + j < T) {
+                const uint32_t k = order_key(sc[t0 + j]);
+                gt[j] = k > prefix;
+                eq[j] = k == prefix;
+                n_gt += gt[j];
+                n_eq += eq[j];
+            }
+        }
+        int total;
+        const int off = scan.excl(n_gt | (n_eq << 16), total, s);
+        int gt_before = gt_base + (off & 0xffff);
+        int eq_before = eq_base + (off >> 16);
+#pragma unroll
+        for (int j = 0; j < SEL_EPT; ++j) {
+            const int dst = gt_before + min(eq_before, (int)remaining);
+            if ((gt[j] || (eq[j] && eq_before < (int)remaining)) && dst < Me) heavy[dst] = t0 + j;
+            gt_before += gt[j];
+            eq_before += eq[j];
+        }
+        gt_base += total & 0xffff;
+        eq_base += total >> 16;
+    }
+    __syncthreads();
+}
+
 // Top-`Me` (0 < Me) of one row of T scores -> heavy[0..Me).  Exact; see the file header.
 __device__ __forceinline__ void select_row(SelShared& s, Scan& scan, const float* __restrict__ sc, int T,
                                            int Me, int32_t* __restrict__ heavy) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const bool vec = (reinterpret_cast<uintptr_t>(sc) & 15u) == 0;
     if (Me == T) {
         for (int i = tid; i < T; i += SEL_THREADS) heavy[i] = i;
     } else if (Me > 0) {
-        int n_cand = 0;        // candidates in shared memory (index order)
-        int need = Me;         // how many of them to take
-        int out_pos = 0;       // heavy entries already emitted
-        bool have_cand = false, global_fallback = false;
-
+        bool done = false;
+        uint32_t kmin = 0xffffffffu, kmax = 0u;            // finite keys of this thread's candidates
+        auto range = [&](uint32_t k) {
+            if (k > KEY_MINUS_INF) kmin = min(kmin, k);
+            kmax = max(kmax, k);
+        };
         if (T <= SEL_CAP) {
+            reinterpret_cast<uint4*>(s.hist)[tid] = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll 4
             for (int i = tid; i < T; i += SEL_THREADS) {
-                s.cand_key[i] = order_key(sc[i]);
+                const uint32_t k = order_key(sc[i]);
+                s.cand_key[i] = k;
                 s.cand_idx[i] = i;
+                range(k);
             }
-            n_cand = T;
-            have_cand = true;
-            __syncthreads();
+            emit_candidates(s, scan, T, Me, 0, Me, kmin, kmax, heavy);
+            done = true;
         } else {
             // ---- main path: cut from a sample, then one streaming pass
             const int stride = T / SEL_SAMPLES;                     // >= 2
@@ -362,7 +545,7 @@ __device__ __forceinline__ void select_row(SelShared& s, Scan& scan, const float
                         fhi = max(fhi, key);
                     }
                 }
-                for (int i = tid; i < SEL_BINS; i += SEL_THREADS) s.hist[i] = 0;
+                reinterpret_cast<uint4*>(s.hist)[tid] = make_uint4(0u, 0u, 0u, 0u);
                 block_minmax(s, flo, fhi);
                 const float fmin = key_to_float(flo), fmax = key_to_float(fhi);
                 float cut = INFINITY;
@@ -394,8 +577,10 @@ __device__ __forceinline__ void select_row(SelShared& s, Scan& scan, const float
                     for (int j = 0; j < SEL_EPT1; ++j) {
                         if (hit & (1u << j)) {
                             if (pos < SEL_CAP) {
-                                s.cand_key[pos] = order_key(cur[j]);
+                                const uint32_t k = order_key(cur[j]);
+                                s.cand_key[pos] = k;
                                 s.cand_idx[pos] = t0 + j;
+                                range(k);
                             }
                             ++pos;
                         }
@@ -404,176 +589,14 @@ __device__ __forceinline__ void select_row(SelShared& s, Scan& scan, const float
 #pragma unroll
                     for (int j = 0; j < SEL_EPT1; ++j) cur[j] = nxt[j];
                 }
-                __syncthreads();
                 if (base_cnt >= Me && base_cnt <= SEL_CAP) {
-                    n_cand = base_cnt;
-                    have_cand = true;
-                }
-            }
-            if (!have_cand) {
-                // ---- two-pass path: sampled range, histogram, threshold bin
-                uint32_t kmin = 0xffffffffu, kmax = 0u;
-                const int sstride = T / (SEL_THREADS * 4);
-                for (int j = 0; j < 4; ++j) {
-                    const float f = sc[(size_t)(tid * 4 + j) * sstride];
-                    if (f > -INFINITY && f < INFINITY) {
-                        const uint32_t k = order_key(f);
-                        kmin = min(kmin, k);
-                        kmax = max(kmax, k);
-                    }
-                }
-#pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) {
-                    kmin = min(kmin, __shfl_xor_sync(FULL, kmin, o));
-                    kmax = max(kmax, __shfl_xor_sync(FULL, kmax, o));
-                }
-                if (lane == 0) {
-                    s.red_lo[warp] = kmin;
-                    s.red_hi[warp] = kmax;
-                }
-                for (int i = tid; i < SEL_BINS; i += SEL_THREADS) s.hist[i] = 0;
-                __syncthreads();
-                kmin = s.red_lo[lane];
-                kmax = s.red_hi[lane];
-#pragma unroll
-                for (int o = 16; o >= 1; o >>= 1) {
-                    kmin = min(kmin, __shfl_xor_sync(FULL, kmin, o));
-                    kmax = max(kmax, __shfl_xor_sync(FULL, kmax, o));
-                }
-                BinMap bin;
-                if (kmin > kmax) {  // no finite sample
-                    bin.lo = 0;
-                    bin.shift = 20;
-                } else {
-                    const uint32_t range = kmax - kmin;
-                    const int bits = 32 - __clz(range | 1u);
-                    bin.lo = kmin;
-                    bin.shift = max(0, bits - 11);
-                }
-                // pass 1: histogram; two independent groups per thread keep 4 x 16 B in flight
-                for (int base = 0; base < T; base += 2 * SEL_CHUNK) {
-                    float fa[SEL_EPT], fb[SEL_EPT];
-                    const int ta = base + tid * SEL_EPT, tb = ta + SEL_CHUNK;
-                    load_scores<SEL_EPT>(sc, ta, T, vec, fa);
-                    load_scores<SEL_EPT>(sc, tb, T, vec, fb);
-#pragma unroll
-                    for (int j = 0; j < SEL_EPT; ++j)
-                        warp_hist_add(s.hist, (uint32_t)bin(order_key(fa[j])), ta + j < T);
-#pragma unroll
-                    for (int j = 0; j < SEL_EPT; ++j)
-                        warp_hist_add(s.hist, (uint32_t)bin(order_key(fb[j])), tb + j < T);
-                }
-                __syncthreads();
-                find_bin_desc(s, scan, Me);
-                const int thr = s.thr_bin;
-                const int above = s.thr_above;
-                const int inbin = s.thr_inbin;
-                if (inbin > SEL_CAP) {
-                    global_fallback = true;
-                } else {
-                    // pass 2: emit the sure ones, keep the threshold bin on chip (index order)
-                    int sure_base = 0, cand_base = 0;
-                    float cur[SEL_EPT], nxt[SEL_EPT];
-                    load_scores<SEL_EPT>(sc, tid * SEL_EPT, T, vec, cur);
-                    for (int base = 0; base < T; base += SEL_CHUNK) {
-                        const int t0 = base + tid * SEL_EPT;
-                        if (base + SEL_CHUNK < T) load_scores<SEL_EPT>(sc, t0 + SEL_CHUNK, T, vec, nxt);
-                        uint32_t k[SEL_EPT];
-                        int cls[SEL_EPT];  // 2 = sure, 1 = candidate
-                        int n_sure = 0, n_cnd = 0;
-#pragma unroll
-                        for (int j = 0; j < SEL_EPT; ++j) {
-                            cls[j] = 0;
-                            k[j] = order_key(cur[j]);
-                            if (t0 + j < T) {
-                                const int b = bin(k[j]);
-                                cls[j] = b > thr ? 2 : (b == thr ? 1 : 0);
-                                n_sure += cls[j] == 2;
-                                n_cnd += cls[j] == 1;
-                            }
-                        }
-                        int total;
-                        const int off = scan.excl(n_sure | (n_cnd << 16), total, s);
-                        int so = sure_base + (off & 0xffff), co = cand_base + (off >> 16);
-#pragma unroll
-                        for (int j = 0; j < SEL_EPT; ++j) {
-                            // bounds hold by construction; the guards keep a row whose scores
-                            // change under the kernel from writing outside its buffers
-                            if (cls[j] == 2) {
-                                if (so < Me) heavy[so] = t0 + j;
-                                ++so;
-                            } else if (cls[j] == 1) {
-                                if (co < SEL_CAP) {
-                                    s.cand_key[co] = k[j];
-                                    s.cand_idx[co] = t0 + j;
-                                }
-                                ++co;
-                            }
-                        }
-                        sure_base += total & 0xffff;
-                        cand_base += total >> 16;
-#pragma unroll
-                        for (int j = 0; j < SEL_EPT; ++j) cur[j] = nxt[j];
-                    }
-                    out_pos = above;
-                    need = Me - above;
-                    n_cand = inbin;
-                    have_cand = true;
-                    __syncthreads();
+                    reinterpret_cast<uint4*>(s.hist)[tid] = make_uint4(0u, 0u, 0u, 0u);
+                    emit_candidates(s, scan, base_cnt, Me, 0, Me, kmin, kmax, heavy);
+                    done = true;
                 }
             }
         }
-
-        if (have_cand) {
-            emit_from_candidates(s, scan, n_cand, need, out_pos, Me, heavy);
-        } else if (global_fallback) {
-            // ---- fallback: radix select over the whole row in global memory
-            uint32_t prefix = 0, mask = 0, remaining = (uint32_t)Me;
-            for (int shift = 24; shift >= 0; shift -= 8) {
-                for (int i = tid; i < SEL_BINS; i += SEL_THREADS) s.hist[i] = 0;
-                __syncthreads();
-                for (int base = 0; base < T; base += SEL_THREADS) {
-                    const int t = base + tid;
-                    const uint32_t k = t < T ? order_key(sc[t]) : 0u;
-                    warp_hist_add_match(s.hist, (k >> shift) & 0xffu, t < T && (k & mask) == prefix);
-                }
-                __syncthreads();
-                find_bin_desc(s, scan, (int)remaining);
-                remaining -= (uint32_t)s.thr_above;
-                prefix |= (uint32_t)s.thr_bin << shift;
-                mask |= 0xffu << shift;
-                __syncthreads();
-            }
-            int gt_base = 0, eq_base = 0;
-            for (int base = 0; base < T; base += SEL_CHUNK) {
-                const int t0 = base + tid * SEL_EPT;
-                int gt[SEL_EPT], eq[SEL_EPT], n_gt = 0, n_eq = 0;
-#pragma unroll
-                for (int j = 0; j < SEL_EPT; ++j) {
-                    gt[j] = eq[j] = 0;
-                    if (t0 + j < T) {
-                        const uint32_t k = order_key(sc[t0 + j]);
-                        gt[j] = k > prefix;
-                        eq[j] = k == prefix;
-                        n_gt += gt[j];
-                        n_eq += eq[j];
-                    }
-                }
-                int total;
-                const int off = scan.excl(n_gt | (n_eq << 16), total, s);
-                int gt_before = gt_base + (off & 0xffff);
-                int eq_before = eq_base + (off >> 16);
-#pragma unroll
-                for (int j = 0; j < SEL_EPT; ++j) {
-                    const int dst = gt_before + min(eq_before, (int)remaining);
-                    if ((gt[j] || (eq[j] && eq_before < (int)remaining)) && dst < Me) heavy[dst] = t0 + j;
-                    gt_before += gt[j];
-                    eq_before += eq[j];
-                }
-                gt_base += total & 0xffff;
-                eq_base += total >> 16;
-            }
-        }
+        if (!done && !select_row_two_pass(s, sc, T, Me, heavy)) select_row_global(s, sc, T, Me, heavy);
     }
 }
 
@@ -585,7 +608,9 @@ __device__ __forceinline__ int write_base(int32_t* __restrict__ out, int T, int 
     const int win_start = max(T - window, sink);
     const int n_win = window > 0 ? T - win_start : 0;
     int nb = sink + n_win;
+#pragma unroll 1
     for (int i = tid; i < sink; i += SEL_THREADS) out[i] = i;
+#pragma unroll 1
     for (int i = tid; i < n_win; i += SEL_THREADS) out[sink + i] = win_start + i;
     if (nb == 0) {
         if (tid == 0) out[0] = T - 1;
@@ -614,8 +639,9 @@ __device__ __forceinline__ void finish_row(SelShared& s, const float* __restrict
             keys[i] = v;
         }
         __syncthreads();
-        for (int k = 2; k <= n2; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
+        // bitonic, descending: exchanges at distances below 32 stay inside a warp and need no barrier
+        for (int k = 2; k <= n2;) {
+            for (int j = k >> 1; j >= 32; j >>= 1) {
                 for (int i = tid; i < n2; i += SEL_THREADS) {
                     const int p = i ^ j;
                     if (p > i) {
@@ -629,6 +655,20 @@ __device__ __forceinline__ void finish_row(SelShared& s, const float* __restrict
                 }
                 __syncthreads();
             }
+            const int k_first = k;
+            for (int i = tid; i < ((n2 + 31) & ~31); i += SEL_THREADS) {      // whole warps; n2 below 32: lanes above it idle along
+                uint64_t v = i < n2 ? keys[i] : 0;
+                for (int kk = k_first; kk <= max(k_first, min(n2, 32)); kk <<= 1) {
+                    for (int j = min(kk >> 1, 16); j > 0; j >>= 1) {
+                        const uint64_t o = __shfl_xor_sync(FULL, v, j);
+                        const bool keep_large = ((i & kk) == 0) == ((i & j) == 0);
+                        v = keep_large ? (v > o ? v : o) : (v < o ? v : o);
+                    }
+                }
+                if (i < n2) keys[i] = v;
+            }
+            __syncthreads();
+            k = max(k_first, min(n2, 32)) << 1;
         }
         for (int i = tid; i < Me; i += SEL_THREADS)
             heavy[i] = (int32_t)(0xffffffffu - (uint32_t)(keys[i] & 0xffffffffu));
@@ -689,6 +729,7 @@ struct CandArgs {
     int32_t* n_fallback;    // statistics: rows that had to be rescored
     int64_t score_stride;
     int chunks_max, cap_w;
+    bool narrow;            // (groups x Tslots) fits 32 bits
     int64_t Tslots, per_cta;
     // for the rescoring path
     const float* lut;
@@ -767,6 +808,31 @@ __device__ __forceinline__ void exact_scores_like_scorer(const float* tab_s, con
     }
 }
 
+// The best `want` of a large band (band order = index order) -> out.  Out of line; begins with a barrier.
+__device__ __noinline__ void rank_band_radix(SelShared& s, const uint32_t* band_e, const int32_t* band_t, int n, int want,
+                                             int32_t* __restrict__ out) {
+    Scan scan;
+    uint32_t quota;
+    const uint32_t kth = smem_kth(s, scan, band_e, n, (uint32_t)want, quota);
+    const int ept = (n + SEL_THREADS - 1) / SEL_THREADS;
+    const int j0 = threadIdx.x * ept, j1 = min(n, j0 + ept);
+    int n_gt = 0, n_eq = 0;
+    for (int jb = j0; jb < j1; ++jb) {
+        n_gt += band_e[jb] > kth;
+        n_eq += band_e[jb] == kth;
+    }
+    int total;
+    const int off = scan.excl(n_gt | (n_eq << 16), total, s);
+    int gt_before = off & 0xffff, eq_before = off >> 16;
+    for (int jb = j0; jb < j1; ++jb) {
+        const uint32_t e = band_e[jb];
+        const int dst = gt_before + min(eq_before, (int)quota);
+        if ((e > kth || (e == kth && eq_before < (int)quota)) && dst < want) out[dst] = band_t[jb];
+        gt_before += e > kth;
+        eq_before += e == kth;
+    }
+}
+
 // Exact top-Me of a row from its packed candidates (the packed words in cand_key, in index order;
 // kmin / kmax = smallest / largest order key of their up_i; hist zero on entry; s_min = smallest S
 // of the row's candidates).  Returns false, with nothing usable written, when the result cannot be proved or
@@ -791,6 +857,7 @@ __device__ __forceinline__ bool emit_packed_candidates(SelShared& s, Scan& scan,
     const int bits = range == 0 ? 0 : 32 - __clz(range);
     const int shift = max(0, bits - 12);
     auto vn_of = [](uint32_t x) { return __half2float(__ushort_as_half((unsigned short)(x & 0x7fffu))); };
+#pragma unroll 2
     for (int base = 0; base < n; base += SEL_THREADS) {
         const int i = base + tid;
         uint32_t k = kmin;
@@ -798,7 +865,7 @@ __device__ __forceinline__ bool emit_packed_candidates(SelShared& s, Scan& scan,
             const uint32_t x = s.cand_key[i];
             k = order_key(packed_upper_sel(x >> 15, K0 + 33.0f, vn_of(x)));
         }
-        warp_hist_add(s.hist, (k - kmin) >> shift, i < n);
+        hist_add(s.hist, (k - kmin) >> shift, i < n);
     }
     // the row's probabilities [L][R] (32 KiB), requested now, stored to shared memory once the
     // classification below has freed cand_key
@@ -820,22 +887,29 @@ __device__ __forceinline__ bool emit_packed_candidates(SelShared& s, Scan& scan,
         return false;
     }
 
-    // ---- classes: 1 = in, 2 = between the brackets, 0 = out; two bits per candidate of this thread
-    const int ept = (n + SEL_THREADS - 1) / SEL_THREADS;          // <= 16
-    const int i0 = tid * ept, i1 = min(n, i0 + ept);
-    uint32_t cls_bits = 0;
-    int n_sure = 0, n_band = 0;
-    for (int i = i0; i < i1; ++i) {
-        const uint32_t x = s.cand_key[i];
-        const float up = packed_upper_sel(x >> 15, K0 + 33.0f, vn_of(x));
-        const float lo = packed_lower_sel(x >> 15, K0 - 1.0f, vn_of(x));
-        const uint32_t cls = lo > UB ? 1u : (up >= LB ? 2u : 0u);
-        cls_bits |= cls << (2 * (i - i0));
-        n_sure += cls == 1u;
-        n_band += cls == 2u;
+    // ---- in for certain, or between the brackets: a bit each per candidate of this thread, consecutive candidates, four to a load
+    const int nq = (n + 4 * SEL_THREADS - 1) / (4 * SEL_THREADS), q0 = tid * nq;      // 4 at most
+    uint32_t sure = 0, band = 0;
+#pragma unroll 1
+    for (int q = 0; q < nq; ++q) {
+        const int i = (q0 + q) * 4;
+        if (i >= n) break;
+        const uint4 w = reinterpret_cast<const uint4*>(s.cand_key)[q0 + q];
+        const uint32_t word[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t x = word[e];
+            const float vn = vn_of(x);
+            const float up = packed_upper_sel(x >> 15, K0 + 33.0f, vn);
+            const float lo = packed_lower_sel(x >> 15, K0 - 1.0f, vn);
+            if (i + e < n) {
+                if (lo > UB) sure |= 1u << (4 * q + e);
+                else if (up >= LB) band |= 1u << (4 * q + e);
+            }
+        }
     }
     int total;
-    const int off = scan.excl(n_sure | (n_band << 16), total, s);
+    const int off = scan.excl(__popc(sure) | (__popc(band) << 16), total, s);
     const int tot_sure = total & 0xffff, tot_band = total >> 16;
     const int want = Me - tot_sure;
     if (tid == 0) {                                   // statistics: keys rescored, rows ranked by the radix path
@@ -855,13 +929,19 @@ __device__ __forceinline__ bool emit_packed_candidates(SelShared& s, Scan& scan,
         reinterpret_cast<float4*>(tab_s)[u * SEL_THREADS + tid] = tab_r[u];
     {
         int spos = off & 0xffff, bpos = off >> 16;
-        for (int i = i0; i < i1; ++i) {
-            const uint32_t cls = (cls_bits >> (2 * (i - i0))) & 3u;
-            if (cls == 1u) {
-                if (spos < Me) heavy[spos] = s.cand_idx[i];
-                ++spos;
-            } else if (cls == 2u) {
-                band_t[bpos++] = s.cand_idx[i];
+#pragma unroll 1
+        for (int q = 0; q < nq; ++q, sure >>= 4, band >>= 4) {
+            if (((sure | band) & 15u) == 0u) continue;
+            const int4 ix = reinterpret_cast<const int4*>(s.cand_idx)[q0 + q];
+            const int32_t idx[4] = {ix.x, ix.y, ix.z, ix.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                if (sure >> c & 1u) {
+                    if (spos < Me) heavy[spos] = idx[c];
+                    ++spos;
+                } else if (band >> c & 1u) {
+                    band_t[bpos++] = idx[c];
+                }
             }
         }
     }
@@ -889,27 +969,56 @@ __device__ __forceinline__ bool emit_packed_candidates(SelShared& s, Scan& scan,
         cnt += __shfl_xor_sync(FULL, cnt, 2);
         if (kb < tot_band && part == 0 && cnt < want) out[cnt] = band_t[kb];
     } else {
-        uint32_t quota;
-        const uint32_t kth = smem_kth(s, scan, band_e, tot_band, (uint32_t)want, quota);
-        const int ept2 = (tot_band + SEL_THREADS - 1) / SEL_THREADS;
-        const int j0 = tid * ept2, j1 = min(tot_band, j0 + ept2);
-        int n_gt = 0, n_eq = 0;
-        for (int jb = j0; jb < j1; ++jb) {
-            n_gt += band_e[jb] > kth;
-            n_eq += band_e[jb] == kth;
-        }
-        int tot2;
-        const int off2 = scan.excl(n_gt | (n_eq << 16), tot2, s);
-        int gt_before = off2 & 0xffff, eq_before = off2 >> 16;
-        for (int jb = j0; jb < j1; ++jb) {
-            const uint32_t e = band_e[jb];
-            const int dst = gt_before + min(eq_before, (int)quota);
-            if ((e > kth || (e == kth && eq_before < (int)quota)) && dst < want) out[dst] = band_t[jb];
-            gt_before += e > kth;
-            eq_before += e == kth;
-        }
+        rank_band_radix(s, band_e, band_t, tot_band, want, out);
     }
     return true;
+}
+
+// Rescore a row (tables added in the scorer's order), then the full-row select.  Out of line; begins with a barrier.
+__device__ __noinline__ void rescore_row(SelShared& s, const CandArgs& a, int64_t row, int g, int hj, int kv, int T, int Me, int why,
+                                         int32_t* __restrict__ heavy) {
+    const int tid = threadIdx.x;
+    float* sc = a.scratch + row * a.score_stride;
+    if (tid == 0) {
+        atomicAdd(a.n_fallback, 1);
+        atomicAdd(a.n_fallback + why, 1);
+    }
+    __syncthreads();
+    float* tab = reinterpret_cast<float*>(s.cand_key);           // [L][R] of this head
+    if (a.probs != nullptr) {
+        // packed step: the row's probabilities are the table ([L][R], the very values the fp32
+        // scorer table holds), and that table is not written
+        const float* pr = a.probs + (size_t)row * a.L * a.R;
+        for (int i = tid; i < a.L * a.R; i += SEL_THREADS) tab[i] = __ldcg(pr + i);
+    } else {
+        const float* lut_g = a.lut + (size_t)g * a.R * a.L * a.ht;
+        const int j = hj % a.ht;
+        for (int i = tid; i < a.L * a.R; i += SEL_THREADS) {
+            const int l = i / a.R, r = i - l * a.R;
+            tab[i] = __ldcg(lut_g + ((size_t)r * a.L + l) * a.ht + j);
+        }
+    }
+    __syncthreads();
+    const uint8_t* cg = a.codes + (size_t)kv * a.Tcap * a.L;
+    const __half* vg = a.v_norm + (size_t)kv * a.Tcap;
+    for (int t = tid; t < T; t += SEL_THREADS) {
+        const uint4* cp = reinterpret_cast<const uint4*>(cg + (size_t)t * a.L);
+        const int m = t & 7;                   // the scorer's table order for this key
+        float sum = 0.f;
+        for (int v = 0; v < a.L / 16; ++v) {
+            const uint4 w4 = __ldcg(cp + v);
+            const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+#pragma unroll
+            for (int q = 0; q < 16; ++q) {
+                const int tb = (q & 8) | ((q & 7) ^ m);
+                sum += tab[(v * 16 + tb) * a.R + ((w[tb >> 2] >> (8 * (tb & 3))) & 0xffu)];
+            }
+        }
+        sc[t] = sum * __half2float(__ldcg(vg + t));
+    }
+    __syncthreads();
+    Scan scan;
+    select_row(s, scan, sc, T, Me, heavy);
 }
 
 static_assert(SC_TAIL <= SEL_THREADS, "one tail entry per thread in the gather");
@@ -917,23 +1026,29 @@ static_assert(SC_TAIL <= SEL_THREADS, "one tail entry per thread in the gather")
 // PACKED: the candidates are packed (S, ||v||) words (score_packed_kernel), else fp32 scores.
 template <bool PACKED>
 __global__ void __launch_bounds__(SEL_THREADS, 1)
-select_cand_kernel(CandArgs a, int64_t T_host, const int32_t* __restrict__ T_dev, int64_t M,
+select_cand_kernel(const __grid_constant__ CandArgs a, int64_t T_host, const int32_t* __restrict__ T_dev, int64_t M,
                    int sink_in, int window_in, int sorted, int32_t* __restrict__ list,
                    int64_t list_row_stride, int32_t* __restrict__ list_len) {
     extern __shared__ __align__(16) char smem_raw[];
     SelShared& s = *reinterpret_cast<SelShared*>(smem_raw);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t row = blockIdx.x;
+    const int64_t row = blockIdx.x;                   // below 2^31, as the grid
     int32_t* out = list + row * list_row_stride;
 
     // which scorer chunks belong to this row's KV-head group
     const int rep = a.H / a.Hkv, tiles = rep / a.ht;
-    const int b = (int)(row / a.H), h = (int)(row - (int64_t)b * a.H);
+    const int b = (int)((unsigned)row / (unsigned)a.H), h = (int)row - b * a.H;
     const int kvh = h / rep, hj = h - kvh * rep;
     const int g = (b * a.Hkv + kvh) * tiles + hj / a.ht;
-    const int64_t first_cta = ((int64_t)g * a.Tslots) / a.per_cta;
-    const int64_t last_cta = ((int64_t)(g + 1) * a.Tslots - 1) / a.per_cta;
-    const int n_runs = (int)(last_cta - first_cta + 1) * SC_WARPS;      // <= 1024
+    int first_cta, last_cta;
+    if (a.narrow) {                                   // slots of all groups below 2^32: a 64-bit division is some sixty instructions
+        first_cta = (int)((uint32_t)g * (uint32_t)a.Tslots / (uint32_t)a.per_cta);
+        last_cta = (int)(((uint32_t)(g + 1) * (uint32_t)a.Tslots - 1u) / (uint32_t)a.per_cta);
+    } else {
+        first_cta = (int)(((int64_t)g * a.Tslots) / a.per_cta);
+        last_cta = (int)(((int64_t)(g + 1) * a.Tslots - 1) / a.per_cta);
+    }
+    const int n_runs = (last_cta - first_cta + 1) * SC_WARPS;      // <= 1024
     const int32_t* cnt = a.cnt + row * a.chunks_max * SC_WARPS;
     constexpr bool packed = PACKED;
     pdl_launch_dependents();
@@ -973,20 +1088,21 @@ select_cand_kernel(CandArgs a, int64_t T_host, const int32_t* __restrict__ T_dev
 
     bool exact = false;
     if (Me > 0 && Me < T) {
-        // ---- run lengths -> offsets (one run per thread), largest cut, overflow flag
-        if (tid == 0) {
-            s.thr_bin = 0;                             // "some run overflowed"
-            s.red_hi[0] = 0u;                          // key of the largest cut
+        // ---- run lengths -> offsets (one run per thread), largest cut, number of runs that overflowed (in the sum's high bits:
+        // 1024 runs of at most 250 entries stay below 2^18)
+        reinterpret_cast<uint4*>(s.hist)[tid] = make_uint4(0u, 0u, 0u, 0u);
+        const int c = min(c_run, a.cap_w);
+        if (warp == 0) {                               // n_runs / SC_WARPS <= 36 chunks
+            uint32_t ck = order_key(cut_chunk);
+            if (tid + 32 < n_runs / SC_WARPS) ck = max(ck, order_key(__ldcg(a.cut + row * a.chunks_max + tid + 32)));
+            ck = __reduce_max_sync(FULL, ck);
+            if (lane == 0) s.cut_key = ck;
         }
-        for (int i = tid; i < SEL_BINS; i += SEL_THREADS) s.hist[i] = 0;
-        __syncthreads();
-        const int c = c_run;
-        if (c > a.cap_w) s.thr_bin = 1;
-        if (tid < n_runs / SC_WARPS) atomicMax(&s.red_hi[0], order_key(cut_chunk));
         int total;
-        const int off = scan.excl(c, total, s);        // two barriers: the flags above are visible after it
-        const bool any_over = s.thr_bin != 0;
-        const uint32_t chi = s.red_hi[0];
+        const int off = scan.excl(c | (c_run > a.cap_w ? 1 << 20 : 0), total, s) & 0xfffff;
+        const bool any_over = total >> 20 != 0;
+        total &= 0xfffff;
+        const uint32_t chi = s.cut_key;
         // the row's newest keys follow the runs: all of them, in index order (they have the largest indices)
         const int n_tail = min(SC_TAIL, T);
         const int total_runs = total;
@@ -994,7 +1110,7 @@ select_cand_kernel(CandArgs a, int64_t T_host, const int32_t* __restrict__ T_dev
         total += n_tail;
         if (!any_over && total >= Me && total <= SEL_CAP) {
             // ---- gather: G lanes per run (G = the power of two at or above the mean run length, 4 to 32),
-            // four runs per lane group in flight, each with its first 3 G entries: all loads of a pass
+            // four runs per lane group in flight, each with its first 2 G entries: all loads of a pass
             // are independent and nothing searches.  Run r's (offset | length << 16) comes from shared
             // memory: the tail of cand_idx while the candidates leave it free, else the histogram bins.
             const bool tail_free = total <= SEL_CAP - 1024;
@@ -1004,45 +1120,47 @@ select_cand_kernel(CandArgs a, int64_t T_host, const int32_t* __restrict__ T_dev
             __syncthreads();
             const uint2* cand = a.cand + row * a.chunks_max * SC_WARPS * a.cap_w;
             const uint2 e_tail = tid < n_tail ? __ldcg(tail + tid) : make_uint2(0u, 0u);   // SC_TAIL <= SEL_THREADS
-            int G = 4;
-            while (G < 32 && G * n_runs < total_runs) G <<= 1;
-            const int rpw = 32 / G, sub = lane / G, li = lane - sub * G;
+            int G = 4, lg = 2;
+            while (G < 32 && G * n_runs < total_runs) {
+                G <<= 1;
+                ++lg;
+            }
+            const int rpw = 32 >> lg, sub = lane >> lg, li = lane & (G - 1);
             const int step_runs = SEL_WARPS * rpw;
+#pragma unroll 1
             for (int r0 = warp * rpw + sub; r0 < n_runs; r0 += 4 * step_runs) {
-                uint2 e[4][3];
-                int o[4], n[4];
+                uint2 e[4][2];
+                int m[4];
+                bool longer = false;
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const int r = r0 + u * step_runs;
-                    const int m = r < n_runs ? meta[r] : 0;
-                    o[u] = m & 0xffff;
-                    n[u] = m >> 16;
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        const int i = li + G * k;
-                        e[u][k] = make_uint2(0u, 0u);
-                        if (i < n[u]) e[u][k] = __ldcg(cand + (size_t)r * a.cap_w + i);
-                    }
+                    m[u] = r < n_runs ? meta[r] : 0;
+                    const uint2* run = cand + (uint32_t)r * (uint32_t)a.cap_w + li;
+                    const int n = m[u] >> 16;
+                    if (li < n) e[u][0] = __ldcg(run);
+                    if (li + G < n) e[u][1] = __ldcg(run + G);
+                    longer |= n > 2 * G;
                 }
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) {
-                        const int i = li + G * k;
-                        if (i < n[u]) put(o[u] + i, e[u][k], kmin, kmax);
-                    }
+                    const int o = (m[u] & 0xffff) + li, n = m[u] >> 16;
+                    if (li < n) put(o, e[u][0], kmin, kmax);
+                    if (li + G < n) put(o + G, e[u][1], kmin, kmax);
                 }
-#pragma unroll
-                for (int u = 0; u < 4; ++u) {                      // runs longer than 3 G: rare
-                    const int r = r0 + u * step_runs;
-                    for (int i = li + 3 * G; i < n[u]; i += G)
-                        put(o[u] + i, __ldcg(cand + (size_t)r * a.cap_w + i), kmin, kmax);
+                if (longer) {                                      // rare
+#pragma unroll 1
+                    for (int u = 0; u < 4; ++u) {
+                        const int r = r0 + u * step_runs, mm = r < n_runs ? meta[r] : 0;
+                        for (int i = li + 2 * G; i < mm >> 16; i += G)
+                            put((mm & 0xffff) + i, __ldcg(cand + (uint32_t)r * (uint32_t)a.cap_w + i), kmin, kmax);
+                    }
                 }
             }
             if (tid < n_tail) put(total_runs + tid, e_tail, kmin, kmax);
             if (!tail_free) {
                 __syncthreads();
-                for (int i = tid; i < SEL_BINS; i += SEL_THREADS) s.hist[i] = 0;
+                reinterpret_cast<uint4*>(s.hist)[tid] = make_uint4(0u, 0u, 0u, 0u);
             }
             if (packed) block_minmax3(s, kmin, kmax, s_min);
             else block_minmax(s, kmin, kmax);          // also the barrier after the gather
@@ -1053,55 +1171,14 @@ select_cand_kernel(CandArgs a, int64_t T_host, const int32_t* __restrict__ T_dev
                                                a.v_norm + (size_t)(b * a.Hkv + kvh) * a.Tcap, heavy, a.n_fallback);
             } else {
                 uint32_t kth = 0;
-                if (!emit_candidates_binned(s, scan, total, Me, Me, kmin, kmax, heavy, kth)) {
-                    __syncthreads();
-                    kth = emit_from_candidates(s, scan, total, Me, 0, Me, heavy);
-                }
+                if (!emit_candidates_binned(s, scan, total, Me, 0, Me, kmin, kmax, heavy, kth))
+                    kth = emit_from_candidates(s, total, Me, 0, Me, heavy);
                 exact = kth >= chi;                    // uniform: kth and chi are block-wide values
             }
         }
         if (!exact) {
-            // ---- rescore this row (tables added in the scorer's order), then the full-row select
-            if (tid == 0) {
-                atomicAdd(a.n_fallback, 1);
-                // why: a run overflowed / too few or too many candidates / result not provable on the candidates
-                atomicAdd(a.n_fallback + (any_over ? 3 : ((total < Me || total > SEL_CAP) ? 4 : 5)), 1);
-            }
-            __syncthreads();
-            float* tab = reinterpret_cast<float*>(s.cand_key);           // [L][R] of this head
-            if (a.probs != nullptr) {
-                // packed step: the row's probabilities are the table ([L][R], the very values the fp32
-                // scorer table holds), and that table is not written
-                const float* pr = a.probs + (size_t)row * a.L * a.R;
-                for (int i = tid; i < a.L * a.R; i += SEL_THREADS) tab[i] = __ldcg(pr + i);
-            } else {
-                const float* lut_g = a.lut + (size_t)g * a.R * a.L * a.ht;
-                const int j = hj % a.ht;
-                for (int i = tid; i < a.L * a.R; i += SEL_THREADS) {
-                    const int l = i / a.R, r = i - l * a.R;
-                    tab[i] = __ldcg(lut_g + ((size_t)r * a.L + l) * a.ht + j);
-                }
-            }
-            __syncthreads();
-            const uint8_t* cg = a.codes + (size_t)(b * a.Hkv + kvh) * a.Tcap * a.L;
-            const __half* vg = a.v_norm + (size_t)(b * a.Hkv + kvh) * a.Tcap;
-            for (int t = tid; t < T; t += SEL_THREADS) {
-                const uint4* cp = reinterpret_cast<const uint4*>(cg + (size_t)t * a.L);
-                const int m = t & 7;                   // the scorer's table order for this key
-                float sum = 0.f;
-                for (int v = 0; v < a.L / 16; ++v) {
-                    const uint4 w4 = __ldcg(cp + v);
-                    const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
-#pragma unroll
-                    for (int q = 0; q < 16; ++q) {
-                        const int tb = (q & 8) | ((q & 7) ^ m);
-                        sum += tab[(v * 16 + tb) * a.R + ((w[tb >> 2] >> (8 * (tb & 3))) & 0xffu)];
-                    }
-                }
-                sc[t] = sum * __half2float(__ldcg(vg + t));
-            }
-            __syncthreads();
-            select_row(s, scan, sc, T, Me, heavy);
+            // why: a run overflowed / too few or too many candidates / result not provable on the candidates
+            rescore_row(s, a, row, g, hj, b * a.Hkv + kvh, T, Me, any_over ? 3 : ((total < Me || total > SEL_CAP) ? 4 : 5), heavy);
         }
     } else if (Me == T) {
         for (int i = tid; i < T; i += SEL_THREADS) heavy[i] = i;
@@ -1155,6 +1232,7 @@ int launch_select_candidates(const float* lut, const uint8_t* codes, const uint1
     a.cap_w = plan.cap_w;
     a.Tslots = plan.Tslots;
     a.per_cta = plan.per_cta;
+    a.narrow = (uint64_t)B * Hkv * ((H / Hkv) / ht) * (uint64_t)plan.Tslots < (1ull << 32);
     a.lut = lut;
     a.codes = codes;
     a.v_norm = reinterpret_cast<const __half*>(v_norm);
