@@ -9,9 +9,10 @@
 // are fetched 32 at a time one batch ahead, so the gather never waits on an index load.
 // Each half-warp then handles one entry at a time (16 lanes x 16 bytes = one 256-byte row),
 // with a private online-softmax state (max, sum, 8 output lanes per thread) in fp32 registers.
-// The half-warp states are merged through shared memory, the CTA writes one partial
-// (max, sum, acc[D]) and takes a ticket; the CTA that draws the last ticket of a row merges
-// the row's partials and writes the output.  No CTA ever waits for another one.
+// The half-warp states are merged through shared memory.  The CTAs of a row (up to eight) are a thread-block cluster: each
+// stores its partial (max, sum, acc[D]) into the first one's shared memory, which merges them and writes the output - 1 us
+// after the slowest CTA, where a fence, a ticket and another CTA's loads through L2 took 3 (32 rows of 1216 entries).  A row
+// of more CTAs has several clusters, whose first CTAs write partials and take a ticket; the last one merges those.
 #include <mutex>
 #include <type_traits>
 
@@ -41,6 +42,10 @@ __host__ __device__ inline size_t align256(size_t x) { return (x + 255) & ~(size
 constexpr int64_t DEC_MAX_ROWS = 65536;
 constexpr size_t DEC_TICKET_BYTES = DEC_MAX_ROWS * sizeof(int32_t);
 
+// CTAs of a row: clusters of one to eight
+struct DecodeSplit {
+    int cluster, groups;
+};
 inline int decode_splits(int64_t rows, int64_t max_len) {
     // Few fat CTAs rather than many thin ones: the block scheduler starts roughly 150 CTAs per
     // microsecond, so a grid of 900 small CTAs spends more time ramping up than gathering.
@@ -53,6 +58,28 @@ inline int decode_splits(int64_t rows, int64_t max_len) {
     if (s < 1) s = 1;
     if (s > 256) s = 256;
     return (int)s;
+}
+constexpr int DEC_CLUSTER = 8;                           // the largest portable cluster
+// As many CTAs as decode_splits allows, in equal clusters; nine become one cluster of eight.  Without clusters where there are
+// three CTAs per SM: not all clusters find a place at once then, and the gather is bound by bandwidth (128 rows of 2368
+// entries in clusters of three: the step 129 us, without 121).
+// fp32 rows: the ring of one CTA takes more than half of an SM's shared memory, so one CTA per SM.
+inline DecodeSplit decode_split(int64_t rows, int64_t max_len, bool f32) {
+    int s = decode_splits(rows, max_len);
+    if (f32 && s > sm_count() / rows) s = sm_count() / rows > 1 ? (int)(sm_count() / rows) : 1;
+    if (s * rows > 2 * sm_count()) return {1, s};
+    if (s <= DEC_CLUSTER + 1) return {s < DEC_CLUSTER ? s : DEC_CLUSTER, 1};
+    const int groups = (s + DEC_CLUSTER - 1) / DEC_CLUSTER;
+    return {s / groups, groups};
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// into the shared memory of the cluster's first CTA, at the place `local` has in this one's
+__device__ __forceinline__ void store_first_cta(const float* local, float v) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(local)));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
 }
 
 // smem_dst: 32-bit shared-window address (converted once per kernel, not per copy)
@@ -127,7 +154,8 @@ template <typename KT> struct DecSmem {
     static constexpr int RING = DEC_WARPS * DEC_STAGES * STAGE;
     static constexpr int IDX = DEC_WARPS * DEC_STAGES * DEC_G * 4;
     static constexpr int MERGE = DEC_HW * (DEC_D + 2) * 4;              // aliases the ring
-    static constexpr int TOTAL = RING + IDX + 16;
+    static constexpr int PART = DEC_CLUSTER * (DEC_D + 2) * 4;          // the cluster's partials, in its first CTA
+    static constexpr int TOTAL = RING + IDX + PART + 16;
     static_assert(MERGE <= RING, "merge buffers alias the ring");
 };
 
@@ -138,14 +166,15 @@ sparse_decode_kernel(const QT* __restrict__ q, const KT* __restrict__ k_cache,
                      const int32_t* __restrict__ list, int64_t list_rs,
                      const int32_t* __restrict__ list_len, int64_t max_len, QT* __restrict__ out,
                      int H, int Hkv, int64_t T, const int32_t* __restrict__ T_dev, int32_t* tickets,
-                     float* ws_ml, float* ws_acc, int32_t* status) {
+                     float* ws_ml, float* ws_acc, int32_t* status, int cluster) {
     using S = DecSmem<KT>;
     constexpr int CPR = S::ROW / 16;                    // 16-byte chunks per row
     constexpr int COPIES = DEC_G * CPR / 32;            // cp.async per lane for the K (or V) rows
     constexpr int EPC = 16 / (int)sizeof(KT);           // elements per chunk
     extern __shared__ __align__(128) char smem[];
     int32_t* sidx_all = reinterpret_cast<int32_t*>(smem + S::RING);
-    int* is_last = reinterpret_cast<int*>(smem + S::RING + S::IDX);
+    float* part_s = reinterpret_cast<float*>(smem + S::RING + S::IDX);     // [rank][D], then [rank][max, sum]
+    int* is_last = reinterpret_cast<int*>(smem + S::RING + S::IDX + S::PART);
 
     const int splits = gridDim.x, split = blockIdx.x;
     const int row = blockIdx.y;                    // b*H + h
@@ -154,6 +183,7 @@ sparse_decode_kernel(const QT* __restrict__ q, const KT* __restrict__ k_cache,
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hw = tid >> 4, hw2 = lane >> 4, hl = tid & 15;
     pdl_launch_dependents();
+    if (cluster > 1) cluster_arrive();             // waited for before the first store into another CTA
 
     // the query is an input of the whole step, so it can be fetched before the list exists
     // 16-bit query and keys of one type: the query stays packed and the scale is applied to the
@@ -351,14 +381,14 @@ sparse_decode_kernel(const QT* __restrict__ q, const KT* __restrict__ k_cache,
         m_s[hw] = m;
         l_s[hw] = l;
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) acc_s[hw * DEC_D + hl * 8 + i] = acc[i];
+    float4* acc4 = reinterpret_cast<float4*>(acc_s + hw * DEC_D + hl * 8);
+    acc4[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    acc4[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
     __syncthreads();
+    float mm = -INFINITY, ll = 0.f, a = 0.f;
     if (tid < DEC_D) {                     // one output element per thread
-        float mm = -INFINITY;
 #pragma unroll
         for (int w = 0; w < DEC_HW; ++w) mm = fmaxf(mm, m_s[w]);
-        float ll = 0.f, a = 0.f;
         if (mm > -INFINITY) {
 #pragma unroll
             for (int w = 0; w < DEC_HW; ++w) {
@@ -367,45 +397,73 @@ sparse_decode_kernel(const QT* __restrict__ q, const KT* __restrict__ k_cache,
                 a += acc_s[w * DEC_D + tid] * f;
             }
         }
-        const size_t slot = (size_t)row * splits + split;
-        ws_acc[slot * DEC_D + tid] = a;
-        if (tid == 0) {
-            ws_ml[slot * 2] = mm;
-            ws_ml[slot * 2 + 1] = ll;
-        }
     }
-    // ---- ticket: the last CTA of this row merges the partials
-    __threadfence();
-    __syncthreads();
-    if (tid == 0) {
-        const int t = atomicAdd(&tickets[row], 1);
-        *is_last = (t == splits - 1);
-    }
-    __syncthreads();
-    if (!*is_last || tid >= DEC_D) return;
-    __threadfence();
-    // one pass, all loads independent of each other: running maximum with rescaling, splits in
-    // ascending order (so the result does not depend on which CTA came last)
-    float mm = -INFINITY, ll = 0.f, a = 0.f;
-#pragma unroll 4
-    for (int i = 0; i < splits; ++i) {
-        const size_t slot = (size_t)row * splits + i;
-        const float2 ml = __ldcg(reinterpret_cast<const float2*>(ws_ml + slot * 2));
-        const float av = __ldcg(ws_acc + slot * DEC_D + tid);
-        if (ml.x > -INFINITY) {
-            const float mn = fmaxf(mm, ml.x);
-            const float fo = exp2f(mm - mn), fn = exp2f(ml.x - mn);
-            ll = ll * fo + ml.y * fn;
-            a = a * fo + av * fn;
+    // another partial of the row, in ascending order (so the result does not depend on which CTA came last)
+    auto add_partial = [&](float pm, float pl, float pa) {
+        if (pm > -INFINITY) {
+            const float mn = fmaxf(mm, pm);
+            const float fo = exp2f(mm - mn), fn = exp2f(pm - mn);
+            ll = ll * fo + pl * fn;
+            a = a * fo + pa * fn;
             mm = mn;
         }
+    };
+    if (cluster > 1) {
+        const int rank = split % cluster;
+        float* ml = part_s + DEC_CLUSTER * DEC_D;
+        cluster_wait();                    // every CTA of the cluster has begun
+        if (tid < DEC_D && rank > 0) {
+            store_first_cta(part_s + rank * DEC_D + tid, a);
+            if (tid == 0) {
+                store_first_cta(ml + 2 * rank, mm);
+                store_first_cta(ml + 2 * rank + 1, ll);
+            }
+        }
+        cluster_arrive();
+        cluster_wait();
+        if (rank > 0) return;
+        if (tid < DEC_D) {
+#pragma unroll 1
+            for (int i = 1; i < cluster; ++i) add_partial(ml[2 * i], ml[2 * i + 1], part_s[i * DEC_D + tid]);
+        }
     }
-    out[(size_t)row * DEC_D + tid] = from_f32<QT>(ll > 0.f ? a / ll : 0.f);
-    if (tid == 0) tickets[row] = 0;   // ready for the next call
+    const int groups = splits / cluster, group = split / cluster;
+    if (groups > 1) {
+        const size_t slot = (size_t)row * groups + group;
+        if (tid < DEC_D) {
+            ws_acc[slot * DEC_D + tid] = a;
+            if (tid == 0) {
+                ws_ml[slot * 2] = mm;
+                ws_ml[slot * 2 + 1] = ll;
+            }
+        }
+        // ---- ticket: the last of the row's clusters merges the partials
+        __threadfence();
+        __syncthreads();
+        if (tid == 0) {
+            const int t = atomicAdd(&tickets[row], 1);
+            *is_last = (t == groups - 1);
+        }
+        __syncthreads();
+        if (!*is_last) return;
+        __threadfence();
+        mm = -INFINITY;
+        ll = a = 0.f;
+        if (tid < DEC_D) {
+#pragma unroll 4
+            for (int i = 0; i < groups; ++i) {
+                const size_t at = (size_t)row * groups + i;
+                const float2 p = __ldcg(reinterpret_cast<const float2*>(ws_ml + at * 2));
+                add_partial(p.x, p.y, __ldcg(ws_acc + at * DEC_D + tid));
+            }
+        }
+        if (tid == 0) tickets[row] = 0;    // ready for the next call
+    }
+    if (tid < DEC_D) out[(size_t)row * DEC_D + tid] = from_f32<QT>(ll > 0.f ? a / ll : 0.f);
 }
 
 template <typename QT, typename KT>
-int decode_launch(dim3 grid, cudaStream_t st, const void* q, const void* k_cache, const void* v_cache,
+int decode_launch(DecodeSplit split, int64_t rows, cudaStream_t st, const void* q, const void* k_cache, const void* v_cache,
                   int64_t kv_bs, int64_t kv_hs, int64_t kv_rs, const int32_t* list, int64_t list_rs,
                   const int32_t* list_len, int64_t max_list_len, void* out, int H, int Hkv, int64_t T,
                   const int32_t* T_dev, int32_t* tickets, float* ws_ml, float* ws_acc, int32_t* status) {
@@ -416,9 +474,26 @@ int decode_launch(dim3 grid, cudaStream_t st, const void* q, const void* k_cache
         if (e != cudaSuccess)
             return fail(SK_ERR_CUDA, "sparse_decode_kernel smem attribute: %s", cudaGetErrorString(e));
     }
-    cudaError_t e = launch_chained(kern, grid, dim3(DEC_THREADS), (size_t)smem, st, (const QT*)q, (const KT*)k_cache,
-                                   (const KT*)v_cache, kv_bs, kv_hs, kv_rs, list, list_rs, list_len, max_list_len,
-                                   (QT*)out, H, Hkv, T, T_dev, tickets, ws_ml, ws_acc, status);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(split.cluster * split.groups), (unsigned)rows);
+    cfg.blockDim = dim3(DEC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    if (pdl_chain_active()) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (split.cluster > 1) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = (unsigned)split.cluster;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
+    cfg.attrs = attr;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (const QT*)q, (const KT*)k_cache, (const KT*)v_cache, kv_bs, kv_hs, kv_rs, list,
+                                             list_rs, list_len, max_list_len, (QT*)out, H, Hkv, T, T_dev, tickets, ws_ml, ws_acc,
+                                             status, split.cluster);
     if (e != cudaSuccess) return fail(SK_ERR_CUDA, "sparse_decode_kernel: %s", cudaGetErrorString(e));
     return check_launch("sparse_decode_kernel");
 }
@@ -447,15 +522,15 @@ int launch_sparse_decode(const void* q, int q_dtype, const void* k_cache, const 
     const size_t need = sparse_decode_workspace_bytes(B, H, D, max_list_len);
     if (workspace_bytes < need)
         return fail(SK_ERR_WORKSPACE, "sk_sparse_decode: workspace %zu < %zu bytes", workspace_bytes, need);
-    const int splits = decode_splits(rows, max_list_len);
+    const int splits = decode_splits(rows, max_list_len);       // at least as many as there are partials
+    const DecodeSplit split = decode_split(rows, max_list_len, kv_dtype == SK_F32);
     char* ws = static_cast<char*>(workspace);
     int32_t* tickets = reinterpret_cast<int32_t*>(ws);
     float* ws_ml = reinterpret_cast<float*>(ws + DEC_TICKET_BYTES);
     float* ws_acc = reinterpret_cast<float*>(ws + DEC_TICKET_BYTES +
                                              align256((size_t)rows * splits * 2 * sizeof(float)));
-    dim3 grid(splits, (unsigned)rows);
 #define SK_DEC_LAUNCH(QT, KT)                                                                        \
-    return decode_launch<QT, KT>(grid, st, q, k_cache, v_cache, kv_bs, kv_hs, kv_rs, list, list_rs,  \
+    return decode_launch<QT, KT>(split, rows, st, q, k_cache, v_cache, kv_bs, kv_hs, kv_rs, list, list_rs,  \
                                  list_len, max_list_len, out, H, Hkv, T, T_dev, tickets, ws_ml,      \
                                  ws_acc, status)
     if (q_dtype == SK_BF16 && kv_dtype == SK_BF16) SK_DEC_LAUNCH(__nv_bfloat16, __nv_bfloat16);
