@@ -1,9 +1,9 @@
 // Key hashing (sign-random-projection codes) and the KV-cache append.
 //
-// Exactness: every projection is accumulated in fp64.  For 16-bit inputs each product is
-// exact in fp64 and so is the 128-term sum for any realistic dynamic range, hence the sign
-// (the hash bit) is the sign of the true dot product and does not depend on the order of
-// summation.
+// Exactness: a hash bit is the sign of the dot product accumulated in fp64.  For 16-bit inputs each
+// product is exact in fp64 and so is the 128-term sum for any realistic dynamic range, hence it is
+// the sign of the true dot product and does not depend on the order of summation.  Where the fp32 sum
+// is too far from zero for its rounding to matter, its sign is taken (hash_body.cuh).
 #include "hash_body.cuh"
 
 namespace sk {
@@ -17,17 +17,17 @@ hash_keys_kernel(const KT* __restrict__ keys, int64_t key_row_stride, const PT* 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int l = blockIdx.y * HASH_WARPS + warp;
     for (int64_t n0 = (int64_t)blockIdx.x * HASH_ROWS; n0 < N; n0 += (int64_t)gridDim.x * HASH_ROWS) {
-        double kd[HASH_ROWS][EPL];
+        float kd[HASH_ROWS][EPL];
         void* code_ptr[HASH_ROWS];
 #pragma unroll
         for (int r = 0; r < HASH_ROWS; ++r) {
             const int64_t n = n0 + r;
             if (n < N) {
-                load_row_f64<KT, EPL>(keys + n * key_row_stride, lane, kd[r]);
+                load_row_f32<KT, EPL>(keys + n * key_row_stride, lane, kd[r]);
                 code_ptr[r] = static_cast<char*>(codes) + n * code_row_stride * code_bytes;
             } else {
 #pragma unroll
-                for (int i = 0; i < EPL; ++i) kd[r][i] = 0.0;
+                for (int i = 0; i < EPL; ++i) kd[r][i] = 0.f;
                 code_ptr[r] = nullptr;
             }
         }
@@ -44,7 +44,7 @@ kv_append_kernel(const KT* __restrict__ k_new, const KT* __restrict__ v_new,
                  int Hkv, int64_t Tcap, int L, int P) {
     kv_append_body<KT, PT, EPL>(k_new, v_new, input_pos, planes, k_cache, v_cache, codes, v_norm,
                                 prefill_len, status, B, S, Hkv, Tcap, L, P,
-                                (int64_t)blockIdx.x * HASH_ROWS, blockIdx.y * HASH_WARPS);
+                                (int64_t)blockIdx.x * HASH_ROWS, (int64_t)gridDim.x * HASH_ROWS, blockIdx.y * HASH_WARPS);
 }
 
 template <typename KT, typename PT>
@@ -69,8 +69,9 @@ int kv_append_dispatch(const void* k_new, const void* v_new, const int64_t* pos,
                        int32_t* status, int B, int S, int Hkv, int D, int64_t Tcap, int L, int P,
                        cudaStream_t st) {
     const int64_t N = (int64_t)B * S * Hkv;
-    const int64_t gx = (N + HASH_ROWS - 1) / HASH_ROWS;
+    int64_t gx = (N + HASH_ROWS - 1) / HASH_ROWS;
     if (gx > 0x7fffffff) return fail(SK_ERR_UNSUPPORTED, "sk_kv_append: too many rows");
+    if (gx > sm_count() * 2) gx = sm_count() * 2;             // blocks keep their planes over many groups of rows
     dim3 grid((unsigned)gx, (unsigned)((L + HASH_WARPS - 1) / HASH_WARPS));
     if (D == 128)
         kv_append_kernel<KT, PT, 4><<<grid, HASH_THREADS, 0, st>>>(

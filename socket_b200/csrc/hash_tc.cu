@@ -507,7 +507,7 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
                 if (piece == j) mine = ss;
             }
             const float s = sqrtf(mine);
-            const bool sure = s >= 6.2e-5f && s <= 65000.f && (__float_as_uint(s) & 0x1fffu) - 0x1000u + 24u > 48u;
+            const bool sure = norm_decides_f16(s);
             const int64_t dm = __shfl_sync(FULL, dst, (2 * piece + part) & 15);
             if (sure && piece < 8 && dm >= 0) ap.v_norm[dm] = __float2half_rn(s);
             uint32_t redo = __ballot_sync(FULL, !sure && piece < 8 && dm >= 0);

@@ -25,7 +25,7 @@ decode_prologue_kernel(const T* __restrict__ q, const T* __restrict__ k_new, con
     if ((int)blockIdx.x < n_append) {
         const int bx = blockIdx.x % append_gx, by = blockIdx.x / append_gx;
         kv_append_body<T, PT, 4>(k_new, v_new, input_pos, planes, k_cache, v_cache, codes, v_norm,
-                                 prefill_len, status, B, 1, Hkv, Tcap, L, P, (int64_t)bx * HASH_ROWS,
+                                 prefill_len, status, B, 1, Hkv, Tcap, L, P, (int64_t)bx * HASH_ROWS, (int64_t)append_gx * HASH_ROWS,
                                  by * HASH_WARPS);
     } else {
         const int i = blockIdx.x - n_append;

@@ -67,6 +67,35 @@ def test_append_of_hostile_rows_is_exact(dtype):
         _both(1, S, 1, S + 2, torch.arange(S, device=DEV), k, v, (planes.float() * 1e-25).to(dtype))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+def test_the_exact_kernel_against_fp64(dtype):
+    """Its fp32 sums decide only what fp64 would decide alike: hostile rows, few rows (the general kernel for every type)."""
+    g = torch.Generator(device=DEV).manual_seed(11)
+    S = 397
+    planes, k, v = (torch.randn(*s, generator=g, device=DEV).to(dtype) for s in ((32, 8, 128), (1, S, 1, 128), (1, S, 1, 128)))
+    planes[0, 0] = 0
+    planes[5, :, 64:] = 0
+    k[0, 5] = 0
+    k[0, 6] = 0
+    k[0, 6, 0, 0], k[0, 6, 0, 1] = planes[3, 2, 1], -planes[3, 2, 0]
+    k[0, 20:60, :, :64] = 0
+    k[0, 60:70] *= 1e-4 if dtype == torch.float16 else 1e-25
+    k[0, 70:80] *= 6e4 if dtype == torch.float16 else 1e37
+    v[0, 70:80] *= 1e3
+    v[0, 60:70] *= 1e-6
+    v[0, 5] = 0
+    k[0, 81, 0, 3], k[0, 82, 0, 3], k[0, 83, 0, 3] = float("inf"), float("-inf"), float("nan")
+    cache = _cache(1, 1, S, dtype)
+    ops.kv_append(*cache, torch.arange(S, device=DEV), k, v, planes)
+    prod = (k.double().view(S, 1, 128) * planes.double().view(1, 256, 128)).sum(-1)
+    sure = ~(prod.abs() <= 1e-13 * k.double().view(S, 1, 128).norm(dim=-1) * planes.double().view(1, 256, 128).norm(dim=-1)) | (prod == 0)
+    bits = (prod >= 0).view(S, 32, 8)
+    got = (cache[2][0, 0, :, :, None] >> torch.arange(7, -1, -1, device=DEV) & 1).bool()
+    assert torch.equal(got & sure.view(S, 32, 8), bits & sure.view(S, 32, 8))
+    want = (v.double() ** 2).sum(-1).sqrt().float().half()[0, :, 0]
+    assert torch.equal(cache[3][0, 0], want)
+
+
 def test_append_where_every_projection_is_near_zero():
     S, planes = 4000, torch.randn(32, 8, 128, device=DEV).bfloat16()
     planes[:, :, 64:] = 0
