@@ -9,7 +9,7 @@ namespace {
 
 static_assert(HASH_THREADS == SH_THREADS, "both roles share one block size");
 
-template <typename T, typename PT>
+template <typename T, typename PT, bool USUAL>
 __global__ void __launch_bounds__(SH_THREADS, 2)
 decode_prologue_kernel(const T* __restrict__ q, const T* __restrict__ k_new, const T* __restrict__ v_new,
                        const int64_t* __restrict__ input_pos, const PT* __restrict__ planes,
@@ -25,12 +25,12 @@ decode_prologue_kernel(const T* __restrict__ q, const T* __restrict__ k_new, con
     if ((int)blockIdx.x < n_append) {
         const int bx = blockIdx.x % append_gx, by = blockIdx.x / append_gx;
         kv_append_body<T, PT, 4>(k_new, v_new, input_pos, planes, k_cache, v_cache, codes, v_norm,
-                                 prefill_len, status, B, 1, Hkv, Tcap, L, P, (int64_t)bx * HASH_ROWS, (int64_t)append_gx * HASH_ROWS,
-                                 by * HASH_WARPS);
+                                 prefill_len, status, B, 1, Hkv, Tcap, L, P, (int64_t)bx * HASH_ROWS,
+                                 (int64_t)append_gx * HASH_ROWS, by * HASH_WARPS);
     } else {
         const int i = blockIdx.x - n_append;
         const int bx = i % sh_gx, g = i / sh_gx;
-        soft_hash_body<T, PT>(q, planes, protos_T, inv_temperature, H, Hkv, 128, L, P, R, ht, g,
+        soft_hash_body<T, PT, USUAL>(q, planes, protos_T, inv_temperature, H, Hkv, 128, L, P, R, ht, g,
                               bx * (SH_WARPS / ht), q_probs, lut, pro_smem, lutq, qpar);
     }
 }
@@ -63,7 +63,8 @@ int launch_decode_prologue(const void* q, const void* k_new, const void* v_new, 
     const unsigned grid = (unsigned)(append_gx * append_gy + sh_total);
 #define SK_PRO_LAUNCH(T, PT)                                                                         \
     do {                                                                                             \
-        auto kern = decode_prologue_kernel<T, PT>;                                                   \
+        auto kern = soft_hash_usual<T, PT>(q, planes, D, P, R, ht) ? decode_prologue_kernel<T, PT, true>             \
+                                                                   : decode_prologue_kernel<T, PT, false>;                                                 \
         if (smem > 48 * 1024)                                                                        \
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
         kern<<<grid, SH_THREADS, smem, st>>>((const T*)q, (const T*)k_new, (const T*)v_new, input_pos, \

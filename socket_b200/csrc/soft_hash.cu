@@ -25,7 +25,7 @@ soft_hash_kernel(const QT* __restrict__ q, const PT* __restrict__ planes,
                  int L, int P, int R, int ht, float* __restrict__ q_probs, float* __restrict__ lut,
                  uint2* __restrict__ lutq, float* __restrict__ qpar) {
     extern __shared__ __align__(16) float sh_smem[];
-    soft_hash_body<QT, PT>(q, planes, protos_T, inv_temperature, H, Hkv, D, L, P, R, ht, blockIdx.y,
+    soft_hash_body<QT, PT, false>(q, planes, protos_T, inv_temperature, H, Hkv, D, L, P, R, ht, blockIdx.y,
                            blockIdx.x * (SH_WARPS / ht), q_probs, lut, sh_smem, lutq, qpar);
 }
 

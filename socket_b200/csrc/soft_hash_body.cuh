@@ -56,15 +56,30 @@ __device__ __forceinline__ uint32_t packed_entry(float p, const PackedQuant& q) 
     return (uint32_t)min(max(e, 0), PK_QMAX);
 }
 
+// The usual shape, which has a body of its own: sizes known, one load per row and lane.
+template <typename QT, typename PT>
+inline bool soft_hash_usual(const void* q, const void* planes, int D, int P, int R, int ht) {
+    return D == 128 && P == 8 && R == 256 && ht == 4 && (uintptr_t)q % (4 * sizeof(QT)) == 0 && (uintptr_t)planes % (4 * sizeof(PT)) == 0;
+}
+template <typename T> struct alignas(4 * sizeof(T)) Four {
+    T e[4];
+};
+
 // One CTA: head tile `g` (= (b*Hkv + kvh)*tiles + tile) and tables [l0, l0 + SH_WARPS/ht).
 // Warp w handles (table l0 + w / ht, head w % ht).  All global loads of a warp are issued
 // before the first use, so a cold call costs one memory round trip.
-template <typename QT, typename PT>
+template <typename QT, typename PT, bool USUAL>
 __device__ __forceinline__ void soft_hash_body(
     const QT* __restrict__ q, const PT* __restrict__ planes, const float* __restrict__ protos_T,
     float inv_temperature, int H, int Hkv, int D, int L, int P, int R, int ht, int g, int l0,
     float* __restrict__ q_probs, float* __restrict__ lut, float* smem,
     uint2* __restrict__ lutq = nullptr, float* __restrict__ qpar = nullptr) {
+    if (USUAL) {
+        D = 128;
+        P = 8;
+        R = 256;
+        ht = 4;
+    }
     const int rep = H / Hkv;
     const int tiles = rep / ht;
     const int tile = g % tiles;
@@ -99,12 +114,25 @@ __device__ __forceinline__ void soft_hash_body(
         if (D == 128 && P == 8) {
             // four consecutive elements per lane: every load of the warp is issued up front
             float qv[4], pv[8][4];
+            if (USUAL) {
+                const Four<QT> qr = reinterpret_cast<const Four<QT>*>(qh)[lane];
+                Four<PT> pr[8];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) qv[i] = to_f32(qh[lane * 4 + i]);
+                for (int p = 0; p < 8; ++p) pr[p] = reinterpret_cast<const Four<PT>*>(pl)[p * 32 + lane];
 #pragma unroll
-            for (int p = 0; p < 8; ++p)
+                for (int i = 0; i < 4; ++i) qv[i] = to_f32(qr.e[i]);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) pv[p][i] = to_f32(pl[p * 128 + lane * 4 + i]);
+                for (int p = 0; p < 8; ++p)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) pv[p][i] = to_f32(pr[p].e[i]);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) qv[i] = to_f32(qh[lane * 4 + i]);
+#pragma unroll
+                for (int p = 0; p < 8; ++p)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) pv[p][i] = to_f32(pl[p * 128 + lane * 4 + i]);
+            }
 #pragma unroll
             for (int p = 0; p < 8; ++p)
 #pragma unroll
@@ -127,11 +155,31 @@ __device__ __forceinline__ void soft_hash_body(
     const float inv_sqrt_d = 1.0f / fmaxf(sqrtf((float)D), 1e-6f);
     // lane p keeps the p-th dot product, so the P tanh evaluations run side by side
     float mine = 0.f;
+    if (USUAL) {
+        // the sums of warp_sum_f in its order (lanes 16 apart first), each exchange halving what a lane carries on: 10 shuffles
+        // in place of 40
+        float v[8];
 #pragma unroll
-    for (int p = 0; p < 16; ++p) {
-        if (p < P) {
-            const float s = warp_sum_f(part[p]);
-            if (lane == p) mine = s;
+        for (int p = 0; p < 8; ++p) v[p] = part[p];
+#pragma unroll
+        for (int step = 16, n = 4; step >= 4; step >>= 1, n >>= 1) {
+            const bool upper = (lane & step) != 0;
+#pragma unroll
+            for (int p = 0; p < n; ++p) {
+                const float send = upper ? v[p] : v[p + n], keep = upper ? v[p + n] : v[p];
+                v[p] = keep + __shfl_xor_sync(FULL, send, step);
+            }
+        }
+        v[0] += __shfl_xor_sync(FULL, v[0], 2);
+        v[0] += __shfl_xor_sync(FULL, v[0], 1);
+        mine = __shfl_sync(FULL, v[0], (lane & 7) << 2);      // product p is in lanes 4 p to 4 p + 3
+    } else {
+#pragma unroll
+        for (int p = 0; p < 16; ++p) {
+            if (p < P) {
+                const float s = warp_sum_f(part[p]);
+                if (lane == p) mine = s;
+            }
         }
     }
     if (lane < P) t_s[warp * 16 + lane] = tanhf(mine) * inv_sqrt_d;
