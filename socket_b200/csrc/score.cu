@@ -25,6 +25,8 @@ namespace {
 // Shared memory after the table: mbarrier | per-head sample statistics for the filter mode.
 constexpr int SC_SAMPLE_WARPS = 16;         // warps whose lanes score one sample key each
 constexpr int SC_SAMPLES = 32 * SC_SAMPLE_WARPS;
+constexpr int SC_CUT_BITS = 12;             // of 23 bits of mantissa: a cut below the sample it comes from by 2^-11 at most
+static_assert(SC_SAMPLE_WARPS <= SC_WARPS - 4, "the warps that search have no sample");
 
 struct FilterShared {
     uint64_t bar;
@@ -48,15 +50,15 @@ struct FilterArgs {
 // Per-head cut from the SC_SAMPLES sample scores (one per thread of the first SC_SAMPLE_WARPS warps,
 // sv[j]), such that the fraction `frac` of the samples lies at or above it: the r-th largest sample,
 // r = frac * SC_SAMPLES, found exactly by one warp per head with a bitwise descent on the order keys
-// (the low 8 key bits are left at zero, which can only lower the cut).  Any value would be correct
+// (the low SC_CUT_BITS key bits are left at zero, which can only lower the cut, by less than a thousandth).  Any value would be correct
 // (the select kernel proves or repairs the result); a cut above the row's k-th score costs the row a
 // full rescoring, and with r around 3 k T^-1 SC_SAMPLES the chance of that is the chance that a third
 // of the expected number of samples above the k-th score turns into all of them.
-// The cuts are returned in cut[] and, for the select kernel's check, written to cut_out[j * cut_stride].
-// Must be called by the whole CTA.
+// filter_cuts_begin stores the samples and lets one warp per head search, the other warps go on at once: each scores its first
+// own key meanwhile (the search of one warp takes about a microsecond).  filter_cuts_end returns the cuts in cut[] and writes them to
+// cut_out[j * cut_stride] for the select kernel's check.  Both must be called by the whole CTA.
 template <int HT>
-__device__ __forceinline__ void filter_cuts(FilterShared& fs, const float (&sv)[HT], bool sampling, float frac,
-                                            float* __restrict__ cut_out, size_t cut_stride, float (&cut)[HT]) {
+__device__ __forceinline__ void filter_cuts_begin(FilterShared& fs, const float (&sv)[HT], bool sampling, float frac) {
     static_assert(HT <= 4 && SC_SAMPLES % 32 == 0, "one selecting warp per head");
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (sampling) {
@@ -67,10 +69,11 @@ __device__ __forceinline__ void filter_cuts(FilterShared& fs, const float (&sv)[
         }
     }
     __syncthreads();
-    if (warp < HT) {
+    const int head = warp - (SC_WARPS - HT);          // the last warps: they have not scored a sample
+    if (head >= 0) {
         uint32_t k[SC_SAMPLES / 32];
 #pragma unroll
-        for (int i = 0; i < SC_SAMPLES / 32; ++i) k[i] = fs.skey[warp][lane + 32 * i];
+        for (int i = 0; i < SC_SAMPLES / 32; ++i) k[i] = fs.skey[head][lane + 32 * i];
         const int r = max(2, min(SC_SAMPLES / 2, (int)(frac * (float)SC_SAMPLES + 0.5f)));
         // the bits above the highest one in which two usable samples differ are common to all of them
         uint32_t kmx = 0u, kmn = 0xffffffffu;
@@ -84,7 +87,7 @@ __device__ __forceinline__ void filter_cuts(FilterShared& fs, const float (&sv)[
         const int top = kmx > kmn ? 31 - __clz(kmx ^ kmn) : 7;          // first bit to decide
         uint32_t prefix = top < 31 ? (kmx >> (top + 1)) << (top + 1) : 0u;
         if (kmx == 0u) prefix = 0u;
-        for (int bit = top; bit >= 8; --bit) {
+        for (int bit = top; bit >= SC_CUT_BITS; --bit) {
             const uint32_t cand = prefix | (1u << bit);
             int c = 0;
 #pragma unroll
@@ -92,8 +95,11 @@ __device__ __forceinline__ void filter_cuts(FilterShared& fs, const float (&sv)[
             c = __reduce_add_sync(FULL, c);
             if (c >= r) prefix = cand;
         }
-        if (lane == 0) fs.cut[warp] = prefix != 0u ? order_key_inverse(prefix) : -INFINITY;   // no usable sample: keep everything
+        if (lane == 0) fs.cut[head] = prefix != 0u ? order_key_inverse(prefix) : -INFINITY;   // no usable sample: keep everything
     }
+}
+template <int HT>
+__device__ __forceinline__ void filter_cuts_end(FilterShared& fs, float* __restrict__ cut_out, size_t cut_stride, float (&cut)[HT]) {
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < HT; ++j) cut[j] = fs.cut[j];
@@ -263,6 +269,7 @@ score_kernel(const float* __restrict__ lut, const uint8_t* __restrict__ codes,
         const int run_stride = fa.chunks_max * SC_WARPS * fa.cap_w;
         const int run_index0 = FILTER ? (((int)row0 * fa.chunks_max + chunk) * SC_WARPS + warp) * fa.cap_w : 0;
 
+        bool cuts_open = false;                       // being searched for
         if (FILTER) {
             // ---- the row-wide sample: scores, cut
             float sv[HT];
@@ -277,12 +284,13 @@ score_kernel(const float* __restrict__ lut, const uint8_t* __restrict__ codes,
             }
             // a short segment (the newest keys of a partly filled chunk, or the few keys a CTA has on
             // one side of a KV-head boundary) keeps everything when its runs have the room
-            if (t1 - t0 <= 1024 && 2 * (t1 - t0) <= slots_per_cta && per_warp <= fa.cap_w) {   // uniform across the CTA
+            cuts_open = !(t1 - t0 <= 1024 && 2 * (t1 - t0) <= slots_per_cta && per_warp <= fa.cap_w);   // uniform across the CTA
+            if (!cuts_open) {
                 if (threadIdx.x < HT) fa.cut[(row0 + threadIdx.x) * fa.chunks_max + chunk] = -INFINITY;
             } else {
                 // the kept fraction is taken of the live length: the capacity the plan was made for may
                 // be several times larger, and a cut for 3M / capacity would drop needed keys
-                filter_cuts<HT>(fs, sv, warp < SC_SAMPLE_WARPS, fminf(__fdividef(fa.keep, (float)Teff), 1.0f), fa.cut + row0 * fa.chunks_max + chunk, (size_t)fa.chunks_max, cutv);
+                filter_cuts_begin<HT>(fs, sv, warp < SC_SAMPLE_WARPS, fminf(__fdividef(fa.keep, (float)Teff), 1.0f));
             }
             // on to the warp's own keys
 #pragma unroll
@@ -296,7 +304,7 @@ score_kernel(const float* __restrict__ lut, const uint8_t* __restrict__ codes,
         }
 
         // ---- main loop over this warp's keys, codes double-buffered in registers
-        for (; t - lane < we; t += 32) {
+        for (bool first = true; first || t - lane < we; t += 32, first = false) {      // once at least: the cuts are met by all
             const bool valid = t < we;
             float sv[HT];
             if (valid) {
@@ -306,6 +314,7 @@ score_kernel(const float* __restrict__ lut, const uint8_t* __restrict__ codes,
 #pragma unroll
                 for (int j = 0; j < HT; ++j) sv[j] = acc[j] * vn;
             }
+            if (FILTER && first && cuts_open) filter_cuts_end<HT>(fs, fa.cut + row0 * fa.chunks_max + chunk, (size_t)fa.chunks_max, cutv);
             if (FILTER) {
                 const bool in_tail = valid && t >= tail_start;
                 if (in_tail) {
@@ -606,6 +615,7 @@ score_packed_kernel(const uint8_t* __restrict__ lutq, const float* __restrict__ 
             }
         };
 
+        bool cuts_open;                               // being searched for; uniform across the CTA
         {
             // ---- the row-wide sample: scores, cut
             float sv[HT];
@@ -613,11 +623,11 @@ score_packed_kernel(const uint8_t* __restrict__ lutq, const float* __restrict__ 
 #pragma unroll
             for (int j = 0; j < HT; ++j) sv[j] = 0.f;
             if (warp < SC_SAMPLE_WARPS) score_cur(pk, sv);          // warp-uniform
-            if (t1 - t0 <= 1024 && 2 * (t1 - t0) <= slots_per_cta && per_warp <= fa.cap_w) {   // uniform across the CTA
+            cuts_open = !(t1 - t0 <= 1024 && 2 * (t1 - t0) <= slots_per_cta && per_warp <= fa.cap_w);
+            if (!cuts_open) {
                 if (threadIdx.x < HT) fa.cut[(row0 + threadIdx.x) * fa.chunks_max + chunk] = -INFINITY;
             } else {
-                filter_cuts<HT>(fs, sv, warp < SC_SAMPLE_WARPS, fminf(__fdividef(fa.keep, (float)Teff), 1.0f),
-                                fa.cut + row0 * fa.chunks_max + chunk, (size_t)fa.chunks_max, cutv);
+                filter_cuts_begin<HT>(fs, sv, warp < SC_SAMPLE_WARPS, fminf(__fdividef(fa.keep, (float)Teff), 1.0f));
             }
         }
         // on to the warp's own keys
@@ -628,11 +638,12 @@ score_packed_kernel(const uint8_t* __restrict__ lutq, const float* __restrict__ 
             ldg256(cg + (size_t)(t + 32) * L, nxt);
             vnxt = __ldcg(reinterpret_cast<const uint16_t*>(vg) + t + 32);
         }
-        for (; t - lane < we; t += 32) {
+        for (bool first = true; first || t - lane < we; t += 32, first = false) {      // once at least: the cuts are met by all
             const bool valid = t < we;
             float sv[HT];
             uint32_t pk[HT];
             score_cur(pk, sv);
+            if (first && cuts_open) filter_cuts_end<HT>(fs, fa.cut + row0 * fa.chunks_max + chunk, (size_t)fa.chunks_max, cutv);
             keep(pk, sv, valid, t);
 #pragma unroll
             for (int i = 0; i < 8; ++i) cur[i] = nxt[i];
