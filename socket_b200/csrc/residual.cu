@@ -29,8 +29,10 @@ embed_rows_kernel(const int64_t* __restrict__ tokens, const T* __restrict__ tabl
 // One CTA per row; the row lives in registers (NV vectors of V elements per thread).
 //   in_mode  0: x stays; 1: x += rms(y) * w_in; 2: x = y + w_in; 3: x += y
 //   out_mode 0: nothing; 1: out = rms(x) * w_out; 2: out = [x ; x0]; 3: out = layer norm of x * w_out
+// A decoded token's rows are bound by latency, a prompt's by memory.  Everything the kernel reads is requested at once: with
+// each norm's weights requested behind its sum, a row of 4096 waited for memory three times.
 template <typename T, typename TY, int V, int NV>
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(V == 8 ? 512 : 1024)
 residual_norm_kernel(sk_residual_params p) {
     __shared__ float red[3][32];
     const int64_t row = blockIdx.x;
@@ -39,43 +41,61 @@ residual_norm_kernel(sk_residual_params p) {
     float* xr = p.x + row * W;
     const T* w_in = (const T*)p.w_in;
     const T* w_out = (const T*)p.w_out;
+    const TY* yr = (const TY*)p.y + row * p.y_ld;
+    const bool norm_out = p.out_mode == 1 || p.out_mode == 3;
+    constexpr bool EARLY = NV * V <= 16;                  // else the weights' registers would be spilled
+    Raw<TY, V> yw[NV];
+    Raw<float, V> xw[NV];
+    Raw<T, V> wi[NV], wo[NV];
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+        const int i = (n * nt + t) * V;
+        if (i < W) {
+            if (p.in_mode != 0) yw[n] = load_raw<TY, V>(yr + i);
+            if (p.in_mode != 2) xw[n] = load_raw<float, V>(xr + i);
+        }
+    }
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+        const int i = (n * nt + t) * V;
+        if (EARLY && i < W) {
+            if (p.in_mode == 1 || p.in_mode == 2) wi[n] = load_raw<T, V>(w_in + i);
+            if (norm_out) wo[n] = load_raw<T, V>(w_out + i);
+        }
+    }
     float xv[NV][V];
     if (p.in_mode != 0) {
-        const TY* yr = (const TY*)p.y + row * p.y_ld;
-        float yv[NV][V], ss = 0.f;
-#pragma unroll
-        for (int n = 0; n < NV; ++n) {
-            const int i = (n * nt + t) * V;
-            if (i < W) {
-                load_vec<TY, V>(yr + i, yv[n]);
-                if (p.in_mode != 2) load_vec<float, V>(xr + i, xv[n]);
-#pragma unroll
-                for (int e = 0; e < V; ++e) ss = fmaf(yv[n][e], yv[n][e], ss);
-            }
-        }
         float inv = 1.f;
-        if (p.in_mode == 1) inv = 1.f / sqrtf(block_sum(ss, red[0]) / (float)W + p.eps);
+        if (p.in_mode == 1) {
+            float ss = 0.f;
+#pragma unroll
+            for (int n = 0; n < NV; ++n)
+                if ((n * nt + t) * V < W)
+#pragma unroll
+                    for (int e = 0; e < V; ++e) ss = fmaf(to_f32(yw[n].e[e]), to_f32(yw[n].e[e]), ss);
+            inv = 1.f / sqrtf(block_sum(ss, red[0]) / (float)W + p.eps);
+        }
 #pragma unroll
         for (int n = 0; n < NV; ++n) {
             const int i = (n * nt + t) * V;
             if (i < W) {
-                float w[V];
-                if (p.in_mode != 3) load_vec<T, V>(w_in + i, w);
+                if (!EARLY && p.in_mode != 3) wi[n] = load_raw<T, V>(w_in + i);
 #pragma unroll
-                for (int e = 0; e < V; ++e)
-                    xv[n][e] = p.in_mode == 1 ? xv[n][e] + yv[n][e] * inv * w[e]
-                                              : (p.in_mode == 2 ? yv[n][e] + w[e] : xv[n][e] + yv[n][e]);
+                for (int e = 0; e < V; ++e) {
+                    const float y = to_f32(yw[n].e[e]);
+                    xv[n][e] = p.in_mode == 1 ? xw[n].e[e] + y * inv * to_f32(wi[n].e[e])
+                                              : (p.in_mode == 2 ? y + to_f32(wi[n].e[e]) : xw[n].e[e] + y);
+                }
                 store_vec<float, V>(xr + i, xv[n]);
             }
         }
     } else {
 #pragma unroll
-        for (int n = 0; n < NV; ++n) {
-            const int i = (n * nt + t) * V;
-            if (i < W) load_vec<float, V>(xr + i, xv[n]);
-        }
+        for (int n = 0; n < NV; ++n)
+#pragma unroll
+            for (int e = 0; e < V; ++e) xv[n][e] = xw[n].e[e];
     }
-    if (p.out_mode == 1 || p.out_mode == 3) {
+    if (norm_out) {
         float mean = 0.f;
         if (p.out_mode == 3) {                            // centred in registers; the stream itself is written already
             float sum = 0.f;
@@ -101,10 +121,10 @@ residual_norm_kernel(sk_residual_params p) {
         for (int n = 0; n < NV; ++n) {
             const int i = (n * nt + t) * V;
             if (i < W) {
-                float w[V], r[V];
-                load_vec<T, V>(w_out + i, w);
+                float r[V];
+                if (!EARLY) wo[n] = load_raw<T, V>(w_out + i);
 #pragma unroll
-                for (int e = 0; e < V; ++e) r[e] = xv[n][e] * inv * w[e];
+                for (int e = 0; e < V; ++e) r[e] = xv[n][e] * inv * to_f32(wo[n].e[e]);
                 store_vec<T, V>(o + i, r);
             }
         }
@@ -114,8 +134,10 @@ residual_norm_kernel(sk_residual_params p) {
         for (int n = 0; n < NV; ++n) {
             const int i = (n * nt + t) * V;
             if (i < W) {
+                const Raw<float, V> x0 = load_raw<float, V>(p.x0 + row * W + i);
                 float r[V];
-                load_vec<float, V>(p.x0 + row * W + i, r);
+#pragma unroll
+                for (int e = 0; e < V; ++e) r[e] = x0.e[e];
                 store_vec<T, V>(o + i, xv[n]);
                 store_vec<T, V>(o + W + i, r);
             }
@@ -172,9 +194,10 @@ template <typename T, typename TY, int V>
 int residual_dispatch(const sk_residual_params& p, cudaStream_t st) {
     const int vecs = (p.width + V - 1) / V;
     // few rows: one vector per thread (latency); many rows: smaller blocks, more of them per SM
-    int nt = p.rows < 296 ? 1024 : 256;
+    const int most = V == 8 ? 512 : 1024;
+    int nt = p.rows < 296 ? most : 256;
     while (nt > 32 && nt / 2 >= vecs) nt /= 2;
-    while (nt < 1024 && (vecs + nt - 1) / nt > 8) nt *= 2;
+    while (nt < most && (vecs + nt - 1) / nt > 8) nt *= 2;
     const int nv = (vecs + nt - 1) / nt;
     dim3 grid((unsigned)p.rows);
     void (*kern)(sk_residual_params) = nullptr;
@@ -203,6 +226,10 @@ int launch_residual_norm(const sk_residual_params& p, cudaStream_t st) {
     const bool v4 = p.width % 4 == 0 && p.y_ld % 4 == 0;
     if (p.dtype == SK_F32) return v4 ? residual_dispatch<float, float, 4>(p, st) : residual_dispatch<float, float, 1>(p, st);
     using bf = __nv_bfloat16;
+    // rows of 16-byte pieces: half the threads and instructions
+    const bool v8 = p.width % 8 == 0 && p.y_ld % 8 == 0 && p.width <= 8 * 512 * 8 &&
+                    ((uintptr_t)p.x | (uintptr_t)p.y | (uintptr_t)p.w_in | (uintptr_t)p.w_out | (uintptr_t)p.x0 | (uintptr_t)p.out) % 16 == 0;
+    if (v8) return p.y_dtype == SK_F32 ? residual_dispatch<bf, float, 8>(p, st) : residual_dispatch<bf, bf, 8>(p, st);
     if (p.y_dtype == SK_F32) return v4 ? residual_dispatch<bf, float, 4>(p, st) : residual_dispatch<bf, float, 1>(p, st);
     return v4 ? residual_dispatch<bf, bf, 4>(p, st) : residual_dispatch<bf, bf, 1>(p, st);
 }

@@ -15,24 +15,27 @@ rms_norm_rows_kernel(const T* x, const T* w, int width, float eps, T* __restrict
     const int64_t row = blockIdx.x;
     const int nt = blockDim.x, t = threadIdx.x;
     float v[NV][V], ss = 0.f;
+    Raw<T, V> g[NV];                                      // requested with the row: one trip to memory
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
         const int i = (n * nt + t) * V;
         if (i < width) {
             load_vec<T, V>(x + row * width + i, v[n]);
-#pragma unroll
-            for (int e = 0; e < V; ++e) ss = fmaf(v[n][e], v[n][e], ss);
+            g[n] = load_raw<T, V>(w + i);
         }
     }
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+        if ((n * nt + t) * V < width)
+#pragma unroll
+            for (int e = 0; e < V; ++e) ss = fmaf(v[n][e], v[n][e], ss);
     const float inv = 1.f / sqrtf(block_sum(ss, red) / (float)width + eps);
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
         const int i = (n * nt + t) * V;
         if (i < width) {
-            float g[V];
-            load_vec<T, V>(w + i, g);
 #pragma unroll
-            for (int e = 0; e < V; ++e) v[n][e] *= inv * g[e];
+            for (int e = 0; e < V; ++e) v[n][e] *= inv * to_f32(g[n].e[e]);
             store_vec<T, V>(out + row * width + i, v[n]);
         }
     }
