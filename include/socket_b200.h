@@ -446,6 +446,11 @@ SK_API int sk_rms_norm(const void* x, const void* w, int dtype, int64_t rows, in
 SK_API int sk_pick_token(const void* logits, int dtype, int64_t ld, int batch, int vocab, int64_t* token, int64_t* pos,
                          int32_t* seqlens, void* stream);
 
+/* The start of a decode step on given tokens, in one launch: token[b] = first[b], seqlens[b] = position, pos[0] = position, and
+ * *lengths[i] = position for the n device words whose addresses the host array `lengths` holds (read during the call). */
+SK_API int sk_begin_token(const int64_t* first, int64_t* token, int batch, int64_t* pos, int32_t* seqlens, int64_t position,
+                          int32_t* const* lengths, int n, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -64,6 +64,10 @@ SK_API int skb_linear_rows(const sk_linear_params* p, void* stream);
 SK_API int skb_pick_token(const void* logits, int dtype, int64_t ld, int batch, int vocab, int64_t* token, int64_t* pos,
                           int32_t* seqlens, void* stream);
 
+/* The start of one, as sk_begin_token. */
+SK_API int skb_begin_token(const int64_t* first, int64_t* token, int batch, int64_t* pos, int32_t* seqlens, int64_t position,
+                           int32_t* const* lengths, int n, void* stream);
+
 /* Gated unit of a feed-forward; gate and up rows are `ld` elements apart, out rows out_ld:
  *   SKB_GLU_CLAMPED  out = g * sigmoid(slope * g) * (u + 1), g = min(gate, limit), u = clamp(up, -limit, limit)
  *   SKB_GLU_SILU     out = gate * sigmoid(gate) * up */

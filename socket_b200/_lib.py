@@ -105,6 +105,7 @@ SIGNATURES = {
     "sk_linear_rows": (_i, [C.POINTER(LinearParams), _p]),
     "sk_rms_norm": (_i, [_p, _p, _i, _i64, _i, _f, _p, _p]),
     "sk_pick_token": (_i, [_p, _i, _i64, _i, _i, _p, _p, _p, _p]),
+    "sk_begin_token": (_i, [_p, _p, _i, _p, _p, _i64, _p, _i, _p]),
 }
 
 
@@ -180,6 +181,7 @@ BLOCK_SIGNATURES = {
     "skb_linear_rows_applicable": (_i, [C.POINTER(LinearParams)]),
     "skb_linear_rows": (_i, [C.POINTER(LinearParams), _p]),
     "skb_pick_token": (_i, [_p, _i, _i64, _i, _i, _p, _p, _p, _p]),
+    "skb_begin_token": (_i, [_p, _p, _i, _p, _p, _i64, _p, _i, _p]),
     "skb_glu": (_i, [_p, _p, _i, _i64, _i, _i64, _i, _f, _f, _p, _i64, _p]),
     "skb_ring_append": (_i, [_p, _p, _i, _i, _i, _i64, _i64, _i64, _i64, _i, _i, _i, _i, _p, _i64, _p, _p, _p]),
     "skb_rotary_rows": (_i, [C.POINTER(RotaryRowsParams), _p]),

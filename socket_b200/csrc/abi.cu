@@ -635,4 +635,9 @@ int sk_pick_token(const void* logits, int dtype, int64_t ld, int batch, int voca
     return pick_token(logits, dtype, ld, batch, vocab, token, pos, seqlens, (cudaStream_t)stream);
 }
 
+int sk_begin_token(const int64_t* first, int64_t* token, int batch, int64_t* pos, int32_t* seqlens, int64_t position,
+                   int32_t* const* lengths, int n, void* stream) {
+    return begin_token(first, token, batch, pos, seqlens, position, lengths, n, (cudaStream_t)stream);
+}
+
 }  // extern "C"

@@ -119,6 +119,11 @@ int skb_pick_token(const void* logits, int dtype, int64_t ld, int batch, int voc
     return pick_token(logits, dtype, ld, batch, vocab, token, pos, seqlens, (cudaStream_t)stream);
 }
 
+int skb_begin_token(const int64_t* first, int64_t* token, int batch, int64_t* pos, int32_t* seqlens, int64_t position,
+                    int32_t* const* lengths, int n, void* stream) {
+    return begin_token(first, token, batch, pos, seqlens, position, lengths, n, (cudaStream_t)stream);
+}
+
 int skb_glu(const void* gate, const void* up, int dtype, int64_t rows, int ff, int64_t ld, int kind, float limit, float slope,
             void* out, int64_t out_ld, void* stream) {
     SK_REQUIRE(gate && up && out && block_dtype(dtype) && rows > 0 && ff > 0 && ld >= ff && out_ld >= ff,

@@ -54,6 +54,9 @@ template <typename T, int V> __device__ __forceinline__ void store_vec(T* p, con
 #pragma unroll
         for (int i = 0; i < 4; ++i) e[i] = from_f32<T>(r[i]);
         *reinterpret_cast<uint2*>(p) = *reinterpret_cast<uint2*>(e);
+    } else if constexpr (V == 8 && sizeof(T) == 4) {
+        reinterpret_cast<float4*>(p)[0] = make_float4(r[0], r[1], r[2], r[3]);
+        reinterpret_cast<float4*>(p)[1] = make_float4(r[4], r[5], r[6], r[7]);
     } else if constexpr (V == 8 && sizeof(T) == 2) {
         T e[8];
 #pragma unroll
@@ -64,6 +67,12 @@ template <typename T, int V> __device__ __forceinline__ void store_vec(T* p, con
         for (int i = 0; i < V; ++i) p[i] = from_f32<T>(r[i]);
     }
 }
+
+// The same in two steps, so that a load can be requested long before its values are needed
+template <typename T, int V> struct alignas(sizeof(T) * V < 16 ? sizeof(T) * V : 16) Raw {
+    T e[V];
+};
+template <typename T, int V> __device__ __forceinline__ Raw<T, V> load_raw(const T* p) { return *reinterpret_cast<const Raw<T, V>*>(p); }
 
 __device__ __forceinline__ float exp2_fast(float x) {
     float y;
@@ -101,6 +110,8 @@ bool linear_rows_applicable(const sk_linear_params& p);
 int linear_rows(const sk_linear_params* p, cudaStream_t st);             // both libraries' entry point, with its checks
 int pick_token(const void* logits, int dtype, int64_t ld, int batch, int vocab, int64_t* token, int64_t* pos, int32_t* seqlens,
                cudaStream_t st);                                         // the same
+int begin_token(const int64_t* first, int64_t* token, int batch, int64_t* pos, int32_t* seqlens, int64_t position, int32_t* const* lengths,
+                int n, cudaStream_t st);                                 // the same
 int rms_norm_rows(const void* x, const void* w, int dtype, int64_t rows, int width, float eps, void* out, cudaStream_t st);
 int launch_glu(const void* gate, const void* up, int dtype, int64_t rows, int ff, int64_t ld, int kind, float limit, float slope,
                void* out, int64_t out_ld, cudaStream_t st);

@@ -120,6 +120,19 @@ inline int check_chained(cudaError_t e, const char* what) {
     return e == cudaSuccess ? SK_OK : fail(SK_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
 }
 
+// ---------------------------------------------------------------- thread-block clusters
+// A first arrive / wait pair tells that every CTA of the cluster has begun, which a store into another one's shared memory
+// needs; a second one that the stores have landed.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// into the shared memory of the cluster's first CTA, at the place `local` has in this one's
+__device__ __forceinline__ void store_first_cta(const void* local, uint32_t v) {
+    uint32_t remote;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(local)));
+    asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(remote), "r"(v) : "memory");
+}
+__device__ __forceinline__ void store_first_cta(const float* local, float v) { store_first_cta((const void*)local, __float_as_uint(v)); }
+
 // ---------------------------------------------------------------- shared-memory histograms
 // Histogram increment by all 32 lanes of a warp.  The lanes that hit the same bin as the first
 // active lane are merged into one atomic (score keys cluster, so one dominant bin per warp is the

@@ -73,15 +73,6 @@ inline DecodeSplit decode_split(int64_t rows, int64_t max_len, bool f32) {
     return {s / groups, groups};
 }
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// into the shared memory of the cluster's first CTA, at the place `local` has in this one's
-__device__ __forceinline__ void store_first_cta(const float* local, float v) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(remote) : "r"((uint32_t)__cvta_generic_to_shared(local)));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
-}
-
 // smem_dst: 32-bit shared-window address (converted once per kernel, not per copy)
 __device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void* gmem_src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(gmem_src) : "memory");

@@ -14,55 +14,65 @@ __device__ __forceinline__ bool picked(float a, int i, float b, int j) {
     return i < j;
 }
 
-// One CTA per sequence.  32768 bf16 logits: 6.6 us at the end of a decoded token, where argmax, copy and two increments by
-// the library take 17.
+// A cluster of eight CTAs per sequence, each an eighth of the row; the first one joins what they found.  32768 logits: one CTA
+// took 6.6 us at the end of a decoded token.
+constexpr int PT_CLUSTER = 8, PT_THREADS = 256;
 template <typename T, int V>
-__global__ void __launch_bounds__(1024)
+__global__ void __launch_bounds__(PT_THREADS)
 pick_token_kernel(const T* logits, int64_t ld, int vocab, int64_t* token, int64_t* pos, int32_t* seqlens) {
     pdl_begin();
-    __shared__ float best_s[32];
-    __shared__ int at_s[32];
-    const int b = blockIdx.x, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    constexpr int WARPS = PT_THREADS / 32;
+    __shared__ float best_s[PT_CLUSTER * WARPS];
+    __shared__ int at_s[PT_CLUSTER * WARPS];
+    cluster_arrive();
+    const int rank = blockIdx.x, b = blockIdx.y, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const T* row = logits + b * ld;
     float best = -INFINITY;
     int at = vocab;                                           // behind every index: a row of -inf alone picks its first
-    constexpr int U = 4;
-    for (int i0 = t * V; i0 < vocab; i0 += U * 1024 * V) {
+    constexpr int U = 4, STEP = PT_CLUSTER * PT_THREADS * V;  // elements of the cluster's one load each
+    for (int64_t i0 = (rank * PT_THREADS + t) * V; i0 < vocab; i0 += U * STEP) {
         float v[U][V];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            if (i0 + u * 1024 * V < vocab) load_vec<T, V>(row + i0 + u * 1024 * V, v[u]);
+            if (i0 + u * STEP < vocab) load_vec<T, V>(row + i0 + u * STEP, v[u]);
 #pragma unroll
         for (int u = 0; u < U; ++u)
 #pragma unroll
             for (int e = 0; e < V; ++e) {
-                const int i = i0 + u * 1024 * V + e;
-                if (i < vocab && picked(v[u][e], i, best, at)) {
+                const int64_t i = i0 + u * STEP + e;
+                if (i < vocab && picked(v[u][e], (int)i, best, at)) {
                     best = v[u][e];
-                    at = i;
+                    at = (int)i;
                 }
             }
     }
+    auto join = [&](float x, int i) {
+        if (picked(x, i, best, at)) {
+            best = x;
+            at = i;
+        }
+    };
     auto reduce = [&]() {
 #pragma unroll
         for (int o = 16; o >= 1; o >>= 1) {
             const float x = __shfl_xor_sync(FULL, best, o);
             const int i = __shfl_xor_sync(FULL, at, o);
-            if (picked(x, i, best, at)) {
-                best = x;
-                at = i;
-            }
+            join(x, i);
         }
     };
     reduce();
+    cluster_wait();                                           // every CTA of the cluster has begun
     if (lane == 0) {
-        best_s[warp] = best;
-        at_s[warp] = at;
+        store_first_cta(best_s + rank * WARPS + warp, best);
+        store_first_cta(at_s + rank * WARPS + warp, (uint32_t)at);
     }
-    __syncthreads();
-    if (warp == 0) {
+    cluster_arrive();
+    cluster_wait();
+    if (rank == 0 && warp == 0) {
+        static_assert(PT_CLUSTER * WARPS == 64, "two results per lane");
         best = best_s[lane];
         at = at_s[lane];
+        join(best_s[lane + 32], at_s[lane + 32]);
         reduce();
         if (lane == 0) {
             token[b] = at;
@@ -78,8 +88,40 @@ int pick_dispatch(const void* logits, int64_t ld, int batch, int vocab, int64_t*
     constexpr int V = 16 / sizeof(T);
     const bool vec = vocab % V == 0 && ld % V == 0 && (uintptr_t)logits % 16 == 0;
     auto kern = vec ? pick_token_kernel<T, V> : pick_token_kernel<T, 1>;
-    return check_chained(launch_after(kern, dim3((unsigned)batch), dim3(1024), 0, st, (const T*)logits, ld, vocab, token, pos, seqlens),
-                         "pick_token_kernel");
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(PT_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = PT_CLUSTER;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    for (int b0 = 0; b0 < batch; b0 += 65535) {               // the grid's second dimension
+        cfg.gridDim = dim3(PT_CLUSTER, (unsigned)(batch - b0 < 65535 ? batch - b0 : 65535));
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (const T*)logits + b0 * ld, ld, vocab, token + b0, b0 == 0 ? pos : (int64_t*)nullptr,
+                                                 seqlens != nullptr ? seqlens + b0 : (int32_t*)nullptr);
+        if (int rc = check_chained(e, "pick_token_kernel")) return rc;
+    }
+    return SK_OK;
+}
+
+// What a decode step begins with, in one launch: the current tokens, the position, and the lengths.
+constexpr int BT_LENGTHS = 64;
+struct BtLengths {
+    int32_t* at[BT_LENGTHS];
+};
+__global__ void __launch_bounds__(128)
+begin_token_kernel(const int64_t* first, int64_t* token, int batch, int64_t* pos, int32_t* seqlens, int64_t position,
+                   const __grid_constant__ BtLengths lengths, int n) {
+    for (int b = threadIdx.x; b < batch; b += 128) {
+        token[b] = first[b];
+        seqlens[b] = (int32_t)position;
+    }
+    if (threadIdx.x == 0) pos[0] = position;
+    for (int i = threadIdx.x; i < n; i += 128) *lengths.at[i] = (int32_t)position;
 }
 
 }  // namespace
@@ -90,6 +132,24 @@ int pick_token(const void* logits, int dtype, int64_t ld, int batch, int vocab, 
     if (dtype == SK_F32) return pick_dispatch<float>(logits, ld, batch, vocab, token, pos, seqlens, st);
     return dtype == SK_BF16 ? pick_dispatch<__nv_bfloat16>(logits, ld, batch, vocab, token, pos, seqlens, st)
                             : pick_dispatch<__half>(logits, ld, batch, vocab, token, pos, seqlens, st);
+}
+
+int begin_token(const int64_t* first, int64_t* token, int batch, int64_t* pos, int32_t* seqlens, int64_t position, int32_t* const* lengths,
+                int n, cudaStream_t st) {
+    SK_REQUIRE(first && token && pos && seqlens && batch > 0 && position >= INT32_MIN && position <= INT32_MAX && n >= 0 && (n == 0 || lengths),
+               "begin_token: null pointer or bad sizes");
+    int i = 0;
+    do {                                                      // more lengths than a launch takes: the rest by themselves
+        BtLengths part{};
+        int m = 0;
+        for (; m < BT_LENGTHS && i < n; ++m, ++i) {
+            SK_REQUIRE(lengths[i] != nullptr, "begin_token: null length");
+            part.at[m] = lengths[i];
+        }
+        begin_token_kernel<<<1, 128, 0, st>>>(first, token, batch, pos, seqlens, position, part, m);
+        if (int rc = check_launch("begin_token_kernel")) return rc;
+    } while (i < n);
+    return SK_OK;
 }
 
 }  // namespace sk

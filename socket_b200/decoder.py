@@ -7,7 +7,7 @@ A model class supplies its layers through a handful of hooks:
 * `_portion(idx, start)`               hidden rows [B, S, width] of S consecutive tokens, caches advanced
 * `_head(hidden)`                      logits of hidden rows
 * `_decode_logits(mode)`               logits [B, vocab] of the token in `_tok` at the device position `_pos`
-* `_setup_decode_layers`, `_start_decode_layers`, `_release_decode_layers`   decode-time buffers
+* `_setup_decode_layers`, `_start_decode_layers`, `_release_decode_layers`, `_decode_lengths`   decode-time buffers
 """
 from __future__ import annotations
 
@@ -55,6 +55,10 @@ class Decoder(nn.Module):
 
     def _start_decode_layers(self, position: int) -> None:
         pass
+
+    def _decode_lengths(self) -> Sequence[Tensor]:
+        """Device words (int32) that a decode step finds its position in, beside `_pos` and `_seqlens`."""
+        return ()
 
     def _release_decode_layers(self) -> None:
         pass
@@ -162,9 +166,16 @@ class Decoder(nn.Module):
             raise RuntimeError(f"start_decode: position {position} outside the caches (max_seq_length="
                                f"{self.max_seq_length})")
         self._host_pos = position                 # host mirror of the device-side position counter
-        self._tok.copy_(first_token)
-        self._pos.fill_(position)
-        self._seqlens.fill_(position)
+        lengths = self._decode_lengths()
+        if self._tok.is_cuda and first_token.device == self._tok.device and first_token.dtype == torch.long and \
+                first_token.shape == self._tok.shape and first_token.is_contiguous():
+            few_rows.begin_token(first_token, self._tok, self._pos, self._seqlens, position, lengths, self.libraries[0])
+        else:
+            self._tok.copy_(first_token)
+            self._pos.fill_(position)
+            self._seqlens.fill_(position)
+            for n in lengths:
+                n.fill_(position)
         self._start_decode_layers(position)
 
     @torch.no_grad()

@@ -4,7 +4,7 @@ the norm; a model calls those of the library it is built on (`library`: "step" o
 from __future__ import annotations
 
 import ctypes as C
-from typing import Optional
+from typing import Optional, Sequence
 
 import torch
 from torch import Tensor
@@ -115,3 +115,16 @@ def pick_token(logits: Tensor, token: Tensor, pos: Tensor, seqlens: Tensor, libr
     logits = _separate_rows(logits)                               # lives until the launch
     _launch(library, "pick_token", ptr(logits), dtype_code(logits), _ld(logits), logits.shape[0], logits.shape[1], ptr(token), ptr(pos),
             ptr(seqlens), stream_ptr(logits.device))
+
+
+def begin_token(first: Tensor, token: Tensor, pos: Tensor, seqlens: Tensor, position: int, lengths: Sequence[Tensor], library: str) -> None:
+    """token [batch, 1] = first, pos = seqlens = every one of `lengths` = position, in one launch."""
+    _require_cuda(first, token)
+    _require_on(first.device, token, pos, seqlens, *lengths)
+    assert first.shape == token.shape and first.dtype == token.dtype == pos.dtype == torch.int64
+    assert first.is_contiguous() and token.is_contiguous() and seqlens.is_contiguous() and pos.numel() == 1
+    assert seqlens.dtype == torch.int32 and token.numel() == seqlens.numel()
+    assert all(t.dtype == torch.int32 and t.numel() == 1 for t in lengths)
+    table = (C.c_void_p * max(len(lengths), 1))(*(ptr(t) for t in lengths))
+    _launch(library, "begin_token", ptr(first), ptr(token), token.numel(), ptr(pos), ptr(seqlens), int(position), table, len(lengths),
+            stream_ptr(first.device))

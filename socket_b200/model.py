@@ -447,7 +447,5 @@ class Transformer(Decoder):
             layer.attention._step = None
             layer.fused_sum = None
 
-    def _start_decode_layers(self, position: int) -> None:
-        if self._mode == "sparse":
-            for layer in self.layers:
-                layer.attention.kv_cache.prefill_len.fill_(position)
+    def _decode_lengths(self) -> list:
+        return [y.attention.kv_cache.prefill_len for y in self.layers] if self._mode == "sparse" else []
