@@ -99,6 +99,13 @@ constexpr float TANH_POLY_RANGE = 0.5f;
 constexpr double TANH_POLY[5] = {0.999999987, -0.333330719, 0.13324829, -0.0529892412, 0.017141319};
 __device__ __forceinline__ float softplus_f32(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 
+// Positions by a chunk or a ring: 64-bit division is some hundred instructions in a row, and positions are rarely that large
+__device__ __forceinline__ int64_t position_div(int64_t i, int n) {
+    return (uint64_t)i >> 32 == 0 ? (int64_t)((uint32_t)i / (uint32_t)n) : i / n;
+}
+__device__ __forceinline__ int64_t position_mod(int64_t i, int n) {
+    return (uint64_t)i >> 32 == 0 ? (int64_t)((uint32_t)i % (uint32_t)n) : i % n;
+}
 // position of the first token of a portion: on the device (decode) or given by the host
 __device__ __forceinline__ int64_t first_position(const int64_t* pos, int64_t start) { return pos != nullptr ? pos[0] : start; }
 

@@ -83,14 +83,22 @@ mlstm_finish_kernel(sk_mlstm_params p) {
     __shared__ float red[32];
     const int64_t row = blockIdx.x;
     const int h = blockIdx.y, nt = blockDim.x, t = threadIdx.x;
-    const float inv_den = 1.f / p.den[row * p.H + h];
     const T* num = (const T*)p.num + (row * p.H + h) * p.P;
     float v[NV][V], ss = 0.f;
+    Raw<T, V> ww[NV], zw[NV];                                     // requested with the rows
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
         const int i = (n * nt + t) * V;
         if (i < p.P) {
             load_vec<T, V>(num + i, v[n]);
+            ww[n] = load_raw<T, V>((const T*)p.norm_w + h * p.P + i);
+            zw[n] = load_raw<T, V>((const T*)p.z + row * p.in_ld + (int64_t)h * p.P + i);
+        }
+    }
+    const float inv_den = 1.f / p.den[row * p.H + h];
+#pragma unroll
+    for (int n = 0; n < NV; ++n) {
+        if ((n * nt + t) * V < p.P) {
 #pragma unroll
             for (int e = 0; e < V; ++e) {
                 v[n][e] *= inv_den;
@@ -107,17 +115,59 @@ mlstm_finish_kernel(sk_mlstm_params p) {
     for (int n = 0; n < NV; ++n) {
         const int i = (n * nt + t) * V;
         if (i < p.P) {
-            float w[V], z[V];
-            load_vec<T, V>((const T*)p.norm_w + h * p.P + i, w);
-            load_vec<T, V>((const T*)p.z + row * p.in_ld + (int64_t)h * p.P + i, z);
 #pragma unroll
-            for (int e = 0; e < V; ++e) v[n][e] *= inv * w[e] * sigmoid_scaled<T>(z[e], 1.f);
+            for (int e = 0; e < V; ++e) v[n][e] *= inv * to_f32(ww[n].e[e]) * sigmoid_scaled<T>(to_f32(zw[n].e[e]), 1.f);
             store_vec<T, V>((T*)p.out + row * p.out_ld + (int64_t)h * p.P + i, v[n]);
         }
     }
 }
 
+// A prompt's rows with values of up to 256 elements, a warp per (token, head) and eight of them per block: with a block each, 256000
+// blocks of one warp took 153 us where their bytes take 60 (now 120).
+__global__ void __launch_bounds__(256)
+mlstm_finish_warps_kernel(sk_mlstm_params p) {
+    pdl_begin();
+    using T = __nv_bfloat16;
+    const uint32_t n = blockIdx.x * 8 + (threadIdx.x >> 5);       // below 2^32: the caller's rule
+    const int lane = threadIdx.x & 31, i = lane * 8;
+    if (n >= (uint32_t)p.B * p.S * p.H) return;
+    const uint32_t r32 = n / (uint32_t)p.H, seq = r32 / (uint32_t)p.S;
+    const int64_t row = r32;
+    const int h = (int)(n - r32 * p.H);
+    const bool live = i < p.P;
+    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    Raw<T, 8> ww, zw;
+    if (live) {
+        load_vec<T, 8>((const T*)p.num + (int64_t)n * p.P + i, v);
+        ww = load_raw<T, 8>((const T*)p.norm_w + h * p.P + i);
+        zw = load_raw<T, 8>((const T*)p.z + row * p.in_ld + (int64_t)h * p.P + i);
+    }
+    const float inv_den = 1.f / p.den[n];
+    float ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        v[e] *= inv_den;
+        ss = fmaf(v[e], v[e], ss);
+    }
+    if (lane == 0 && r32 - seq * p.S == (uint32_t)p.S - 1) {
+        const int64_t head = (int64_t)seq * p.H + h;
+        p.m_state[head] = p.m_next[head];
+    }
+    const float inv = 1.f / sqrtf(warp_sum(ss) / (float)p.P + p.eps);
+    if (live) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] *= inv * to_f32(ww.e[e]) * sigmoid_scaled<T>(to_f32(zw.e[e]), 1.f);
+        store_vec<T, 8>((T*)p.out + row * p.out_ld + (int64_t)h * p.P + i, v);
+    }
+}
+
 template <typename T, int V> int finish_dispatch(const sk_mlstm_params& p, cudaStream_t st) {
+    if constexpr (V == 8) {
+        const int64_t warps = (int64_t)p.B * p.S * p.H;
+        if (p.P <= 256 && warps > 4 * 148 * 8 && warps < (int64_t)1 << 32)
+            return check_chained(launch_after(mlstm_finish_warps_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, st, p),
+                                 "mlstm_finish_warps_kernel");
+    }
     const int vecs = (p.P + V - 1) / V;
     int nt = 256;
     while (nt > 32 && nt / 2 >= vecs) nt /= 2;

@@ -29,10 +29,12 @@ embed_rows_kernel(const int64_t* __restrict__ tokens, const T* __restrict__ tabl
 // One CTA per row; the row lives in registers (NV vectors of V elements per thread).
 //   in_mode  0: x stays; 1: x += rms(y) * w_in; 2: x = y + w_in; 3: x += y
 //   out_mode 0: nothing; 1: out = rms(x) * w_out; 2: out = [x ; x0]; 3: out = layer norm of x * w_out
-// A decoded token's rows are bound by latency, a prompt's by memory.  Everything the kernel reads is requested at once: with
-// each norm's weights requested behind its sum, a row of 4096 waited for memory three times.
+// A decoded token's rows (NV = 1) are bound by latency: everything is requested at once, as with each norm's weights requested
+// behind its sum a row of 4096 waited for memory three times.  A prompt's are bound by memory, and the registers that would hold
+// the weights keep rows in flight instead; vectors of 8 leave every other 16 bytes of the fp32 stream to a second access
+// (8000 rows of 4096: 125 us, so 95).
 template <typename T, typename TY, int V, int NV>
-__global__ void __launch_bounds__(V == 8 ? 512 : 1024)
+__global__ void __launch_bounds__(1024)
 residual_norm_kernel(sk_residual_params p) {
     __shared__ float red[3][32];
     const int64_t row = blockIdx.x;
@@ -43,7 +45,7 @@ residual_norm_kernel(sk_residual_params p) {
     const T* w_out = (const T*)p.w_out;
     const TY* yr = (const TY*)p.y + row * p.y_ld;
     const bool norm_out = p.out_mode == 1 || p.out_mode == 3;
-    constexpr bool EARLY = NV * V <= 16;                  // else the weights' registers would be spilled
+    constexpr bool EARLY = NV == 1;
     Raw<TY, V> yw[NV];
     Raw<float, V> xw[NV];
     Raw<T, V> wi[NV], wo[NV];
@@ -172,21 +174,29 @@ glu_kernel(const T* gate, const T* up, int64_t rows, int ff, int64_t ld, float l
 
 // The newest tokens of a portion, from token s0 on, into a ring of `ring` rows (row of position p: p % ring).
 // s0 leaves out what no later token sees, so that no two tokens of a portion meet in one row.
-template <typename T>
+// E: the unit of a copy, as large as rows and strides allow: 4096 tokens of 1024 + 1024 elements of 2 bytes in 14 us, one element at
+// a time 34
+template <typename E>
 __global__ void __launch_bounds__(256)
-ring_append_kernel(const T* k, const T* v, int64_t k_bs, int64_t k_ss, int64_t v_bs,
+ring_append_kernel(const E* k, const E* v, int64_t k_bs, int64_t k_ss, int64_t v_bs,
                    int64_t v_ss, int k_row, int v_row, int ring, const int64_t* pos, int64_t start, int s0,
-                   T* __restrict__ k_cache, T* __restrict__ v_cache) {
+                   E* __restrict__ k_cache, E* __restrict__ v_cache) {
     pdl_begin();
     const int s = s0 + blockIdx.x, b = blockIdx.y;
-    const int64_t slot = (first_position(pos, start) + s) % ring;
-    const T* ks = k + b * k_bs + s * k_ss;
-    T* kd = k_cache + ((int64_t)b * ring + slot) * k_row;
-    for (int i = threadIdx.x; i < k_row; i += blockDim.x) kd[i] = ks[i];
-    if (v != nullptr) {
-        const T* vs = v + b * v_bs + s * v_ss;
-        T* vd = v_cache + ((int64_t)b * ring + slot) * v_row;
-        for (int i = threadIdx.x; i < v_row; i += blockDim.x) vd[i] = vs[i];
+    const E* ks = k + b * k_bs + s * k_ss;
+    const E* vs = v + b * v_bs + s * v_ss;                    // v_row is zero without values
+    const int i = threadIdx.x, j = i - k_row;                 // the first piece is requested with the position
+    E first;
+    if (i < k_row) first = ks[i];
+    else if (j < v_row) first = vs[j];
+    const int64_t slot = position_mod(first_position(pos, start) + s, ring);
+    E* kd = k_cache + ((int64_t)b * ring + slot) * k_row;
+    E* vd = v_cache + ((int64_t)b * ring + slot) * v_row;
+    if (i < k_row) kd[i] = first;
+    else if (j < v_row) vd[j] = first;
+    for (int n = i + blockDim.x; n < k_row + v_row; n += blockDim.x) {
+        if (n < k_row) kd[n] = ks[n];
+        else vd[n - k_row] = vs[n - k_row];
     }
 }
 
@@ -194,10 +204,9 @@ template <typename T, typename TY, int V>
 int residual_dispatch(const sk_residual_params& p, cudaStream_t st) {
     const int vecs = (p.width + V - 1) / V;
     // few rows: one vector per thread (latency); many rows: smaller blocks, more of them per SM
-    const int most = V == 8 ? 512 : 1024;
-    int nt = p.rows < 296 ? most : 256;
+    int nt = p.rows < 296 ? 1024 : 256;
     while (nt > 32 && nt / 2 >= vecs) nt /= 2;
-    while (nt < most && (vecs + nt - 1) / nt > 8) nt *= 2;
+    while (nt < 1024 && (vecs + nt - 1) / nt > 8) nt *= 2;
     const int nv = (vecs + nt - 1) / nt;
     dim3 grid((unsigned)p.rows);
     void (*kern)(sk_residual_params) = nullptr;
@@ -226,10 +235,6 @@ int launch_residual_norm(const sk_residual_params& p, cudaStream_t st) {
     const bool v4 = p.width % 4 == 0 && p.y_ld % 4 == 0;
     if (p.dtype == SK_F32) return v4 ? residual_dispatch<float, float, 4>(p, st) : residual_dispatch<float, float, 1>(p, st);
     using bf = __nv_bfloat16;
-    // rows of 16-byte pieces: half the threads and instructions
-    const bool v8 = p.width % 8 == 0 && p.y_ld % 8 == 0 && p.width <= 8 * 512 * 8 &&
-                    ((uintptr_t)p.x | (uintptr_t)p.y | (uintptr_t)p.w_in | (uintptr_t)p.w_out | (uintptr_t)p.x0 | (uintptr_t)p.out) % 16 == 0;
-    if (v8) return p.y_dtype == SK_F32 ? residual_dispatch<bf, float, 8>(p, st) : residual_dispatch<bf, bf, 8>(p, st);
     if (p.y_dtype == SK_F32) return v4 ? residual_dispatch<bf, float, 4>(p, st) : residual_dispatch<bf, float, 1>(p, st);
     return v4 ? residual_dispatch<bf, bf, 4>(p, st) : residual_dispatch<bf, bf, 1>(p, st);
 }
@@ -261,14 +266,20 @@ int launch_ring_append(const void* k, const void* v, int dtype, int B, int S, in
     // first position to write: of the last block of `ring` positions, or of the last `ring` positions
     const int64_t first = keep == SKB_RING_CHUNK ? (start + S - 1) / ring * ring : start + S - ring;
     const int s0 = pos == nullptr && first > start ? (int)(first - start) : 0;   // a device position: one token
-    dim3 grid((unsigned)(S - s0), (unsigned)B);
-    if (dtype == SK_BF16)
-        return check_chained(launch_after(ring_append_kernel<__nv_bfloat16>, grid, dim3(256), 0, st, (const __nv_bfloat16*)k,
-                                          (const __nv_bfloat16*)v, k_bs, k_ss, v_bs, v_ss, k_row, v_row, ring, pos, start, s0,
-                                          (__nv_bfloat16*)k_cache, (__nv_bfloat16*)v_cache), "ring_append_kernel");
-    return check_chained(launch_after(ring_append_kernel<float>, grid, dim3(256), 0, st, (const float*)k, (const float*)v, k_bs, k_ss,
-                                      v_bs, v_ss, k_row, v_row, ring, pos, start, s0, (float*)k_cache, (float*)v_cache),
-                         "ring_append_kernel");
+    const int es = dtype == SK_BF16 ? 2 : 4, e16 = 16 / es;
+    const bool vec = k_row % e16 == 0 && k_bs % e16 == 0 && k_ss % e16 == 0 && ((uintptr_t)k | (uintptr_t)k_cache) % 16 == 0 &&
+                     (v == nullptr || (v_row % e16 == 0 && v_bs % e16 == 0 && v_ss % e16 == 0 && ((uintptr_t)v | (uintptr_t)v_cache) % 16 == 0));
+    if (v == nullptr) v_row = 0;
+    auto run = [&](auto unit, int per) {                       // `per` elements in a unit
+        using E = decltype(unit);
+        const int pieces = k_row / per + v_row / per;
+        const unsigned nt = pieces >= 256 ? 256u : (unsigned)((pieces + 31) / 32 * 32);
+        return check_chained(launch_after(ring_append_kernel<E>, dim3((unsigned)(S - s0), (unsigned)B), dim3(nt), 0, st, (const E*)k,
+                                          (const E*)v, k_bs / per, k_ss / per, v_bs / per, v_ss / per, k_row / per, v_row / per, ring, pos,
+                                          start, s0, (E*)k_cache, (E*)v_cache), "ring_append_kernel");
+    };
+    if (vec) return run(uint4{}, e16);
+    return dtype == SK_BF16 ? run(uint16_t{}, 1) : run(uint32_t{}, 1);
 }
 
 }  // namespace sk

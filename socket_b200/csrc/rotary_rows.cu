@@ -19,7 +19,7 @@ rotary_rows_kernel(const sk_rotary_rows_params p) {
     const int64_t first = first_position(p.pos, p.start);
     T* rows = (T*)p.rows_out + (int64_t)b * p.rows_cap * p.G * hrow;
     if (row < p.prev) {
-        const int64_t slot = (first - p.prev + row) % p.ring_rows;
+        const int64_t slot = position_mod(first - p.prev + row, p.ring_rows);
         const T* src = (const T*)p.ring + ((int64_t)b * p.ring_rows + slot) * p.G * hrow;
         for (int i = t * V; i < p.G * hrow; i += RR_THREADS * V) {
             float r[V];
@@ -34,7 +34,7 @@ rotary_rows_kernel(const sk_rotary_rows_params p) {
         if (t == 0 && p.status != nullptr) atomicOr(p.status, SK_DEV_POS_OUT_OF_RANGE);
         return;
     }
-    T* dst_row = rows + (p.pos != nullptr ? i % p.rows_cap : row) * p.G * hrow;
+    T* dst_row = rows + (p.pos != nullptr ? position_mod(i, p.rows_cap) : row) * p.G * hrow;
     const int64_t in = ((int64_t)b * p.S + s) * p.in_ld;
     const float* cs = p.angles + i * rot;                    // [half][cos, sin]
     const int n_rest = rest / V, per = n_rest + half / V;    // vectors of a head: unturned ones, then pairs

@@ -10,7 +10,7 @@ namespace {
 // ---------------------------------------------------------------- convolution
 // in  = the [x | B | C] columns of the input projection, rows `ld` apart
 // One thread: V channels of CONV_TOK consecutive tokens.
-constexpr int CONV_TOK = 16;
+constexpr int CONV_TOK = 32;
 
 template <typename T, int V>
 __device__ __forceinline__ void conv_tap_input(const sk_ssm_params& p, int b, int s, int ch, bool fresh, int channels, float (&r)[V]) {
@@ -46,11 +46,19 @@ ssm_conv_kernel(sk_ssm_params p) {
             for (int e = 0; e < V; ++e) wt[j][e] = to_f32(w[(int64_t)(ch + e) * K + j]);
 #pragma unroll
         for (int j = 1; j < K; ++j) conv_tap_input<T, V>(p, b, s0 - K + j, ch, fresh, channels, win[j]);
-        constexpr int U = 4;                                      // tokens requested together
-        for (int s = s0; s < s1; s += U) {
-            float in[U][V];
+        // four tokens are computed while the next four are on their way, in the type they come in (8 channels of four tokens
+        // in fp32 are 32 registers): 8000 tokens of 10240 channels in 96 us, in 183 with the requests of a group behind the last
+        constexpr int U = 4;
+        const T* in0 = (const T*)p.xbc_in + (int64_t)b * p.S * p.in_ld + ch;
+        Raw<T, V> cur[U], nxt[U];
+        auto request = [&](int s, Raw<T, V> (&r)[U]) {
 #pragma unroll
-            for (int u = 0; u < U; ++u) conv_tap_input<T, V>(p, b, s + u < s1 ? s + u : s1 - 1, ch, fresh, channels, in[u]);
+            for (int u = 0; u < U; ++u) r[u] = load_raw<T, V>(in0 + (int64_t)(s + u < s1 ? s + u : s1 - 1) * p.in_ld);
+        };
+        request(s0, cur);
+#pragma unroll 1
+        for (int s = s0; s < s1; s += U) {
+            if (s + U < s1) request(s + U, nxt);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 float acc[V];
@@ -58,7 +66,7 @@ ssm_conv_kernel(sk_ssm_params p) {
                 for (int e = 0; e < V; ++e) {
 #pragma unroll
                     for (int j = 0; j + 1 < K; ++j) win[j][e] = win[j + 1][e];
-                    win[K - 1][e] = in[u][e];
+                    win[K - 1][e] = to_f32(cur[u].e[e]);
                     acc[e] = bias[e];
 #pragma unroll
                     for (int j = 0; j < K; ++j) acc[e] = fmaf(wt[j][e], win[j][e], acc[e]);
@@ -66,6 +74,8 @@ ssm_conv_kernel(sk_ssm_params p) {
                 }
                 if (s + u < s1) store_vec<T, V>((T*)p.xbc + ((int64_t)b * p.S + s + u) * p.xbc_ld + ch, acc);
             }
+#pragma unroll
+            for (int u = 0; u < U; ++u) cur[u] = nxt[u];
         }
     } else
     for (int s = s0; s < s1; ++s) {
@@ -180,6 +190,10 @@ gated_group_norm_kernel(const T* y, const T* z, int64_t z_ld, const T* w, int in
     const int64_t row = blockIdx.x;
     const int c0 = blockIdx.y * part, nt = blockDim.x, t = threadIdx.x;
     float v[NV][V], ss = 0.f;
+    Raw<T, V> ww[NV];                                             // requested with the rows
+#pragma unroll
+    for (int n = 0; n < NV; ++n)
+        if ((n * nt + t) * V < part) ww[n] = load_raw<T, V>(w + c0 + (n * nt + t) * V);
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
         const int i = (n * nt + t) * V;
@@ -199,10 +213,8 @@ gated_group_norm_kernel(const T* y, const T* z, int64_t z_ld, const T* w, int in
     for (int n = 0; n < NV; ++n) {
         const int i = (n * nt + t) * V;
         if (i < part) {
-            float ww[V];
-            load_vec<T, V>(w + c0 + i, ww);
 #pragma unroll
-            for (int e = 0; e < V; ++e) v[n][e] *= inv * ww[e];
+            for (int e = 0; e < V; ++e) v[n][e] *= inv * to_f32(ww[n].e[e]);
             store_vec<T, V>(out + row * inner + c0 + i, v[n]);
         }
     }
@@ -244,7 +256,8 @@ template <typename T> int conv_dispatch(const sk_ssm_params& p, cudaStream_t st)
     };
     const int V = p.S == 1 ? 1 : sizeof(T) == 2 && vec(8) && p.taps == 4 ? 8 : (vec(4) ? 4 : 1);
     dim3 grid((unsigned)((channels + 128 * V - 1) / (128 * V)), (unsigned)((p.S + CONV_TOK - 1) / CONV_TOK), (unsigned)p.B);
-    auto kern = V == 4 && p.taps == 4 ? ssm_conv_kernel<T, 4, 4> : V == 4 ? ssm_conv_kernel<T, 4, 0> : ssm_conv_kernel<T, 1, 0>;
+    auto kern = V == 4 && p.taps == 4 ? ssm_conv_kernel<T, 4, 4> : V == 4 ? ssm_conv_kernel<T, 4, 0>
+              : p.taps == 4 ? ssm_conv_kernel<T, 1, 4> : ssm_conv_kernel<T, 1, 0>;
     if constexpr (sizeof(T) == 2)
         if (V == 8) kern = ssm_conv_kernel<T, 8, 4>;
     if (int rc = check_chained(launch_after(kern, grid, dim3(128), 0, st, p), "ssm_conv_kernel")) return rc;
