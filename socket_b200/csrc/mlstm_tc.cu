@@ -4,8 +4,10 @@
 //   num_t = 2^(m_in - M_t) q_t^T S_in + sum_{s <= t} 2^(a_s - M_t) (q_t . k_s) v_s         (n likewise, with v = 1)
 //   S_out = 2^(m_in - M_end) S_in + sum_s 2^(a_s - M_end) k_s v_s^T,    m_out = b_end + M_end
 // 1. gates: a, A, b of every chunk;  2. sums: sum_s 2^(a_s - A_end) k_s;  3. carry: m_in and n_in of every chunk, in order.
-// 4. states: a CTA owns 128 x 64 elements of one head's S in tensor memory and walks the chunks in order; K comes by
-//    TMA, the weighted values are made by four warps, and the state a chunk starts with goes to memory by TMA.
+// 4. states: a CTA owns 128 x 64 elements of one head's S in registers and walks the chunks in order; K comes by TMA, the
+//    weighted values are made by eight warps, the products of a chunk run ahead of the state (they do not depend on it), so
+//    that the chain from chunk to chunk is a multiply-add; the state a chunk starts with goes to memory by TMA.  8000 tokens,
+//    32 heads of 128 x 128: 367 us (445 with the state in tensor memory, where a chunk's products waited for the one before).
 // 5. outputs: every (chunk, head, 128 value columns) by itself: scores Q K^T, weights back into tensor memory,
 //    Q S_in beside them, weights times V, and the two parts joined in fp32.
 // Whatever carries a gate or the state enters a product as two bf16 numbers, value and remainder (16 significant
@@ -159,12 +161,14 @@ mlstm_tc_carry_kernel(const __grid_constant__ MtShape p) {
 
 // ---------------------------------------------------------------- states
 constexpr int ST_P = 64;                                      // value columns of a CTA; 128 key columns
-constexpr int ST_THREADS = 288;                               // warps 0-3: tensor memory; 4-7: weighted values; 8: TMA and MMA
-constexpr int ST_KSTAGES = 4;                                 // chunks of K in flight
-constexpr uint32_t ST_SMEM = (ST_KSTAGES + 2 + 1) * 2 * MT_PANEL + 1024;   // K; two stages of weighted V; the outgoing state
+// warps 0-7: the state; 8-15: weighted values; 16: MMA; 17: TMA.  Two of each kind per scheduler: alone on one, a warp issues every
+// fifth cycle, and four warps of either kind took as long for a chunk as everything else
+constexpr int ST_MMA_WARP = 16, ST_TMA_WARP = 17, ST_THREADS = 18 * 32;
+constexpr int ST_KSTAGES = 3;                                 // chunks of K in flight
+constexpr uint32_t ST_SMEM = (ST_KSTAGES + 2 + 2) * 2 * MT_PANEL + 1024;   // K; two stages of weighted V and of the outgoing state
 
 struct StShared {
-    uint64_t k_full[ST_KSTAGES], v_full[2], v_empty[2], s_ready, mma_done, drained;
+    uint64_t k_full[ST_KSTAGES], k_empty[ST_KSTAGES], v_full[2], v_empty[2], u_full[2], u_empty[2], drained;
     uint32_t tmem_base;
     int failed;
 };
@@ -176,13 +180,13 @@ __device__ __forceinline__ void split8(const float (&x)[8], uint4& hi, uint4& lo
     split_bf16(x[6], x[7], hi.w, lo.w);
 }
 
-// barrier 1 of 128 threads, and whether `ok` held for all of them
-__device__ __forceinline__ bool all_of_128(bool ok) {
+// barrier 1 of 256 threads, and whether `ok` held for all of them
+__device__ __forceinline__ bool all_of_256(bool ok) {
     uint32_t r;
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 p, %1, 0;\n\t"
-        "bar.red.and.pred q, 1, 128, p;\n\t"
+        "bar.red.and.pred q, 1, 256, p;\n\t"
         "selp.u32 %0, 1, 0, q;\n\t}"
         : "=r"(r)
         : "r"(ok ? 1u : 0u)
@@ -197,25 +201,28 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     __shared__ StShared sh;
     char* k_s = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(st_raw) + 1023) & ~(uintptr_t)1023);   // [stage][panel]
     char* v_s = k_s + ST_KSTAGES * 2 * MT_PANEL;              // [stage][value, remainder]
-    char* o_s = v_s + 2 * 2 * MT_PANEL;                       // [value, remainder]
+    char* o_s = v_s + 2 * 2 * MT_PANEL;                       // [stage][value, remainder]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int p0 = blockIdx.x * ST_P, n0 = blockIdx.y * 128, b = blockIdx.z / p.H, h = blockIdx.z - b * p.H;
     const int64_t head = (int64_t)b * p.H + h;
     volatile int* failed = &sh.failed;
     if (tid == 0) {
-        for (int s = 0; s < ST_KSTAGES; ++s) mbar_init_count(&sh.k_full[s], 1);
-        for (int s = 0; s < 2; ++s) {
-            mbar_init_count(&sh.v_full[s], 4);
-            mbar_init_count(&sh.v_empty[s], 1);
+        for (int s = 0; s < ST_KSTAGES; ++s) {
+            mbar_init_count(&sh.k_full[s], 1);
+            mbar_init_count(&sh.k_empty[s], 1);
         }
-        mbar_init_count(&sh.s_ready, 4);
-        mbar_init_count(&sh.mma_done, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init_count(&sh.v_full[s], 8);
+            mbar_init_count(&sh.v_empty[s], 1);
+            mbar_init_count(&sh.u_full[s], 1);
+            mbar_init_count(&sh.u_empty[s], 8);
+        }
         mbar_init_count(&sh.drained, 1);
         sh.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 8) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sh.tmem_base)), "r"(64u)
+    if (warp == ST_MMA_WARP) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sh.tmem_base)), "r"(256u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -226,94 +233,88 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
     const float* top_end = p.top + head * p.chunks * MT_TOK + MT_TOK - 1;      // A_end of chunk c: [c * 128]
     const float* m_in = p.m_in + head * p.chunks;
 
-    if (warp < 4) {
-        // ---- the state between two chunks: thread = key column
-        const int r = warp * 32 + lane, n = n0 + r;
-        const uint32_t row = tmem + ((uint32_t)(warp * 32) << 16);
-        float* gst = p.S_state + (head * p.N + n) * p.P + p0;
-        const int cols = n >= p.N ? 0 : (p.P - p0 < ST_P ? p.P - p0 : ST_P);
-        float mi = m_in[0], tp = top_end[0];
+    if (warp < 8) {
+        // ---- the state: a key column and half of the value columns per thread
+        const int half = warp >> 2, r = (warp & 3) * 32 + lane, n = n0 + r, c0 = p0 + half * 32;
+        const uint32_t row = tmem + ((uint32_t)((warp & 3) * 32) << 16) + half * 32;
+        float* gst = p.S_state + (head * p.N + n) * p.P + c0;
+        const int cols = n >= p.N ? 0 : (p.P - c0 < 32 ? p.P - c0 : 32);
+        float mi = m_in[0], tp = top_end[0], s[32];
         bool ok = true;
-        for (int c = 0; c <= p.chunks; ++c) {
-            float s[2][32];
-            if (c > 0) ok = *failed == 0 && mbar_wait_bounded(&sh.mma_done, (uint32_t)((c - 1) & 1));
-            // the copy before has left the buffer; and the four warps agree on whether to go on
-            if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-            ok = all_of_128(ok);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) s[j] = p.start > 0 && j < cols ? gst[j] : 0.f;
+#pragma unroll 1
+        for (int c = 0; c < p.chunks; ++c) {
+            const int st = c & 1;
+            // the copy before the last has left its buffer; and the eight warps agree on whether to go on
+            if (tid == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            ok = all_of_256(ok && *failed == 0);
             if (!ok) break;
-            if (c == 0) {
-#pragma unroll
-                for (int j = 0; j < 64; ++j) s[j >> 5][j & 31] = p.start > 0 && j < cols ? gst[j] : 0.f;
-            } else {
-                tc_fence_after();
-                tmem_ld32(row, reinterpret_cast<uint32_t(&)[32]>(s[0]));
-                tmem_ld32(row + 32, reinterpret_cast<uint32_t(&)[32]>(s[1]));
-            }
-            if (c == p.chunks) {                              // what the portion leaves
-#pragma unroll
-                for (int j = 0; j < 64; j += 8)
-                    if (j < cols) {                           // P is a multiple of 8
-                        *reinterpret_cast<float4*>(gst + j) = make_float4(s[j >> 5][j & 31], s[j >> 5][(j & 31) + 1], s[j >> 5][(j & 31) + 2], s[j >> 5][(j & 31) + 3]);
-                        *reinterpret_cast<float4*>(gst + j + 4) = make_float4(s[j >> 5][(j & 31) + 4], s[j >> 5][(j & 31) + 5], s[j >> 5][(j & 31) + 6], s[j >> 5][(j & 31) + 7]);
-                    }
-                break;
-            }
-            const float f = exp2f(mi - fmaxf(mi, tp));
-#pragma unroll
-            for (int half = 0; half < 2; ++half) {
-                uint32_t w[32];
-#pragma unroll
-                for (int j = 0; j < 32; ++j) w[j] = __float_as_uint(s[half][j] * f);
-                tmem_st32(row + half * 32, w);
-            }
-            tmem_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&sh.s_ready);
-            if (c + 1 < p.chunks) {
-                mi = m_in[c + 1];
-                tp = top_end[(int64_t)(c + 1) * MT_TOK];
-            }
             // the state the chunk starts with, to memory
+            char* out = o_s + st * 2 * MT_PANEL;
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
+            for (int j = 0; j < 4; ++j) {
                 float x[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e) x[e] = s[j >> 2][(j & 3) * 8 + e];
+                for (int e = 0; e < 8; ++e) x[e] = s[j * 8 + e];
                 uint4 hi, lo;
                 split8(x, hi, lo);
-                char* dst = o_s + r * 128 + ((j ^ (r & 7)) << 4);
+                char* dst = out + r * 128 + (((half * 4 + j) ^ (r & 7)) << 4);
                 *reinterpret_cast<uint4*>(dst) = hi;
                 *reinterpret_cast<uint4*>(dst + MT_PANEL) = lo;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            asm volatile("bar.sync 1, 128;" ::: "memory");
+            asm volatile("bar.sync 1, 256;" ::: "memory");
             if (tid == 0) {
                 const int hc = (int)(head * p.chunks + c);
 #pragma unroll
                 for (int part = 0; part < 2; ++part)
                     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(&map_s),
-                                 "r"(p0), "r"(part), "r"(n0), "r"(hc), "r"(smem_addr(o_s + part * MT_PANEL))
+                                 "r"(p0), "r"(part), "r"(n0), "r"(hc), "r"(smem_addr(out + part * MT_PANEL))
                                  : "memory");
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
+            const float f = exp2f(mi - fmaxf(mi, tp));
+            if (c + 1 < p.chunks) {
+                mi = m_in[c + 1];
+                tp = top_end[(int64_t)(c + 1) * MT_TOK];
+            }
+            ok = __all_sync(FULL, mbar_wait_bounded(&sh.u_full[st], (uint32_t)((c >> 1) & 1)));
+            if (!ok) continue;                                // told to the other warps above
+            tc_fence_after();
+            float u[32];                                      // products with the remainders, then with the values
+            tmem_ld32(row + st * 128 + 64, reinterpret_cast<uint32_t(&)[32]>(u));
+#pragma unroll
+            for (int j = 0; j < 32; ++j) s[j] = fmaf(f, s[j], u[j]);
+            tmem_ld32(row + st * 128, reinterpret_cast<uint32_t(&)[32]>(u));
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sh.u_empty[st]);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) s[j] += u[j];
         }
-        if (!ok) *failed = 1;
+        if (ok) {                                             // what the portion leaves
+#pragma unroll
+            for (int j = 0; j < 32; j += 4)
+                if (j < cols) *reinterpret_cast<float4*>(gst + j) = make_float4(s[j], s[j + 1], s[j + 2], s[j + 3]);     // P is a multiple of 8
+        } else {
+            *failed = 1;
+        }
         if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         tc_fence_before();
-    } else if (warp < 8) {
-        // ---- weighted values: eight lanes along a token's 64 columns, 16 tokens at a time
-        const int vw = warp - 4, piece = lane & 7;
+    } else if (warp < 16) {
+        // ---- weighted values: eight lanes along a token's 64 columns, 32 tokens at a time
+        const int vw = warp - 8, piece = lane & 7;
         const bool live_col = p0 + piece * 8 < p.P;
         const __nv_bfloat16* v = p.v + (int64_t)b * p.S * p.in_ld + (int64_t)h * p.P + p0 + piece * 8;
         const float* a = p.a + head * p.chunks * MT_TOK;
         // a chunk's values are requested two chunks ahead
-        uint4 raw[2][8];
-        float e[2][8], mi[2], tp[2];
-        auto load = [&](int c, uint4 (&r)[8], float (&x)[8], float& m, float& t) {
+        uint4 raw[2][4];
+        float e[2][4], mi[2], tp[2];
+        auto load = [&](int c, uint4 (&r)[4], float (&x)[4], float& m, float& t) {
 #pragma unroll
-            for (int it = 0; it < 8; ++it) {
-                const int s = it * 16 + vw * 4 + (lane >> 3), tok = c * MT_TOK + s;
+            for (int it = 0; it < 4; ++it) {
+                const int s = it * 32 + vw * 4 + (lane >> 3), tok = c * MT_TOK + s;
                 r[it] = live_col && tok < p.S ? __ldg(reinterpret_cast<const uint4*>(v + (int64_t)tok * p.in_ld)) : make_uint4(0, 0, 0, 0);
                 x[it] = a[(int64_t)c * MT_TOK + s];
             }
@@ -337,8 +338,8 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             const float mm = fmaxf(mi[stage], tp[stage]);
             char* dst = v_s + stage * 2 * MT_PANEL;
 #pragma unroll
-            for (int it = 0; it < 8; ++it) {
-                const int s = it * 16 + vw * 4 + (lane >> 3);
+            for (int it = 0; it < 4; ++it) {
+                const int s = it * 32 + vw * 4 + (lane >> 3);
                 const float w = exp2_fast(e[stage][it] - mm);
                 const uint32_t q[4] = {raw[stage][it].x, raw[stage][it].y, raw[stage][it].z, raw[stage][it].w};
                 float x[8];
@@ -358,52 +359,53 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             if (lane == 0) mbar_arrive(&sh.v_full[stage]);
             if (c + 2 < p.chunks) load(c + 2, raw[stage], e[stage], mi[stage], tp[stage]);
         }
-    } else {
-        // ---- K by TMA, MMAs: S += K^T (weighted V).  The warp stays converged, one lane issues (see umma_ss_by)
+    } else if (warp == ST_MMA_WARP) {
+        // ---- MMAs: K^T against the weighted values and their remainders side by side.  The warp stays converged, one lane
+        // issues (see umma_ss_by)
         const bool leader = elect_one();
         auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(FULL, mbar_wait_bounded(bar, parity)) != 0; };
-        auto fetch = [&](int c) {
-            const int s = c % ST_KSTAGES;
-            char* dst = k_s + s * 2 * MT_PANEL;
-            if (leader) {
-                mbar_expect(&sh.k_full[s], 2 * MT_PANEL);
-                for (int q = 0; q < 2; ++q) tma_load_4d(dst + q * MT_PANEL, &map_k, n0 + q * 64, h, c * MT_TOK, b, &sh.k_full[s]);
-            }
-            __syncwarp();
-        };
-        const uint32_t idesc = umma_idesc_bf16(ST_P, true) | UMMA_A_MN;
+        const uint32_t idesc = umma_idesc_bf16(2 * ST_P, true) | UMMA_A_MN;
         const uint64_t k_desc = umma_desc_sw128_mn(smem_addr(k_s), MT_PANEL), v_desc = umma_desc_sw128_mn(smem_addr(v_s), MT_PANEL);
-        int sent = 0;
-        for (; sent < p.chunks && sent < ST_KSTAGES; ++sent) fetch(sent);
         bool ok = true;
-        int c = 0;
-        for (; c < p.chunks && !__any_sync(FULL, *failed != 0); ++c) {
-            const int stage = c & 1;
-            ok = wait_all(&sh.s_ready, (uint32_t)(c & 1));                    // which follows the MMAs of chunk c - 1
-            if (!ok) break;
-            if (c >= 1 && sent < p.chunks) fetch(sent++);                     // into the stage chunk c - 1 has left
-            ok = wait_all(&sh.k_full[c % ST_KSTAGES], (uint32_t)((c / ST_KSTAGES) & 1)) && wait_all(&sh.v_full[stage], (uint32_t)((c >> 1) & 1));
+#pragma unroll 1
+        for (int c = 0; c < p.chunks && !__any_sync(FULL, *failed != 0); ++c) {
+            const int stage = c & 1, ks = c % ST_KSTAGES;
+            ok = wait_all(&sh.k_full[ks], (uint32_t)((c / ST_KSTAGES) & 1)) && wait_all(&sh.v_full[stage], (uint32_t)((c >> 1) & 1)) &&
+                 (c < 2 || wait_all(&sh.u_empty[stage], (uint32_t)(((c >> 1) - 1) & 1)));
             if (!ok) break;
             tc_fence_after();
-            const uint64_t kd = umma_desc_at(k_desc, (c % ST_KSTAGES) * (2 * MT_PANEL >> 4)), vd = umma_desc_at(v_desc, stage * (2 * MT_PANEL >> 4));
+            const uint64_t kd = umma_desc_at(k_desc, ks * (2 * MT_PANEL >> 4)), vd = umma_desc_at(v_desc, stage * (2 * MT_PANEL >> 4));
 #pragma unroll
-            for (int part = 0; part < 2; ++part)
-#pragma unroll
-                for (int k = 0; k < MT_TOK / 16; ++k)
-                    umma_ss_by(leader, tmem, umma_desc_at(kd, k * (2048 >> 4)), umma_desc_at(vd, part * (MT_PANEL >> 4) + k * (2048 >> 4)), idesc, 1);
-            umma_commit_by(leader, &sh.mma_done);
+            for (int k = 0; k < MT_TOK / 16; ++k)
+                umma_ss_by(leader, tmem + stage * 128, umma_desc_at(kd, k * (2048 >> 4)), umma_desc_at(vd, k * (2048 >> 4)), idesc, k > 0);
+            umma_commit_by(leader, &sh.u_full[stage]);
             umma_commit_by(leader, &sh.v_empty[stage]);
+            umma_commit_by(leader, &sh.k_empty[ks]);
         }
         if (!ok && lane == 0) *failed = 1;
-        if (c < p.chunks)                                     // left early: no copy stays in flight
-            for (int q = c; q < sent; ++q) mbar_wait_bounded(&sh.k_full[q % ST_KSTAGES], (uint32_t)((q / ST_KSTAGES) & 1));
         umma_commit_by(leader, &sh.drained);
         mbar_wait_bounded(&sh.drained, 0);
+    } else if (warp == ST_TMA_WARP && lane == 0) {
+        // ---- K by TMA
+        int c = 0;
+        for (; c < p.chunks && !*failed; ++c) {
+            const int s = c % ST_KSTAGES;
+            if (c >= ST_KSTAGES && !mbar_wait_bounded(&sh.k_empty[s], (uint32_t)((c / ST_KSTAGES - 1) & 1))) {
+                *failed = 1;
+                break;
+            }
+            char* dst = k_s + s * 2 * MT_PANEL;
+            mbar_expect(&sh.k_full[s], 2 * MT_PANEL);
+            for (int q = 0; q < 2; ++q) tma_load_4d(dst + q * MT_PANEL, &map_k, n0 + q * 64, h, c * MT_TOK, b, &sh.k_full[s]);
+        }
+        if (c < p.chunks)                                     // left early: no copy stays in flight
+            for (int q = c > ST_KSTAGES ? c - ST_KSTAGES : 0; q < c; ++q)
+                mbar_wait_bounded(&sh.k_full[q % ST_KSTAGES], (uint32_t)((q / ST_KSTAGES) & 1));
     }
     __syncthreads();
     if (tid == 0 && sh.failed && p.status != nullptr) atomicOr(p.status, SK_DEV_WAIT_TIMEOUT);
-    if (warp == 8)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(64u) : "memory");
+    if (warp == ST_MMA_WARP)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
 }
 
 // ---------------------------------------------------------------- outputs
