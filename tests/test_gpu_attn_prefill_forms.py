@@ -64,6 +64,23 @@ def test_forms(S, H, G, D, E, start, kv_start, bias_len, chunk, window, cap, sin
             assert bool(((got[i, h] - want).abs() <= 2.0 ** -8 * mag + 2.0 ** -8 * want.abs() + 1e-6).all()), (i, h)
 
 
+@pytest.mark.parametrize("growth", [0.1, 0.6, -0.6])
+@pytest.mark.parametrize("D,E,window,cap,bias_len", [(128, 128, 0, 0.0, 0), (192, 128, 300, 0.0, 0), (128, 64, 0, 0.0, 90), (64, 128, 0, 900.0, 0)])
+def test_maximum_that_moves(growth, D, E, window, cap, bias_len):
+    """Scores that rise from key to key, so that a tile's first weights are taken again and the sums before are scaled, or fall."""
+    from socket_b200 import block_ops as ops
+    q, k, v, kw = _case(400, 2, 1, D, E, 260, 0, bias_len, 0, window, cap, True, D + E)
+    q[..., 0], k[..., 0] = 8.0, (growth * torch.arange(k.shape[1], device="cuda"))[None, :, None].bfloat16()
+    q[:, ::3, :, 0] = 0.0                                          # every third row as it was, in the same warps
+    kw["scale"] = 0.125
+    got = ops.attn(q, k, v, path="prefill_tc", **kw)[0].double()
+    for i in (0, 1, 2, 95, 127, 128, 255, 256, 300, 398, 399):
+        for h in range(2):
+            want, mag = _plain(q, k, v, kw, i, h)
+            # as above; scores of at most 2^9 in fp32
+            assert bool(((got[i, h] - want).abs() <= 2.0 ** -8 * mag + 2.0 ** -8 * want.abs() + 1e-6).all()), (i, h)
+
+
 @pytest.mark.parametrize("kv_start", [2 ** 31 - 300, 2 ** 31 + 7, 2 ** 40])
 @pytest.mark.parametrize("chunk,window,cap", [(0, 0, 0.0), (0, 200, 30.0), (2 ** 30, 0, 0.0)])
 def test_positions_beyond_two_billion(kv_start, chunk, window, cap):
