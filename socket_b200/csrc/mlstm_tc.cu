@@ -4,10 +4,11 @@
 //   num_t = 2^(m_in - M_t) q_t^T S_in + sum_{s <= t} 2^(a_s - M_t) (q_t . k_s) v_s         (n likewise, with v = 1)
 //   S_out = 2^(m_in - M_end) S_in + sum_s 2^(a_s - M_end) k_s v_s^T,    m_out = b_end + M_end
 // 1. gates: a, A, b of every chunk;  2. sums: sum_s 2^(a_s - A_end) k_s;  3. carry: m_in and n_in of every chunk, in order.
-// 4. states: a CTA owns 128 x 64 elements of one head's S in registers and walks the chunks in order; K comes by TMA, the
+// 4. states: a CTA owns 128 x 16 to 64 elements of one head's S in registers and walks the chunks in order; K comes by TMA, the
 //    weighted values are made by eight warps, the products of a chunk run ahead of the state (they do not depend on it), so
-//    that the chain from chunk to chunk is a multiply-add; the state a chunk starts with goes to memory by TMA.  8000 tokens,
-//    32 heads of 128 x 128: 367 us (445 with the state in tensor memory, where a chunk's products waited for the one before).
+//    that the chain from chunk to chunk is a multiply-add; the state a chunk starts with goes to memory by TMA.  32000 tokens,
+//    8 heads of 128 x 256: 367 us with 64 columns (445 with the state in tensor memory, where a chunk's products waited for the one
+//    before), 200 with 16.
 // 5. outputs: every (chunk, head, 128 value columns) by itself: scores Q K^T, weights back into tensor memory,
 //    Q S_in beside them, weights times V, and the two parts joined in fp32.
 // Whatever carries a gate or the state enters a product as two bf16 numbers, value and remainder (16 significant
@@ -160,12 +161,17 @@ mlstm_tc_carry_kernel(const __grid_constant__ MtShape p) {
 }
 
 // ---------------------------------------------------------------- states
-constexpr int ST_P = 64;                                      // value columns of a CTA; 128 key columns
 // warps 0-7: the state; 8-15: weighted values; 16: MMA; 17: TMA.  Two of each kind per scheduler: alone on one, a warp issues every
 // fifth cycle, and four warps of either kind took as long for a chunk as everything else
 constexpr int ST_MMA_WARP = 16, ST_TMA_WARP = 17, ST_THREADS = 18 * 32;
 constexpr int ST_KSTAGES = 3;                                 // chunks of K in flight
-constexpr uint32_t ST_SMEM = (ST_KSTAGES + 2 + 2) * 2 * MT_PANEL + 1024;   // K; two stages of weighted V and of the outgoing state
+// SP: value columns of a CTA, beside 128 key columns.  Weighted values and their remainders are one operand of 2 SP columns, in panels of 64
+template <int SP> struct StTile {
+    static constexpr uint32_t V_STAGE = MT_PANEL * (SP == 64 ? 2 : 1);
+    static constexpr uint32_t LO = SP == 64 ? MT_PANEL : 0;   // where the remainders begin: a panel further, or SP columns
+    static constexpr uint32_t O_PART = MT_TOK * SP * 2;       // the outgoing state: 128 rows of SP bf16
+    static constexpr uint32_t SMEM = ST_KSTAGES * 2 * MT_PANEL + 2 * V_STAGE + 2 * 2 * O_PART + 1024;
+};
 
 struct StShared {
     uint64_t k_full[ST_KSTAGES], k_empty[ST_KSTAGES], v_full[2], v_empty[2], u_full[2], u_empty[2], drained;
@@ -194,16 +200,19 @@ __device__ __forceinline__ bool all_of_256(bool ok) {
     return r != 0;
 }
 
+template <int SP>
 __global__ void __launch_bounds__(ST_THREADS, 1)
 mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_s,
                        const __grid_constant__ MtShape p) {
+    using Tile = StTile<SP>;
+    constexpr int C = SP / 2;                                 // state columns of a thread
     extern __shared__ char st_raw[];
     __shared__ StShared sh;
     char* k_s = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(st_raw) + 1023) & ~(uintptr_t)1023);   // [stage][panel]
     char* v_s = k_s + ST_KSTAGES * 2 * MT_PANEL;              // [stage][value, remainder]
-    char* o_s = v_s + 2 * 2 * MT_PANEL;                       // [stage][value, remainder]
+    char* o_s = v_s + 2 * Tile::V_STAGE;                       // [stage][value, remainder]
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int p0 = blockIdx.x * ST_P, n0 = blockIdx.y * 128, b = blockIdx.z / p.H, h = blockIdx.z - b * p.H;
+    const int p0 = blockIdx.x * SP, n0 = blockIdx.y * 128, b = blockIdx.z / p.H, h = blockIdx.z - b * p.H;
     const int64_t head = (int64_t)b * p.H + h;
     volatile int* failed = &sh.failed;
     if (tid == 0) {
@@ -235,14 +244,14 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 
     if (warp < 8) {
         // ---- the state: a key column and half of the value columns per thread
-        const int half = warp >> 2, r = (warp & 3) * 32 + lane, n = n0 + r, c0 = p0 + half * 32;
-        const uint32_t row = tmem + ((uint32_t)((warp & 3) * 32) << 16) + half * 32;
+        const int half = warp >> 2, r = (warp & 3) * 32 + lane, n = n0 + r, c0 = p0 + half * C;
+        const uint32_t row = tmem + ((uint32_t)((warp & 3) * 32) << 16) + half * C;
         float* gst = p.S_state + (head * p.N + n) * p.P + c0;
-        const int cols = n >= p.N ? 0 : (p.P - c0 < 32 ? p.P - c0 : 32);
-        float mi = m_in[0], tp = top_end[0], s[32];
+        const int cols = n >= p.N ? 0 : (p.P - c0 < C ? p.P - c0 : C);
+        float mi = m_in[0], tp = top_end[0], s[C];
         bool ok = true;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) s[j] = p.start > 0 && j < cols ? gst[j] : 0.f;
+        for (int j = 0; j < C; ++j) s[j] = p.start > 0 && j < cols ? gst[j] : 0.f;
 #pragma unroll 1
         for (int c = 0; c < p.chunks; ++c) {
             const int st = c & 1;
@@ -251,17 +260,17 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             ok = all_of_256(ok && *failed == 0);
             if (!ok) break;
             // the state the chunk starts with, to memory
-            char* out = o_s + st * 2 * MT_PANEL;
+            char* out = o_s + st * 2 * Tile::O_PART;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
+            for (int j = 0; j < C / 8; ++j) {
                 float x[8];
 #pragma unroll
                 for (int e = 0; e < 8; ++e) x[e] = s[j * 8 + e];
                 uint4 hi, lo;
                 split8(x, hi, lo);
-                char* dst = out + r * 128 + (((half * 4 + j) ^ (r & 7)) << 4);
+                char* dst = out + r * SP * 2 + (((half * (C / 8) + j) ^ (r * SP * 2 >> 7 & (SP / 8 - 1))) << 4);
                 *reinterpret_cast<uint4*>(dst) = hi;
-                *reinterpret_cast<uint4*>(dst + MT_PANEL) = lo;
+                *reinterpret_cast<uint4*>(dst + Tile::O_PART) = lo;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -270,7 +279,7 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 #pragma unroll
                 for (int part = 0; part < 2; ++part)
                     asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.bulk_group [%0, {%1, %2, %3, %4}], [%5];" ::"l"(&map_s),
-                                 "r"(p0), "r"(part), "r"(n0), "r"(hc), "r"(smem_addr(out + part * MT_PANEL))
+                                 "r"(p0), "r"(part), "r"(n0), "r"(hc), "r"(smem_addr(out + part * Tile::O_PART))
                                  : "memory");
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
@@ -282,20 +291,20 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
             ok = __all_sync(FULL, mbar_wait_bounded(&sh.u_full[st], (uint32_t)((c >> 1) & 1)));
             if (!ok) continue;                                // told to the other warps above
             tc_fence_after();
-            float u[32];                                      // products with the remainders, then with the values
-            tmem_ld32(row + st * 128 + 64, reinterpret_cast<uint32_t(&)[32]>(u));
+            float u[C];                                      // products with the remainders, then with the values
+            tmem_ld(row + st * 2 * SP + SP, reinterpret_cast<uint32_t(&)[C]>(u));
 #pragma unroll
-            for (int j = 0; j < 32; ++j) s[j] = fmaf(f, s[j], u[j]);
-            tmem_ld32(row + st * 128, reinterpret_cast<uint32_t(&)[32]>(u));
+            for (int j = 0; j < C; ++j) s[j] = fmaf(f, s[j], u[j]);
+            tmem_ld(row + st * 2 * SP, reinterpret_cast<uint32_t(&)[C]>(u));
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&sh.u_empty[st]);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) s[j] += u[j];
+            for (int j = 0; j < C; ++j) s[j] += u[j];
         }
         if (ok) {                                             // what the portion leaves
 #pragma unroll
-            for (int j = 0; j < 32; j += 4)
+            for (int j = 0; j < C; j += 4)
                 if (j < cols) *reinterpret_cast<float4*>(gst + j) = make_float4(s[j], s[j + 1], s[j + 2], s[j + 3]);     // P is a multiple of 8
         } else {
             *failed = 1;
@@ -303,18 +312,19 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
         tc_fence_before();
     } else if (warp < 16) {
-        // ---- weighted values: eight lanes along a token's 64 columns, 32 tokens at a time
-        const int vw = warp - 8, piece = lane & 7;
+        // ---- weighted values: a lane has eight of a token's columns
+        constexpr int PIECES = SP / 8, TOKS = 32 / PIECES, TURNS = MT_TOK / (8 * TOKS);       // tokens of a warp at a time
+        const int vw = warp - 8, piece = lane % PIECES, own = vw * TOKS + lane / PIECES;
         const bool live_col = p0 + piece * 8 < p.P;
         const __nv_bfloat16* v = p.v + (int64_t)b * p.S * p.in_ld + (int64_t)h * p.P + p0 + piece * 8;
         const float* a = p.a + head * p.chunks * MT_TOK;
         // a chunk's values are requested two chunks ahead
-        uint4 raw[2][4];
-        float e[2][4], mi[2], tp[2];
-        auto load = [&](int c, uint4 (&r)[4], float (&x)[4], float& m, float& t) {
+        uint4 raw[2][TURNS];
+        float e[2][TURNS], mi[2], tp[2];
+        auto load = [&](int c, uint4 (&r)[TURNS], float (&x)[TURNS], float& m, float& t) {
 #pragma unroll
-            for (int it = 0; it < 4; ++it) {
-                const int s = it * 32 + vw * 4 + (lane >> 3), tok = c * MT_TOK + s;
+            for (int it = 0; it < TURNS; ++it) {
+                const int s = it * 8 * TOKS + own, tok = c * MT_TOK + s;
                 r[it] = live_col && tok < p.S ? __ldg(reinterpret_cast<const uint4*>(v + (int64_t)tok * p.in_ld)) : make_uint4(0, 0, 0, 0);
                 x[it] = a[(int64_t)c * MT_TOK + s];
             }
@@ -336,10 +346,10 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 break;
             }
             const float mm = fmaxf(mi[stage], tp[stage]);
-            char* dst = v_s + stage * 2 * MT_PANEL;
+            char* dst = v_s + stage * Tile::V_STAGE;
 #pragma unroll
-            for (int it = 0; it < 4; ++it) {
-                const int s = it * 32 + vw * 4 + (lane >> 3);
+            for (int it = 0; it < TURNS; ++it) {
+                const int s = it * 8 * TOKS + own;
                 const float w = exp2_fast(e[stage][it] - mm);
                 const uint32_t q[4] = {raw[stage][it].x, raw[stage][it].y, raw[stage][it].z, raw[stage][it].w};
                 float x[8];
@@ -350,9 +360,8 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                 }
                 uint4 hi, lo;
                 split8(x, hi, lo);
-                char* d = dst + s * 128 + ((piece ^ (s & 7)) << 4);
-                *reinterpret_cast<uint4*>(d) = hi;
-                *reinterpret_cast<uint4*>(d + MT_PANEL) = lo;
+                *reinterpret_cast<uint4*>(dst + s * 128 + ((piece ^ (s & 7)) << 4)) = hi;
+                *reinterpret_cast<uint4*>(dst + Tile::LO + s * 128 + (((SP == 64 ? piece : piece + PIECES) ^ (s & 7)) << 4)) = lo;
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
@@ -364,7 +373,7 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
         // issues (see umma_ss_by)
         const bool leader = elect_one();
         auto wait_all = [&](uint64_t* bar, uint32_t parity) { return __all_sync(FULL, mbar_wait_bounded(bar, parity)) != 0; };
-        const uint32_t idesc = umma_idesc_bf16(2 * ST_P, true) | UMMA_A_MN;
+        const uint32_t idesc = umma_idesc_bf16(2 * SP, true) | UMMA_A_MN;
         const uint64_t k_desc = umma_desc_sw128_mn(smem_addr(k_s), MT_PANEL), v_desc = umma_desc_sw128_mn(smem_addr(v_s), MT_PANEL);
         bool ok = true;
 #pragma unroll 1
@@ -374,10 +383,10 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
                  (c < 2 || wait_all(&sh.u_empty[stage], (uint32_t)(((c >> 1) - 1) & 1)));
             if (!ok) break;
             tc_fence_after();
-            const uint64_t kd = umma_desc_at(k_desc, ks * (2 * MT_PANEL >> 4)), vd = umma_desc_at(v_desc, stage * (2 * MT_PANEL >> 4));
+            const uint64_t kd = umma_desc_at(k_desc, ks * (2 * MT_PANEL >> 4)), vd = umma_desc_at(v_desc, stage * (Tile::V_STAGE >> 4));
 #pragma unroll
             for (int k = 0; k < MT_TOK / 16; ++k)
-                umma_ss_by(leader, tmem + stage * 128, umma_desc_at(kd, k * (2048 >> 4)), umma_desc_at(vd, k * (2048 >> 4)), idesc, k > 0);
+                umma_ss_by(leader, tmem + stage * 2 * SP, umma_desc_at(kd, k * (2048 >> 4)), umma_desc_at(vd, k * (2048 >> 4)), idesc, k > 0);
             umma_commit_by(leader, &sh.u_full[stage]);
             umma_commit_by(leader, &sh.v_empty[stage]);
             umma_commit_by(leader, &sh.k_empty[ks]);
@@ -691,7 +700,11 @@ int launch_mlstm_tc(const sk_mlstm_params& p, cudaStream_t st) {
     if (int rc = make_head_map(&mq, p.q, p.N, p.H, p.S, p.B, p.N, p.in_ld, bs, MT_TOK)) return rc;
     if (int rc = make_head_map(&mk, p.k, p.N, p.H, p.S, p.B, p.N, p.in_ld, bs, MT_TOK)) return rc;
     if (int rc = make_head_map(&mv, p.v, p.P, p.H, p.S, p.B, p.P, p.in_ld, bs, MT_TOK)) return rc;
-    if (int rc = make_head_map(&ms_out, states, p.P, 2, p.N, (int)hc, np, p.P, 2 * np, MT_TOK)) return rc;
+    // The walk over the chunks is a chain, so a head's state is dealt out to as many CTAs as there is room for: 32000 tokens, 8 heads of
+    // 128 x 256: 200 us with 128 CTAs of 16 columns, 271 with 64 of 32, 367 with 32 of 64.  More CTAs than SMs would walk it twice
+    auto ctas = [&](int sp) { return (int64_t)((p.P + sp - 1) / sp) * ((p.N + 127) / 128) * p.B * p.H; };
+    const int sp = ctas(32) > 148 ? 64 : ctas(16) > 148 ? 32 : 16;
+    if (int rc = make_head_map(&ms_out, states, p.P, 2, p.N, (int)hc, np, p.P, 2 * np, MT_TOK, sp)) return rc;
     if (int rc = make_head_map(&ms_in, states, p.P, 2, p.N, (int)hc, np, p.P, 2 * np, 64)) return rc;
 
     mlstm_tc_gates_kernel<<<dim3((unsigned)chunks, (unsigned)((p.H + MT_GATE_HEADS - 1) / MT_GATE_HEADS), (unsigned)p.B), 256, 0, st>>>(m);
@@ -700,10 +713,12 @@ int launch_mlstm_tc(const sk_mlstm_params& p, cudaStream_t st) {
     if (int rc = check_launch("mlstm_tc_sums_kernel")) return rc;
     mlstm_tc_carry_kernel<<<dim3((unsigned)p.H, (unsigned)p.B), 256, 0, st>>>(m);
     if (int rc = check_launch("mlstm_tc_carry_kernel")) return rc;
-    cudaError_t e = cudaFuncSetAttribute(mlstm_tc_states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ST_SMEM);
+    auto states_kernel = sp == 64 ? mlstm_tc_states_kernel<64> : sp == 32 ? mlstm_tc_states_kernel<32> : mlstm_tc_states_kernel<16>;
+    const uint32_t st_smem = sp == 64 ? StTile<64>::SMEM : sp == 32 ? StTile<32>::SMEM : StTile<16>::SMEM;
+    cudaError_t e = cudaFuncSetAttribute(states_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)st_smem);
     if (e != cudaSuccess) return fail(SK_ERR_CUDA, "mlstm_tc_states_kernel smem attribute: %s", cudaGetErrorString(e));
-    mlstm_tc_states_kernel<<<dim3((unsigned)((p.P + ST_P - 1) / ST_P), (unsigned)((p.N + 127) / 128), (unsigned)(p.B * p.H)), ST_THREADS,
-                             ST_SMEM, st>>>(mk, ms_out, m);
+    states_kernel<<<dim3((unsigned)((p.P + sp - 1) / sp), (unsigned)((p.N + 127) / 128), (unsigned)(p.B * p.H)), ST_THREADS, st_smem, st>>>(
+        mk, ms_out, m);
     if (int rc = check_launch("mlstm_tc_states_kernel")) return rc;
     const uint32_t smem = (uint32_t)((p.N + 63) / 64) * MT_PANEL + OT_STAGES * OT_STAGE + 1024;
     e = cudaFuncSetAttribute(mlstm_tc_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -41,3 +41,25 @@ def test_ring_append_of_every_layout(G, D, E, pad, dtype):
     for s in range(max(first - start, 0), S):
         slot = (start + s) % ring
         assert torch.equal(kc[:, slot], k[:, s]) and torch.equal(vc[:, slot], v[:, s])
+
+
+@pytest.mark.parametrize("N,P,S", [(128, 256, 300), (136, 264, 700), (40, 72, 129), (256, 512, 257)])
+def test_memory_states_of_every_width(N, P, S):
+    """A head's state in parts of 16, 32 and 64 value columns, by how many sequences there are."""
+    H = 8
+    g = torch.Generator(device=DEV).manual_seed(N)
+    r = lambda *s: torch.randn(*s, generator=g, device=DEV)  # noqa: E731
+    base, base_gates = r(S, 2 * H * (N + P)).to(BF16), r(S, 2 * H)
+    bias, w = (torch.zeros(H, device=DEV), torch.full((H,), 3.0, device=DEV)), (1 + 0.1 * r(H * P)).to(BF16)
+
+    def run(B):
+        rows, gates = base.repeat(B, 1), base_gates.repeat(B, 1)
+        q, k, v, z = rows.split([H * N, H * N, H * P, H * P], 1)
+        state = [torch.zeros(B, H, N, P, device=DEV), torch.zeros(B, H, N, device=DEV), torch.zeros(B, H, device=DEV)]
+        out = torch.empty(B * S, H * P, dtype=BF16, device=DEV)
+        ops.mlstm(q, k, v, z, gates, *bias, w, *state, out, S=S, cap=15.0, q_scale=N ** -0.5, eps=1e-5)
+        return out.view(B, S, -1), state[0]
+
+    runs = [run(B) for B in (1, 2, 4, 9)]
+    for out, state in runs[1:]:                                # the same sums in the same order, in every sequence
+        assert torch.equal(out, runs[0][0].expand_as(out)) and torch.equal(state, runs[0][1].expand_as(state))
