@@ -140,13 +140,18 @@ class ChunkedAttention(nn.Module):
             y = ops.attn(q, cache.k, cache.v, pos=at.pos, ring=True, workspace=at.workspace, **args)
         else:
             lo = at.start // self.chunk * self.chunk
-            if lo < at.start:                      # the portion starts inside a chunk: its kept keys come first
-                n = at.start - lo
+            n, end = at.start - lo, at.end - lo
+            kept = 0 < n and end <= cache.k.shape[1]
+            if kept:                               # the portion starts and ends inside a chunk: the ring has all of its rows in order
+                ops.ring_append(k, v, cache.k[:B], cache.v[:B], start=at.start)
+                ka, va = cache.k[:B, :end], cache.v[:B, :end]
+            elif 0 < n:                            # it runs into the next chunk, whose rows replace the kept ones
                 ka, va = torch.cat([cache.k[:B, :n], k], 1), torch.cat([cache.v[:B, :n], v], 1)
             else:
                 ka, va = k, v
             y = ops.attn(q, ka, va, start=at.start, kv_start=lo, **args)
-            ops.ring_append(k, v, cache.k[:B], cache.v[:B], start=at.start)
+            if not kept:
+                ops.ring_append(k, v, cache.k[:B], cache.v[:B], start=at.start)
         return matmul(y.view(B * S, self.H * self.E), self.wo, at.chained)
 
 

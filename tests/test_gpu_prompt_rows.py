@@ -63,3 +63,24 @@ def test_memory_states_of_every_width(N, P, S):
     runs = [run(B) for B in (1, 2, 4, 9)]
     for out, state in runs[1:]:                                # the same sums in the same order, in every sequence
         assert torch.equal(out, runs[0][0].expand_as(out)) and torch.equal(state, runs[0][1].expand_as(state))
+
+
+@pytest.mark.parametrize("start,S,chunk,length", [(5, 40, 64, 256), (5, 59, 64, 256), (5, 60, 64, 256), (70, 50, 64, 256), (60, 100, 64, 256), (9, 70, 512, 100)])
+def test_portion_inside_a_chunk_and_across(start, S, chunk, length):
+    """A portion that attends on the ring's own rows, and one whose rows replace them, against both halves in one portion."""
+    from socket_b200 import mixers
+    torch.manual_seed(S)
+    m = mixers.ChunkedAttention(64, 4, 2, 16, 24, chunk, 0.25, 12, 50.0).to(DEV).to(BF16)
+    for p in m.parameters():
+        p.data.copy_(0.3 * torch.randn_like(p))
+    m.finish_loading()
+    h = torch.randn(2, start + S, 64, device=DEV).to(BF16)
+    whole, parts = (m.make_cache(2, length, BF16, DEV) for _ in range(2))
+    flat = lambda x: x.reshape(-1, 64).contiguous()  # noqa: E731
+    want = m(flat(h), whole, mixers.Portion(2, start + S, 0)).view(2, start + S, -1)
+    m(flat(h[:, :start]), parts, mixers.Portion(2, start, 0))
+    got = m(flat(h[:, start:]), parts, mixers.Portion(2, S, start)).view(2, S, -1)
+    err = (got.float() - want[:, start:].float()).abs().max()
+    assert err <= 2.0 ** -6 * want.float().abs().max(), float(err)               # weights, outputs and the projection in bf16
+    kept = (start + S - 1) % chunk + 1                         # rows of the last token's chunk
+    assert torch.equal(parts.k[:, :kept], whole.k[:, :kept]) and torch.equal(parts.v[:, :kept], whole.v[:, :kept])
