@@ -52,7 +52,7 @@ struct FpShared {
     uint64_t drained;
     uint32_t tmem_base;
     int failed;
-    float xch[FP_TILE * 4];                  // what the two threads of a row tell each other
+    float xch[FP_TILE * 4];                  // what the threads of a row, or the CTAs of a block, tell each other
 };
 
 // Dynamic shared memory: operand tiles, bias, FpShared.  Its start is a multiple of 1024 when there is no static shared
@@ -74,11 +74,40 @@ enum { FP_CAP_NONE = 0, FP_CAP = 1, FP_CAP_BOUND = 2 };
 constexpr float FP_CAP_BOUND_LOG2 = 80.f;
 
 // first key row (counted from kv_start: rows of the call, below 2^30, whatever the positions are) that query row i sees
-__device__ __forceinline__ int fp_first_row(const FpShape& p, int i) {
+__host__ __device__ __forceinline__ int fp_first_row(const FpShape& p, int i) {
     int64_t lo = -p.kv_start;
     if (p.chunk > 0) lo = position_div(i + p.kv_start, p.chunk) * p.chunk - p.kv_start;
     if (p.window > 0 && i - p.window + 1 > lo) lo = i - p.window + 1;
-    return (int)max(lo, (int64_t)0);
+    return (int)(lo > 0 ? lo : 0);
+}
+// the range [beg, end) of key tiles that each of the two query tiles from query q0 on visits; tiles count from key row `base`
+__host__ __device__ __forceinline__ void fp_tiles(const FpShape& p, int q0, int (&i0)[2], int (&beg)[2], int (&end)[2], int& base) {
+    base = 0;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+        const int first = q0 + t * FP_TILE;
+        i0[t] = (int)(p.start - p.kv_start) + first;
+        const int lo = fp_first_row(p, i0[t]);
+        if (t == 0) base = lo;
+        const int rows = p.S - first < FP_TILE ? p.S - first : FP_TILE;
+        beg[t] = (lo - base) / FP_TILE;
+        end[t] = rows > 0 ? (i0[t] + rows - 1 - base) / FP_TILE + 1 : 0;
+        if (rows <= 0) beg[t] = 0;
+    }
+}
+__device__ __forceinline__ float4 load_cta(const void* local, int rank) {      // shared memory of the cluster's CTA `rank`, in its place here
+    uint32_t at;
+    float4 v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_addr(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+    return v;
+}
+__device__ __forceinline__ float load_cta1(const void* local, int rank) {
+    uint32_t at;
+    float v;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(smem_addr(local)), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(at));
+    return v;
 }
 
 // s <- cap_out tanh(s cap_in): two small scores
@@ -120,7 +149,8 @@ template <int N> __device__ __forceinline__ void fp_cap_all(const FpShape& p, fl
     }
 }
 
-template <bool BIAS, int CAP, int PER>
+// SPLIT: CTAs, a cluster, that share a block's keys
+template <bool BIAS, int CAP, int PER, int SPLIT>
 __global__ void __launch_bounds__(FpRoles<PER>::THREADS, 1)
 attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const FpShape p) {
@@ -132,7 +162,8 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // heads side by side, long rows first: the last blocks to start are short ones.  (Heads in groups whose keys and values fit
     // the L2 end in a short group of long rows: 24000 tokens, 16 heads of 192 / 128 in groups of 3: 2975 us, so 2643; 8000
     // tokens, 32 heads in groups of 9: 699 us, so 677.  16000 tokens, 16 heads were 1177 us in groups and are 1207 so.)
-    const int b = blockIdx.y, back = blockIdx.x / p.H, h = blockIdx.x - back * p.H, g = h / (p.H / p.G);
+    const int unit = blockIdx.x / SPLIT, rank = blockIdx.x % SPLIT;
+    const int b = blockIdx.y, back = unit / p.H, h = unit - back * p.H, g = h / (p.H / p.G);
     const int np = (p.dqk + 63) / 64, nvp = (p.dv + 63) / 64;
     char* q_s = tiles;                                        // [tile][panel]
     char* k_s = q_s + 2 * np * FP_PANEL;                      // [stage][panel]
@@ -142,19 +173,26 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
     // query tiles, and the range [beg, end) of key tiles each of them visits; key rows count from kv_start
     const int q0 = (p.q_blocks - 1 - back) * 2 * FP_TILE;
-    int i0[2], beg[2], end[2], base = 0;                      // rows of a call: below 2^30
+    int i0[2], beg[2], end[2], base;                          // rows of a call: below 2^30
+    fp_tiles(p, q0, i0, beg, end, base);
+    int n = end[1] > end[0] ? end[1] : end[0];
+    if constexpr (SPLIT > 1) {                                        // this CTA's share of them
+        const int first = n * rank / SPLIT;
+        n = n * (rank + 1) / SPLIT - first;
+        base += first * FP_TILE;
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-        const int first = q0 + t * FP_TILE;
-        i0[t] = (int)(p.start - p.kv_start) + first;
-        const int lo = fp_first_row(p, i0[t]);
-        if (t == 0) base = lo;
-        const int rows = p.S - first < FP_TILE ? p.S - first : FP_TILE;
-        beg[t] = (lo - base) / FP_TILE;
-        end[t] = rows > 0 ? (i0[t] + rows - 1 - base) / FP_TILE + 1 : 0;
-        if (rows <= 0) beg[t] = 0;
+        for (int t = 0; t < 2; ++t) {
+            beg[t] = max(beg[t] - first, 0);
+            end[t] = min(end[t] - first, n);
+            if (end[t] <= beg[t]) beg[t] = end[t] = 0;
+        }
     }
-    const int n = end[1] > end[0] ? end[1] : end[0];
+    // all threads of the cluster, warp by warp
+    auto meet = [] {
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+    };
     uint32_t room;                                            // the tiles end inside what was launched, wherever shared memory begins
     asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(room));
     const uint32_t used = (uint32_t)((char*)(&sh + 1) - fp_raw);
@@ -234,6 +272,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     mbar_wait_bounded(&sh.v_full[i % p.nv], (uint32_t)((i / p.nv) & 1));
             }
         }
+        if constexpr (SPLIT > 1) {
+            meet();
+            meet();
+        }
     } else if (warp == Roles::MMA_WARP) {
         // ---- MMA issuer.  The whole warp walks the tiles and waits, one lane issues: operands then are warp-uniform, and an
         // MMA costs an addition per descriptor (built in one lane's loop, each took about 200 cycles to issue and 64 to run)
@@ -306,6 +348,10 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (!ok && lane == 0) *failed = 1;
         umma_commit_by(leader, &sh.drained);                  // leave no MMA and no barrier arrival in flight
         mbar_wait_bounded(&sh.drained, 0);
+        if constexpr (SPLIT > 1) {
+            meet();
+            meet();
+        }
     } else if (warp < Roles::SOFTMAX_WARPS) {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Roles::REGS_SOFTMAX));
         // ---- softmax
@@ -447,7 +493,90 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             unpack2(add2(ls[0], ls[1]), l0, l1);
             l += l0 + l1;
         }
-        if (end[t] > 0) {
+        if constexpr (SPLIT > 1) {
+            // ---- the CTAs' parts of a block: each leaves its sums and unscaled rows of O where its operands were (no product
+            // is in flight any more), then takes every SPLIT-th row of all of them
+            const int pitch = nvp * 64, row = t * FP_TILE + a;               // floats of a row, 16-byte pieces permuted
+            float* rows = reinterpret_cast<float*>(tiles);
+            ok = __all_sync(FULL, mbar_wait_bounded(&sh.drained, 0)) && ok;
+            sh.xch[PER == 1 ? row : half * 2 * FP_TILE + row] = PER == 1 ? m : l;
+            if (PER == 1) sh.xch[2 * FP_TILE + row] = l;
+            if (ok && end[t] > 0) {
+                tc_fence_after();
+                for (int c = half * KEYS; c < p.dv && c < (half + 1) * KEYS; c += 32) {
+                    uint32_t r[32];
+                    tmem_ld32(o_addr + c, r);
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        *reinterpret_cast<uint4*>(rows + row * pitch + (((c >> 2) + e) ^ (row & 7)) * 4) =
+                            make_uint4(r[4 * e], r[4 * e + 1], r[4 * e + 2], r[4 * e + 3]);
+                }
+            }
+            meet();
+            {
+                constexpr int N = SPLIT;
+                float wt[N], sum[N], top = -INFINITY, total = 0.f;
+                uint32_t seen = 0;                            // parts with visible keys; the others have no rows either
+#pragma unroll
+                for (int q = 0; q < N; ++q) {
+                    wt[q] = load_cta1(&sh.xch[row], q);
+                    sum[q] = load_cta1(&sh.xch[2 * FP_TILE + row], q);
+                }
+#pragma unroll
+                for (int q = 0; q < N; ++q) {
+                    if (PER == 2) {
+                        sum[q] += wt[q];
+                        wt[q] = 0.f;
+                    }
+                    if (sum[q] != 0.f) {
+                        seen |= 1u << q;
+                        wt[q] = fmaxf(wt[q], -3.0e38f);       // of NaN alone there is no maximum, but a sum
+                        top = fmaxf(top, wt[q]);
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < N; ++q) {
+                    wt[q] = seen >> q & 1 ? exp2_fast(wt[q] - top) : 0.f;
+                    total = fmaf(wt[q], sum[q], total);
+                }
+                if (p.sink != nullptr) total += exp2f(p.sink[h] * FP_LOG2E - top);
+                const float inv = 1.f / total;
+                // a row at a time, its columns along the lanes: another CTA's memory is read in whole rows, four of them requested together
+                constexpr int STEP = N * PER, U = 4;
+                for (int e0 = rank + (PER == 1 ? 0 : half * N); e0 < 32; e0 += STEP * U) {
+                    float4 x[U][N];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int r1 = row - lane + ((e0 + u * STEP) & 31);
+#pragma unroll
+                        for (int q = 0; q < N; ++q) x[u][q] = load_cta(rows + r1 * pitch + (((lane * 4 < pitch ? lane : 0)) ^ (r1 & 7)) * 4, q);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const int e = e0 + u * STEP, s_row = q0 + row - lane + e;
+                        const float inv1 = __shfl_sync(FULL, inv, e & 31);
+                        const uint32_t seen1 = __shfl_sync(FULL, seen, e & 31);
+                        float v[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                        for (int q = 0; q < N; ++q) {
+                            const float w = __shfl_sync(FULL, wt[q], e & 31);
+                            if (seen1 >> q & 1) {
+                                v[0] = fmaf(w, x[u][q].x, v[0]);
+                                v[1] = fmaf(w, x[u][q].y, v[1]);
+                                v[2] = fmaf(w, x[u][q].z, v[2]);
+                                v[3] = fmaf(w, x[u][q].w, v[3]);
+                            }
+                        }
+                        if (e < 32 && s_row < p.S && lane * 4 < p.dv) {
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) v[k] *= inv1;
+                            store_vec<__nv_bfloat16, 4>((__nv_bfloat16*)p.out + (int64_t)b * p.o_bs + (int64_t)s_row * p.o_ss + h * p.o_hs + lane * 4, v);
+                        }
+                    }
+                }
+            }
+            meet();                                           // nobody leaves while its rows are read
+        } else if (end[t] > 0) {
             if (ok) ok = __all_sync(FULL, mbar_wait_bounded(&sh.o_full[t], 0));
             if (PER == 2) {                                   // the sum of both threads of a row
                 sh.xch[warp * 32 + lane] = l;
@@ -485,6 +614,9 @@ attn_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
         if (!ok) *failed = 1;
         tc_fence_before();
+    } else if (SPLIT > 1) {
+        meet();
+        meet();
     }
     __syncthreads();
     if (tid == 0 && sh.failed && p.status != nullptr) atomicOr(p.status, SK_DEV_WAIT_TIMEOUT);
@@ -505,6 +637,31 @@ uint32_t plan_smem(int dqk, int dv, bool bias, int* nk, int* nv) {
         }
     }
     return 0;
+}
+
+// CTAs that share a block's keys.  A call of few blocks leaves most SMs idle while its blocks walk over all keys: where two or four CTAs
+// a block find a place at once (32 clusters of four are certain to), they share it.  What joining costs shows where they don't: 8000
+// tokens, 16 heads are 512 blocks, 222 us alone, 266 by pairs, 401 by fours.  By the longest block's key tiles (one CTA | two | four):
+// 28 tiles, 32 blocks 65 | 45 | 35 us; 35 tiles of 192 / 128, 64 blocks 82 | 55 us; 16 tiles under a cap, 64 blocks 47 | 34 us; 6 tiles of
+// 256 / 128, 24 blocks 28.7 | 22.5 | 22.5 us.
+int fp_split(const FpShape& f, int B) {
+    const int64_t blocks = (int64_t)B * f.H * f.q_blocks;
+    const int np = (f.dqk + 63) / 64, nvp = (f.dv + 63) / 64;
+    if (blocks > 72 || (2 + f.nk) * np + f.nv * nvp < 4 * nvp) return 1;             // O's rows take the operands' place
+    int most = 0;
+    for (int k = 0; k < f.q_blocks; ++k) {
+        int i0[2], beg[2], end[2], base;
+        fp_tiles(f, k * 2 * FP_TILE, i0, beg, end, base);
+        for (int e : end) most = e > most ? e : most;
+    }
+    return most < 6 ? 1 : most < 16 || blocks > 32 ? 2 : 4;
+}
+
+template <int SPLIT> auto fp_kernel(bool bias, float softcap, bool bound) {
+    if (softcap > 0.f)
+        return bias ? attn_prefill_kernel<true, FP_CAP, 1, SPLIT>
+                    : bound ? attn_prefill_kernel<false, FP_CAP_BOUND, 2, SPLIT> : attn_prefill_kernel<false, FP_CAP, 1, SPLIT>;
+    return bias ? attn_prefill_kernel<true, FP_CAP_NONE, 1, SPLIT> : attn_prefill_kernel<false, FP_CAP_NONE, 1, SPLIT>;
 }
 
 }  // namespace
@@ -547,17 +704,25 @@ int launch_attn_prefill_tc(const sk_attn_params& p, cudaStream_t st) {
     if (int rc = make_head_map(&mq, p.q, p.dqk, p.H, p.S, p.B, p.q_hs, p.q_ss, p.q_bs, FP_TILE)) return rc;
     if (int rc = make_head_map(&mk, p.k, p.dqk, p.G, p.kv_rows, p.B, p.k_hs, p.k_ts, p.k_bs, FP_TILE)) return rc;
     if (int rc = make_head_map(&mv, p.v, p.dv, p.G, p.kv_rows, p.B, p.v_hs, p.v_ts, p.v_bs, FP_TILE)) return rc;
-    auto kern = p.bias != nullptr ? attn_prefill_kernel<true, FP_CAP_NONE, 1> : attn_prefill_kernel<false, FP_CAP_NONE, 1>;
     const bool bound = p.softcap > 0.f && p.bias == nullptr && f.cap_out <= FP_CAP_BOUND_LOG2;
-    if (p.softcap > 0.f)
-        kern = p.bias != nullptr ? attn_prefill_kernel<true, FP_CAP, 1>
-                                 : bound ? attn_prefill_kernel<false, FP_CAP_BOUND, 2> : attn_prefill_kernel<false, FP_CAP, 1>;
+    f.q_blocks = (p.S + 2 * FP_TILE - 1) / (2 * FP_TILE);
+    const int split = fp_split(f, p.B);
+    const auto kern = split == 1 ? fp_kernel<1>(p.bias != nullptr, p.softcap, bound)
+                    : split == 2 ? fp_kernel<2>(p.bias != nullptr, p.softcap, bound) : fp_kernel<4>(p.bias != nullptr, p.softcap, bound);
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(SK_ERR_CUDA, "attn_prefill_kernel smem attribute: %s", cudaGetErrorString(e));
-    f.q_blocks = (p.S + 2 * FP_TILE - 1) / (2 * FP_TILE);
-    dim3 grid((unsigned)(p.H * f.q_blocks), (unsigned)p.B);
-    kern<<<grid, bound ? FpRoles<2>::THREADS : FpRoles<1>::THREADS, smem, st>>>(mq, mk, mv, f);
-    return check_launch("attn_prefill_kernel");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(p.H * f.q_blocks * split), (unsigned)p.B);
+    cfg.blockDim = dim3(bound ? FpRoles<2>::THREADS : FpRoles<1>::THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)split;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = split > 1 ? 1 : 0;
+    return check_chained(cudaLaunchKernelEx(&cfg, kern, mq, mk, mv, f), "attn_prefill_kernel");
 }
 
 }  // namespace sk

@@ -100,7 +100,7 @@ constexpr double TANH_POLY[5] = {0.999999987, -0.333330719, 0.13324829, -0.05298
 __device__ __forceinline__ float softplus_f32(float x) { return fmaxf(x, 0.f) + log1pf(expf(-fabsf(x))); }
 
 // Positions by a chunk or a ring: 64-bit division is some hundred instructions in a row, and positions are rarely that large
-__device__ __forceinline__ int64_t position_div(int64_t i, int n) {
+__host__ __device__ __forceinline__ int64_t position_div(int64_t i, int n) {
     return (uint64_t)i >> 32 == 0 ? (int64_t)((uint32_t)i / (uint32_t)n) : i / n;
 }
 __device__ __forceinline__ int64_t position_mod(int64_t i, int n) {

@@ -81,6 +81,25 @@ def test_maximum_that_moves(growth, D, E, window, cap, bias_len):
             assert bool(((got[i, h] - want).abs() <= 2.0 ** -8 * mag + 2.0 ** -8 * want.abs() + 1e-6).all()), (i, h)
 
 
+@pytest.mark.parametrize("S,H,G,D,E,start,bias_len,chunk,window,cap,sink", [
+    (129, 2, 1, 128, 128, 3000, 0, 0, 0, 0.0, True),             # few blocks of many key tiles
+    (40, 1, 1, 64, 128, 100, 50, 0, 0, 0.0, False),              # fewer tiles than parts
+    (700, 2, 2, 192, 128, 0, 0, 0, 0, 0.0, True),                # first blocks of two tiles
+    (300, 2, 1, 128, 72, 900, 0, 0, 200, 30.0, True),            # relative to zero; a part without one of the query tiles
+    (257, 3, 1, 256, 40, 700, 90, 512, 0, 50.0, False),
+])
+def test_keys_shared_by_blocks(S, H, G, D, E, start, bias_len, chunk, window, cap, sink):
+    """One sequence, whose blocks are shared by CTAs, against many, whose blocks are not."""
+    from socket_b200 import block_ops as ops
+    q, k, v, kw = _case(S, H, G, D, E, start, 0, bias_len, chunk, window, cap, sink, S)
+    one = ops.attn(q, k, v, path="prefill_tc", **kw)[0].float()
+    n = 592 // (H * ((S + 255) // 256)) + 1
+    many = ops.attn(*(x.expand(n, *x.shape[1:]).contiguous() for x in (q, k, v)), path="prefill_tc", **kw).float()
+    assert torch.equal(many[0].expand_as(many), many)
+    # weights rounded to bf16 relative to another maximum, the results rounded
+    assert bool(((one - many[0]).abs() <= 2.0 ** -7 * one.abs() + 2.0 ** -8 * v.abs().max().item()).all())
+
+
 @pytest.mark.parametrize("kv_start", [2 ** 31 - 300, 2 ** 31 + 7, 2 ** 40])
 @pytest.mark.parametrize("chunk,window,cap", [(0, 0, 0.0), (0, 200, 30.0), (2 ** 30, 0, 0.0)])
 def test_positions_beyond_two_billion(kv_start, chunk, window, cap):
