@@ -420,21 +420,27 @@ mlstm_tc_states_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_c
 // ---------------------------------------------------------------- outputs
 constexpr int OT_P = 128;                                     // value columns of a CTA
 constexpr int OT_THREADS = 192;                               // warps 0-3: token rows; 4: TMA; 5: MMA
+// Up to 128 key columns two CTAs share an SM, one in its loads and products while the other is in its rows: 256 columns of tensor memory
+// each, two stages instead of four.  32000 tokens, 8 heads of 128 x 256: 149 us, 219 with one.  More key columns leave no room for two.
 constexpr int OT_STAGES = 4;
 constexpr uint32_t OT_STAGE = 2 * MT_PANEL;                   // two K panels, 64 rows of the state, or V
 constexpr uint32_t OT_S_PANEL = 64 * 128;                     // 64 key columns x 64 value columns of the state
 
 struct OtShared {
-    uint64_t q_full, full[OT_STAGES], empty[OT_STAGES], s_full, p_full, done, drained;
+    uint64_t q_full, full[OT_STAGES], empty[OT_STAGES], s_full, qs_full, p_full, done, drained;
     uint32_t tmem_base;
     int failed;
-    float a[MT_TOK], n[256];
+    alignas(16) float a[MT_TOK];             // read four at a time
+    float n[256];
 };
 
-__global__ void __launch_bounds__(OT_THREADS, 1)
+template <int STAGES>
+__global__ void __launch_bounds__(OT_THREADS, STAGES == 2 ? 2 : 1)
 mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_s,
                     const __grid_constant__ MtShape p) {
+    // in 256 columns the weights' products go on top of Q S, scaled before, and the weights over their scores
+    constexpr bool JOINED = STAGES == 2;
     extern __shared__ char ot_raw[];
     __shared__ __align__(16) OtShared sh;
     const int np = (p.N + 63) / 64;
@@ -447,11 +453,12 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     volatile int* failed = &sh.failed;
     if (tid == 0) {
         mbar_init_count(&sh.q_full, 1);
-        for (int s = 0; s < OT_STAGES; ++s) {
+        for (int s = 0; s < STAGES; ++s) {
             mbar_init_count(&sh.full[s], 1);
             mbar_init_count(&sh.empty[s], 1);
         }
         mbar_init_count(&sh.s_full, 1);
+        mbar_init_count(&sh.qs_full, 1);
         mbar_init_count(&sh.p_full, 4);
         mbar_init_count(&sh.done, 1);
         mbar_init_count(&sh.drained, 1);
@@ -459,7 +466,7 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 5) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sh.tmem_base)), "r"(512u)
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&sh.tmem_base)), "r"(JOINED ? 256u : 512u)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -468,8 +475,8 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = sh.tmem_base;                       // columns: Q S | weights V | scores | weights, 128 each
-    const uint32_t t_qs = tmem, t_wv = tmem + 128, t_sc = tmem + 256, t_w = tmem + 384;
+    const uint32_t tmem = sh.tmem_base;                       // columns: Q S | scores | weights V | weights, 128 each
+    const uint32_t t_qs = tmem, t_sc = tmem + 128, t_wv = JOINED ? t_qs : tmem + 256, t_w = JOINED ? t_sc : tmem + 384;
 
     if (warp == 4) {
         if (lane == 0) {
@@ -477,9 +484,9 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int q = 0; q < np; ++q) tma_load_4d(q_s + q * MT_PANEL, &map_q, q * 64, h, c * MT_TOK, b, &sh.q_full);
             int i = 0;
             for (; i < items && !*failed; ++i) {
-                const int s = i % OT_STAGES;
+                const int s = i % STAGES;
                 char* dst = ring + s * OT_STAGE;
-                if (i >= OT_STAGES && !mbar_wait_bounded(&sh.empty[s], (uint32_t)((i / OT_STAGES - 1) & 1))) {
+                if (i >= STAGES && !mbar_wait_bounded(&sh.empty[s], (uint32_t)((i / STAGES - 1) & 1))) {
                     *failed = 1;
                     break;
                 }
@@ -498,8 +505,8 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
             if (*failed) {                                    // leave no copy in flight
                 mbar_wait_bounded(&sh.q_full, 0);
-                for (int q = i > OT_STAGES ? i - OT_STAGES : 0; q < i; ++q)
-                    mbar_wait_bounded(&sh.full[q % OT_STAGES], (uint32_t)((q / OT_STAGES) & 1));
+                for (int q = i > STAGES ? i - STAGES : 0; q < i; ++q)
+                    mbar_wait_bounded(&sh.full[q % STAGES], (uint32_t)((q / STAGES) & 1));
             }
         }
     } else if (warp == 5) {
@@ -512,10 +519,10 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         const int k16 = (p.N + 15) / 16;
         bool ok = wait_all(&sh.q_full, 0);
         for (int i = 0; ok && i < items && !__any_sync(FULL, *failed != 0); ++i) {
-            const int s = i % OT_STAGES;
+            const int s = i % STAGES;
             const uint32_t at = s * (OT_STAGE >> 4);
             if (i == items - 1) ok = wait_all(&sh.p_full, 0);
-            ok = ok && wait_all(&sh.full[s], (uint32_t)((i / OT_STAGES) & 1));
+            ok = ok && wait_all(&sh.full[s], (uint32_t)((i / STAGES) & 1));
             if (!ok) break;
             tc_fence_after();
             if (i < k_items) {                                // scores
@@ -536,13 +543,15 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         if (j * 4 + k < k16)
                             umma_ss_by(leader, t_qs, umma_desc_at(qd, k * 2), umma_desc_at(sd, (part * 2 * OT_S_PANEL + k * 2048) >> 4),
                                        id_mn, j > 0 || k > 0 || part > 0);
-            } else {                                          // weights V, value and remainder
+                if (i == items - 2) umma_commit_by(leader, &sh.qs_full);
+            } else {                                          // weights V, value and remainder, 32 keys of each side by side
                 const uint64_t vd = umma_desc_at(ring_v, at);
 #pragma unroll
                 for (int part = 0; part < 2; ++part)
 #pragma unroll
                     for (int k = 0; k < MT_TOK / 16; ++k)
-                        umma_ts_by(leader, t_wv, t_w + part * 64 + k * 8, umma_desc_at(vd, k * (2048 >> 4)), id_mn, k > 0 || part > 0);
+                        umma_ts_by(leader, t_wv, t_w + (k >> 1) * 32 + part * 16 + (k & 1) * 8, umma_desc_at(vd, k * (2048 >> 4)), id_mn,
+                                   JOINED || k > 0 || part > 0);
                 umma_commit_by(leader, &sh.done);
             }
             umma_commit_by(leader, &sh.empty[s]);
@@ -596,8 +605,22 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 }
 #pragma unroll
                 for (int e = 0; e < 16; ++e) split_bf16(s[2 * e], s[2 * e + 1], hi[e], lo[e]);
-                tmem_st16(t_w + lane_base + c0 / 2, hi);
-                tmem_st16(t_w + lane_base + 64 + c0 / 2, lo);
+                tmem_st16(t_w + lane_base + c0, hi);
+                tmem_st16(t_w + lane_base + c0 + 16, lo);
+            }
+            if (JOINED) ok = __all_sync(FULL, mbar_wait_bounded(&sh.qs_full, 0));
+        }
+        if (ok) {
+            tc_fence_after();
+            if constexpr (JOINED) {                           // Q S to the weights' scale
+#pragma unroll
+                for (int c0 = 0; c0 < OT_P; c0 += 32) {
+                    float x[32];
+                    tmem_ld32(t_qs + lane_base + c0, reinterpret_cast<uint32_t(&)[32]>(x));
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) x[e] *= carry;
+                    tmem_st32(t_qs + lane_base + c0, reinterpret_cast<uint32_t(&)[32]>(x));
+                }
             }
             tmem_wait_st();
             tc_fence_before();
@@ -612,18 +635,17 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 tc_fence_after();
                 __nv_bfloat16* o = p.num + (((int64_t)b * p.S + tok) * p.H + h) * p.P + p0;
                 const int cols = tok < p.S ? p.P - p0 : 0;
-                const float fq = carry * p.q_scale;
 #pragma unroll
                 for (int c0 = 0; c0 < OT_P; c0 += 32) {
                     float x[32], y[32];
-                    tmem_ld32(t_qs + lane_base + c0, reinterpret_cast<uint32_t(&)[32]>(x));
                     tmem_ld32(t_wv + lane_base + c0, reinterpret_cast<uint32_t(&)[32]>(y));
+                    if constexpr (!JOINED) tmem_ld32(t_qs + lane_base + c0, reinterpret_cast<uint32_t(&)[32]>(x));
 #pragma unroll
                     for (int e = 0; e < 32; e += 8) {
                         if (c0 + e < cols) {
                             float r[8];
 #pragma unroll
-                            for (int j = 0; j < 8; ++j) r[j] = fmaf(fq, x[e + j], y[e + j] * p.q_scale);
+                            for (int j = 0; j < 8; ++j) r[j] = JOINED ? y[e + j] * p.q_scale : fmaf(carry * p.q_scale, x[e + j], y[e + j] * p.q_scale);
                             store_vec<__nv_bfloat16, 8>(o + c0 + e, r);
                         }
                     }
@@ -636,7 +658,7 @@ mlstm_tc_out_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     __syncthreads();
     if (tid == 0 && sh.failed && p.status != nullptr) atomicOr(p.status, SK_DEV_WAIT_TIMEOUT);
     if (warp == 5)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(JOINED ? 256u : 512u) : "memory");
 }
 
 int mt_chunks(const sk_mlstm_params& p) { return (p.S + MT_TOK - 1) / MT_TOK; }
@@ -720,11 +742,12 @@ int launch_mlstm_tc(const sk_mlstm_params& p, cudaStream_t st) {
     states_kernel<<<dim3((unsigned)((p.P + sp - 1) / sp), (unsigned)((p.N + 127) / 128), (unsigned)(p.B * p.H)), ST_THREADS, st_smem, st>>>(
         mk, ms_out, m);
     if (int rc = check_launch("mlstm_tc_states_kernel")) return rc;
-    const uint32_t smem = (uint32_t)((p.N + 63) / 64) * MT_PANEL + OT_STAGES * OT_STAGE + 1024;
-    e = cudaFuncSetAttribute(mlstm_tc_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int stages = p.N <= 128 ? 2 : OT_STAGES;
+    auto out_kernel = stages == 2 ? mlstm_tc_out_kernel<2> : mlstm_tc_out_kernel<OT_STAGES>;
+    const uint32_t smem = (uint32_t)((p.N + 63) / 64) * MT_PANEL + stages * OT_STAGE + 1024;
+    e = cudaFuncSetAttribute(out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return fail(SK_ERR_CUDA, "mlstm_tc_out_kernel smem attribute: %s", cudaGetErrorString(e));
-    mlstm_tc_out_kernel<<<dim3((unsigned)((p.P + OT_P - 1) / OT_P), (unsigned)chunks, (unsigned)(p.B * p.H)), OT_THREADS, smem, st>>>(
-        mq, mk, mv, ms_in, m);
+    out_kernel<<<dim3((unsigned)((p.P + OT_P - 1) / OT_P), (unsigned)chunks, (unsigned)(p.B * p.H)), OT_THREADS, smem, st>>>(mq, mk, mv, ms_in, m);
     return check_launch("mlstm_tc_out_kernel");
 }
 
