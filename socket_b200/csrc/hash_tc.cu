@@ -396,7 +396,8 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             ok = wait_all(&ts.norm_full[i % TC_NSLOTS], (uint32_t)((i / TC_NSLOTS) & 1)) &&
                  (i < TC_STAGES || wait_all(&ts.near_empty[s], par ^ 1u));
             if (!ok) break;
-            const float knorm = valid ? ts.knorm[i % TC_NSLOTS][r_in_tile] : 0.f;
+            // rows behind the last must not look like rows of zeros, whose careful path costs a warp's tile 16 us
+            const float knorm = valid ? ts.knorm[i % TC_NSLOTS][r_in_tile] : 1.f;
             const float thr = TC_BAND * knorm;
             const float thr_max = valid ? thr * ts.plane_norm[TC_N] : -1.f;  // cheap first test, exact test inside
             if (!(ok = wait_all(&ts.acc_full[s], par))) break;
