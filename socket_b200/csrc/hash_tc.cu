@@ -63,14 +63,20 @@ __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t da, uint64_t 
         : "memory");
 }
 
-constexpr int TC_STAGES = 2;          // accumulators in tensor memory, masks of near-zero projections
+constexpr int TC_STAGES = 2;          // accumulators in tensor memory
+constexpr int TC_MASKS = 4;           // masks of near-zero projections: tiles whose decisions may be outstanding
 constexpr int TC_ARING = 4;           // K tiles in flight
 constexpr int TC_NSLOTS = 8;          // norm slots
 constexpr int TC_NORM_WARPS = 4;      // one thread per row of the K tile: its norm, and later its near-zero projections
-constexpr int TC_EPI_WARPS = 8;       // two threads per accumulator row, 128 columns each
+// two threads per accumulator row, 128 columns each; four of 64 where no warps move rows
+template <bool APPEND> constexpr int TC_EPI_WARPS = APPEND ? 8 : 16;
 constexpr int TC_MOVE_WARPS = 8;      // APPEND: 16 rows each
-constexpr int TC_PIPE_THREADS = 32 * (2 + TC_NORM_WARPS + TC_EPI_WARPS);   // TMA warp, MMA warp, norm warps, epilogue warps
-constexpr int TC_APPEND_THREADS = TC_PIPE_THREADS + 32 * TC_MOVE_WARPS;
+// Without APPEND: one thread per row of every second tile, for its near-zero projections.  Bulk hashing is bound by the tiles' roles, not by
+// memory, and decisions take longest: 4194304 rows 638 us by the norm warps, 525 by four warps of their own, 444 with the masks of four
+// tiles instead of two and keys from global memory, 386 by eight.
+constexpr int TC_FIX_WARPS = 8;
+// TMA warp, MMA warp, norm warps, epilogue warps, moving or deciding warps
+template <bool APPEND> constexpr int TC_THREADS = 32 * (2 + TC_NORM_WARPS + TC_EPI_WARPS<APPEND> + (APPEND ? TC_MOVE_WARPS : TC_FIX_WARPS));
 constexpr int TC_FIX_TOGETHER = 256;  // up to so many near-zero projections of 32 rows, a warp takes them one by one
 
 struct TcShared {
@@ -80,13 +86,13 @@ struct TcShared {
     uint64_t norm_full[TC_NSLOTS];     // row norms of tile i are in knorm[i % 8]
     uint64_t acc_full[TC_STAGES];      // accumulator is complete
     uint64_t acc_empty[TC_STAGES];     // accumulator has been read back
-    uint64_t near_full[TC_STAGES];     // codes are written and the mask is complete
-    uint64_t near_empty[TC_STAGES];    // the mask has been read
+    uint64_t near_full[TC_MASKS];     // codes are written and the mask is complete
+    uint64_t near_empty[TC_MASKS];    // the mask has been read
     uint32_t tmem_base;
     int failed;                        // some bounded wait ran out
     float plane_norm[TC_N + 1];        // [TC_N] = the largest norm
     float knorm[TC_NSLOTS][TC_ROWS];   // |k| * 1.001 of the rows of tile i in slot i % 8 (inf: decide every bit exactly)
-    __align__(16) uint32_t near_zero[TC_STAGES][TC_ROWS][TC_N / 32];   // bit k of word c: column 32 c + k
+    __align__(16) uint32_t near_zero[TC_MASKS][TC_ROWS][TC_N / 32];   // bit k of word c: column 32 c + k
 };
 
 // Where an append writes; unused fields without APPEND
@@ -145,16 +151,16 @@ __device__ __forceinline__ void patch_code(uint8_t* row_codes, int col, bool set
 
 // Persistent, warp-specialised: every CTA keeps the 256 plane rows in shared memory and walks the
 // K tiles blockIdx.x, blockIdx.x + gridDim.x, ...  Warp 0 feeds a ring of K tiles by TMA, warp 1 issues the
-// MMAs into one of two accumulators in tensor memory, warps 6-13 read the other accumulator back
+// MMAs into one of two accumulators in tensor memory, the eight (APPEND) or sixteen warps from 6 on read the other accumulator back
 // (tcgen05.ld), take the signs, apply the near-zero test and write the code bytes; warps 2-5 compute the
 // row norms that test needs from the K tile in shared memory, and one tile later decide its near-zero
-// projections; warps 14-21 (APPEND) move the rows.  So the load of tile i+1, the MMAs of tile i+1 and the
+// projections (APPEND; else the last eight warps do); warps 14-21 (APPEND) move the rows.  So the load of tile i+1, the MMAs of tile i+1 and the
 // epilogue of tile i overlap.  Every wait is bounded; a wait that runs out raises `failed`, which makes
 // every role leave its loop, and the status flag.
 template <typename T, bool APPEND>
-__global__ void __launch_bounds__(APPEND ? TC_APPEND_THREADS : TC_PIPE_THREADS, 1)
+__global__ void __launch_bounds__(TC_THREADS<APPEND>, 1)
 hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_p,
-               const T* __restrict__ planes, int64_t N, uint8_t* codes, int64_t code_row_stride,
+               const T* __restrict__ planes, const T* __restrict__ keys, int64_t key_row_stride, int64_t N, uint8_t* codes, int64_t code_row_stride,
                const int64_t* __restrict__ dst_row, const __grid_constant__ TcAppend ap, int32_t* status) {
     extern __shared__ char tc_raw[];
     __shared__ TcShared ts;
@@ -176,9 +182,11 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         for (int s = 0; s < TC_NSLOTS; ++s) mbar_init_count(&ts.norm_full[s], TC_NORM_WARPS);
         for (int s = 0; s < TC_STAGES; ++s) {
             mbar_init_count(&ts.acc_full[s], 1);
-            mbar_init_count(&ts.acc_empty[s], TC_EPI_WARPS);
-            mbar_init_count(&ts.near_full[s], TC_EPI_WARPS);
-            mbar_init_count(&ts.near_empty[s], TC_NORM_WARPS);
+            mbar_init_count(&ts.acc_empty[s], TC_EPI_WARPS<APPEND>);
+        }
+        for (int s = 0; s < TC_MASKS; ++s) {
+            mbar_init_count(&ts.near_full[s], TC_EPI_WARPS<APPEND>);
+            mbar_init_count(&ts.near_empty[s], 4);               // four warps decide a tile
         }
         ts.failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -197,7 +205,7 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     volatile int* failed = &ts.failed;
     // |plane| * 1.001 of the 256 planes, by the norm and the epilogue warps while the first tiles come in (every CTA
     // computes them for itself: 64 KiB from L2, cheaper than a launch of its own)
-    constexpr int NORMERS = TC_NORM_WARPS + TC_EPI_WARPS;
+    constexpr int NORMERS = TC_NORM_WARPS + TC_EPI_WARPS<APPEND>;
     if (warp >= 2 && warp < 2 + NORMERS) {
         constexpr int U = 4;                                  // planes in flight per warp
         for (int n0 = (warp - 2) * U; n0 < TC_N; n0 += NORMERS * U) {
@@ -239,6 +247,74 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         if (n >= N) return -1;
         if (APPEND) return ap.row(n, pos);
         return dst_row != nullptr ? dst_row[n] : n;
+    };
+
+    // near-zero projections of 32 rows of tile j, whose codes are written: exact fp64 dot products patch their bits
+    auto decide = [&](int64_t j, int quad) {
+        const int s = (int)(j % TC_MASKS), ra = (int)(j % TC_ARING), r_in_tile = quad * 32 + lane;
+        const int64_t dst = code_row(first_row(j) + r_in_tile);
+        if (!wait_all(&ts.near_full[s], (uint32_t)((j / TC_MASKS) & 1))) return false;
+        uint32_t left[TC_N / 32];
+        int mine = 0;
+#pragma unroll
+        for (int w = 0; w < TC_N / 32; w += 4) {
+            const uint4 x = *reinterpret_cast<const uint4*>(&ts.near_zero[s][r_in_tile][w]);
+            left[w] = x.x;
+            left[w + 1] = x.y;
+            left[w + 2] = x.z;
+            left[w + 3] = x.w;
+            mine += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+        }
+        if (dst < 0) mine = 0;
+        const int count = __reduce_add_sync(FULL, mine);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ts.near_empty[s]);                 // the mask is in registers
+        // this lane's next projection
+        auto next = [&]() {
+            int col = 0;
+            bool found = false;
+#pragma unroll
+            for (int w = 0; w < TC_N / 32; ++w)
+                if (!found && left[w] != 0) {
+                    col = w * 32 + __ffs(left[w]) - 1;
+                    left[w] &= left[w] - 1;
+                    found = true;
+                }
+            --mine;
+            return col;
+        };
+        const char* a = a_base + (size_t)ra * 2 * TC_A_HALF_BYTES;
+        // four elements of a row of the tile: of an append, whose K tiles wait for the moving warps anyhow, from shared memory; else
+        // from global memory, which leaves the tile to the next load
+        auto key_piece = [&](int row, int i4) {
+            if constexpr (APPEND) return tile_piece(a + (i4 >> 4) * TC_A_HALF_BYTES, row, i4 & 15);
+            else return __ldg(reinterpret_cast<const uint2*>(keys + (first_row(j) + row) * key_row_stride) + i4);
+        };
+        const int h = lane >> 4, q = lane & 15;
+        if (count <= TC_FIX_TOGETHER) {                                // a projection at a time, four elements per lane
+            for (unsigned have = __ballot_sync(FULL, mine > 0); have != 0; have = __ballot_sync(FULL, mine > 0)) {
+                const int src = __ffs(have) - 1, row = quad * 32 + src;
+                const int col = __shfl_sync(FULL, lane == src ? next() : 0, src);
+                const uint2 kr = key_piece(row, lane), pr = tile_piece(tiles + h * TC_B_HALF_BYTES, col, q);
+                const double d = warp_sum_f64(dot4<Ty>(kr, pr, 0.0));
+                if (lane == src) patch_code(codes + dst * code_row_stride, col, d >= 0.0);
+            }
+        } else {                                                       // hostile inputs: every lane its own row
+            while (mine > 0) {
+                const int col = next();
+                double d = 0.0;
+#pragma unroll 2
+                for (int i4 = 0; i4 < 32; ++i4)
+                    d = dot4<Ty>(key_piece(r_in_tile, i4), tile_piece(tiles + (i4 >> 4) * TC_B_HALF_BYTES, col, i4 & 15), d);
+                patch_code(codes + dst * code_row_stride, col, d >= 0.0);
+            }
+            __syncwarp();
+        }
+        if (APPEND) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ts.a_empty[ra]);
+        }
+        return true;
     };
 
     if (warp == 0) {
@@ -299,7 +375,7 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         const int r_in_tile = (warp - 2) * 32 + lane;
         bool ok = wait_all(&ts.b_full, 0);                             // the near-zero decisions read the planes
 #pragma unroll 1
-        for (int64_t i = 0; ok && i <= my_tiles && !gone(); ++i) {
+        for (int64_t i = 0; ok && i < my_tiles + (APPEND ? 1 : 0) && !gone(); ++i) {
             // norms of tile i.  They go to slot i % 8, which has a barrier of its own (these warps may be
             // ahead of the epilogue, and a barrier must not complete two phases ahead of a waiter): tile i
             // can only have been loaded after the MMAs of tile i-4 were done, which started after the
@@ -310,9 +386,9 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
                 float ss = 0.f;
                 uint32_t any = 0;
                 const char* a = a_base + (size_t)ra * 2 * TC_A_HALF_BYTES + (size_t)r_in_tile * 128;
-#pragma unroll 1                       // the roles together have to fit the instruction cache
+#pragma unroll(APPEND ? 1 : 2)         // the roles of an append together have to fit the instruction cache
                 for (int h = 0; h < 2; ++h) {
-#pragma unroll 4
+#pragma unroll(APPEND ? 4 : 8)
                     for (int c = 0; c < 8; ++c) {
                         const uint4 w = *reinterpret_cast<const uint4*>(a + h * TC_A_HALF_BYTES + ((c ^ (r_in_tile & 7)) << 4));
                         const uint32_t u[4] = {w.x, w.y, w.z, w.w};
@@ -332,57 +408,16 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&ts.norm_full[i % TC_NSLOTS]);
             }
-            if (i == 0) continue;
-            // near-zero projections of tile i - 1, whose codes are written: exact fp64 dot products patch their bits
-            const int64_t j = i - 1;
-            const int s = (int)(j & 1), ra = (int)(j % TC_ARING);
-            const int64_t dst = code_row(first_row(j) + r_in_tile);
-            if (!(ok = wait_all(&ts.near_full[s], (uint32_t)((j >> 1) & 1)))) break;
-            const uint32_t* near = ts.near_zero[s][r_in_tile];
-            int count = 0;
-#pragma unroll 1
-            for (int w = 0; w < TC_N / 32; w += 4) {
-                const uint4 x = *reinterpret_cast<const uint4*>(near + w);
-                count += __popc(x.x) + __popc(x.y) + __popc(x.z) + __popc(x.w);
+            if (!APPEND) {
+                if (lane == 0) mbar_arrive(&ts.a_empty[i % TC_ARING]);
+            } else if (i > 0) {
+                ok = decide(i - 1, warp - 2);
             }
-            count = __reduce_add_sync(FULL, dst >= 0 ? count : 0);
-            const char* a = a_base + (size_t)ra * 2 * TC_A_HALF_BYTES;
-            const int h = lane >> 4, q = lane & 15;
-#pragma unroll 1
-            for (int w = 0; count > 0 && w < TC_N / 32; ++w) {
-                uint32_t left = dst >= 0 ? near[w] : 0;
-                if (count <= TC_FIX_TOGETHER) {                        // a projection at a time, four elements per lane
-                    for (unsigned have = __ballot_sync(FULL, left != 0); have != 0; have = __ballot_sync(FULL, left != 0)) {
-                        const int src = __ffs(have) - 1;
-                        const int col = w * 32 + __ffs(__shfl_sync(FULL, left, src)) - 1, row = (warp - 2) * 32 + src;
-                        const uint2 kr = tile_piece(a + h * TC_A_HALF_BYTES, row, q), pr = tile_piece(tiles + h * TC_B_HALF_BYTES, col, q);
-                        const double d = warp_sum_f64(dot4<Ty>(kr, pr, 0.0));
-                        if (lane == src) {
-                            patch_code(codes + dst * code_row_stride, col, d >= 0.0);
-                            left &= left - 1;
-                        }
-                    }
-                } else {                                               // hostile inputs: every lane its own row
-                    for (; left != 0; left &= left - 1) {
-                        const int col = w * 32 + __ffs(left) - 1;
-                        double d = 0.0;
-#pragma unroll 2
-                        for (int i4 = 0; i4 < 32; ++i4)
-                            d = dot4<Ty>(tile_piece(a + (i4 >> 4) * TC_A_HALF_BYTES, r_in_tile, i4 & 15),
-                                         tile_piece(tiles + (i4 >> 4) * TC_B_HALF_BYTES, col, i4 & 15), d);
-                        patch_code(codes + dst * code_row_stride, col, d >= 0.0);
-                    }
-                    __syncwarp();
-                }
-            }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ts.near_empty[s]);
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ts.a_empty[ra]);
         }
-    } else if (warp < 2 + TC_NORM_WARPS + TC_EPI_WARPS) {
-        // ---- epilogue: the two warps with the same (warp % 4) share the 32 accumulator lanes of that
-        // quarter, half of the columns each; a thread owns one row and 128 columns = 16 tables
+    } else if (warp < 2 + TC_NORM_WARPS + TC_EPI_WARPS<APPEND>) {
+        // ---- epilogue: the two or four warps with the same (warp % 4) share the 32 accumulator lanes of that
+        // quarter, a part of the columns each; a thread owns one row and 128 or 64 columns
+        constexpr int CHUNKS = 32 / TC_EPI_WARPS<APPEND>;       // of 32 columns, a thread
         const int quad = warp & 3, ch = (warp - 2 - TC_NORM_WARPS) >> 2;
         const int r_in_tile = quad * 32 + lane;
         bool ok = true;
@@ -394,7 +429,7 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             const bool valid = row < N;
             const int64_t dst = code_row(row);                      // requested before the waits below
             ok = wait_all(&ts.norm_full[i % TC_NSLOTS], (uint32_t)((i / TC_NSLOTS) & 1)) &&
-                 (i < TC_STAGES || wait_all(&ts.near_empty[s], par ^ 1u));
+                 (i < TC_MASKS || wait_all(&ts.near_empty[i % TC_MASKS], (uint32_t)((i / TC_MASKS - 1) & 1)));
             if (!ok) break;
             // rows behind the last must not look like rows of zeros, whose careful path costs a warp's tile 16 us
             const float knorm = valid ? ts.knorm[i % TC_NSLOTS][r_in_tile] : 1.f;
@@ -402,10 +437,10 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             const float thr_max = valid ? thr * ts.plane_norm[TC_N] : -1.f;  // cheap first test, exact test inside
             if (!(ok = wait_all(&ts.acc_full[s], par))) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            uint32_t words[4] = {0u, 0u, 0u, 0u};
-#pragma unroll 1
-            for (int c4 = 0; c4 < 4; ++c4) {
-                const int c = ch * 4 + c4;
+            uint32_t words[CHUNKS] = {};
+#pragma unroll(APPEND ? 1 : CHUNKS)
+            for (int c4 = 0; c4 < CHUNKS; ++c4) {
+                const int c = ch * CHUNKS + c4;
                 const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)s * TC_N + c * 32;
                 uint32_t r[32];
                 tmem_ld32(at, r);
@@ -442,25 +477,33 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
                     }
                 }
 #pragma unroll
-                for (int x = 0; x < 4; ++x) words[x] = x == c4 ? word : words[x];
-                ts.near_zero[s][r_in_tile][c] = mark;
+                for (int x = 0; x < CHUNKS; ++x) words[x] = x == c4 ? word : words[x];
+                ts.near_zero[i % TC_MASKS][r_in_tile][c] = mark;
             }
             // the accumulator is free again
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&ts.acc_empty[s]);
-            if (dst >= 0)                                          // negative = row not to be written
-                reinterpret_cast<uint4*>(codes + dst * code_row_stride)[ch] = make_uint4(words[0], words[1], words[2], words[3]);
+            if (dst >= 0) {                                        // negative = row not to be written
+                if constexpr (CHUNKS == 4) reinterpret_cast<uint4*>(codes + dst * code_row_stride)[ch] = make_uint4(words[0], words[1], words[2], words[3]);
+                else reinterpret_cast<uint2*>(codes + dst * code_row_stride)[ch] = make_uint2(words[0], words[1]);
+            }
             __syncwarp();
-            if (lane == 0) mbar_arrive(&ts.near_full[s]);          // releases the codes to the warps that may patch them
+            if (lane == 0) mbar_arrive(&ts.near_full[i % TC_MASKS]);          // releases the codes to the warps that may patch them
         }
+    } else if (!APPEND) {
+        // ---- decisions
+        const int own = warp - 2 - TC_NORM_WARPS - TC_EPI_WARPS<APPEND>;
+        bool ok = wait_all(&ts.b_full, 0);
+#pragma unroll 1
+        for (int64_t i = own >> 2; ok && i < my_tiles && !gone(); i += 2) ok = decide(i, own & 3);
     } else {
         // ---- APPEND: 16 rows of the tile to the cache, half a warp per row and 16 bytes per lane.  v_norm is the number the
         // general append stores, the fp64 norm rounded to fp32 and then to fp16; fp64 arithmetic runs at a few lanes a cycle
         // here (the sums alone took 9 of a tile's 10 us), so the norm is taken in fp32, whose error is far below 24 units of
         // its last place, and in fp64 only where that could change the rounding to fp16 (one row in 170), or fp32 or fp16
         // leaves its normal range.
-        const int m0 = (warp - 2 - TC_NORM_WARPS - TC_EPI_WARPS) * 16, part = lane >> 4, piece = lane & 15;
+        const int m0 = (warp - 2 - TC_NORM_WARPS - TC_EPI_WARPS<APPEND>) * 16, part = lane >> 4, piece = lane & 15;
         bool bad = false, ok = true;
         int32_t max_len = 0;
 #pragma unroll 1
@@ -596,8 +639,8 @@ int hash_tc_launch(const void* keys, int64_t key_row_stride, const void* planes,
     if (e != cudaSuccess) return fail(SK_ERR_CUDA, "hash_tc_kernel smem attribute: %s", cudaGetErrorString(e));
     const int64_t tiles = (N + TC_ROWS - 1) / TC_ROWS;
     const unsigned n_cta = (unsigned)(tiles < sm_count() ? tiles : sm_count());
-    kern<<<n_cta, APPEND ? TC_APPEND_THREADS : TC_PIPE_THREADS, smem, st>>>(map_k, map_p, static_cast<const T*>(planes), N, codes,
-                                                                           code_row_stride, dst_row, ap, status);
+    kern<<<n_cta, TC_THREADS<APPEND>, smem, st>>>(map_k, map_p, static_cast<const T*>(planes), static_cast<const T*>(keys), key_row_stride, N, codes,
+                                              code_row_stride, dst_row, ap, status);
     return check_launch("hash_tc_kernel");
 }
 
