@@ -511,7 +511,7 @@ def measure(args, wl, K, W, world, rank, local_rank, full):
             "frac_of_bf16_peak": None if tf_peak is None else round(flops / t_us / 1e6 / tf_peak, 4),
             "frac_of_bf16_sustained": None if tf_sus is None else round(flops / t_us / 1e6 / tf_sus, 4),
             "gbs": round(n_rows * (D * 2 + cfg.L) / t_us / 1e3, 1),
-            "note": "sk_hash_keys_tc incl. its fix-up launch; not in the step"}
+            "note": "sk_hash_keys_tc; not in the step"}
         del keys2d
         # the whole prefill cache write (copy K/V + v_norm + codes) of S tokens; the tokens are the
         # cache's own first S rows, so the cache is left unchanged
@@ -536,7 +536,7 @@ def measure(args, wl, K, W, world, rank, local_rank, full):
         stages["prefill_kv_append"] = {
             "us": round(t_us, 1), "rows": rows_pf, "gbs": round(bytes_pf / t_us / 1e3, 1),
             "frac_of_hbm_peak": round(bytes_pf / t_us / 1e3 / peak, 4),
-            "note": "sk_kv_append_tc: copy + v_norm kernel, then tensor-core hashing; not in the step"}
+            "note": "sk_kv_append: copies, norms and tensor-core hashing in one launch; not in the step"}
         del k_pf, v_pf
     # context figure, not on the path: dense attention of the same query over the whole cache
     # (library kernels), i.e. what the sparse path replaces per layer and token
