@@ -11,9 +11,11 @@
 // (warp w runs on scheduler w % 4 and can reach the accumulator rows 32 (w % 4) on only; later tokens have more keys, so the
 // weighted values, which any warp can make, go to the schedulers of the earlier tokens.)
 // Whatever carries a decay or the state enters a product as two bf16 numbers, value and remainder (16 significant bits);
-// sums are fp32.  The skip D x_t is an addition to the weight of a token with itself.
-// Measured (one GPU, inside a decoder; the form in blocks of 64 tokens in brackets): 8000 tokens, 128 heads of 128 x 64, 234 us
-// (904); 1501 tokens, 64 heads, 43 us (105).  A chunk takes about 5000 cycles: 80 KiB come in over L2 (3000 cycles when 128
+// sums are fp32, and so is the skip D x_t, added to the finished ones (8000 tokens, 128
+// heads, with the convolution 291 us; as an addition to the weight of a token with itself, 16 bits of D, 280; with x read again from
+// global memory 298).
+// Measured (one GPU, inside a decoder; the form in blocks of 64 tokens in brackets): 8000 tokens, 128 heads of 128 x 64, 245 us
+// (904); 1501 tokens, 64 heads, 45 us (105).  A chunk takes about 5000 cycles: 80 KiB come in over L2 (3000 cycles when 128
 // blocks do so), and the 56 MMAs read 290 KiB of operands from shared memory (3400).  The roles' code has to stay small:
 // with every loop of a chunk unrolled (90 KiB of instructions, of which each warp walks its own part once per chunk) a chunk
 // took 6900 cycles.
@@ -142,6 +144,7 @@ ssm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
         const float skip = p.skip[h];
         float carry = 0.f, next = 0.f;
+        uint4 x_own[4], x_out[4];                             // the token's x, 32 columns: of this chunk, and of the one before
 #pragma unroll 1
         for (int c = 0; ok && c <= p.chunks; ++c) {
             if (c < p.chunks) {
@@ -184,7 +187,7 @@ ssm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 #pragma unroll
                                 for (int q = 0; q < 4; ++q) {
                                     const float v = s[e + q] * (exp2_fast(ct - cv[q]) * dv[q]);
-                                    s[e + q] = e + q < lane ? v : e + q == lane ? v + skip : 0.f;
+                                    s[e + q] = e + q <= lane ? v : 0.f;
                                 }
                             }
                         }
@@ -193,6 +196,10 @@ ssm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                     }
                     tmem_st32(col, w);
                 }
+                // the skip is added to the finished sums, when the stage may be gone; it stays until this warp's weights are there
+                const char* x_s = stage_s + st * TS_STAGE + 4 * TS_PANEL + t * 128;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) x_own[e] = *reinterpret_cast<const uint4*>(x_s + (((half * 4 + e) ^ (t & 7)) << 4));
                 tmem_wait_st();
                 tc_fence_before();
                 __syncwarp();
@@ -202,25 +209,35 @@ ssm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 ok = wait_all(&sh.y_full, (uint32_t)((c - 1) & 1)) && !gone();
                 if (!ok) break;
                 tc_fence_after();
-                float x[32], y[32];
-                tmem_ld32(t_qs + lane_base + half * 32, reinterpret_cast<uint32_t(&)[32]>(x));
-                tmem_ld32(t_wx + lane_base + half * 32, reinterpret_cast<uint32_t(&)[32]>(y));
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&sh.y_empty);
                 const int tok = (c - 1) * TS_TOK + t;
                 const int cols = tok < p.S ? p.P - p0 - half * 32 : 0;
                 __nv_bfloat16* o = p.y + (((int64_t)b * p.S + tok) * p.H + h) * p.P + p0 + half * 32;
 #pragma unroll
-                for (int e = 0; e < 32; e += 8) {
-                    if (e < cols) {                           // P is a multiple of 8
+                for (int q = 0; q < 2; ++q) {
+                    float x[16], y[16];
+                    tmem_ld(t_qs + lane_base + half * 32 + q * 16, reinterpret_cast<uint32_t(&)[16]>(x));
+                    tmem_ld(t_wx + lane_base + half * 32 + q * 16, reinterpret_cast<uint32_t(&)[16]>(y));
+                    if (q == 1) {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&sh.y_empty);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 16; e += 8) {
+                        const uint4 own = x_out[q * 2 + e / 8];
+                        const uint32_t w[4] = {own.x, own.y, own.z, own.w};
                         float r[8];
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) r[j] = fmaf(carry, x[e + j], y[e + j]);
-                        store_vec<__nv_bfloat16, 8>(o + e, r);
+                        for (int j = 0; j < 8; ++j) {
+                            const float xt = __uint_as_float(j & 1 ? w[j >> 1] & 0xffff0000u : w[j >> 1] << 16);
+                            r[j] = fmaf(skip, xt, fmaf(carry, x[e + j], y[e + j]));
+                        }
+                        if (q * 16 + e < cols) store_vec<__nv_bfloat16, 8>(o + q * 16 + e, r);       // P is a multiple of 8
                     }
                 }
             }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x_out[e] = x_own[e];
             carry = next;
         }
     } else if (warp < 12) {

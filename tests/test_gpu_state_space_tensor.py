@@ -65,3 +65,20 @@ def test_many_chunks_and_heads():
     assert torch.isfinite(got[1][0]).all()
     assert (got[0][1] - got[1][1]).abs().max() <= 6e-5 * got[0][1].abs().max()
     assert (got[0][0] - got[1][0]).abs().max() <= 2.0 ** -7 * got[0][0].abs().max()
+
+
+def test_the_skip_is_one_fp32_product():
+    """Without queries an output is the skip alone: D x in fp32, rounded once to the output's type, as the block form leaves it."""
+    c, B, S = dict(H=64, P=24, N=16, G=2, taps=1), 2, 333     # many skips: an input has 128 mantissas only
+    proj, w, inner, ch = _ssm_inputs(c, B, S, BF16, seed=5)
+    n_qk = c["G"] * c["N"]
+    w["conv_b"][inner + n_qk:inner + 2 * n_qk] = 0
+    proj[:, inner + inner + n_qk:inner + inner + 2 * n_qk] = 0
+    w["D"] *= 10.0 ** torch.linspace(-3, 3, c["H"])
+    w = {k: v.to(DEV) for k, v in w.items()}
+    got = []
+    for path in ("chunks", "auto"):
+        conv, state = torch.zeros(B, 0, ch, dtype=BF16, device=DEV), torch.zeros(B, c["H"], c["N"], c["P"], device=DEV)
+        got.append(_scan(proj.to(DEV), w, c, B, S, inner, state, conv, path=path))
+    assert (got[0] != 0).float().mean() > 0.9
+    assert torch.equal(got[0], got[1])
