@@ -420,8 +420,10 @@ ssm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 for (int part = 0; part < 2; ++part)
 #pragma unroll
                     for (int k = 0; k < TS_TOK / 16; ++k)
-                        umma_ts_by(leader, t_wx, t_sc + st * 128 + (k >> 1) * 32 + part * 16 + (k & 1) * 8,
-                                   umma_desc_at(x_mn, at + k * (2048 >> 4)), id_mn, part > 0 || k > 0);
+                        // rows before these 16 keys have weights of zero for them, which an infinite or NaN x would not leave without
+                        // effect: they are left out (k = 0, which all rows take, comes first)
+                        umma_ts_from(leader, t_wx, t_sc + st * 128 + (k >> 1) * 32 + part * 16 + (k & 1) * 8,
+                                     umma_desc_at(x_mn, at + k * (2048 >> 4)), id_mn, part > 0 || k > 0, k * 16);
                 if (nq > nw) umma_commit_by(leader, &sh.y_full);
                 if (nu > nw && nq > nw) umma_commit_by(leader, &sh.empty[st]);
                 ++nw;

@@ -246,6 +246,24 @@ __device__ __forceinline__ void umma_ts_by(bool leader, uint32_t tmem_d, uint32_
         ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader)
         : "memory");
 }
+// the same, which leaves the accumulator's rows before first_row (a constant to the compiler) as they are
+__device__ __forceinline__ void umma_ts_from(bool leader, uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate,
+                                             int first_row) {
+    uint32_t off[4];                                          // a bit per row that is left out
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        const int n = first_row - 32 * w;
+        off[w] = n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u;
+    }
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%6, %7, %8, %9}, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate), "r"((uint32_t)leader), "r"(off[0]), "r"(off[1]), "r"(off[2]),
+          "r"(off[3])
+        : "memory");
+}
 __device__ __forceinline__ void umma_commit_by(bool leader, uint64_t* bar) {
     asm volatile(
         "{\n\t.reg .pred q;\n\t"

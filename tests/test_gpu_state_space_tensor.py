@@ -82,3 +82,25 @@ def test_the_skip_is_one_fp32_product():
         got.append(_scan(proj.to(DEV), w, c, B, S, inner, state, conv, path=path))
     assert (got[0] != 0).float().mean() > 0.9
     assert torch.equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("at", [0, 37, 127, 128, 200, 383])
+def test_a_value_that_is_not_finite_reaches_no_token_before_its_16(at, value):
+    """One such x: its column from its 16 tokens on, as in the block form; every other output as without it, bit for bit."""
+    c, B, S, col = dict(H=2, P=72, N=24, G=1, taps=1), 1, 400, 72 + 67      # head 1, beyond its first 64 columns
+    proj, w, inner, ch = _ssm_inputs(c, B, S, BF16, seed=7)
+    w = {k: v.to(DEV) for k, v in w.items()}
+    got = []
+    for x in (None, value):
+        rows = proj.clone()
+        if x is not None:
+            rows[at, inner + col] = x
+        conv, state = torch.zeros(B, 0, ch, dtype=BF16, device=DEV), torch.zeros(B, 2, 24, 72, device=DEV)
+        got.append((_scan(rows.to(DEV), w, c, B, S, inner, state, conv), state.transpose(2, 3).reshape(B, inner, -1)))
+    (y0, st0), (y1, st1) = got
+    assert torch.isfinite(y0).all() and not torch.isfinite(y1[at, col]) and not torch.isfinite(st1[:, col]).any()
+    first = at // 16 * 16
+    assert torch.equal(y0[:first], y1[:first])
+    others = torch.arange(inner, device=DEV) != col
+    assert torch.equal(y0[:, others], y1[:, others]) and torch.equal(st0[:, others], st1[:, others])
