@@ -13,6 +13,7 @@
 // stores its partial (max, sum, acc[D]) into the first one's shared memory, which merges them and writes the output - 1 us
 // after the slowest CTA, where a fence, a ticket and another CTA's loads through L2 took 3 (32 rows of 1216 entries).  A row
 // of more CTAs has several clusters, whose first CTAs write partials and take a ticket; the last one merges those.
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -33,6 +34,8 @@ constexpr int DEC_G = 8;                   // list entries per stage and warp
 constexpr int DEC_STAGES = 2;
 constexpr int DEC_D = 128;
 constexpr float LOG2E = 1.4426950408889634f;
+// shared memory of an SM, of it what each CTA takes beside its own, and the most that one CTA can have
+constexpr int DEC_SM_SMEM = 228 * 1024, DEC_CTA_SMEM = 1024, DEC_MAX_SMEM = 227 * 1024;
 
 __host__ __device__ inline size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
@@ -60,18 +63,6 @@ inline int decode_splits(int64_t rows, int64_t max_len) {
     return (int)s;
 }
 constexpr int DEC_CLUSTER = 8;                           // the largest portable cluster
-// As many CTAs as decode_splits allows, in equal clusters; nine become one cluster of eight.  Without clusters where there are
-// three CTAs per SM: not all clusters find a place at once then, and the gather is bound by bandwidth (128 rows of 2368
-// entries in clusters of three: the step 129 us, without 121).
-// fp32 rows: the ring of one CTA takes more than half of an SM's shared memory, so one CTA per SM.
-inline DecodeSplit decode_split(int64_t rows, int64_t max_len, bool f32) {
-    int s = decode_splits(rows, max_len);
-    if (f32 && s > sm_count() / rows) s = sm_count() / rows > 1 ? (int)(sm_count() / rows) : 1;
-    if (s * rows > 2 * sm_count()) return {1, s};
-    if (s <= DEC_CLUSTER + 1) return {s < DEC_CLUSTER ? s : DEC_CLUSTER, 1};
-    const int groups = (s + DEC_CLUSTER - 1) / DEC_CLUSTER;
-    return {s / groups, groups};
-}
 
 // smem_dst: 32-bit shared-window address (converted once per kernel, not per copy)
 __device__ __forceinline__ void cp_async16(uint32_t smem_dst, const void* gmem_src) {
@@ -150,14 +141,14 @@ template <typename KT> struct DecSmem {
     static_assert(MERGE <= RING, "merge buffers alias the ring");
 };
 
-template <typename QT, typename KT>
-__global__ void __launch_bounds__(DEC_THREADS)
+template <typename QT, typename KT, bool CLUSTERS>
+__global__ void __launch_bounds__(DEC_THREADS, 3)          // 80 registers: with the 64 the compiler took of itself 40 x 4096 15.4 us, so 15.0
 sparse_decode_kernel(const QT* __restrict__ q, const KT* __restrict__ k_cache,
                      const KT* __restrict__ v_cache, int64_t kv_bs, int64_t kv_hs, int64_t kv_rs,
                      const int32_t* __restrict__ list, int64_t list_rs,
                      const int32_t* __restrict__ list_len, int64_t max_len, QT* __restrict__ out,
                      int H, int Hkv, int64_t T, const int32_t* __restrict__ T_dev, int32_t* tickets,
-                     float* ws_ml, float* ws_acc, int32_t* status, int cluster) {
+                     float* ws_ml, float* ws_acc, int32_t* status, int cluster_size) {
     using S = DecSmem<KT>;
     constexpr int CPR = S::ROW / 16;                    // 16-byte chunks per row
     constexpr int COPIES = DEC_G * CPR / 32;            // cp.async per lane for the K (or V) rows
@@ -165,16 +156,16 @@ sparse_decode_kernel(const QT* __restrict__ q, const KT* __restrict__ k_cache,
     extern __shared__ __align__(128) char smem[];
     int32_t* sidx_all = reinterpret_cast<int32_t*>(smem + S::RING);
     float* part_s = reinterpret_cast<float*>(smem + S::RING + S::IDX);     // [rank][D], then [rank][max, sum]
-    int* is_last = reinterpret_cast<int*>(smem + S::RING + S::IDX + S::PART);
+    int* is_last = reinterpret_cast<int*>(smem + S::RING + S::IDX + (CLUSTERS ? S::PART : 0));
 
-    const int splits = gridDim.x, split = blockIdx.x;
+    const int splits = gridDim.x, split = blockIdx.x, cluster = CLUSTERS ? cluster_size : 1;
     const int row = blockIdx.y;                    // b*H + h
     const int b = row / H, h = row - b * H;
     const int kvh = h / (H / Hkv);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int hw = tid >> 4, hw2 = lane >> 4, hl = tid & 15;
     pdl_launch_dependents();
-    if (cluster > 1) cluster_arrive();             // waited for before the first store into another CTA
+    if (CLUSTERS) cluster_arrive();                // waited for before the first store into another CTA
 
     // the query is an input of the whole step, so it can be fetched before the list exists
     // 16-bit query and keys of one type: the query stays packed and the scale is applied to the
@@ -399,7 +390,7 @@ sparse_decode_kernel(const QT* __restrict__ q, const KT* __restrict__ k_cache,
             mm = mn;
         }
     };
-    if (cluster > 1) {
+    if (CLUSTERS) {
         const int rank = split % cluster;
         float* ml = part_s + DEC_CLUSTER * DEC_D;
         cluster_wait();                    // every CTA of the cluster has begun
@@ -420,8 +411,8 @@ sparse_decode_kernel(const QT* __restrict__ q, const KT* __restrict__ k_cache,
     }
     const int groups = splits / cluster, group = split / cluster;
     if (groups > 1) {
-        const size_t slot = (size_t)row * groups + group;
         if (tid < DEC_D) {
+            const size_t slot = (size_t)row * groups + group;
             ws_acc[slot * DEC_D + tid] = a;
             if (tid == 0) {
                 ws_ml[slot * 2] = mm;
@@ -436,16 +427,22 @@ sparse_decode_kernel(const QT* __restrict__ q, const KT* __restrict__ k_cache,
             *is_last = (t == groups - 1);
         }
         __syncthreads();
-        if (!*is_last) return;
+        if (!*is_last || tid >= DEC_D) return;
         __threadfence();
         mm = -INFINITY;
         ll = a = 0.f;
-        if (tid < DEC_D) {
+        // add_partial spelt out: called here, it left the loads one behind another (36 x 4096 bf16 13.8 us, so 13.6)
 #pragma unroll 4
-            for (int i = 0; i < groups; ++i) {
-                const size_t at = (size_t)row * groups + i;
-                const float2 p = __ldcg(reinterpret_cast<const float2*>(ws_ml + at * 2));
-                add_partial(p.x, p.y, __ldcg(ws_acc + at * DEC_D + tid));
+        for (int i = 0; i < groups; ++i) {
+            const size_t at = (size_t)row * groups + i;
+            const float2 p = __ldcg(reinterpret_cast<const float2*>(ws_ml + at * 2));
+            const float v = __ldcg(ws_acc + at * DEC_D + tid);
+            if (p.x > -INFINITY) {
+                const float mn = fmaxf(mm, p.x);
+                const float fo = exp2f(mm - mn), fn = exp2f(p.x - mn);
+                ll = ll * fo + p.y * fn;
+                a = a * fo + v * fn;
+                mm = mn;
             }
         }
         if (tid == 0) tickets[row] = 0;    // ready for the next call
@@ -453,18 +450,96 @@ sparse_decode_kernel(const QT* __restrict__ q, const KT* __restrict__ k_cache,
     if (tid < DEC_D) out[(size_t)row * DEC_D + tid] = from_f32<QT>(ll > 0.f ? a / ll : 0.f);
 }
 
+// Clusters of `cluster` CTAs that find a place at once with `per_sm` CTAs on an SM; asked of the driver once per device.
+template <typename QT, typename KT> int cluster_room(int cluster, int per_sm) {
+    constexpr int MAX_DEV = 64, PER = 3;
+    static std::atomic<int> known[MAX_DEV][DEC_CLUSTER + 1][PER + 1];        // plus one; 0: not asked yet
+    int dev = -1;
+    if (cluster < 1 || cluster > DEC_CLUSTER || per_sm < 1 || per_sm > PER || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEV)
+        return 0;
+    std::atomic<int>& k = known[dev][cluster][per_sm];
+    int n = k.load(std::memory_order_relaxed);
+    if (n > 0) return n - 1;
+    // shared memory that leaves an SM room for per_sm CTAs
+    const int share = (DEC_SM_SMEM / per_sm - DEC_CTA_SMEM) / 1024 * 1024;
+    const int smem = share > DecSmem<KT>::TOTAL ? (share < DEC_MAX_SMEM ? share : DEC_MAX_SMEM) : DecSmem<KT>::TOTAL;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)cluster);
+    cfg.blockDim = dim3(DEC_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = (unsigned)cluster;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    auto kern = sparse_decode_kernel<QT, KT, true>;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_MAX_SMEM) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();               // no clusters then, and no error of the next launch
+        n = 0;
+    }
+    k.store(n + 1, std::memory_order_relaxed);
+    return n;
+}
+
+// The CTAs of a row as clusters, of as many CTAs as decode_splits allows and as find a place at once for all rows: a cluster has to fit
+// one GPC, and what does not fit waits for a whole one to end.  Measured alone, us, rows x entries:
+//   bf16   16 x 1216: a cluster of 8 6.2, three of 6 8.5, 18 CTAs without clusters 8.1;  48 x 2368: 5 12.4, 6 (some SMs with three CTAs, some
+//          with one) 13.9, 6 without clusters 12.8;  64 x 2368, three CTAs an SM: 6 14.8, without 15.7
+//   fp32   24 x 2368: 5 12.5, 6 (which do not fit) 19.8;  48 x 2368: 3 without clusters 21.4, 3 (which do not fit) 34.1, 2 24.0
+// Inside a step the CTAs become resident while the select of other rows still runs: three an SM there, evenly spread or not (steps with 48 x
+// 2368: 6 46.5, 5 47.6; with 96 x 1216: 3 52.7, without 54.0), but no clusters where all three are needed (a step of 128 rows of 131072 keys: 117
+// with clusters of 3, 109 without).
+struct DecodeRule {
+    // a list of more entries has several clusters (bf16 16 x 4096: two of 8 9.5, one 11.0; 16 x 2368: one 8.2)
+    static constexpr int64_t GROUP_LEN = 3072;
+    // entries a CTA up to which latency counts more than the spread over the SMs; from which CTAs count more than a cluster; from which all do
+    static constexpr int64_t SHORT = 128, LONG = 256, FULL = 448;
+    static constexpr int64_t F32_LONG = 2048;
+};
+template <typename QT, typename KT> DecodeSplit decode_split(int64_t rows, int64_t max_len) {
+    int s = decode_splits(rows, max_len);
+    const int sms = sm_count();
+    const bool chained = pdl_chain_active(), thirds = s * rows > 2 * sms;
+    int per_sm = chained || thirds || max_len <= DecodeRule::SHORT * s ? 3 : 2;
+    if (std::is_same<KT, float>::value) {
+        // One CTA an SM, and so no more than there are SMs (32 x 1216: 9.9 us, in two waves 15.7), except where the rows alone are more (160 x
+        // 2368: 78.5, one a row 91.0) and where one a row leaves much of the chip without work (80 x 2368: 38.7, one a row 42.3; 80 x 1216:
+        // 24.3 and 23.5; 90 x 2368: 47.1 and 42.8).
+        per_sm = 1;
+        const int64_t once = sms / rows;
+        if (once > 1) s = s < once ? s : (int)once;
+        else if (once == 1 && !(7 * rows <= 4 * sms && max_len >= DecodeRule::F32_LONG)) s = 1;
+    } else if (chained && thirds) {
+        return {1, s};
+    }
+    for (int c = s < DEC_CLUSTER ? s : DEC_CLUSTER; c > 1; --c) {
+        int64_t groups = cluster_room<QT, KT>(c, per_sm) / rows;
+        if (groups < 1) continue;
+        const int64_t wanted = (max_len + DecodeRule::GROUP_LEN - 1) / DecodeRule::GROUP_LEN;
+        if (groups > wanted) groups = wanted;
+        if (groups > s / c) groups = s / c;
+        // fewer CTAs than without clusters: not much fewer, except of short lists, and where they are bound by their entries hardly any
+        const int64_t n = groups * c;
+        if (4 * n < 3 * s && (c < DEC_CLUSTER || max_len > DecodeRule::LONG * s)) break;
+        if (8 * n <= 7 * s && max_len > DecodeRule::FULL * s) break;
+        return {c, (int)groups};
+    }
+    return {1, s};
+}
+
 template <typename QT, typename KT>
-int decode_launch(DecodeSplit split, int64_t rows, cudaStream_t st, const void* q, const void* k_cache, const void* v_cache,
+int decode_launch(int64_t rows, cudaStream_t st, const void* q, const void* k_cache, const void* v_cache,
                   int64_t kv_bs, int64_t kv_hs, int64_t kv_rs, const int32_t* list, int64_t list_rs,
                   const int32_t* list_len, int64_t max_list_len, void* out, int H, int Hkv, int64_t T,
                   const int32_t* T_dev, int32_t* tickets, float* ws_ml, float* ws_acc, int32_t* status) {
-    auto kern = sparse_decode_kernel<QT, KT>;
-    constexpr int smem = DecSmem<KT>::TOTAL;
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess)
-            return fail(SK_ERR_CUDA, "sparse_decode_kernel smem attribute: %s", cudaGetErrorString(e));
-    }
+    const DecodeSplit split = decode_split<QT, KT>(rows, max_list_len);
+    auto kern = sparse_decode_kernel<QT, KT, false>;
+    if (split.cluster > 1) kern = sparse_decode_kernel<QT, KT, true>;
+    const int smem = split.cluster > 1 ? DecSmem<KT>::TOTAL : DecSmem<KT>::TOTAL - DecSmem<KT>::PART;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, split.cluster > 1 ? DEC_MAX_SMEM : smem);
+    if (e != cudaSuccess) return fail(SK_ERR_CUDA, "sparse_decode_kernel smem attribute: %s", cudaGetErrorString(e));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(split.cluster * split.groups), (unsigned)rows);
     cfg.blockDim = dim3(DEC_THREADS);
@@ -481,8 +556,8 @@ int decode_launch(DecodeSplit split, int64_t rows, cudaStream_t st, const void* 
         attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
         ++cfg.numAttrs;
     }
-    cfg.attrs = attr;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (const QT*)q, (const KT*)k_cache, (const KT*)v_cache, kv_bs, kv_hs, kv_rs, list,
+    cfg.attrs = cfg.numAttrs ? attr : nullptr;
+    e = cudaLaunchKernelEx(&cfg, kern, (const QT*)q, (const KT*)k_cache, (const KT*)v_cache, kv_bs, kv_hs, kv_rs, list,
                                              list_rs, list_len, max_list_len, (QT*)out, H, Hkv, T, T_dev, tickets, ws_ml, ws_acc,
                                              status, split.cluster);
     if (e != cudaSuccess) return fail(SK_ERR_CUDA, "sparse_decode_kernel: %s", cudaGetErrorString(e));
@@ -513,15 +588,14 @@ int launch_sparse_decode(const void* q, int q_dtype, const void* k_cache, const 
     const size_t need = sparse_decode_workspace_bytes(B, H, D, max_list_len);
     if (workspace_bytes < need)
         return fail(SK_ERR_WORKSPACE, "sk_sparse_decode: workspace %zu < %zu bytes", workspace_bytes, need);
-    const int splits = decode_splits(rows, max_list_len);       // at least as many as there are partials
-    const DecodeSplit split = decode_split(rows, max_list_len, kv_dtype == SK_F32);
+    const int splits = decode_splits(rows, max_list_len);       // no fewer than there are partials
     char* ws = static_cast<char*>(workspace);
     int32_t* tickets = reinterpret_cast<int32_t*>(ws);
     float* ws_ml = reinterpret_cast<float*>(ws + DEC_TICKET_BYTES);
     float* ws_acc = reinterpret_cast<float*>(ws + DEC_TICKET_BYTES +
                                              align256((size_t)rows * splits * 2 * sizeof(float)));
 #define SK_DEC_LAUNCH(QT, KT)                                                                        \
-    return decode_launch<QT, KT>(split, rows, st, q, k_cache, v_cache, kv_bs, kv_hs, kv_rs, list, list_rs,  \
+    return decode_launch<QT, KT>(rows, st, q, k_cache, v_cache, kv_bs, kv_hs, kv_rs, list, list_rs,  \
                                  list_len, max_list_len, out, H, Hkv, T, T_dev, tickets, ws_ml,      \
                                  ws_acc, status)
     if (q_dtype == SK_BF16 && kv_dtype == SK_BF16) SK_DEC_LAUNCH(__nv_bfloat16, __nv_bfloat16);
