@@ -166,7 +166,8 @@ SK_API int skb_latent_up(const void* o, int dtype, const void* uv, int64_t rows,
  * inputs conv_state [B, taps - 1, channels].  skb_ssm_scan: the recurrence on those rows,
  * state [B, H, N, P] fp32, y [B, S, H P] (with the skip D x).  Position 0 starts from zero state.
  * `path`: SKB_SSM_STEPS walks token by token, SKB_SSM_CHUNKS uses matrix products per block of 64 tokens; SKB_SSM_AUTO
- * also has chunks of 128 tokens on the tensor cores (skb_ssm_path then says SKB_SSM_TENSOR). */
+ * also has chunks of 128 tokens on the tensor cores (skb_ssm_path then says SKB_SSM_TENSOR).  `status`: NULL, or a device word
+ * that collects SK_DEV_WAIT_TIMEOUT; the head's outputs and state are NaN then. */
 enum { SKB_SSM_AUTO = 0, SKB_SSM_STEPS = 1, SKB_SSM_CHUNKS = 2, SKB_SSM_TENSOR = 3 };
 typedef struct sk_ssm_params {
     const void *xbc_in, *dt_in, *conv_w, *conv_b;
@@ -178,6 +179,7 @@ typedef struct sk_ssm_params {
     size_t workspace_bytes;
     int64_t in_ld, xbc_ld, start;
     int dtype, B, S, H, P, N, G, taps, path;
+    int32_t* status;
 } sk_ssm_params;
 SK_API int skb_ssm_conv(const sk_ssm_params* p, void* stream);
 SK_API size_t skb_ssm_workspace_bytes(const sk_ssm_params* p);

@@ -157,6 +157,7 @@ class SsmParams(C.Structure):
         ("dt_bias", _p), ("A_log", _p), ("D", _p), ("state", _p), ("pos", _p),
         ("workspace", _p), ("workspace_bytes", _sz), ("in_ld", _i64), ("xbc_ld", _i64), ("start", _i64),
         ("dtype", _i), ("B", _i), ("S", _i), ("H", _i), ("P", _i), ("N", _i), ("G", _i), ("taps", _i), ("path", _i),
+        ("status", _p),
     ]
 
 

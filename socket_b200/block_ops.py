@@ -241,7 +241,7 @@ def latent_up(o: Tensor, uv: Tensor, vdim: int) -> Tensor:
 
 def ssm(proj: Tensor, inner: int, conv_w: Tensor, conv_b: Tensor, dt_bias: Tensor, A_log: Tensor, D: Tensor,
         conv_state: Tensor, state: Tensor, *, S: int, groups: int, start: int = 0, pos: Optional[Tensor] = None,
-        path: str = "auto") -> Tensor:
+        path: str = "auto", status: Optional[Tensor] = None) -> Tensor:
     """proj rows [z | x | B | C | dt] (B*S of them, strided) -> y [B*S, inner] before the gate; conv_state
     [B, taps - 1, channels] and state [B, H, N, P] (fp32) are advanced by the portion."""
     _require_cuda(proj, conv_w, conv_b, dt_bias, A_log, D, conv_state, state)
@@ -262,7 +262,7 @@ def ssm(proj: Tensor, inner: int, conv_w: Tensor, conv_b: Tensor, dt_bias: Tenso
     p.dt_bias, p.A_log, p.D, p.state, p.pos, p.start = ptr(dt_bias), ptr(A_log), ptr(D), ptr(state), ptr(pos), start
     p.in_ld, p.xbc_ld = proj.stride(0), xbc_ld
     p.dtype, p.B, p.S, p.H, p.P, p.N, p.G, p.taps = dtype_code(proj), B, S, H, P, N, groups, taps
-    p.path = SSM_PATHS[path]
+    p.path, p.status = SSM_PATHS[path], ptr(status)
     need = int(blocks().skb_ssm_workspace_bytes(C.byref(p)))
     ws = torch.empty(need, dtype=torch.uint8, device=proj.device) if need else None
     p.workspace, p.workspace_bytes = ptr(ws), need

@@ -19,7 +19,7 @@
 // blocks do so), and the 56 MMAs read 290 KiB of operands from shared memory (3400).  The roles' code has to stay small:
 // with every loop of a chunk unrolled (90 KiB of instructions, of which each warp walks its own part once per chunk) a chunk
 // took 6900 cycles.
-// Every wait is bounded; if one runs out, all roles leave and the head's columns of y and its state become NaN.
+// Every wait is bounded; if one runs out, all roles leave, the head's columns of y and its state become NaN, and the status word says so.
 #include "blocks.cuh"
 #include "tcgen05.cuh"
 #include "tensor_map.cuh"
@@ -39,6 +39,7 @@ struct TsShape {
     const float *dt, *cum;            // [B, H, chunks, 128]
     const float* skip;
     float* state;                     // [B, H, N, P]
+    int32_t* status;
     __nv_bfloat16* y;                 // [B S, H P]
     int64_t start;
     int S, H, P, N, rep, chunks;
@@ -437,7 +438,8 @@ ssm_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     }
     if (!ok && lane == 0) *failed = 1;
     __syncthreads();
-    if (sh.failed) {                                          // loud, and without a status word
+    if (sh.failed) {
+        if (tid == 0 && p.status != nullptr) atomicOr(p.status, SK_DEV_WAIT_TIMEOUT);
         const int c = tid & (TS_P - 1);
         if (p0 + c < p.P) {
 #pragma unroll 1
@@ -487,6 +489,7 @@ int launch_ssm_tc(const sk_ssm_params& p, cudaStream_t st) {
     s.cum = cum;
     s.skip = p.D;
     s.state = p.state;
+    s.status = p.status;
     s.y = (__nv_bfloat16*)p.y;
     s.start = p.start;
     s.S = p.S;

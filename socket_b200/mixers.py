@@ -415,7 +415,8 @@ class Mamba2(nn.Module):
     def forward(self, h: Tensor, cache: StateCache, at: Portion) -> Tensor:
         proj = matmul(h, self.w_in, at.chained)
         y = ops.ssm(proj, self.inner, self.conv_w, self.conv_b, self.dt_bias_f32, self.A_log_f32, self.skip_f32,
-                    cache.conv[:at.B], cache.state[:at.B], S=at.S, groups=self.G, start=at.start, pos=at.pos)
+                    cache.conv[:at.B], cache.state[:at.B], S=at.S, groups=self.G, start=at.start, pos=at.pos,
+                    status=at.status)
         y = ops.gated_group_norm(y, proj, self.norm_w, self.parts, self.eps)
         return matmul(y, self.wo, at.chained)
 

@@ -2,8 +2,9 @@
 import ctypes as C
 
 import pytest
+import torch
 
-from socket_b200 import _lib
+from socket_b200 import _lib, block_ops, mixers
 
 AUTO, STEPS, CHUNKS, TENSOR = 0, 1, 2, 3
 
@@ -28,3 +29,31 @@ def test_route_and_workspace(kw, path):
     assert lib.skb_ssm_path(C.byref(p)) == path
     blocks = {TENSOR: -(-p.S // 128) * 128, CHUNKS: -(-p.S // 64) * 64, STEPS: 0}[path]
     assert lib.skb_ssm_workspace_bytes(C.byref(p)) == 8 * p.B * p.H * blocks
+
+
+def test_the_models_status_word_reaches_the_scan(monkeypatch):
+    """A wait that runs out in the tensor-core form is reported in the word that `device_flags()` reads."""
+    seen = []
+
+    class Library:
+        def skb_ssm_workspace_bytes(self, p):
+            return 0
+
+        def skb_ssm_conv(self, p, stream):
+            return 0
+
+        def skb_ssm_scan(self, p, stream):
+            seen.append(p._obj.status)
+            return 0
+
+    monkeypatch.setattr(block_ops, "blocks", Library)
+    monkeypatch.setattr(block_ops, "_require_cuda", lambda *t: None)
+    monkeypatch.setattr(block_ops, "stream_ptr", lambda device: None)
+    monkeypatch.setattr(block_ops, "gated_group_norm", lambda y, *a: torch.zeros_like(y))
+    layer = mixers.Mamba2(32, heads=4, vdim=8, state=16, groups=2, taps=4, norm_groups=2, eps=1e-5)
+    layer.finish_loading()
+    cache = layer.make_cache(1, 200, torch.float32, "cpu")
+    status = torch.zeros(1, dtype=torch.int32)
+    layer(torch.zeros(100, 32), cache, mixers.Portion(1, 100, 0, status=status))
+    layer(torch.zeros(100, 32), cache, mixers.Portion(1, 100, 100))
+    assert seen == [status.data_ptr(), None]
