@@ -167,7 +167,8 @@ SK_API int skb_latent_up(const void* o, int dtype, const void* uv, int64_t rows,
  * state [B, H, N, P] fp32, y [B, S, H P] (with the skip D x).  Position 0 starts from zero state.
  * `path`: SKB_SSM_STEPS walks token by token, SKB_SSM_CHUNKS uses matrix products per block of 64 tokens; SKB_SSM_AUTO
  * also has chunks of 128 tokens on the tensor cores (skb_ssm_path then says SKB_SSM_TENSOR).  `status`: NULL, or a device word
- * that collects SK_DEV_WAIT_TIMEOUT; the head's outputs and state are NaN then. */
+ * that collects SK_DEV_WAIT_TIMEOUT; the head's outputs and state are NaN then.  A workspace that is not 16-byte aligned leaves
+ * that form out. */
 enum { SKB_SSM_AUTO = 0, SKB_SSM_STEPS = 1, SKB_SSM_CHUNKS = 2, SKB_SSM_TENSOR = 3 };
 typedef struct sk_ssm_params {
     const void *xbc_in, *dt_in, *conv_w, *conv_b;
@@ -193,7 +194,7 @@ SK_API int skb_ssm_path(const sk_ssm_params* p);
  *   o = q_scale S'^T q / (max(|q_scale n' . q|, exp(-m')) + 1e-6),
  *   out = o / rms(o) * norm_w * sigmoid(z)              out rows [H P], out_ld apart
  * State: S [B, H, N, P], n [B, H, N], m [B, H], all fp32; position 0 starts from zero state and m = 0.
- * num [B S, H P] (of dtype), den [B S, H] and m_next [B, H] (fp32) are scratch.
+ * num [B S, H P] (of dtype), den [B S, H] and m_next [B, H] (fp32) are scratch; the workspace is 16-byte aligned.
  * `path`: SKB_SSM_STEPS walks token by token, SKB_SSM_CHUNKS uses warp-level matrix products per block of 64
  * tokens, SKB_SSM_TENSOR tensor-memory ones per chunk of 128, all chunks of a portion side by side. */
 typedef struct sk_mlstm_params {

@@ -236,6 +236,7 @@ int skb_mlstm(const sk_mlstm_params* p, void* stream) {
         return fail(SK_ERR_UNSUPPORTED, "skb_mlstm: shape outside the block kernels");
     if (mlstm_workspace(*p) > 0 && (p->workspace == nullptr || p->workspace_bytes < mlstm_workspace(*p)))
         return fail(SK_ERR_WORKSPACE, "skb_mlstm: workspace of %zu bytes needed, %zu given", mlstm_workspace(*p), p->workspace_bytes);
+    if (path == SKB_SSM_TENSOR) SK_ALIGNED(p->workspace, 16, "skb_mlstm: workspace");
     const int rc = path == SKB_SSM_TENSOR ? launch_mlstm_tc(*p, st) : path == SKB_SSM_CHUNKS ? launch_mlstm_chunks(*p, st)
                                                                                             : launch_mlstm_steps(*p, st);
     return rc != SK_OK ? rc : launch_mlstm_finish(*p, st);

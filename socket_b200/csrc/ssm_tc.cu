@@ -461,6 +461,8 @@ size_t ssm_tc_workspace(const sk_ssm_params& p) {             // step sizes and 
 }
 
 bool ssm_tc_applicable(const sk_ssm_params& p) {
+    // step sizes and decays are written and copied 16 bytes at a time (no workspace yet: a query)
+    if ((uintptr_t)p.workspace % 16 != 0) return false;
     if (p.dtype != SK_BF16 || p.pos != nullptr || p.N % 8 != 0 || p.N > 128 || p.P % 8 != 0) return false;
     const __nv_bfloat16* x = (const __nv_bfloat16*)p.xbc;
     const __nv_bfloat16* k = x + (int64_t)p.H * p.P;

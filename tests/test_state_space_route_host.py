@@ -31,6 +31,26 @@ def test_route_and_workspace(kw, path):
     assert lib.skb_ssm_workspace_bytes(C.byref(p)) == 8 * p.B * p.H * blocks
 
 
+@pytest.mark.parametrize("off", [4, 8, 12])
+def test_a_workspace_off_16_bytes(off):
+    """The tensor-core forms move their scratch 16 bytes at a time.  The state space takes the blocks of 64 tokens instead, for which the
+    scratch asked for without a workspace is enough; the matrix memory refuses before any launch."""
+    lib, p = _lib.blocks(), _params()
+    asked = lib.skb_ssm_workspace_bytes(C.byref(p))
+    p.workspace = (1 << 24) + off
+    assert lib.skb_ssm_path(C.byref(p)) == CHUNKS and lib.skb_ssm_workspace_bytes(C.byref(p)) <= asked
+    p.workspace = (1 << 24) + 16
+    assert lib.skb_ssm_path(C.byref(p)) == TENSOR and lib.skb_ssm_workspace_bytes(C.byref(p)) == asked
+    m = _lib.MlstmParams()
+    for name in ("q", "k", "v", "z", "norm_w", "gates", "i_bias", "f_bias", "S_state", "n_state", "m_state", "num", "den", "m_next", "out"):
+        setattr(m, name, 1 << 20)
+    m.dtype, m.B, m.S, m.H, m.N, m.P, m.cap = _lib.SK_BF16, 1, 300, 4, 64, 64, 15.0
+    m.in_ld, m.gates_ld, m.out_ld = 2048, 8, 256
+    assert lib.skb_mlstm_path(C.byref(m)) == TENSOR
+    m.workspace, m.workspace_bytes = (1 << 24) + off, lib.skb_mlstm_workspace_bytes(C.byref(m))
+    assert lib.skb_mlstm(C.byref(m), None) == -3 and b"workspace" in lib.skb_last_error()
+
+
 def test_the_models_status_word_reaches_the_scan(monkeypatch):
     """A wait that runs out in the tensor-core form is reported in the word that `device_flags()` reads."""
     seen = []
