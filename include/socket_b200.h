@@ -91,9 +91,9 @@ SK_API int sk_kv_append(const void* k_new, const void* v_new, int kv_dtype, cons
  * bit.  bf16 keys and planes, D = 128, L = 32, P = 8; codes are uint8.
  *   dst_row    NULL, or [N] int64: row n's codes go to codes + dst_row[n] * code_row_stride
  *              (negative = skip the row); lets a [B,S,Hkv] batch land in a [B,Hkv,Tcap] cache
- *   workspace  sk_hash_keys_tc_workspace_bytes(N) bytes, 256-byte aligned
+ *   workspace  not used (its query says 0 bytes): may be NULL
  * sk_kv_append_tc = sk_kv_append for many tokens at once (prefill) on that path, which sk_kv_append also takes by
- * itself for bf16 or fp16 rows from 512 on.  The kernel needs no scratch; the workspace stays part of the interface.
+ * itself for bf16 or fp16 rows from 512 on.  The same of its workspace.
  * Replaces the same reference code as sk_hash_keys / sk_kv_append.
  * ---------------------------------------------------------------------------------- */
 SK_API size_t sk_hash_keys_tc_workspace_bytes(int64_t N);

@@ -295,9 +295,8 @@ int launch_score_select_cluster(const float* lut, const uint8_t* codes, const ui
                                 int32_t* status, cudaStream_t st);
 
 // Tensor-core bulk hashing (bf16, head_dim 128, L*P = 256)
-size_t hash_keys_tc_workspace_bytes(int64_t N);
 int launch_hash_keys_tc(const void* keys, int64_t key_row_stride, const void* planes, int64_t N, uint8_t* codes,
-                        int64_t code_row_stride, const int64_t* dst_row, size_t workspace_bytes, int32_t* status, cudaStream_t st);
+                        int64_t code_row_stride, const int64_t* dst_row, int32_t* status, cudaStream_t st);
 bool kv_append_tc_applicable(const void* k_new, const void* v_new, int kv_dtype, const void* planes, int plane_dtype,
                              const void* k_cache, const void* v_cache, const uint8_t* codes, int64_t N, int D, int L, int P);
 int launch_kv_append_tc(const void* k_new, const void* v_new, int kv_dtype, const int64_t* input_pos, const void* planes,

@@ -646,20 +646,10 @@ int hash_tc_launch(const void* keys, int64_t key_row_stride, const void* planes,
 
 }  // namespace
 
-constexpr size_t TC_WS_HEADER = 256 + (TC_N + 16) * sizeof(float);
-
-// The kernel keeps its near-zero projections on chip; callers still bring the workspace that the interface names.
-size_t hash_keys_tc_workspace_bytes(int64_t N) {
-    const int64_t cap = N > 4096 ? N : 4096;
-    return TC_WS_HEADER + (size_t)cap * sizeof(uint32_t);
-}
-
 int launch_hash_keys_tc(const void* keys, int64_t key_row_stride, const void* planes, int64_t N, uint8_t* codes,
-                        int64_t code_row_stride, const int64_t* dst_row, size_t workspace_bytes, int32_t* status, cudaStream_t st) {
+                        int64_t code_row_stride, const int64_t* dst_row, int32_t* status, cudaStream_t st) {
     if (N == 0) return SK_OK;
     if (N >= TC_MAX_ROWS) return fail(SK_ERR_UNSUPPORTED, "sk_hash_keys_tc: at most 2^24 - 1 rows per call");
-    if (workspace_bytes < TC_WS_HEADER + 1024 * sizeof(uint32_t))
-        return fail(SK_ERR_WORKSPACE, "sk_hash_keys_tc: workspace %zu bytes is too small", workspace_bytes);
     return hash_tc_launch<__nv_bfloat16, false>(keys, key_row_stride, planes, N, codes, code_row_stride, dst_row, TcAppend{}, status, st);
 }
 

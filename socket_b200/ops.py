@@ -66,11 +66,10 @@ def hash_keys_tc(keys: torch.Tensor, planes: torch.Tensor, status: Optional[torc
     planes = planes.contiguous()
     N = keys.numel() // D
     codes = torch.empty(*keys.shape[:-1], L, dtype=torch.uint8, device=keys.device)
-    ws = torch.empty(int(lib().sk_hash_keys_tc_workspace_bytes(N)), dtype=torch.uint8, device=keys.device)
     if dtype_code(keys) != _lib.SK_BF16 or dtype_code(planes) != _lib.SK_BF16:
         raise RuntimeError("hash_keys_tc needs bf16 keys and planes")
-    check(lib().sk_hash_keys_tc(ptr(keys), D, ptr(planes), N, D, L, P, ptr(codes), L, None, ptr(ws), ws.numel(),
-                                ptr(status), stream_ptr(keys.device)), "sk_hash_keys_tc")
+    check(lib().sk_hash_keys_tc(ptr(keys), D, ptr(planes), N, D, L, P, ptr(codes), L, None, None, 0, ptr(status),
+                                stream_ptr(keys.device)), "sk_hash_keys_tc")
     return codes
 
 

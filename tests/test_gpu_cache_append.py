@@ -3,7 +3,7 @@ select): the same cache rows, codes, norms and length, bit for bit."""
 import pytest
 import torch
 
-from socket_b200 import ops
+from socket_b200 import _lib, ops
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -111,3 +111,32 @@ def test_rows_that_do_not_start_on_16_bytes_take_the_general_kernel():
     raw = torch.randn(2, S * 128 + 1, device=DEV).half()
     k, v = (t[1:].view(1, S, 1, 128) for t in raw)
     _both(1, S, 1, S, torch.arange(S, device=DEV), k, v, planes)
+
+
+def test_entry_points_by_name_with_strides_rows_elsewhere_and_no_workspace():
+    """`sk_hash_keys_tc` on rows 136 elements apart, whose codes go to rows 48 bytes apart in another order (negative: nowhere), and
+    `sk_kv_append_tc`: neither reads a workspace."""
+    g = torch.Generator(device=DEV).manual_seed(23)
+    N, planes = 1000, torch.randn(32, 8, 128, generator=g, device=DEV).bfloat16()
+    wide = torch.randn(N, 136, generator=g, device=DEV).bfloat16()
+    wide[40:400, :64] = 0                                    # near zero against a table's planes: decided from the rows in memory
+    planes[5, :, 64:] = 0
+    k, st = wide[:, :128].contiguous(), torch.cuda.current_stream().cuda_stream
+    want = ops.hash_keys(k, planes)
+    to = torch.randperm(N, generator=g, device=DEV)
+    to[::7] = -1
+    codes = torch.full((N, 48), 9, dtype=torch.uint8, device=DEV)
+    lib = _lib.lib()
+    assert lib.sk_hash_keys_tc_workspace_bytes(N) == lib.sk_kv_append_tc_workspace_bytes(1, N, 1) == 0
+    assert lib.sk_hash_keys_tc(wide.data_ptr(), 136, planes.data_ptr(), N, 128, 32, 8, codes.data_ptr(), 48, to.data_ptr(), None, 0, None, st) == 0
+    expect = torch.full_like(codes, 9)
+    expect[to[to >= 0], :32] = want[to >= 0]
+    assert torch.equal(codes, expect)
+    v, pos = torch.randn(1, N, 1, 128, generator=g, device=DEV).bfloat16(), torch.arange(N, device=DEV)
+    for S in (100, N):                                       # fewer rows than the general entry point would bring here, and more
+        got, ref = _cache(1, 1, N, torch.bfloat16), _cache(1, 1, N, torch.bfloat16)
+        kc, vc, cc, nc, length = got
+        assert lib.sk_kv_append_tc(k.data_ptr(), v.data_ptr(), _lib.SK_BF16, pos.data_ptr(), planes.data_ptr(), _lib.SK_BF16, kc.data_ptr(),
+                                   vc.data_ptr(), cc.data_ptr(), nc.data_ptr(), length.data_ptr(), None, 1, S, 1, 128, N, 32, 8, None, 0, st) == 0
+        ops.kv_append(*ref, pos[:S], k.view(1, N, 1, 128)[:, :S], v[:, :S], planes.float())
+        assert all(torch.equal(a, b) for a, b in zip(got, ref))
