@@ -1,5 +1,6 @@
-"""Cache appends of 16-bit rows in one tensor-core launch, against the exact fp64 kernel (which fp32 planes of the same values
-select): the same cache rows, codes, norms and length, bit for bit."""
+"""Cache appends of 16-bit rows in one tensor-core launch, against the general kernel (which fp32 planes of the same values
+select): the same cache rows, codes, norms and length, bit for bit.  Both let fp32 sums decide a sign outside the same band, so
+codes and norms of both are also compared with float64 sums."""
 import pytest
 import torch
 
@@ -15,6 +16,24 @@ def _cache(B, Hkv, T, dtype):
             torch.zeros((), dtype=torch.int32, device=DEV)]
 
 
+def _against_fp64(cache, pos, k, v, planes):
+    """Codes of the rows at their positions: signs of float64 sums, where no order of summing 128 products can change them.  Norms: float64
+    ones rounded to fp32 and then to fp16."""
+    live = (pos >= 0) & (pos < cache[0].shape[2])
+    k, v, at = k[:, live].double(), v[:, live].double(), pos[live]
+    flat = planes.double().view(256, 128)
+    for h in range(k.shape[2]):
+        kh = k[:, :, h]
+        prod = (kh @ flat.t()).nan_to_num(nan=-1.0, posinf=1.0, neginf=-1.0)
+        finite = torch.isfinite(kh).all(-1, keepdim=True) & torch.isfinite(flat).all(-1)
+        band = 1e-13 * kh.nan_to_num(0.0, 0.0, 0.0).norm(dim=-1, keepdim=True) * flat.nan_to_num(0.0, 0.0, 0.0).norm(dim=-1)
+        sure = (prod.abs() > band) | (prod == 0) | ~finite
+        codes = cache[2][:, h, at]
+        bits = (codes[..., None] >> torch.arange(7, -1, -1, device=DEV) & 1).bool().flatten(2)
+        assert torch.equal(bits & sure, (prod >= 0) & sure)
+        assert torch.equal(cache[3][:, h, at], (v[:, :, h] ** 2).sum(-1).sqrt().float().half())
+
+
 def _both(B, S, Hkv, T, pos, k, v, planes):
     got, want = _cache(B, Hkv, T, k.dtype), _cache(B, Hkv, T, k.dtype)
     flags = [torch.zeros((), dtype=torch.int32, device=DEV) for _ in range(2)]
@@ -23,6 +42,7 @@ def _both(B, S, Hkv, T, pos, k, v, planes):
     for name, g, w in zip(("keys", "values", "codes", "norms", "length"), got, want):
         assert torch.equal(g.view(torch.uint8) if g.dim() else g, w.view(torch.uint8) if w.dim() else w), name
     assert int(flags[0]) == int(flags[1])
+    _against_fp64(got, pos, k, v, planes)
     return got, int(flags[0])
 
 
