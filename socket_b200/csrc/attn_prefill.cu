@@ -640,21 +640,22 @@ uint32_t plan_smem(int dqk, int dv, bool bias, int* nk, int* nv) {
 }
 
 // CTAs that share a block's keys.  A call of few blocks leaves most SMs idle while its blocks walk over all keys: where two or four CTAs
-// a block find a place at once (32 clusters of four are certain to), they share it.  What joining costs shows where they don't: 8000
+// a block find a place at once, they share it: half as many pairs as there are SMs do, and two clusters of four for nine SMs (33 on 148, as
+// each GPC may leave some SMs over).  What joining costs shows where they don't: 8000
 // tokens, 16 heads are 512 blocks, 222 us alone, 266 by pairs, 401 by fours.  By the longest block's key tiles (one CTA | two | four):
 // 28 tiles, 32 blocks 65 | 45 | 35 us; 35 tiles of 192 / 128, 64 blocks 82 | 55 us; 16 tiles under a cap, 64 blocks 47 | 34 us; 6 tiles of
 // 256 / 128, 24 blocks 28.7 | 22.5 | 22.5 us.
 int fp_split(const FpShape& f, int B) {
-    const int64_t blocks = (int64_t)B * f.H * f.q_blocks;
+    const int64_t blocks = (int64_t)B * f.H * f.q_blocks, sms = sm_count();
     const int np = (f.dqk + 63) / 64, nvp = (f.dv + 63) / 64;
-    if (blocks > 72 || (2 + f.nk) * np + f.nv * nvp < 4 * nvp) return 1;             // O's rows take the operands' place
+    if (2 * blocks > sms || (2 + f.nk) * np + f.nv * nvp < 4 * nvp) return 1;             // O's rows take the operands' place
     int most = 0;
     for (int k = 0; k < f.q_blocks; ++k) {
         int i0[2], beg[2], end[2], base;
         fp_tiles(f, k * 2 * FP_TILE, i0, beg, end, base);
         for (int e : end) most = e > most ? e : most;
     }
-    return most < 6 ? 1 : most < 16 || blocks > 32 ? 2 : 4;
+    return most < 6 ? 1 : most < 16 || 9 * blocks > 2 * sms ? 2 : 4;
 }
 
 template <int SPLIT> auto fp_kernel(bool bias, float softcap, bool bound) {

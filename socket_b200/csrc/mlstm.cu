@@ -164,7 +164,7 @@ mlstm_finish_warps_kernel(sk_mlstm_params p) {
 template <typename T, int V> int finish_dispatch(const sk_mlstm_params& p, cudaStream_t st) {
     if constexpr (V == 8) {
         const int64_t warps = (int64_t)p.B * p.S * p.H;
-        if (p.P <= 256 && warps > 4 * 148 * 8 && warps < (int64_t)1 << 32)
+        if (p.P <= 256 && warps > (int64_t)sm_count() * 4 * 8 && warps < (int64_t)1 << 32)
             return check_chained(launch_after(mlstm_finish_warps_kernel, dim3((unsigned)((warps + 7) / 8)), dim3(256), 0, st, p),
                                  "mlstm_finish_warps_kernel");
     }

@@ -725,7 +725,7 @@ int launch_mlstm_tc(const sk_mlstm_params& p, cudaStream_t st) {
     // The walk over the chunks is a chain, so a head's state is dealt out to as many CTAs as there is room for: 32000 tokens, 8 heads of
     // 128 x 256: 200 us with 128 CTAs of 16 columns, 271 with 64 of 32, 367 with 32 of 64.  More CTAs than SMs would walk it twice
     auto ctas = [&](int sp) { return (int64_t)((p.P + sp - 1) / sp) * ((p.N + 127) / 128) * p.B * p.H; };
-    const int sp = ctas(32) > 148 ? 64 : ctas(16) > 148 ? 32 : 16;
+    const int sp = ctas(32) > sm_count() ? 64 : ctas(16) > sm_count() ? 32 : 16;
     if (int rc = make_head_map(&ms_out, states, p.P, 2, p.N, (int)hc, np, p.P, 2 * np, MT_TOK, sp)) return rc;
     if (int rc = make_head_map(&ms_in, states, p.P, 2, p.N, (int)hc, np, p.P, 2 * np, 64)) return rc;
 
