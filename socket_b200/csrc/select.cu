@@ -999,30 +999,31 @@ __device__ __noinline__ void rescore_row(SelShared& s, const CandArgs& a, int64_
         }
     }
     __syncthreads();
-    const int L = a.L, R = a.R;
+    constexpr int L = 32;                      // of every call that comes here: the filtering scorers have 32 tables
+    const int R = a.R;
     const uint8_t* cg = a.codes + (size_t)kv * a.Tcap * L;
     const __half* vg = a.v_norm + (size_t)kv * a.Tcap;
     // a key's codes are requested while the key before is scored, and taken apart by byte selection: a word chosen by the
     // key's table order would be a read of local memory for every table (a step of 128 rows of 131072 keys, one of them
     // rescored: 421 us, so 516)
-    uint4 c0 = make_uint4(0, 0, 0, 0), c1 = c0;
+    uint4 next[2] = {};
     __half norm = __float2half(0.f);
     auto request = [&](int t) {
         const uint4* cp = reinterpret_cast<const uint4*>(cg + (size_t)t * L);
-        c0 = __ldcg(cp);
-        if (L > 16) c1 = __ldcg(cp + 1);
+        next[0] = __ldcg(cp);
+        next[1] = __ldcg(cp + 1);
         norm = __ldcg(vg + t);
     };
     if (tid < T) request(tid);
     for (int t = tid; t < T; t += SEL_THREADS) {
-        const uint4 now[2] = {c0, c1};
+        const uint4 now[2] = {next[0], next[1]};
         const float vn = __half2float(norm);
         if (t + SEL_THREADS < T) request(t + SEL_THREADS);
         const int m = t & 7;                   // the scorer's table order for this key
         float sum = 0.f;
+#pragma unroll
         for (int v = 0; v < L / 16; ++v) {
-            const uint4 w4 = v == 0 ? now[0] : v == 1 ? now[1] : __ldcg(reinterpret_cast<const uint4*>(cg + (size_t)t * L) + v);
-            const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+            const uint32_t w[4] = {now[v].x, now[v].y, now[v].z, now[v].w};
 #pragma unroll
             for (int q = 0; q < 16; ++q) {
                 const int tb = (q & 8) | ((q & 7) ^ m);
