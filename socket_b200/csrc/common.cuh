@@ -294,7 +294,7 @@ int launch_score_select_cluster(const float* lut, const uint8_t* codes, const ui
                                 int sink, int window, int32_t* list, int64_t list_row_stride, int32_t* list_len,
                                 int32_t* status, cudaStream_t st);
 
-// Tensor-core bulk hashing (bf16, head_dim 128, L*P = 256)
+// Tensor-core bulk hashing (bf16; appends also fp16; head_dim 128, L*P = 256)
 int launch_hash_keys_tc(const void* keys, int64_t key_row_stride, const void* planes, int64_t N, uint8_t* codes,
                         int64_t code_row_stride, const int64_t* dst_row, int32_t* status, cudaStream_t st);
 bool kv_append_tc_applicable(const void* k_new, const void* v_new, int kv_dtype, const void* planes, int plane_dtype,

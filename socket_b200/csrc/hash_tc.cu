@@ -4,9 +4,9 @@
 // Persistent CTAs, one per SM, walk the 128-row tiles of K.  The 256 plane rows stay in shared
 // memory; TMA (cp.async.bulk.tensor, 128-byte swizzle) feeds a ring of K tiles, one elected thread
 // issues eight tcgen05.mma.kind::f16 (M=128, N=256, K=16) per tile into one of two fp32
-// accumulators in tensor memory, and eight epilogue warps read the other accumulator back
-// with tcgen05.ld (two threads per row), take the signs and write 32 code bytes per row, so
-// loading, multiplying and the epilogue of consecutive tiles overlap.
+// accumulators in tensor memory, and the epilogue warps (sixteen, four threads per row; eight and two
+// with APPEND) read the other accumulator back with tcgen05.ld, take the signs and write 32 code bytes
+// per row, so loading, multiplying and the epilogue of consecutive tiles overlap.
 //
 // The same kernel with APPEND writes the rest of a cache append: eight warps move K (from the tile in
 // shared memory) and V (straight through registers) to their cache rows and take ||v||, so K is read
@@ -19,9 +19,10 @@
 // Exactness.  16-bit products are exact in fp32, only the accumulation rounds, so a sign
 // can be wrong only when |acc| is tiny compared with |k|.|p|.  Every projection with
 // |acc| <= 2^-16 |k| |p| (a bound far above the accumulation error of 128 terms) is marked in a
-// bit mask of the tile and decided again from the exact fp64 dot product of the rows in shared
-// memory, which patches the bit; ~1e-4 of the projections (five per tile) take that path, and a mask
-// has room for all of them.  Rows of zeros hash to all-ones bytes directly.
+// bit mask of the tile and decided again from the exact fp64 dot product, which patches the bit: with APPEND
+// by the norm warps from the rows in shared memory, without by eight warps of their own that read the key from
+// global memory again.  ~1e-4 of the projections (five per tile) take that path, and a mask has room for all of
+// them.  Rows of zeros hash to all-ones bytes directly.
 #include <cuda.h>
 
 #include "hash_body.cuh"
@@ -67,7 +68,7 @@ constexpr int TC_STAGES = 2;          // accumulators in tensor memory
 constexpr int TC_MASKS = 4;           // masks of near-zero projections: tiles whose decisions may be outstanding
 constexpr int TC_ARING = 4;           // K tiles in flight
 constexpr int TC_NSLOTS = 8;          // norm slots
-constexpr int TC_NORM_WARPS = 4;      // one thread per row of the K tile: its norm, and later its near-zero projections
+constexpr int TC_NORM_WARPS = 4;      // one thread per row of the K tile: its norm, and with APPEND later its near-zero projections
 // two threads per accumulator row, 128 columns each; four of 64 where no warps move rows
 template <bool APPEND> constexpr int TC_EPI_WARPS = APPEND ? 8 : 16;
 constexpr int TC_MOVE_WARPS = 8;      // APPEND: 16 rows each
@@ -373,7 +374,7 @@ hash_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         // ---- one thread per row of the K tile, read from the swizzled tile in shared memory
         // (16-byte chunk c of row r sits at chunk c ^ (r & 7))
         const int r_in_tile = (warp - 2) * 32 + lane;
-        bool ok = wait_all(&ts.b_full, 0);                             // the near-zero decisions read the planes
+        bool ok = wait_all(&ts.b_full, 0);                             // the near-zero decisions (APPEND) read the planes
 #pragma unroll 1
         for (int64_t i = 0; ok && i < my_tiles + (APPEND ? 1 : 0) && !gone(); ++i) {
             // norms of tile i.  They go to slot i % 8, which has a barrier of its own (these warps may be
