@@ -1,6 +1,8 @@
 // Everything between two matrix products that touches the fp32 residual stream: the scaled embedding,
 // the residual update with a norm on the sublayer's output fused with the norm of the next sublayer's
 // input, and the gated units of the feed-forwards.
+#include <type_traits>
+
 #include "blocks.cuh"
 
 namespace sk {
@@ -29,12 +31,13 @@ embed_rows_kernel(const int64_t* __restrict__ tokens, const T* __restrict__ tabl
 // One CTA per row; the row lives in registers (NV vectors of V elements per thread).
 //   in_mode  0: x stays; 1: x += rms(y) * w_in; 2: x = y + w_in; 3: x += y
 //   out_mode 0: nothing; 1: out = rms(x) * w_out; 2: out = [x ; x0]; 3: out = layer norm of x * w_out
-// A decoded token's rows (NV = 1) are bound by latency: everything is requested at once, as with each norm's weights requested
-// behind its sum a row of 4096 waited for memory three times.  A prompt's are bound by memory, and the registers that would hold
-// the weights keep rows in flight instead; vectors of 8 leave every other 16 bytes of the fp32 stream to a second access
-// (8000 rows of 4096: 125 us, so 95).
-template <typename T, typename TY, int V, int NV>
-__global__ void __launch_bounds__(1024)
+// EARLY: a decoded token's rows are bound by latency: everything is requested at once, as with each norm's weights requested behind its sum
+// a row of 4096 waited for memory three times.  Other rows are bound by memory, and the registers that would hold the weights keep
+// rows in flight instead (290 rows of 4096, 1024 threads each: 5.3 us early, 4.0 late, two rows an SM); vectors of 8 leave every other 16
+// bytes of the fp32 stream to a second access (8000 rows of 4096: 125 us, so 95).
+// IN: false where in_mode is 0, which then takes fewer registers (32000 rows of 4096 with a norm out: 129 us, so 113)
+template <typename T, typename TY, int V, int NV, bool EARLY, bool IN>
+__global__ void __launch_bounds__(1024, !EARLY && NV <= 4 && V * NV <= 8 ? 2 : 1)
 residual_norm_kernel(sk_residual_params p) {
     __shared__ float red[3][32];
     const int64_t row = blockIdx.x;
@@ -45,28 +48,24 @@ residual_norm_kernel(sk_residual_params p) {
     const T* w_out = (const T*)p.w_out;
     const TY* yr = (const TY*)p.y + row * p.y_ld;
     const bool norm_out = p.out_mode == 1 || p.out_mode == 3;
-    constexpr bool EARLY = NV == 1;
     Raw<TY, V> yw[NV];
-    Raw<float, V> xw[NV];
+    Raw<float, V> xw[NV], x0w[NV];
     Raw<T, V> wi[NV], wo[NV];
+    auto request = [&](bool wanted, auto* from, auto& raw) {
+        if (!wanted) return;
 #pragma unroll
-    for (int n = 0; n < NV; ++n) {
-        const int i = (n * nt + t) * V;
-        if (i < W) {
-            if (p.in_mode != 0) yw[n] = load_raw<TY, V>(yr + i);
-            if (p.in_mode != 2) xw[n] = load_raw<float, V>(xr + i);
-        }
-    }
-#pragma unroll
-    for (int n = 0; n < NV; ++n) {
-        const int i = (n * nt + t) * V;
-        if (EARLY && i < W) {
-            if (p.in_mode == 1 || p.in_mode == 2) wi[n] = load_raw<T, V>(w_in + i);
-            if (norm_out) wo[n] = load_raw<T, V>(w_out + i);
-        }
+        for (int n = 0; n < NV; ++n)
+            if ((n * nt + t) * V < W) raw[n] = load_raw<std::remove_const_t<std::remove_pointer_t<decltype(from)>>, V>(from + (n * nt + t) * V);
+    };
+    request(IN && p.in_mode != 0, yr, yw);                    // (known to be true, the registers of four vectors spill)
+    request(p.in_mode != 2, xr, xw);
+    if (EARLY) {
+        request(IN && (p.in_mode == 1 || p.in_mode == 2), w_in, wi);
+        request(norm_out, w_out, wo);
+        request(p.out_mode == 2, p.x0 + row * W, x0w);
     }
     float xv[NV][V];
-    if (p.in_mode != 0) {
+    if (IN && p.in_mode != 0) {
         float inv = 1.f;
         if (p.in_mode == 1) {
             float ss = 0.f;
@@ -136,10 +135,10 @@ residual_norm_kernel(sk_residual_params p) {
         for (int n = 0; n < NV; ++n) {
             const int i = (n * nt + t) * V;
             if (i < W) {
-                const Raw<float, V> x0 = load_raw<float, V>(p.x0 + row * W + i);
+                if (!EARLY) x0w[n] = load_raw<float, V>(p.x0 + row * W + i);
                 float r[V];
 #pragma unroll
-                for (int e = 0; e < V; ++e) r[e] = x0.e[e];
+                for (int e = 0; e < V; ++e) r[e] = x0w[n].e[e];
                 store_vec<T, V>(o + i, xv[n]);
                 store_vec<T, V>(o + W + i, r);
             }
@@ -203,19 +202,30 @@ ring_append_kernel(const E* k, const E* v, int64_t k_bs, int64_t k_ss, int64_t v
 template <typename T, typename TY, int V>
 int residual_dispatch(const sk_residual_params& p, cudaStream_t st) {
     const int vecs = (p.width + V - 1) / V;
-    // few rows: one vector per thread (latency); many rows: smaller blocks, more of them per SM
+    // few rows: one vector per thread (latency); many rows: smaller blocks, more of them per SM, with two to four vectors per thread: of one,
+    // 8000 rows of 1024 took 20.0 us (of two 16.6), of eight, whose registers spill, 8000 rows of 5120 119 us (of four 86)
     int nt = p.rows < 296 ? 1024 : 256;
     while (nt > 32 && nt / 2 >= vecs) nt /= 2;
+    if (p.rows >= 296 && nt >= vecs && nt > 64) nt /= 2;
+    if (vecs > 4 * nt) nt = vecs > 4 * 1024 ? 1024 : (vecs + 127) / 128 * 32;
     while (nt < 1024 && (vecs + nt - 1) / nt > 8) nt *= 2;
     const int nv = (vecs + nt - 1) / nt;
-    dim3 grid((unsigned)p.rows);
+    // Weights early (us, cold, of 2048 or 4096 elements): 8 rows of both norms 3.5, late 3.7, 100 rows 4.0 and 3.8; without a second norm 2.6 and 2.3; of
+    // two vectors a thread (5120) 4.2 and 4.9; small rows (54) 2.2 and 2.9
+    const bool few = p.rows <= sm_count();
+    const bool early = nt <= 128 || (few && (nv > 1 || p.in_mode == 0 || p.out_mode == 2 || (p.out_mode != 0 && p.rows <= 32)));
     void (*kern)(sk_residual_params) = nullptr;
-    if (nv <= 1) kern = residual_norm_kernel<T, TY, V, 1>;
-    else if (nv <= 2) kern = residual_norm_kernel<T, TY, V, 2>;
-    else if (nv <= 4) kern = residual_norm_kernel<T, TY, V, 4>;
-    else if (nv <= 8) kern = residual_norm_kernel<T, TY, V, 8>;
-    else return fail(SK_ERR_UNSUPPORTED, "sk_residual_norm: width %d is too large", p.width);
-    return check_chained(launch_after(kern, grid, dim3((unsigned)nt), 0, st, p), "residual_norm_kernel");
+    auto pick = [&](auto in) {
+        constexpr bool IN = decltype(in)::value;
+        if (nv <= 1) kern = early ? residual_norm_kernel<T, TY, V, 1, true, IN> : residual_norm_kernel<T, TY, V, 1, false, IN>;
+        else if (nv <= 2) kern = early ? residual_norm_kernel<T, TY, V, 2, true, IN> : residual_norm_kernel<T, TY, V, 2, false, IN>;
+        else if (nv <= 4) kern = early && V == 1 ? residual_norm_kernel<T, TY, V, 4, V == 1, IN> : residual_norm_kernel<T, TY, V, 4, false, IN>;
+        else if (nv <= 8) kern = residual_norm_kernel<T, TY, V, 8, false, IN>;
+    };
+    if (p.in_mode != 0) pick(std::true_type{});
+    else pick(std::false_type{});
+    if (kern == nullptr) return fail(SK_ERR_UNSUPPORTED, "sk_residual_norm: width %d is too large", p.width);
+    return check_chained(launch_after(kern, dim3((unsigned)p.rows), dim3((unsigned)nt), 0, st, p), "residual_norm_kernel");
 }
 
 }  // namespace
