@@ -6,8 +6,9 @@ namespace sk {
 namespace {
 
 // One CTA per row, the row in registers.  Latency-bound: one pass over 8 KB (4096 x bf16), 2.9 us inside a decoded token
-// where the library's norm takes 6.3.
-template <typename T, int V, int NV>
+// where the library's norm takes 6.3.  EARLY: the weights are requested with the row, one trip to memory; of more rows than SMs they would keep
+// other rows off (3000 rows of 8192: 47 us early, 28 late).
+template <typename T, int V, int NV, bool EARLY>
 __global__ void __launch_bounds__(512)
 rms_norm_rows_kernel(const T* x, const T* w, int width, float eps, T* __restrict__ out) {
     pdl_begin();
@@ -15,13 +16,13 @@ rms_norm_rows_kernel(const T* x, const T* w, int width, float eps, T* __restrict
     const int64_t row = blockIdx.x;
     const int nt = blockDim.x, t = threadIdx.x;
     float v[NV][V], ss = 0.f;
-    Raw<T, V> g[NV];                                      // requested with the row: one trip to memory
+    Raw<T, V> g[NV];
 #pragma unroll
     for (int n = 0; n < NV; ++n) {
         const int i = (n * nt + t) * V;
         if (i < width) {
             load_vec<T, V>(x + row * width + i, v[n]);
-            g[n] = load_raw<T, V>(w + i);
+            if (EARLY) g[n] = load_raw<T, V>(w + i);
         }
     }
 #pragma unroll
@@ -34,6 +35,7 @@ rms_norm_rows_kernel(const T* x, const T* w, int width, float eps, T* __restrict
     for (int n = 0; n < NV; ++n) {
         const int i = (n * nt + t) * V;
         if (i < width) {
+            if (!EARLY) g[n] = load_raw<T, V>(w + i);
 #pragma unroll
             for (int e = 0; e < V; ++e) v[n][e] *= inv * to_f32(g[n].e[e]);
             store_vec<T, V>(out + row * width + i, v[n]);
@@ -78,9 +80,11 @@ int rms_dispatch(const void* x, const void* w, int64_t rows, int width, float ep
         return check_chained(launch_after(kern, dim3((unsigned)rows), dim3((unsigned)nt), 0, st, (const T*)x, (const T*)w, width, eps,
                                           (T*)out), "rms_norm_rows_kernel");
     };
-    if (vec)
-        return nv <= 1 ? run(rms_norm_rows_kernel<T, V, 1>) : nv <= 4 ? run(rms_norm_rows_kernel<T, V, 4>) : run(rms_norm_long_rows_kernel<T, V>);
-    return nv <= 4 ? run(rms_norm_rows_kernel<T, 1, 4>) : run(rms_norm_long_rows_kernel<T, 1>);
+    const bool few = rows <= sm_count();
+    if (vec && nv <= 1) return run(rms_norm_rows_kernel<T, V, 1, true>);
+    if (vec && nv <= 4) return few ? run(rms_norm_rows_kernel<T, V, 4, true>) : run(rms_norm_rows_kernel<T, V, 4, false>);
+    if (!vec && nv <= 4) return few ? run(rms_norm_rows_kernel<T, 1, 4, true>) : run(rms_norm_rows_kernel<T, 1, 4, false>);
+    return vec ? run(rms_norm_long_rows_kernel<T, V>) : run(rms_norm_long_rows_kernel<T, 1>);
 }
 
 }  // namespace
