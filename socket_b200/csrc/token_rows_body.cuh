@@ -15,22 +15,23 @@ __device__ __forceinline__ bool picked(float a, int i, float b, int j) {
 }
 
 // A cluster of eight CTAs per sequence, each an eighth of the row; the first one joins what they found.  32768 logits: one CTA
-// took 6.6 us at the end of a decoded token.
-constexpr int PT_CLUSTER = 8, PT_THREADS = 256;
-template <typename T, int V>
-__global__ void __launch_bounds__(PT_THREADS)
+// took 6.6 us at the end of a decoded token.  A short row is one larger CTA's: 1000 logits 2.7 us, by a cluster 3.2.
+constexpr int PT_CLUSTER = 8, PT_ALONE = 4096;
+template <int CL> constexpr int PT_THREADS = CL == 1 ? 1024 : 256;
+template <typename T, int V, int CL>
+__global__ void __launch_bounds__(PT_THREADS<CL>)
 pick_token_kernel(const T* logits, int64_t ld, int vocab, int64_t* token, int64_t* pos, int32_t* seqlens) {
     pdl_begin();
-    constexpr int WARPS = PT_THREADS / 32;
-    __shared__ float best_s[PT_CLUSTER * WARPS];
-    __shared__ int at_s[PT_CLUSTER * WARPS];
-    cluster_arrive();
+    constexpr int WARPS = PT_THREADS<CL> / 32;
+    __shared__ float best_s[CL * WARPS];
+    __shared__ int at_s[CL * WARPS];
+    if (CL > 1) cluster_arrive();
     const int rank = blockIdx.x, b = blockIdx.y, t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const T* row = logits + b * ld;
     float best = -INFINITY;
     int at = vocab;                                           // behind every index: a row of -inf alone picks its first
-    constexpr int U = 4, STEP = PT_CLUSTER * PT_THREADS * V;  // elements of the cluster's one load each
-    for (int64_t i0 = (rank * PT_THREADS + t) * V; i0 < vocab; i0 += U * STEP) {
+    constexpr int U = CL == 1 ? 1 : 4, STEP = CL * PT_THREADS<CL> * V;      // elements of the cluster's one load each
+    for (int64_t i0 = (rank * PT_THREADS<CL> + t) * V; i0 < vocab; i0 += U * STEP) {
         float v[U][V];
 #pragma unroll
         for (int u = 0; u < U; ++u)
@@ -61,18 +62,26 @@ pick_token_kernel(const T* logits, int64_t ld, int vocab, int64_t* token, int64_
         }
     };
     reduce();
-    cluster_wait();                                           // every CTA of the cluster has begun
-    if (lane == 0) {
-        store_first_cta(best_s + rank * WARPS + warp, best);
-        store_first_cta(at_s + rank * WARPS + warp, (uint32_t)at);
+    if (CL > 1) {
+        cluster_wait();                                       // every CTA of the cluster has begun
+        if (lane == 0) {
+            store_first_cta(best_s + rank * WARPS + warp, best);
+            store_first_cta(at_s + rank * WARPS + warp, (uint32_t)at);
+        }
+        cluster_arrive();
+        cluster_wait();
+    } else {
+        if (lane == 0) {
+            best_s[warp] = best;
+            at_s[warp] = at;
+        }
+        __syncthreads();
     }
-    cluster_arrive();
-    cluster_wait();
     if (rank == 0 && warp == 0) {
-        static_assert(PT_CLUSTER * WARPS == 64, "two results per lane");
+        static_assert(CL * WARPS % 32 == 0, "as many results for every lane");
         best = best_s[lane];
         at = at_s[lane];
-        join(best_s[lane + 32], at_s[lane + 32]);
+        if (CL * WARPS > 32) join(best_s[(lane + 32) % (CL * WARPS)], at_s[(lane + 32) % (CL * WARPS)]);
         reduce();
         if (lane == 0) {
             token[b] = at;
@@ -87,20 +96,22 @@ int pick_dispatch(const void* logits, int64_t ld, int batch, int vocab, int64_t*
                   cudaStream_t st) {
     constexpr int V = 16 / sizeof(T);
     const bool vec = vocab % V == 0 && ld % V == 0 && (uintptr_t)logits % 16 == 0;
-    auto kern = vec ? pick_token_kernel<T, V> : pick_token_kernel<T, 1>;
+    const int cl = vocab <= PT_ALONE ? 1 : PT_CLUSTER;
+    auto kern = cl == 1 ? (vec ? pick_token_kernel<T, V, 1> : pick_token_kernel<T, 1, 1>)
+                        : (vec ? pick_token_kernel<T, V, PT_CLUSTER> : pick_token_kernel<T, 1, PT_CLUSTER>);
     cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(PT_THREADS);
+    cfg.blockDim = dim3(cl == 1 ? PT_THREADS<1> : PT_THREADS<PT_CLUSTER>);
     cfg.stream = st;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = PT_CLUSTER;
+    attr[1].val.clusterDim.x = (unsigned)cl;
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = cl > 1 ? 2 : 1;
     for (int b0 = 0; b0 < batch; b0 += 65535) {               // the grid's second dimension
-        cfg.gridDim = dim3(PT_CLUSTER, (unsigned)(batch - b0 < 65535 ? batch - b0 : 65535));
+        cfg.gridDim = dim3((unsigned)cl, (unsigned)(batch - b0 < 65535 ? batch - b0 : 65535));
         const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (const T*)logits + b0 * ld, ld, vocab, token + b0, b0 == 0 ? pos : (int64_t*)nullptr,
                                                  seqlens != nullptr ? seqlens + b0 : (int32_t*)nullptr);
         if (int rc = check_chained(e, "pick_token_kernel")) return rc;
