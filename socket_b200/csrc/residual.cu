@@ -206,7 +206,7 @@ int residual_dispatch(const sk_residual_params& p, cudaStream_t st) {
     // 8000 rows of 1024 took 20.0 us (of two 16.6), of eight, whose registers spill, 8000 rows of 5120 119 us (of four 86)
     int nt = p.rows < 296 ? 1024 : 256;
     while (nt > 32 && nt / 2 >= vecs) nt /= 2;
-    if (p.rows >= 296 && nt >= vecs && nt > 64) nt /= 2;
+    if (p.rows >= 2048 && nt >= vecs && nt > 64) nt /= 2;         // (400 rows of 512: 2.7 us of one vector a thread, 3.1 of two)
     if (vecs > 4 * nt) nt = vecs > 4 * 1024 ? 1024 : (vecs + 127) / 128 * 32;
     while (nt < 1024 && (vecs + nt - 1) / nt > 8) nt *= 2;
     const int nv = (vecs + nt - 1) / nt;
