@@ -212,8 +212,8 @@ int residual_dispatch(const sk_residual_params& p, cudaStream_t st) {
     const int nv = (vecs + nt - 1) / nt;
     // Weights early (us, cold, of 2048 or 4096 elements): 8 rows of both norms 3.5, late 3.7, 100 rows 4.0 and 3.8; without a second norm 2.6 and 2.3; of
     // two vectors a thread (5120) 4.2 and 4.9; small rows (54) 2.2 and 2.9
-    const bool few = p.rows <= sm_count();
-    const bool early = nt <= 128 || (few && (nv > 1 || p.in_mode == 0 || p.out_mode == 2 || (p.out_mode != 0 && p.rows <= 32)));
+    const bool few = p.rows <= sm_count(), own = p.out_mode == 2 && p.x0 == p.x;      // the stream itself as x0 is read behind its update
+    const bool early = !own && (nt <= 128 || (few && (nv > 1 || p.in_mode == 0 || p.out_mode == 2 || (p.out_mode != 0 && p.rows <= 32))));
     void (*kern)(sk_residual_params) = nullptr;
     auto pick = [&](auto in) {
         constexpr bool IN = decltype(in)::value;

@@ -49,6 +49,15 @@ def test_residual_rows(rows, width):
                 _near(o, torch.cat([stream, x0.double()], -1))
 
 
+@pytest.mark.parametrize("width", [54, 2048, 5120])
+@pytest.mark.parametrize("rows", [1, 200])
+def test_the_stream_itself_as_second_half(rows, width):
+    g = torch.Generator(device=DEV).manual_seed(width)
+    x, y, w = _r(g, rows, width), _r(g, rows, width, dtype=BF16), _r(g, width, dtype=BF16)
+    o = ops.residual_norm(x, EPS, y=y, w_in=w, x0=x, dtype=BF16)
+    assert torch.equal(o, torch.cat([x, x], -1).to(BF16))
+
+
 @pytest.mark.parametrize("inner,parts", [(4096, 8), (8192, 1), (8192, 8), (4096, 1), (3000, 3), (512, 1)])
 @pytest.mark.parametrize("rows", [1, 18, 19, 148, 149, 300])
 def test_gated_rows(rows, inner, parts):
